@@ -3,6 +3,7 @@
 #include "ops.cuh"
 
 #include "phase_gemv.cuh"
+#include "q2.cuh"
 #include "gemm_tc.cuh"
 #include "token_kernel.cuh"
 
@@ -32,7 +33,9 @@ struct bn_model {
     cudaGraphExec_t token_graph = nullptr;   // one whole token + advance, captured on first use
     std::vector<cudaGraphExec_t> stage_graphs;   // pipeline stage: one captured schedule per stream (its state pointers are baked in)
     uint32_t *PACK_H, *PACK_F;
-    int *SWCNT = nullptr;                 // arrival counters of swiglu_pack (one per Hadamard block of the FFN width)
+    uint8_t *q2 = nullptr;                // two-bit tiles of the local projections (q2.cuh), one allocation
+    uint8_t *SGN = nullptr;               // sign values as bits, 8 per byte: hidden, then ffn
+    const uint8_t *q2_head = nullptr;
     float *GEMV_SCRATCH;
     // persistent state
     float *gdn_state = nullptr, *conv_hist = nullptr, *conv_hist2 = nullptr;   // conv taps: two buffers (position parity)
@@ -64,6 +67,8 @@ struct bn_model {
         const uint32_t *q_w, *k_w, *v_w, *o_w;
         const float *q_norm, *k_norm;
         int idx;   // index among its kind
+        // two-bit tiles: [qkv | gate] or [q | k | v], ssm_out / attn_output, [gate, up] sharing tiles, down
+        const uint8_t *q2_in = nullptr, *q2_out = nullptr, *q2_ffn = nullptr, *q2_down = nullptr;
     };
     std::vector<Layer> layers;
     // multi-sequence pass (bn_model_stage_batch): per-column arenas, shared activation images, tile-major weights
@@ -207,60 +212,70 @@ void attn_plain(bn_model *m, const bn_model::Layer &L) {
     bnk::add_inplace(st, m->RES, m->D, h.hidden);
 }
 
-// ---- fused path: one "phase" kernel per projection group (phase_gemv.cu) -------------------------------
-// Projections that read the same rotated input and lie back to back in device memory run as one matrix.
-bnk::PhaseArgs phase_base(bn_model *m, const uint32_t *W, int M, int K, const int32_t *sg) {
-    bnk::PhaseArgs a = {};
-    a.W = reinterpret_cast<const uint8_t *>(W); a.M = M; a.K = K;
-    a.signs = sg; a.hat_block = m->hp.hat_block; a.hat_inv = 1.0f / sqrtf(float(m->hp.hat_block)); a.eps = m->hp.rms_eps;
+// ---- fused path: one kernel per projection group, its input preparation in front (q2_gemv.cu) -----------------------------
+// Projections that read the same input are one matrix of two-bit tiles.
+bnk::Q2Args phase_base(bn_model *m, const uint8_t *W, int M, int K) {
+    bnk::Q2Args a = {};
+    a.W = W; a.M = M; a.K = K;
+    a.sgn = m->SGN;
+    a.hat_block = m->hp.hat_block; a.hat_inv = 1.0f / sqrtf(float(m->hp.hat_block)); a.eps = m->hp.rms_eps;
     a.err = m->ctx->err_dev;
     if (m->stamps && m->stamp_idx < 256) a.stamps = m->stamps + 8 * (m->stamp_idx++);
     return a;
 }
-void launch(bn_model *m, const bnk::PhaseArgs &a) {
+void launch(bn_model *m, const bnk::Q2Args &a) {
     if (m->mixers_only) return;
-    cudaError_t e = bnk::launch_phase(m->ctx->stream, m->ctx->sm_count, a, m->use_pdl);
+    cudaError_t e = bnk::launch_q2_gemv(m->ctx->stream, m->ctx->sm_count, a, m->use_pdl);
     if (e != cudaSuccess && m->launch_err == cudaSuccess) m->launch_err = e;
 }
 bool adjacent(const uint32_t *a, size_t a_bytes, const uint32_t *b) {
     return reinterpret_cast<const uint8_t *>(a) + a_bytes == reinterpret_cast<const uint8_t *>(b);
 }
+// the projection that follows in the schedule, for the L2 prefetch
+bnk::Q2Next q2_next(const uint8_t *W, int M, int K, const float *w) {
+    bnk::Q2Next n;
+    n.W = W; n.units = (M + 15) / 16; n.unit_bytes = K / 512 * bnk::Q2_PIECE;
+    n.w = w; n.w_bytes = w ? K * 4 : 0;
+    return n;
+}
+// the first projection after block b (the next block's, else the output head; b = b0 - 1: block b0's, which follows the head in the next token)
+bnk::Q2Next next_after(const bn_model *m, int b) {
+    const bn_hparams &h = m->hp;
+    const int QD = h.n_head * h.head_dim, KD = h.n_kv * h.head_dim, IN = h.gdn_heads * h.gdn_dim, C = 2 * h.gdn_qk_heads * h.gdn_dim + IN;
+    if (b + 1 < m->b1) {
+        const bn_model::Layer &L = m->layers[b + 1];
+        return q2_next(L.q2_in, L.attn ? 2 * QD + 2 * KD : C + IN, h.hidden, L.attn_norm);
+    }
+    return m->b1 == h.n_layer ? q2_next(m->q2_head, h.vocab, h.hidden, m->out_norm) : bnk::Q2Next();
+}
+// x = rms_norm(RES) * w through one projection group
+void norm_project(bn_model *m, const uint8_t *W, int M, const float *w, float *out, const bnk::Q2Next &next, float *inv_out = nullptr, bool swiglu = false) {
+    bnk::Q2Args a = phase_base(m, W, M, m->hp.hidden);
+    a.next = next;
+    a.pro = bnk::Q2_NORM; a.x0 = m->RES; a.w = w; a.out = out; a.inv_out = inv_out; a.swiglu = swiglu;
+    launch(m, a);
+}
+// RES += W x
+void project_add(bn_model *m, const uint8_t *W, int K, const float *x, const bnk::Q2Next &next) {
+    bnk::Q2Args a = phase_base(m, W, m->hp.hidden, K);
+    a.next = next;
+    if (x == m->FS) a.sgn = m->SGN + m->hp.hidden / 8;
+    a.pro = bnk::Q2_PLAIN; a.x0 = x; a.resid_in = m->RES; a.resid_out = m->RES;
+    launch(m, a);
+}
 
 void ffn_fused(bn_model *m, const bn_model::Layer &L) {
     const bn_hparams &h = m->hp;
-    bnk::PhaseArgs a = phase_base(m, L.ffn_gate, h.ffn, h.hidden, m->signs);
-    a.pro = bnk::PRO_NORM; a.x0 = m->RES; a.w = L.post_norm;
-    if (adjacent(L.ffn_gate, ptq_bytes(h.ffn, h.hidden), L.ffn_up)) { a.M = 2 * h.ffn; a.out = m->FG; launch(m, a); }
-    else { a.out = m->FG; launch(m, a); a.W = reinterpret_cast<const uint8_t *>(L.ffn_up); a.out = m->FU; launch(m, a); }
-    bnk::PhaseArgs d = phase_base(m, L.ffn_down, h.hidden, h.ffn, m->signs + h.hidden);
-    // silu needs a double-precision exp per element: computed once by a small kernel, not by every CTA. (Measured: folding it
-    // into the gate / up projection's epilogue costs that launch 2.8 us and saves nothing - the small kernel overlaps the
-    // neighbouring launches under programmatic dependent launch.)
-    // The same small kernel also prepares the down projection's input (signs, three Hadamard blocks, q8_1): its three blocks
-    // in parallel, once, instead of one after the other in every CTA of the projection (8.2 -> 2.5 us of prologue there,
-    // 3.5 us more in the small kernel).
-    if (bnk::swiglu_pack_supported(h.ffn, h.hat_block)) {
-        if (!m->phases_only) bnk::swiglu_pack(m->ctx->stream, m->FG, m->FU, h.ffn, m->signs + h.hidden, d.hat_inv, m->FS, m->PACK_F, m->SWCNT);
-        d.pro = bnk::PRO_PACKED; d.pack = m->PACK_F;
-    } else {
-        if (!m->phases_only) bnk::swiglu(m->ctx->stream, m->FG, m->FU, h.ffn, m->FS);
-        d.pro = bnk::PRO_PLAIN; d.x0 = m->FS;
-    }
-    d.resid_in = m->RES; d.resid_out = m->RES;
-    launch(m, d);
+    // gate and up rows share tiles, so the CTA that has a row's two sums writes silu(gate) * up; the down projection walks the
+    // FFN width's Hadamard blocks in its preparation
+    norm_project(m, L.q2_ffn, 2 * h.ffn, L.post_norm, m->FS, q2_next(L.q2_down, h.hidden, h.ffn, nullptr), nullptr, true);
+    project_add(m, L.q2_down, h.ffn, m->FS, next_after(m, int(&L - m->layers.data())));
 }
 
 void gdn_fused(bn_model *m, const bn_model::Layer &L) {
     const bn_hparams &h = m->hp;
     const int NH = h.gdn_heads, NQ = h.gdn_qk_heads, D = h.gdn_dim, C = 2 * NQ * D + NH * D, IN = NH * D;
-    bnk::PhaseArgs a = phase_base(m, L.qkv, C, h.hidden, m->signs);
-    a.pro = bnk::PRO_NORM; a.x0 = m->RES; a.w = L.attn_norm;
-    a.inv_out = m->G + 48;      // the norm factor, for the layer core's two small projections
-    if (adjacent(L.qkv, ptq_bytes(C, h.hidden), L.gate_w)) { a.M = C + IN; a.out = m->QKV; launch(m, a); }
-    else {
-        a.out = m->QKV; launch(m, a);
-        a.inv_out = nullptr; a.W = reinterpret_cast<const uint8_t *>(L.gate_w); a.M = IN; a.out = m->Z; launch(m, a);
-    }
+    norm_project(m, L.q2_in, C + IN, L.attn_norm, m->QKV, q2_next(L.q2_out, h.hidden, IN, nullptr), m->G + 48);      // (the norm factor also goes to the layer core's two small projections)
     if (!m->phases_only) {
         const bnk::GdnDims gd{NH, NQ, D};
         float *h0 = conv_of(m, 0, L.idx), *h1 = conv_of(m, 1, L.idx);
@@ -272,10 +287,7 @@ void gdn_fused(bn_model *m, const bn_model::Layer &L) {
             bnk::gdn_core_fused(m->ctx->stream, gd, h.hidden, m->QKV, L.conv_w, h0, h1, m->POS, m->RES, m->G + 48, L.attn_norm,
                                 L.alpha_w, L.beta_w, L.dt_bias, L.ssm_a, gdn_state_of(m, L.idx), m->Z, L.ssm_norm, h.rms_eps, m->X1);
     }
-    bnk::PhaseArgs o = phase_base(m, L.ssm_out, h.hidden, IN, m->signs);
-    o.pro = bnk::PRO_PLAIN; o.x0 = m->X1;
-    o.resid_in = m->RES; o.resid_out = m->RES;
-    launch(m, o);
+    project_add(m, L.q2_out, IN, m->X1, q2_next(L.q2_ffn, 2 * h.ffn, h.hidden, L.post_norm));
 }
 
 void attn_fused(bn_model *m, const bn_model::Layer &L) {
@@ -284,23 +296,12 @@ void attn_fused(bn_model *m, const bn_model::Layer &L) {
     const int QD = h.n_head * h.head_dim, KD = h.n_kv * h.head_dim;
     const bnk::AttnDims ad = attn_dims(m);
     const bnk::KvLayer kv = kv_layer(m, L.idx);
-    bnk::PhaseArgs a = phase_base(m, L.q_w, 2 * QD, h.hidden, m->signs);
-    a.pro = bnk::PRO_NORM; a.x0 = m->RES; a.w = L.attn_norm;
-    if (adjacent(L.q_w, ptq_bytes(2 * QD, h.hidden), L.k_w) && adjacent(L.k_w, ptq_bytes(KD, h.hidden), L.v_w)) {
-        a.M = 2 * QD + 2 * KD; a.out = m->QKV; launch(m, a);
-    } else {
-        a.out = m->QKV; launch(m, a);
-        a.W = reinterpret_cast<const uint8_t *>(L.k_w); a.M = KD; a.out = m->KBUF; launch(m, a);
-        a.W = reinterpret_cast<const uint8_t *>(L.v_w); a.out = m->VBUF; launch(m, a);
-    }
+    norm_project(m, L.q2_in, 2 * QD + 2 * KD, L.attn_norm, m->QKV, q2_next(L.q2_out, h.hidden, QD, nullptr));
     if (!m->phases_only) {
         bnk::attn_prep(st, ad, m->QKV, m->KBUF, m->VBUF, L.q_norm, L.k_norm, m->POS, kv, m->Q16F, m->GATEB);
         bnk::attn_decode(st, ad, m->Q16F, m->GATEB, m->POS, kv, m->SCORE, m->P16F, m->ESUM, m->PVPART, m->pv_splits, nullptr, m->GOUT, true);
     }
-    bnk::PhaseArgs o = phase_base(m, L.o_w, h.hidden, QD, m->signs);
-    o.pro = bnk::PRO_PLAIN; o.x0 = m->GOUT;
-    o.resid_in = m->RES; o.resid_out = m->RES;
-    launch(m, o);
+    project_add(m, L.q2_out, QD, m->GOUT, q2_next(L.q2_ffn, 2 * h.ffn, h.hidden, L.post_norm));
 }
 
 // enqueue one token: TOK[0], POS[0] hold the token id and its absolute position
@@ -319,9 +320,7 @@ void enqueue_token(bn_model *m, int stop_after, bool want_logits) {
     }
     if (!want_logits || m->b1 != h.n_layer) return;
     if (m->fused) {
-        bnk::PhaseArgs a = phase_base(m, m->out_w, h.vocab, h.hidden, m->signs);
-        a.pro = bnk::PRO_NORM; a.x0 = m->RES; a.w = m->out_norm; a.out = m->LOGITS;
-        launch(m, a);
+        norm_project(m, m->q2_head, h.vocab, m->out_norm, m->LOGITS, next_after(m, m->b0 - 1));
     } else {
         bnk::rms_norm(st, m->RES, m->out_norm, 1, h.hidden, h.rms_eps, m->AN);
         rot_project(m, m->AN, m->signs, h.hidden, m->PACK_H, m->out_w, h.vocab, m->LOGITS);
@@ -343,6 +342,7 @@ bool build_token_ops(bn_model *m) {
     if (!getenv("BONSAI_TOKEN_KERNEL")) return false;
     if (!m->fused || m->b0 != 0 || m->b1 != h.n_layer) return false;
     if (!bnk::token_supported(sm, h.hat_block, h.hidden)) return false;
+    if (!bnk::phase_supported(h.hidden, h.hidden, h.hat_block) || !bnk::phase_supported(h.hidden, h.ffn, h.hat_block)) return false;
     if (h.hidden > 4096 || h.ffn % 16 || D != 128) return false;               // swiglu pairs need one chunk of K
     if (h.n_head != 4 * h.n_kv) return false;                                   // its attention phases are written for four query heads per kv head
     if ((h.cap + m->pv_splits - 1) / m->pv_splits > 512) return false;         // probabilities of one split in shared memory
@@ -446,6 +446,40 @@ int run_token_kernel(bn_model *m, int tok, int pos0, int n_steps, int stop_after
     BN_CUDA(cudaMemsetAsync(m->tok_bar, 0, 4, st));
     BN_CUDA(bnk::launch_token(st, m->ctx->sm_count, ta));
     return BN_OK;
+}
+
+// ---- two-bit tiles of the local projections -------------------------------------------------------------------------------
+int build_q2(bn_model *m) {
+    const bn_hparams &h = m->hp;
+    const int NH = h.gdn_heads, NQ = h.gdn_qk_heads, D = h.gdn_dim, C = 2 * NQ * D + NH * D, IN = NH * D;
+    const int QD = h.n_head * h.head_dim, KD = h.n_kv * h.head_dim;
+    struct Part { const uint32_t *w; int M, K; size_t off; int half; };
+    std::vector<Part> parts;
+    size_t total = 0;
+    std::vector<std::pair<const uint8_t **, size_t>> where;
+    auto matrix = [&](const uint8_t **dst) { where.push_back({dst, total}); };
+    auto part = [&](const uint32_t *w, int M, int K) { parts.push_back({w, M, K, total, -1}); total += bnk::q2_bytes(M, K); };   // (heights are multiples of 16)
+    for (int b = m->b0; b < m->b1; ++b) {
+        bn_model::Layer &L = m->layers[b];
+        matrix(&L.q2_in);
+        if (L.attn) { part(L.q_w, 2 * QD, h.hidden); part(L.k_w, KD, h.hidden); part(L.v_w, KD, h.hidden); }
+        else { part(L.qkv, C, h.hidden); part(L.gate_w, IN, h.hidden); }
+        matrix(&L.q2_out);
+        part(L.attn ? L.o_w : L.ssm_out, h.hidden, h.hidden);
+        matrix(&L.q2_ffn);
+        parts.push_back({L.ffn_gate, h.ffn, h.hidden, total, 0});
+        parts.push_back({L.ffn_up, h.ffn, h.hidden, total, 1});
+        total += 2 * bnk::q2_bytes(h.ffn, h.hidden);
+        matrix(&L.q2_down);
+        part(L.ffn_down, h.hidden, h.ffn);
+    }
+    if (m->b1 == h.n_layer) { matrix(&m->q2_head); part(m->out_w, h.vocab, h.hidden); }
+    BN_CUDA(cudaMalloc(&m->q2, total));
+    BN_CUDA(cudaMalloc(&m->SGN, size_t(h.hidden + h.ffn) / 8));
+    for (auto &w : where) *w.first = m->q2 + w.second;
+    for (const Part &p : parts) bnk::q2_repack(m->ctx->stream, p.w, p.M, p.K, m->q2 + p.off, p.half);
+    bnk::pack_sign_bits(m->ctx->stream, m->signs, h.hidden + h.ffn, m->SGN);
+    return bn_launch_check(m->ctx, "two-bit tiles");
 }
 
 // ---- multi-sequence pass ---------------------------------------------------------------------------------
@@ -802,15 +836,13 @@ int bn_model_finalize(bn_model *m) {
     m->ncols = h.batch_cols > 0 ? h.batch_cols : 1;
     BN_CUDA(cudaSetDevice(m->ctx->device));
     BN_CUDA(cudaMalloc(&m->arena, m->arena_bytes * m->ncols));
-    BN_CUDA(cudaMalloc(&m->SWCNT, 64 * sizeof(int)));
-    BN_CUDA(cudaMemset(m->SWCNT, 0, 64 * sizeof(int)));
     for (auto &s : slots) *s.p = m->arena + s.o;
     m->Z = m->QKV + C;               // [qkv | gate] of a GDN block, [q | k | v] of an attention block
     m->KBUF = m->QKV + 2 * QD;
     m->VBUF = m->KBUF + KD;
     m->FU = m->FG + h.ffn;           // [gate | up]
-    m->fused = h.act_mode == 0 && getenv("BONSAI_NO_FUSE") == nullptr && bnk::phase_supported(h.hidden, h.hidden, h.hat_block) &&
-               bnk::phase_supported(h.hidden, h.ffn, h.hat_block);
+    m->fused = h.act_mode == 0 && getenv("BONSAI_NO_FUSE") == nullptr && bnk::q2_gemv_supported(h.hidden, h.hat_block) &&
+               bnk::q2_gemv_supported(h.ffn, h.hat_block);
     m->use_pdl = getenv("BONSAI_NO_PDL") == nullptr;
     bnk::g_pdl = m->use_pdl;
     // persistent state
@@ -831,6 +863,10 @@ int bn_model_finalize(bn_model *m) {
         m->kv_v_scale_off = al(h.v_mode == 0 ? n / 32 * 2 : 0);
         m->kv_layer_bytes = o;
         BN_CUDA(cudaMalloc(&m->kv, m->kv_layer_bytes * m->n_attn * S));
+    }
+    if (m->fused) {
+        rc = build_q2(m);
+        if (rc != BN_OK) return rc;
     }
     if (h.batch_cols > 0) {
         rc = build_batch_side(m);
@@ -854,7 +890,6 @@ int bn_model_reset(bn_model *m) {
     const int NH = h.gdn_heads, NQ = h.gdn_qk_heads, D = h.gdn_dim, C = 2 * NQ * D + NH * D;
     cudaStream_t st = m->ctx->stream;
     BN_CUDA(cudaMemsetAsync(m->arena, 0, m->arena_bytes * m->ncols, st));
-    BN_CUDA(cudaMemsetAsync(m->SWCNT, 0, 64 * sizeof(int), st));       // (a launch that gave up may have left a count behind)
     if (m->n_gdn) {
         const int S = h.n_streams > 0 ? h.n_streams : 1;
         BN_CUDA(cudaMemsetAsync(m->gdn_state, 0, m->gdn_stream_stride * S * 4, st));
@@ -897,7 +932,8 @@ void bn_model_destroy(bn_model *m) {
     if (m->IMG_HD) cudaFree(m->IMG_HD);
     if (m->IMG_F) cudaFree(m->IMG_F);
     if (m->GROUPS) cudaFree(m->GROUPS);
-    if (m->SWCNT) cudaFree(m->SWCNT);
+    if (m->q2) cudaFree(m->q2);
+    if (m->SGN) cudaFree(m->SGN);
     if (m->CAND) cudaFree(m->CAND);
     delete m;
 }
@@ -1148,9 +1184,7 @@ int bn_model_prefill(bn_model *m, const int *toks, int n, int pos0, int *next_to
         BN_CUDA(cudaMemcpyAsync(m->POS, m->POS + size_t(n - 1) * AS, 4, cudaMemcpyDeviceToDevice, st));
         BN_CUDA(cudaMemcpyAsync(m->TOK, m->TOK + size_t(n - 1) * AS, 4, cudaMemcpyDeviceToDevice, st));
     }
-    bnk::PhaseArgs a = phase_base(m, m->out_w, h.vocab, h.hidden, m->signs);
-    a.pro = bnk::PRO_NORM; a.x0 = m->RES; a.w = m->out_norm; a.out = m->LOGITS;
-    launch(m, a);
+    norm_project(m, m->q2_head, h.vocab, m->out_norm, m->LOGITS, next_after(m, m->b0 - 1));
     bnk::argmax_first(st, m->LOGITS, h.vocab, m->NEXT, m->AMV, m->AMI);
     if (next_tok) {
         BN_CUDA(cudaMemcpyAsync(next_tok, m->NEXT, 4, cudaMemcpyDeviceToHost, st));
@@ -1236,9 +1270,7 @@ int bn_model_gemv_sweep(bn_model *m, int reps, float *ms_per_sweep) {
         if (m->fused) {      // the production launches: every fused projection kernel of one token, nothing else
             m->phases_only = true;
             for (const bn_model::Layer &L : m->layers) { if (L.attn) attn_fused(m, L); else gdn_fused(m, L); ffn_fused(m, L); }
-            bnk::PhaseArgs a = phase_base(m, m->out_w, h.vocab, h.hidden, m->signs);
-            a.pro = bnk::PRO_NORM; a.x0 = m->RES; a.w = m->out_norm; a.out = m->LOGITS;
-            launch(m, a);
+            norm_project(m, m->q2_head, h.vocab, m->out_norm, m->LOGITS, next_after(m, m->b0 - 1));
             m->phases_only = false;
             return;
         }

@@ -1,0 +1,83 @@
+// q2.cuh - the load-time weight layout of the projections ("two-bit tiles") and the kernels' common pieces.
+//
+// A PTQ1_0 block packs five trits into a byte, and unpacking them is what bounds a projection that reads it directly: two
+// integer operations per trit against 0.22 bytes of memory traffic. The model therefore keeps its projection weights a
+// second time with two bits per trit (34 bytes per 128 weights instead of 28), arranged so that ONE bitwise AND turns
+// four packed trits into a ready int8 tensor-core operand register:
+//   * the four two-bit fields of a byte belong to the four 32-weight sub-blocks of its block, so the field that is masked
+//     out selects the sub-block, and the value in place is 4^s * code (code = trit + 1 in {0, 1, 2}, at most 128: a u8);
+//   * the factor 4^s stays in the exact int32 dot and is taken out through the activation scale: fma(d / 4^s, 4^s * I, -s)
+//     is the same float as fma(d, I, -s), because scaling by a power of two is exact (d is an fp16 value, far from the
+//     fp32 underflow range; 4^s * I < 2^22).
+// A piece = 16 rows x 4 blocks (512 weights of K) = 2176 bytes, contiguous: 4 x 512 bytes of codes, then 128 bytes of fp16
+// block scales. Within the codes lane (g = lane / 4, t = lane % 4) of a warp finds at [quarter q = 2R + m][lane] 16 bytes:
+// row 8R + g, blocks 2m and 2m + 1, packed dwords 2t and 2t + 1 of each. Packed dword d, byte b, field s holds element
+// 32s + 4d + b of the block. Scales: word [g][block] = (row g | row g + 8 << 16). Pieces follow each other group (of four
+// blocks) by group, then row tile by row tile. Rows beyond M are zero.
+// That is the m16n8k32 A-fragment order for "all 32 k-slots from one sub-block": the single-sequence kernel gives the eight
+// columns of the instruction to (block, sub-block parity), the multi-column kernel to eight activation vectors.
+#pragma once
+#include "ops.cuh"
+
+namespace bnk {
+
+constexpr int Q2_PIECE = 2176, Q2_SCALES = 2048;
+
+inline size_t q2_bytes(int M, int K) { return size_t((M + 15) / 16) * size_t(K / 512) * Q2_PIECE; }
+// native row-major PTQ1_0 -> two-bit tiles. half = 0 / 1: the matrix is the first / second of a pair whose rows share tiles
+// (rows 0..7 of a tile from the first, 8..15 from the second: gate and up of an FFN). K % 512 == 0; pairs: M % 8 == 0.
+void q2_repack(cudaStream_t st, const uint32_t *W, int M, int K, uint8_t *out, int half = -1);
+// sign values -> one bit per value (set = -1), 8 values per byte
+void pack_sign_bits(cudaStream_t st, const int32_t *signs, int n, uint8_t *bits);
+
+enum Q2Prologue { Q2_PLAIN = 0, Q2_NORM = 1 };
+// what follows this projection in the schedule: its weights (and norm weights) are prefetched into L2 from here
+struct Q2Share { int q, r; };             // CTA c takes q units, the first r CTAs one more
+constexpr int Q2_NEXT_BYTES = 256 << 10;  // per CTA: 38 MB in all, more than any projection of a block; the output head would push everything else out of L2
+struct Q2Next {
+    const uint8_t *W = nullptr;
+    int units = 0, unit_bytes = 0;        // row tiles and their bytes
+    int max_bytes = Q2_NEXT_BYTES;        // per CTA
+    const float *w = nullptr;
+    int w_bytes = 0;
+    Q2Share share = {0, 0};               // filled in by the launch
+};
+struct Q2Args {
+    const uint8_t *W;            // two-bit tiles
+    int M, K;                    // valid rows; K % 512 == 0, K <= 16384
+    int swiglu;                  // a pair of matrices: out[r] = silu(first_r) * second_r, M = rows of both together
+    float *out;                  // optional
+    const float *resid_in;       // with resid_out: resid_out = sum + resid_in
+    float *resid_out;
+    int pro;
+    const float *x0, *w;         // input; Q2_NORM: x = rms_norm(x0) * w
+    const uint8_t *sgn;          // sign bits of the K values
+    int hat_block;
+    float hat_inv, eps;
+    float inv_k;                 // filled in by the launch: 1 / K when K is a power of two, else 0 (divide);
+    int log_hat;                 // log2(hat_block);
+    Q2Share share;               // the CTAs' shares of the row tiles;
+    int slots;                   // ring slots
+    float *inv_out;              // Q2_NORM, optional: 1/sqrt(mean(x0^2) + eps)
+    Q2Next next;
+    int *err;                    // device error word (bounded waits)
+    unsigned long long *stamps;  // optional, 8 device time stamps of CTA 0 (see PhaseArgs)
+};
+bool q2_gemv_supported(int K, int hat_block);
+cudaError_t launch_q2_gemv(cudaStream_t st, int sm_count, const Q2Args &a, bool pdl);
+
+#ifdef __CUDACC__
+constexpr int Q2_MAGIC = 0x4B400000;           // bits of 12582912.0f: adding an int |i| < 2^22 gives the bits of 12582912 + i
+
+// D = A (u8) x B (s8) + C; the first instruction of a chain takes its C from constants
+__device__ __forceinline__ void q2_mma_first(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(Q2_MAGIC));
+}
+__device__ __forceinline__ void q2_mma(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+#endif
+
+}  // namespace bnk

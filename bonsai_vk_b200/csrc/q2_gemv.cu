@@ -1,0 +1,453 @@
+// q2_gemv.cu - the projection of one activation vector over the two-bit weight tiles (q2.cuh), with the preparation of its
+// input in front: [rms norm] -> signs -> Hadamard -> q8_1, then int8 tensor-core dots, then the fp32 combination of the
+// contract (t_sb = fma(d, I, -s); v = d_w ((t0 + t1) + (t2 + t3)); p_g = (v0 + v1) + (v2 + v3); out = p_0 + p_1 + ...).
+//
+// What bounds it: memory when it streams (two-bit tiles read 34 bytes per 128 weights), a latency chain of about 1 us in the
+// preparation otherwise. Per 16 x 512 piece a warp issues 64 ANDs, 16 mma, 5 loads and about 40 instructions of epilogue -
+// 2 warp instructions per 128-weight row-block against 9.1 of the kernel that unpacks base-3 bytes in the loop.
+//
+// Work split. A CTA of 16 warps owns a run of 16-row tiles over all of K; the pieces (tile, group of four blocks) of that run
+// are dealt to the warps in memory order, so with K = 4096 (8 groups) a warp keeps one group. A piece's group sums p_g go to
+// shared memory, and after a barrier one thread per row adds them in ascending order: no atomics, no sums that leave the CTA.
+// Data movement. A CTA's share of the matrix is one contiguous range; a 17th warp brings it into shared memory with a few bulk
+// copies (one piece per warp each), and every projection asks for the NEXT one's weights to be fetched into L2 at its own
+// start. Measured beside it: pieces loaded straight into registers (one or two ahead, 8 % slower on the output head, where the
+// ring runs at the DRAM's rate), one bulk copy per piece and warp (the issue sits on each warp's chain: 66 against 44 us for the
+// head), 16-byte cp.async (1.5 us of load/store-unit time before the first wait), products of one piece interleaved with the
+// sums of the one before (spills). One CTA per SM: with two resident (the next projection's beside this one's) the block
+// scheduler puts two CTAs of one projection on the same SM and leaves others idle (1.71 against 1.42 ms per token).
+#include "q2.cuh"
+#include "rotate_quant.cuh"
+#include "phase_gemv.cuh"
+
+#include <algorithm>
+
+namespace {
+using namespace bnk;
+
+constexpr int NT = 512, NW = NT / 32;          // compute threads; a 17th warp issues the copies
+constexpr int CHUNK = NW * Q2_PIECE;           // one piece per warp, contiguous in memory: one bulk copy
+constexpr int EARLY = 1, MAX_SLOTS = 6, SMEM_MAX = 227 << 10;
+struct Lay {                                    // dynamic shared memory, bytes
+    int bars, codes, ds, red, xs, ring;
+};
+__host__ __device__ constexpr Lay layout(int K) {
+    Lay l{};
+    l.bars = 0;
+    l.codes = 128;
+    l.ds = l.codes + K;
+    l.red = l.ds + (K / 32) * 4;
+    l.xs = l.red + 256 * 4;
+    l.ring = (l.xs + (K + 4095) / 4096 * XS8_SPAN * 4 + 127) & ~127;
+    return l;
+}
+constexpr int PBUF = XS8_SPAN;                 // floats of the transform's buffer that hold group sums afterwards
+
+__device__ __forceinline__ unsigned long long gtime() { unsigned long long t; asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t)); return t; }
+#define Q2_STAMP(i) do { if (a.stamps && blockIdx.x == 0 && threadIdx.x == 0) a.stamps[i] = gtime(); } while (0)
+
+__device__ __forceinline__ void load8(const float *p, f32pair (&v)[4]) {
+    const ulonglong2 *q = reinterpret_cast<const ulonglong2 *>(p);
+    const ulonglong2 a = q[0], b = q[1];
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+// barrier over the 16 compute warps (the copy warp never joins it)
+__device__ __forceinline__ void csync() { asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory"); }
+// bounded wait: on giving up the error word is set and the caller goes on to its end without waiting again (results are then
+// invalid)
+__device__ __forceinline__ bool slot_wait(uint32_t bar, uint32_t parity, int *err) {
+    for (int it = 0; it < (1 << 22); ++it) {
+        uint32_t ok;
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (__builtin_expect(ok != 0u, 1)) return true;
+    }
+    atomicExch(err, 1);
+    return false;
+}
+__device__ __forceinline__ void prefetch_l2(const uint8_t *p, int bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+// sign bits 2k and 2k + 1 of a byte as a pair of sign masks
+__device__ __forceinline__ f32pair sign_pair(uint32_t sg, int k) {
+    return (unsigned long long)((sg << (31 - 2 * k)) & 0x80000000u) | (unsigned long long)((sg << (30 - 2 * k)) & 0x80000000u) << 32;
+}
+
+// SPANS: spans of 4096 values whose inputs a thread holds at once (1: K <= 4096; 4: up to 16384)
+template <int SPANS>
+__global__ void __launch_bounds__(NT + 32, 1) k_q2_gemv(const Q2Args a) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const Lay L = layout(a.K);
+    unsigned char *codes = smem + L.codes;
+    uint32_t *dsw = reinterpret_cast<uint32_t *>(smem + L.ds);
+    float *red = reinterpret_cast<float *>(smem + L.red), *xs = reinterpret_cast<float *>(smem + L.xs);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tig = lane & 3;
+    Q2_STAMP(0);
+
+    // ---- this CTA's tiles ------------------------------------------------------------------------------------------
+    const int ng = a.K >> 9, cta = blockIdx.x, slots = a.slots;
+    const int t0 = cta * a.share.q + min(cta, a.share.r), nt = a.share.q + (cta < a.share.r);
+    const int npieces = nt * ng, nchunks = (npieces + NW - 1) / NW;
+    const uint32_t full = uint32_t(__cvta_generic_to_shared(smem + L.bars)), empty = full + MAX_SLOTS * 8;
+
+    if (warp == NW) {
+        // ---- copy warp. Before the previous kernel is done: one chunk of weights into the ring (more would hold up the input
+        // vector, which follows it through the same queue, by up to a microsecond) and the NEXT projection's weights (the
+        // share that this CTA's successor reads) towards L2; the other slots once the input vector is in registers; refills.
+        const uint8_t *W = a.W + size_t(t0) * ng * Q2_PIECE;
+        auto request = [&](int i, int s) {
+            const uint32_t bytes = uint32_t(min(NW, npieces - i * NW)) * Q2_PIECE;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full + s * 8), "r"(bytes) : "memory");
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         ::"r"(uint32_t(__cvta_generic_to_shared(smem + L.ring)) + s * CHUNK), "l"(W + size_t(i) * CHUNK), "r"(bytes), "r"(full + s * 8) : "memory");
+        };
+        if (lane == 0) {
+            for (int s = 0; s < slots; ++s) {
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full + s * 8));
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty + s * 8), "n"(NW));
+            }
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            for (int i = 0; i < min(EARLY, slots); ++i) request(i, i);
+            if (a.next.W) {
+                const Q2Next &n = a.next;
+                const uint8_t *src = n.W + size_t(cta * n.share.q + min(cta, n.share.r)) * n.unit_bytes;
+                const int bytes = min((n.share.q + (cta < n.share.r)) * n.unit_bytes, n.max_bytes);
+                for (int o = 0; o < bytes; o += 16384) prefetch_l2(src + o, min(16384, bytes - o));
+                if (cta == 0 && n.w) for (int o = 0; o < n.w_bytes; o += 16384) prefetch_l2(reinterpret_cast<const uint8_t *>(n.w) + o, min(16384, n.w_bytes - o));
+            }
+        }
+        __syncwarp();
+        asm volatile("bar.arrive 2, %0;" ::"n"(NT + 32) : "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        asm volatile("bar.sync 3, %0;" ::"n"(NT + 32) : "memory");
+        if (lane == 0) for (int i = EARLY; i < min(slots, nchunks); ++i) request(i, i);
+        for (int i = slots, s = 0, ph = 0; i < nchunks; ++i) {
+            if (!slot_wait(empty + s * 8, ph, a.err)) break;
+            if (lane == 0) request(i, s);
+            if (++s == slots) { s = 0; ph ^= 1; }
+        }
+        return;
+    }
+
+    // constants of the preparation depend on no earlier kernel: norm weights with the signs applied to them (the sign of the
+    // product is the product of the signs), or the signs as masks
+    const int base = tid * 8, nspan = SPANS == 1 ? 1 : (a.K + 4095) >> 12;
+    f32pair nw[4] = {0, 0, 0, 0};
+    uint32_t sg[SPANS];
+#pragma unroll
+    for (int s = 0; s < SPANS; ++s) sg[s] = base + s * 4096 < a.K ? a.sgn[(base >> 3) + s * 512] : 0u;
+    if (SPANS == 1 && a.pro == Q2_NORM && base < a.K) load8(a.w + base, nw);
+    Q2_STAMP(1);
+    // The next kernel may start now: whatever it does before its own wait touches constants only.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (SPANS == 1) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) nw[k] ^= sign_pair(sg[0], k);
+    }
+    asm volatile("bar.sync 2, %0;" ::"n"(NT + 32) : "memory");          // the ring's barriers are initialised
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    Q2_STAMP(2);
+
+    // ---- input preparation -------------------------------------------------------------------------------------------
+    f32pair v[SPANS][4];
+#pragma unroll
+    for (int s = 0; s < SPANS; ++s)
+        if (base + s * 4096 < a.K) load8(a.x0 + base + s * 4096, v[s]);
+        else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[s][k] = 0ull;
+        }
+    // the residual of the row this thread finishes first
+    float resid = 0.0f;
+    const int row0 = t0 * 16 + tid;
+    if (a.resid_out && tid < nt * 16 && row0 < a.M) resid = a.resid_in[row0];
+    f32pair inv2 = pair_of(1.0f, 1.0f);
+    if (a.pro == Q2_NORM) {
+        // rms_norm.comp order: 256 lanes sum the squares of their run of `per` consecutive values ascending, then the tree
+        const int per = (a.K + 255) >> 8;
+        if (SPANS == 1 && per == 16) {             // K = 4096: a lane's run is two neighbouring threads' values
+            float sq = 0.0f, e[8];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) split_pair(pair_mul(v[0][k], v[0][k]), e[2 * k], e[2 * k + 1]);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) sq = __fadd_rn(sq, e[k]);
+            sq = __shfl_up_sync(0xFFFFFFFFu, sq, 1);         // (an odd thread goes on from its even neighbour's sum)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) sq = __fadd_rn(sq, e[k]);
+            if (tid & 1) red[tid >> 1] = sq;
+        } else if (tid < 256) {
+            float sq = 0.0f;
+            for (int i = 0; i < per; ++i) {
+                const int d = tid * per + i;
+                if (d < a.K) { const float x = a.x0[d]; sq = __fadd_rn(sq, __fmul_rn(x, x)); }
+            }
+            red[tid] = sq;
+        }
+        csync();
+        const float ss = norm_tree256(red, lane);
+        const float inv = __frcp_rn(__fsqrt_rn(__fadd_rn(a.inv_k != 0.0f ? __fmul_rn(ss, a.inv_k) : __fdiv_rn(ss, float(a.K)), a.eps)));
+        if (a.inv_out && cta == 0 && tid == 0) a.inv_out[0] = inv;
+        inv2 = pair_of(inv, inv);
+    }
+    Q2_STAMP(3);
+#pragma unroll
+    for (int s = 0; s < SPANS; ++s) {
+        if (s < nspan) {
+            if (SPANS > 1) {
+                if (a.pro == Q2_NORM && base + s * 4096 < a.K) {
+                    load8(a.w + base + s * 4096, nw);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) v[s][k] = pair_mul(pair_mul(v[s][k], inv2), nw[k]);
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[s][k] ^= sign_pair(sg[s], k);
+            } else if (a.pro == Q2_NORM) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[s][k] = pair_mul(pair_mul(v[s][k], inv2), nw[k]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[s][k] ^= nw[k];
+            }
+            fwht_pairs8(v[s], 3);                  // the stages h = 1, 2, 4
+            span_store8(xs + s * XS8_SPAN, tid, v[s]);
+        }
+    }
+    asm volatile("bar.arrive 3, %0;" ::"n"(NT + 32) : "memory");          // to the copy warp: the input is here
+    fwht_spans(xs, tid, nspan, a.log_hat, [] { csync(); });
+    Q2_STAMP(4);
+#pragma unroll 1
+    for (int s = 0; s < nspan; ++s) {
+        f32pair y[4];
+        span_load8(xs + s * XS8_SPAN, tid, y);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) y[k] = pair_mul(y[k], pair_of(a.hat_inv, a.hat_inv));
+        const Q8x8 q = quant8_pairs(y);
+        const int at = base + s * 4096;
+        if (at < a.K) {
+            // codes of (block, sub-block b, elements 8t .. 8t + 7) at block * 128 + (b & 1) * 64 + t * 16 + (b >> 1) * 8
+            const int b = (at >> 5) & 3, e8 = (at >> 3) & 3;
+            *reinterpret_cast<uint2 *>(codes + (at & ~127) + (b & 1) * 64 + e8 * 16 + (b >> 1) * 8) = make_uint2(q.w0, q.w1);
+            if (e8 == 0) dsw[at >> 5] = float_to_half_bits(q.d) | (float_to_half_bits(__fmul_rn(q.d, float(q.sum))) << 16);
+        }
+    }
+    csync();
+    Q2_STAMP(5);
+
+    // ---- pieces ------------------------------------------------------------------------------------------------------
+    uint2 B[4][4];                                 // operand B of [block][sub-block]: the codes in the lanes of column 2j + (s & 1), zero in the others
+    f32pair d01 = 0, d23 = 0, n01 = 0, n23 = 0;    // block tig: (d0, d1/4), (d2/16, d3/64), (-s0, -s1), (-s2, -s3)
+    int group = -1;
+    auto set_group = [&](int gr) {
+        const uint4 own = *reinterpret_cast<const uint4 *>(codes + (gr * 4 + (g >> 1)) * 128 + (g & 1) * 64 + tig * 16);   // sub-blocks (g & 1) and (g & 1) + 2
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            B[c >> 1][c & 1] = g == c ? make_uint2(own.x, own.y) : make_uint2(0u, 0u);
+            B[c >> 1][(c & 1) + 2] = g == c ? make_uint2(own.z, own.w) : make_uint2(0u, 0u);
+        }
+        const uint4 ds = *reinterpret_cast<const uint4 *>(dsw + (gr * 4 + tig) * 4);
+        d01 = pair_of(half_bits_to_float(ds.x), half_bits_to_float(ds.y) * 0.25f);
+        d23 = pair_of(half_bits_to_float(ds.z) * 0.0625f, half_bits_to_float(ds.w) * 0.015625f);
+        n01 = pair_of(-half_bits_to_float(ds.x >> 16), -half_bits_to_float(ds.y >> 16));
+        n23 = pair_of(-half_bits_to_float(ds.z >> 16), -half_bits_to_float(ds.w >> 16));
+        group = gr;
+    };
+    const f32pair magic2 = pair_of(__int_as_float(Q2_MAGIC), __int_as_float(Q2_MAGIC));
+    // tiles per run of group sums: what the transform's buffer holds
+    const int run = max(1, PBUF / (16 * ng)), gstep = NW % ng;
+    int u = warp, gr = warp % ng, slot = 0;
+    uint32_t phase = 0;
+    bool alive = true;
+    // one piece: its group sums p_g of 16 rows go to `dst`
+    auto piece = [&](float *dst) {
+        if (gr != group) set_group(gr);
+        gr += gstep; if (gr >= ng) gr -= ng;
+        if (alive) alive = slot_wait(full + slot * 8, phase, a.err);
+        const unsigned char *src = smem + L.ring + slot * CHUNK + warp * Q2_PIECE;
+        uint4 c[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) c[q] = *reinterpret_cast<const uint4 *>(src + lane * 16 + q * 512);
+        const uint32_t dw = *reinterpret_cast<const uint32_t *>(src + Q2_SCALES + lane * 4);
+        if (u - warp + slots * NW < npieces) {     // the slot is refilled: this warp's part of it is in registers
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty + slot * 8) : "memory");
+        }
+        if (++slot == slots) { slot = 0; phase ^= 1; }
+        int e[4], f[4];                            // sub-blocks (0, 1) and (2, 3) of block tig, rows g and g + 8
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint4 &lo = c[j >> 1], &hi = c[2 + (j >> 1)];
+            const uint32_t l0 = (j & 1) ? lo.z : lo.x, l1 = (j & 1) ? lo.w : lo.y, h0 = (j & 1) ? hi.z : hi.x, h1 = (j & 1) ? hi.w : hi.y;
+            constexpr uint32_t m0 = 0x03030303u, m1 = m0 << 2, m2 = m0 << 4, m3 = m0 << 6;
+            if (j == 0) {
+                q2_mma_first(e, l0 & m0, h0 & m0, l1 & m0, h1 & m0, B[j][0].x, B[j][0].y);
+                q2_mma_first(f, l0 & m2, h0 & m2, l1 & m2, h1 & m2, B[j][2].x, B[j][2].y);
+            } else {
+                q2_mma(e, l0 & m0, h0 & m0, l1 & m0, h1 & m0, B[j][0].x, B[j][0].y);
+                q2_mma(f, l0 & m2, h0 & m2, l1 & m2, h1 & m2, B[j][2].x, B[j][2].y);
+            }
+            q2_mma(e, l0 & m1, h0 & m1, l1 & m1, h1 & m1, B[j][1].x, B[j][1].y);
+            q2_mma(f, l0 & m3, h0 & m3, l1 & m3, h1 & m3, B[j][3].x, B[j][3].y);
+        }
+        auto block_sum = [&](int e0, int e1, int f0, int f1, uint32_t w) {
+            float x0, x1, x2, x3;
+            split_pair(pair_fma(d01, pair_sub(pair_of(__int_as_float(e0), __int_as_float(e1)), magic2), n01), x0, x1);
+            split_pair(pair_fma(d23, pair_sub(pair_of(__int_as_float(f0), __int_as_float(f1)), magic2), n23), x2, x3);
+            return __fmul_rn(half_bits_to_float(w), __fadd_rn(__fadd_rn(x0, x1), __fadd_rn(x2, x3)));
+        };
+        float va = block_sum(e[0], e[1], f[0], f[1], dw), vb = block_sum(e[2], e[3], f[2], f[3], dw >> 16);
+        va = __fadd_rn(va, __shfl_xor_sync(0xFFFFFFFFu, va, 1)); vb = __fadd_rn(vb, __shfl_xor_sync(0xFFFFFFFFu, vb, 1));
+        va = __fadd_rn(va, __shfl_xor_sync(0xFFFFFFFFu, va, 2)); vb = __fadd_rn(vb, __shfl_xor_sync(0xFFFFFFFFu, vb, 2));
+        if (tig < 2) dst[g + 8 * tig] = tig ? vb : va;
+    };
+    Q2_STAMP(6);
+    for (int c0 = 0; c0 < nt; c0 += run) {
+        const int c1 = min(nt, c0 + run), uend = c1 * ng, rows = (c1 - c0) * 16;
+        // what the sums below need, worked out ahead of the barrier
+        const float *own = xs + (tid >> 4) * ng * 16 + (tid & 15);
+        const int row = (t0 + c0) * 16 + tid;
+        for (; u < uend; u += NW) piece(xs + (u - c0 * ng) * 16);
+        csync();
+        for (int i0 = 0; i0 < rows; i0 += NT, own += (NT / 16) * ng * 16) {
+            const bool on = i0 + tid < rows;
+            float s = 0.0f;
+            if (on) {
+                if (ng == 8) {                     // (loads first, then the adds in ascending order)
+                    float x[8];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) x[k] = own[k * 16];
+                    s = x[0];
+#pragma unroll
+                    for (int k = 1; k < 8; ++k) s = __fadd_rn(s, x[k]);
+                } else {
+                    s = own[0];
+                    int k = 1;
+                    for (; k + 8 <= ng; k += 8) {
+                        float x[8];
+#pragma unroll
+                        for (int b = 0; b < 8; ++b) x[b] = own[(k + b) * 16];
+#pragma unroll
+                        for (int b = 0; b < 8; ++b) s = __fadd_rn(s, x[b]);
+                    }
+#pragma unroll 4
+                    for (; k < ng; ++k) s = __fadd_rn(s, own[k * 16]);
+                }
+                if (!a.swiglu && row + i0 < a.M) {
+                    if (a.out) a.out[row + i0] = s;
+                    if (a.resid_out) a.resid_out[row + i0] = __fadd_rn(s, row + i0 == row0 ? resid : a.resid_in[row + i0]);
+                }
+            }
+            if (a.swiglu) {                        // rows r and r + 8 of a tile: gate and up of one FFN row
+                const float up = __shfl_down_sync(0xFFFFFFFFu, s, 8);
+                if (on && !(tid & 8)) a.out[((row + i0) >> 4) * 8 + (tid & 7)] = __fmul_rn(silu_f(s), up);
+            }
+        }
+        if (c1 < nt) csync();
+    }
+    Q2_STAMP(7);
+}
+
+// one thread per (row, block): five base-3 digits per byte -> the four two-bit fields of the piece (unpacking as in the
+// multi-column kernel: T_t = (b * 3^(t+1)) >> 8 is the base-3 prefix of byte b, digit t = T_t - 3 T_(t-1))
+__device__ __forceinline__ void unpack4(uint32_t w, uint32_t *o, int stride) {
+    const uint32_t e = __byte_perm(w, 0u, 0x4240u), d = __byte_perm(w, 0u, 0x4341u);
+    uint32_t prev = 0u, p = 3u;
+#pragma unroll
+    for (int t = 0; t < 5; ++t, p *= 3u) {
+        const uint32_t T = __byte_perm(e * p, d * p, 0x7351u);
+        o[t * stride] = T - 3u * prev;
+        prev = T;
+    }
+}
+__global__ void __launch_bounds__(256) k_q2_repack(const uint32_t *__restrict__ W, int M, int nb, uint8_t *__restrict__ out, int half) {
+    pdl_sync();
+    const int ng = nb >> 2, ntiles = (M + 15) >> 4;
+    const size_t total = size_t(ntiles) * 16 * nb;
+    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
+        const int b = int(i % nb), row = int(i / nb), r = half < 0 ? row & 15 : (row & 7) + 8 * half, tile = half < 0 ? row >> 4 : row >> 3, j = b & 3;
+        uint32_t o[32], w[7] = {0, 0, 0, 0, 0, 0, 0};
+        if (row < M) {
+#pragma unroll
+            for (int k = 0; k < 7; ++k) w[k] = W[(size_t(row) * nb + b) * 7 + k];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) unpack4(w[k], o + k, 4);
+        unpack4(w[4], o + 20, 2);
+        unpack4(w[5], o + 21, 2);
+        const uint32_t v = __byte_perm(w[6], 0u, 0x4140u);
+        const uint32_t ta = __byte_perm(v * 3u, v * 9u, 0x7531u), tb = __byte_perm(v * 27u, v * 81u, 0x7531u);
+        o[30] = ta - 3u * (ta << 16);
+        o[31] = tb - 3u * __byte_perm(ta, tb, 0x5432u);
+        uint8_t *piece = out + (size_t(tile) * ng + (b >> 2)) * Q2_PIECE;
+        uint8_t *dst = piece + ((r >> 3) * 2 + (j >> 1)) * 512 + (r & 7) * 64 + (j & 1) * 8;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            uint2 p;
+            p.x = o[2 * t] | o[8 + 2 * t] << 2 | o[16 + 2 * t] << 4 | o[24 + 2 * t] << 6;
+            p.y = o[2 * t + 1] | o[9 + 2 * t] << 2 | o[17 + 2 * t] << 4 | o[25 + 2 * t] << 6;
+            *reinterpret_cast<uint2 *>(dst + t * 16) = p;
+        }
+        *reinterpret_cast<uint16_t *>(piece + Q2_SCALES + ((r & 7) * 4 + j) * 4 + (r >> 3) * 2) = uint16_t(w[6] >> 16);
+    }
+}
+__global__ void k_sign_bits(const int32_t *__restrict__ signs, int nwords, uint8_t *__restrict__ bits) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nwords) return;
+    uint32_t b = 0;
+    for (int k = 0; k < 8; ++k) b |= (signs[i * 8 + k] < 0 ? 1u : 0u) << k;
+    bits[i] = uint8_t(b);
+}
+
+template <int SPANS>
+cudaError_t launch_spans(cudaStream_t st, int sm_count, Q2Args a, bool pdl) {
+    static int smem_set = 0;
+    // as many chunks of weights as fit beside the rest, and at least half of an SM's shared memory in all, so that two CTAs of a
+    // launch never share an SM (see above)
+    const int ng = a.K / 512, tiles = (a.M + 15) / 16, grid = tiles < sm_count ? tiles : sm_count;
+    a.share = {tiles / grid, tiles % grid};
+    const int chunks = ((a.share.q + (a.share.r > 0)) * ng + NW - 1) / NW;
+    a.slots = std::min({chunks, MAX_SLOTS, (SMEM_MAX - layout(a.K).ring) / CHUNK});
+    const int smem = std::max(layout(a.K).ring + a.slots * CHUNK, 116 << 10);
+    if (smem > smem_set) {
+        cudaError_t e = cudaFuncSetAttribute(k_q2_gemv<SPANS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        smem_set = smem;
+    }
+    a.inv_k = (a.K & (a.K - 1)) == 0 ? 1.0f / float(a.K) : 0.0f;
+    a.log_hat = 31 - __builtin_clz(unsigned(a.hat_block));
+    if (a.next.W) a.next.share = {a.next.units / grid, a.next.units % grid};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(NT + 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl ? 1 : 0;
+    BN_COUNT(1);
+    return cudaLaunchKernelEx(&cfg, k_q2_gemv<SPANS>, a);
+}
+
+}  // namespace
+
+namespace bnk {
+
+bool q2_gemv_supported(int K, int hat_block) {
+    return K >= 512 && K % 512 == 0 && K <= 16384 && hat_block >= 16 && hat_block <= 4096 && (hat_block & (hat_block - 1)) == 0 && K % hat_block == 0;
+}
+
+cudaError_t launch_q2_gemv(cudaStream_t st, int sm_count, const Q2Args &a, bool pdl) {
+    return a.K <= 4096 ? launch_spans<1>(st, sm_count, a, pdl) : launch_spans<4>(st, sm_count, a, pdl);
+}
+
+void q2_repack(cudaStream_t st, const uint32_t *W, int M, int K, uint8_t *out, int half) {
+    const size_t total = size_t((M + 15) / 16) * 16 * (K / 128);
+    launch(k_q2_repack, dim3(unsigned(std::min<size_t>((total + 255) / 256, 148 * 16))), dim3(256), 0, st, W, M, K / 128, out, half);
+}
+void pack_sign_bits(cudaStream_t st, const int32_t *signs, int n, uint8_t *bits) {
+    BN_COUNT(1);
+    k_sign_bits<<<(n / 8 + 255) / 256, 256, 0, st>>>(signs, n / 8, bits);
+}
+
+}  // namespace bnk
