@@ -1,5 +1,6 @@
 // gemm_abi.cu - C entry points of the multi-column tensor-core projection (declared in include/bonsai_cuda.h).
 #include "gemm_tc.cuh"
+#include "q2.cuh"
 #include "phase_gemv.cuh"
 
 #include <cstdio>
@@ -35,16 +36,16 @@ int bn_gemm_act_quant(bn_ctx *ctx, const bn_buf *x, size_t x_off, size_t x_strid
 
 size_t bn_gemm_tiled_bytes(int M, int K) {
     if (M <= 0 || K <= 0 || K % 1024) return 0;
-    return bnk::gemm_tiled_bytes(M, K);
+    return bnk::q2_bytes(M, K);
 }
 
 int bn_gemm_repack(bn_ctx *ctx, const bn_buf *w, size_t w_off, int M, int K, bn_buf *tiled, size_t tiled_off) {
     BN_REQUIRE(ctx, BN_ERR_ARG, "bn_gemm_repack: null context");
     BN_REQUIRE(M > 0 && K > 0 && K % 1024 == 0, BN_ERR_ARG, "bn_gemm_repack: bad shape M=%d K=%d (K %% 1024 != 0)", M, K);
     BN_RANGE(w, w_off, size_t(M) * (K / 128) * 28, 4, "bn_gemm_repack W");
-    BN_RANGE(tiled, tiled_off, bnk::gemm_tiled_bytes(M, K), 128, "bn_gemm_repack out");
-    bnk::repack_tiles(ctx->stream, bn_ptr<uint32_t>(w, w_off), M, K, bn_ptr<uint32_t>(tiled, tiled_off));
-    return bn_launch_check(ctx, "k_repack_tiles");
+    BN_RANGE(tiled, tiled_off, bnk::q2_bytes(M, K), 128, "bn_gemm_repack out");
+    bnk::q2_repack(ctx->stream, bn_ptr<uint32_t>(w, w_off), M, K, bn_ptr<uint8_t>(tiled, tiled_off));
+    return bn_launch_check(ctx, "k_q2_repack");
 }
 
 int bn_gemm_q81(bn_ctx *ctx, const bn_buf *w, size_t w_off, int w_tiled, int M, int K, const bn_buf *image, size_t image_off, int ncol,
@@ -53,12 +54,20 @@ int bn_gemm_q81(bn_ctx *ctx, const bn_buf *w, size_t w_off, int w_tiled, int M, 
     BN_REQUIRE(bnk::gemm_supported(M, K, ncol), BN_ERR_ARG, "bn_gemm_q81: unsupported shape M=%d K=%d columns=%d (K %% 1024 == 0, 1..%d columns)",
                M, K, ncol, bnk::GEMM_MAX_COLS);
     BN_REQUIRE(out_stride >= size_t(M), BN_ERR_ARG, "bn_gemm_q81: column stride %zu is shorter than M", out_stride);
-    if (w_tiled) BN_RANGE(w, w_off, bnk::gemm_tiled_bytes(M, K), 128, "bn_gemm_q81 W (tiled)");
+    if (w_tiled) BN_RANGE(w, w_off, bnk::q2_bytes(M, K), 128, "bn_gemm_q81 W (tiled)");
     else BN_RANGE(w, w_off, size_t(M) * (K / 128) * 28, 16, "bn_gemm_q81 W");
     BN_RANGE(image, image_off, bnk::gemm_image_bytes(K, ncol), 128, "bn_gemm_q81 image");
     BN_RANGE(out, out_off, (size_t(ncol - 1) * out_stride + M) * 4, 4, "bn_gemm_q81 out");
+    if (w_tiled) {
+        bnk::Q2GemmArgs q = {};
+        q.W = bn_ptr<uint8_t>(w, w_off); q.M = M; q.K = K; q.image = bn_ptr<uint8_t>(image, image_off); q.ncol = ncol;
+        q.out = bn_ptr<float>(out, out_off); q.out_stride = out_stride; q.err = ctx->err_dev;
+        cudaError_t e = bnk::launch_q2_gemm(ctx->stream, ctx->sm_count, q, bnk::g_pdl);
+        if (e != cudaSuccess) return bn_cuda_fail(e, "k_q2_gemm");
+        return bn_launch_check(ctx, "k_q2_gemm");
+    }
     bnk::GemmArgs a = {};
-    a.W = bn_ptr<uint8_t>(w, w_off); a.M = M; a.K = K; a.tiled = w_tiled ? 1 : 0;
+    a.W = bn_ptr<uint8_t>(w, w_off); a.M = M; a.K = K; a.tiled = 0;
     a.image = bn_ptr<uint8_t>(image, image_off); a.ncol = ncol;
     a.out = bn_ptr<float>(out, out_off); a.out_stride = out_stride;
     a.err = ctx->err_dev;

@@ -513,158 +513,6 @@ __global__ void __launch_bounds__(Cfg<NCP>::NWARPS * 32, Cfg<NCP>::CTAS) k_ptq_g
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tb), "r"(uint32_t(C::TMEM_COLS)) : "memory");
 }
 
-// ---- activation image: [rms norm] -> signs -> Hadamard per hat_block -> q8_1 codes and scales -----------------
-// grid (K / chunk, padded columns), 512 threads; chunk = hat_block (or 1024 without rotation)
-// chunk = the values one CTA takes: a Hadamard block (hb), or 32 when the Hadamard block is smaller than a q8_1 sub-block
-__global__ void __launch_bounds__(512) k_prep_cols(const PrepArgs a, int chunk, int hb, int ncp) {
-    pdl_sync();
-    extern __shared__ __align__(16) float s[];     // chunk floats
-    __shared__ float part[256];
-    const int cg = blockIdx.y, tid = threadIdx.x;
-    const int c = cg;
-    const size_t base = size_t(blockIdx.x) * chunk;
-    const size_t blk_bytes = size_t(ncp) * IMG_COL;
-    unsigned char *image = a.image;
-    if (cg >= a.ncol) {                             // padding column: zero codes and scales
-        for (int e = tid * 16; e < chunk; e += 512 * 16) {
-            const size_t b = (base + e) / 128;
-            const int sb = int((base + e) & 127) >> 5, kh = (e >> 4) & 1;
-            *reinterpret_cast<uint4 *>(image + b * blk_bytes + (c / 8) * 1024 + (sb * 2 + kh) * 128 + (c & 7) * 16) = make_uint4(0, 0, 0, 0);
-        }
-        for (int e = tid * 32; e < chunk; e += 512 * 32) {
-            const size_t b = (base + e) / 128;
-            float *ent = reinterpret_cast<float *>(image + b * blk_bytes + size_t(ncp) * 128 + (c / 8) * 256 + (((int((base + e) & 127) >> 5) * 4) + ((c & 7) >> 1)) * 16);
-            ent[c & 1] = 0.0f; ent[2 + (c & 1)] = 0.0f;
-        }
-        return;
-    }
-    const float *x = a.x + size_t(cg) * a.x_stride;
-    float inv = 1.0f;
-    const int lane_id = tid & 31, warp_id = tid >> 5;
-    if (a.mode == PREP_NORM) {
-        // same partial sums as the stand-alone norm kernel: 256 lanes, each its consecutive run, then the fixed tree
-        // p[i] += p[i + s], s = 128 .. 1 - run by every warp on its own (the same adds in the same order give the same float
-        // in every warp), so one barrier instead of nine
-        const int per = (a.K + 255) / 256;
-        if (tid < 256) {
-            float acc = 0.0f;
-            if (per == 16 && a.K == 4096) {
-                const float4 *xv = reinterpret_cast<const float4 *>(x + tid * 16);
-                const float4 v0 = xv[0], v1 = xv[1], v2 = xv[2], v3 = xv[3];
-                const float e[16] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w, v2.x, v2.y, v2.z, v2.w, v3.x, v3.y, v3.z, v3.w};
-#pragma unroll
-                for (int i = 0; i < 16; ++i) acc = __fadd_rn(acc, __fmul_rn(e[i], e[i]));
-            } else {
-                for (int i = 0; i < per; ++i) {
-                    const int d = tid * per + i;
-                    if (d < a.K) { const float v = x[d]; acc = __fadd_rn(acc, __fmul_rn(v, v)); }
-                }
-            }
-            part[tid] = acc;
-        }
-        __syncthreads();
-        float v[8];
-#pragma unroll
-        for (int w = 0; w < 8; ++w) v[w] = part[32 * w + lane_id];
-        float t = __fadd_rn(__fadd_rn(__fadd_rn(v[0], v[4]), __fadd_rn(v[2], v[6])),
-                            __fadd_rn(__fadd_rn(v[1], v[5]), __fadd_rn(v[3], v[7])));
-#pragma unroll
-        for (int s2 = 16; s2 > 0; s2 >>= 1) t = __fadd_rn(t, __shfl_xor_sync(0xFFFFFFFFu, t, s2));
-        inv = __frcp_rn(__fsqrt_rn(__fadd_rn(mean_of(t, a.K), a.eps)));
-        if (a.inv_out && blockIdx.x == 0 && tid == 0) a.inv_out[size_t(cg) * a.inv_stride] = inv;
-    }
-    if (a.signs && chunk >= 256) {
-        // Sylvester butterflies (a+c, a-c), h ascending, as hat4096.comp:41-60: h = 1, 2, 4 inside a thread's 8
-        // consecutive elements, h = 8..128 across lanes; then through shared memory (h = 256..1024 inside a thread and
-        // h = 2048 between lanes l and l^16 when the chunk is 4096). Same pairs, same order: bit-identical to the plain loop.
-        if (tid < chunk / 8) {
-            const size_t tb = base + size_t(tid) * 8;
-            const float4 x0 = *reinterpret_cast<const float4 *>(x + tb), x1 = *reinterpret_cast<const float4 *>(x + tb + 4);
-            const int4 g0 = *reinterpret_cast<const int4 *>(a.signs + tb), g1 = *reinterpret_cast<const int4 *>(a.signs + tb + 4);
-            float v[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-            const int sg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-            if (a.mode == PREP_NORM) {
-                const float4 n0 = *reinterpret_cast<const float4 *>(a.w + tb), n1 = *reinterpret_cast<const float4 *>(a.w + tb + 4);
-                const float ne[8] = {n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, n1.z, n1.w};
-#pragma unroll
-                for (int r = 0; r < 8; ++r) v[r] = __fmul_rn(__fmul_rn(v[r], inv), ne[r]);
-            }
-#pragma unroll
-            for (int r = 0; r < 8; ++r) v[r] = __fmul_rn(v[r], float(sg[r]));
-            fwht_regs_lanes(v, lane_id);
-            float4 *dst = reinterpret_cast<float4 *>(s + tid * 8);
-            dst[0] = make_float4(v[0], v[1], v[2], v[3]);
-            dst[1] = make_float4(v[4], v[5], v[6], v[7]);
-        }
-        __syncthreads();
-        const float hinv = 1.0f / sqrtf(float(chunk));
-        if (chunk == 4096) {
-            fwht_4096_tail(s, warp_id, lane_id, hinv);
-        } else {
-            for (int h = 256; h < chunk; h <<= 1) {
-                for (int i = tid; i < (chunk >> 1); i += 512) {
-                    const int j = ((i & ~(h - 1)) << 1) | (i & (h - 1));
-                    const float p = s[j], r = s[j + h];
-                    s[j] = __fadd_rn(p, r);
-                    s[j + h] = __fsub_rn(p, r);
-                }
-                __syncthreads();
-            }
-            for (int i = tid; i < chunk; i += 512) s[i] = __fmul_rn(s[i], hinv);
-        }
-    } else {
-        for (int i = tid; i < chunk; i += 512) {
-            float v = x[base + i];
-            if (a.mode == PREP_NORM) v = __fmul_rn(__fmul_rn(v, inv), a.w[base + i]);
-            if (a.signs) v = __fmul_rn(v, float(a.signs[base + i]));
-            s[i] = v;
-        }
-        if (a.signs) {
-            const float hinv = 1.0f / sqrtf(float(hb));
-            for (int h = 1; h < hb; h <<= 1) {
-                __syncthreads();
-                for (int i = tid; i < (chunk >> 1); i += 512) {
-                    const int j = ((i & ~(h - 1)) << 1) | (i & (h - 1));
-                    const float p = s[j], r = s[j + h];
-                    s[j] = __fadd_rn(p, r);
-                    s[j + h] = __fsub_rn(p, r);
-                }
-            }
-            __syncthreads();
-            for (int i = tid; i < chunk; i += 512) s[i] = __fmul_rn(s[i], hinv);
-        }
-    }
-    __syncthreads();
-    // q8_1 per 32 values: four threads per sub-block, eight consecutive values each (quant8_of32); the eight codes are one
-    // 8-byte store into the image, (d, s) rounded to fp16 as the q8_1 record keeps them and stored as fp32 d and -s
-    for (int sbk0 = 0; sbk0 < chunk / 32; sbk0 += 128) {
-        const int sbk = sbk0 + (tid >> 2), q4 = tid & 3;
-        const bool live = sbk < chunk / 32;
-        float e[8];
-        if (live) {
-            const float4 *src = reinterpret_cast<const float4 *>(s + sbk * 32 + q4 * 8);
-            const float4 v0 = src[0], v1 = src[1];
-            e[0] = v0.x; e[1] = v0.y; e[2] = v0.z; e[3] = v0.w; e[4] = v1.x; e[5] = v1.y; e[6] = v1.z; e[7] = v1.w;
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) e[i] = 0.0f;
-        }
-        const Q8x8 q = quant8_of32(e);
-        if (live) {
-            const int e0 = sbk * 32 + q4 * 8;
-            const size_t b = (base + e0) / 128;
-            const int sb = int((base + e0) & 127) >> 5, kh = (e0 >> 4) & 1;       // (a chunk may be a part of a 128-value block)
-            unsigned char *blk = image + b * blk_bytes;
-            *reinterpret_cast<uint2 *>(blk + (c / 8) * 1024 + (sb * 2 + kh) * 128 + (c & 7) * 16 + (e0 & 15)) = make_uint2(q.w0, q.w1);
-            if (q4 == 0) {
-                float *ent = reinterpret_cast<float *>(blk + size_t(ncp) * 128 + (c / 8) * 256 + (sb * 4 + ((c & 7) >> 1)) * 16);
-                ent[c & 1] = half_bits_to_float(float_to_half_bits(q.d));
-                ent[2 + (c & 1)] = -half_bits_to_float(float_to_half_bits(__fmul_rn(q.d, float(q.sum))));
-            }
-        }
-    }
-}
-
 // native row-major PTQ1_0 -> per (tile of 128 rows, 8 blocks of K): [block][word 0..6][row] dwords; rows beyond M are zero
 __global__ void k_repack_tiles(const uint32_t *__restrict__ W, int M, int nb, uint32_t *__restrict__ out, size_t total) {
     pdl_sync();
@@ -770,14 +618,6 @@ size_t gemm_tiled_bytes(int M, int K) { return size_t((M + 127) / 128) * (K / 12
 void repack_tiles(cudaStream_t st, const uint32_t *W, int M, int K, uint32_t *out) {
     const size_t total = gemm_tiled_bytes(M, K) / 4;
     launch(k_repack_tiles, dim3(unsigned(std::min<size_t>((total + 255) / 256, 148 * 16))), dim3(256), 0, st, W, M, K / 128, out, total);
-}
-
-void prep_cols(cudaStream_t st, const PrepArgs &a) {
-    const int chunk = a.signs ? (a.hat_block < 32 ? 32 : a.hat_block) : 1024;
-    const int ncp = gemm_padded_cols(a.ncol);
-    static bool attr = false;
-    if (!attr) { cudaFuncSetAttribute(k_prep_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, 4096 * 4); attr = true; }
-    launch(k_prep_cols, dim3(a.K / chunk, ncp), dim3(512), size_t(chunk) * 4, st, a, chunk, a.signs ? a.hat_block : chunk, ncp);
 }
 
 cudaError_t launch_wait_selftest_tc(cudaStream_t st, int *err) {

@@ -75,11 +75,7 @@ struct bn_model {
     int ncols = 1;
     uint8_t *IMG_H = nullptr, *IMG_F = nullptr;
     uint8_t *IMG_HD = nullptr;            // sharded head: its own activation image, so that the head may run beside a stage pass
-    float *GROUPS = nullptr;              // group sums of the projections that are split over K (gemm_tc.cuh)
-    uint8_t *tiled = nullptr;
-    struct TiledLayer { const uint8_t *in = nullptr, *out = nullptr, *ffn_in = nullptr, *ffn_down = nullptr; };
-    std::vector<TiledLayer> tl;
-    const uint8_t *t_head = nullptr;
+    const uint8_t *q2_shard = nullptr;    // this model's rows of the output head (all of them unless it is sharded)
     int head_r0 = 0, head_r1 = 0;         // rows of the output head this model holds for the multi-sequence pass
     bool head_sharded = false;            // bn_model_set_head_rows: the head runs through bn_model_head_batch, not in the last stage
     float *CAND = nullptr;                // [batch_cols][2] candidates of a head shard
@@ -474,17 +470,17 @@ int build_q2(bn_model *m) {
         part(L.ffn_down, h.hidden, h.ffn);
     }
     if (m->b1 == h.n_layer) { matrix(&m->q2_head); part(m->out_w, h.vocab, h.hidden); }
+    else if (m->head_sharded) { matrix(&m->q2_shard); part(m->out_w + size_t(m->head_r0) * (h.hidden / 128) * 7, m->head_r1 - m->head_r0, h.hidden); }
     BN_CUDA(cudaMalloc(&m->q2, total));
     BN_CUDA(cudaMalloc(&m->SGN, size_t(h.hidden + h.ffn) / 8));
     for (auto &w : where) *w.first = m->q2 + w.second;
+    if (m->q2_head) m->q2_shard = m->q2_head + size_t(m->head_sharded ? m->head_r0 / 16 : 0) * (h.hidden / 512) * bnk::Q2_PIECE;
     for (const Part &p : parts) bnk::q2_repack(m->ctx->stream, p.w, p.M, p.K, m->q2 + p.off, p.half);
     bnk::pack_sign_bits(m->ctx->stream, m->signs, h.hidden + h.ffn, m->SGN);
     return bn_launch_check(m->ctx, "two-bit tiles");
 }
 
 // ---- multi-sequence pass ---------------------------------------------------------------------------------
-// Tile-major copies of the local projection weights (one allocation). Projections that read the same input are
-// stacked into one matrix whatever their placement in memory: every part is a whole number of 128-row tiles.
 int build_batch_side(bn_model *m) {
     const bn_hparams &h = m->hp;
     const int NH = h.gdn_heads, NQ = h.gdn_qk_heads, D = h.gdn_dim, C = 2 * NQ * D + NH * D, IN = NH * D;
@@ -493,53 +489,13 @@ int build_batch_side(bn_model *m) {
     BN_REQUIRE(h.hidden % 1024 == 0 && h.ffn % 1024 == 0, BN_ERR_ARG, "bn_model_finalize: the multi-sequence pass needs hidden and ffn to be multiples of 1024");
     BN_REQUIRE(C % 128 == 0 && IN % 128 == 0 && (2 * QD) % 128 == 0 && KD % 128 == 0 && h.ffn % 128 == 0 && h.hidden % 128 == 0, BN_ERR_ARG,
                "bn_model_finalize: the multi-sequence pass needs every projection height to be a multiple of 128");
-    struct Part { const uint32_t *w; int M; };
-    struct Group { std::vector<Part> parts; int K; const uint8_t **dst; };
-    std::vector<Group> groups;
-    m->tl.assign(h.n_layer, bn_model::TiledLayer());
-    for (int b = m->b0; b < m->b1; ++b) {
-        const bn_model::Layer &L = m->layers[b];
-        bn_model::TiledLayer &T = m->tl[b];
-        if (L.attn) {
-            groups.push_back({{{L.q_w, 2 * QD}, {L.k_w, KD}, {L.v_w, KD}}, h.hidden, &T.in});
-            groups.push_back({{{L.o_w, h.hidden}}, QD, &T.out});
-        } else {
-            groups.push_back({{{L.qkv, C}, {L.gate_w, IN}}, h.hidden, &T.in});
-            groups.push_back({{{L.ssm_out, h.hidden}}, IN, &T.out});
-        }
-        groups.push_back({{{L.ffn_gate, h.ffn}, {L.ffn_up, h.ffn}}, h.hidden, &T.ffn_in});
-        groups.push_back({{{L.ffn_down, h.hidden}}, h.ffn, &T.ffn_down});
-    }
-    if (m->head_sharded) groups.push_back({{{m->out_w + size_t(m->head_r0) * (h.hidden / 128) * 7, m->head_r1 - m->head_r0}}, h.hidden, &m->t_head});
-    else if (m->b1 == h.n_layer) { groups.push_back({{{m->out_w, h.vocab}}, h.hidden, &m->t_head}); m->head_r0 = 0; m->head_r1 = h.vocab; }
-    size_t total = 0;
-    for (const Group &g : groups) for (const Part &p : g.parts) total += bnk::gemm_tiled_bytes(p.M, g.K);
-    BN_CUDA(cudaMalloc(&m->tiled, total));
-    size_t off = 0;
-    for (const Group &g : groups) {
-        *g.dst = m->tiled + off;
-        for (const Part &p : g.parts) {
-            bnk::repack_tiles(m->ctx->stream, p.w, p.M, g.K, reinterpret_cast<uint32_t *>(m->tiled + off));
-            off += bnk::gemm_tiled_bytes(p.M, g.K);
-        }
-    }
+    if (!m->head_sharded && m->b1 == h.n_layer) { m->head_r0 = 0; m->head_r1 = h.vocab; }
     BN_CUDA(cudaMalloc(&m->IMG_H, bnk::gemm_image_bytes(h.hidden, h.batch_cols)));
     BN_CUDA(cudaMalloc(&m->IMG_F, bnk::gemm_image_bytes(h.ffn, h.batch_cols)));
-    {
-        size_t need = 0;
-        for (const Group &g : groups) {
-            int M = 0;
-            for (const Part &p : g.parts) M += p.M;
-            if (bnk::gemm_wants_split(m->ctx->sm_count, M, g.K, 1) || bnk::gemm_wants_split(m->ctx->sm_count, M, g.K, h.batch_cols))
-                need = std::max(need, bnk::gemm_group_floats(M, g.K, h.batch_cols));
-        }
-        if (need) BN_CUDA(cudaMalloc(&m->GROUPS, need * 4));
-    }
     if (m->head_sharded) {
         BN_CUDA(cudaMalloc(&m->CAND, size_t(h.batch_cols) * 8));
         BN_CUDA(cudaMalloc(&m->IMG_HD, bnk::gemm_image_bytes(h.hidden, h.batch_cols)));
     }
-    BN_CUDA(cudaStreamSynchronize(m->ctx->stream));
     return BN_OK;
 }
 
@@ -580,12 +536,11 @@ void enqueue_batch(bn_model *m, int ncol, bool one_sequence = false) {
         a.image = img; a.inv_out = inv_out; a.inv_stride = AS; a.mode = mode;
         bnk::prep_cols(st, a);
     };
-    auto gemm = [&](const uint8_t *Wt, int M, int K, const uint8_t *img, float *out, const float *resid) {
-        bnk::GemmArgs a = {};
-        a.W = Wt; a.M = M; a.K = K; a.tiled = 1; a.image = img; a.ncol = ncol; a.out = out; a.out_stride = AS;
-        a.resid = resid; a.resid_stride = AS; a.err = m->ctx->err_dev;
-        if (m->GROUPS && bnk::gemm_wants_split(m->ctx->sm_count, M, K, ncol)) a.groups = m->GROUPS;
-        cudaError_t e = bnk::launch_gemm(st, m->ctx->sm_count, a, m->use_pdl);
+    auto gemm = [&](const uint8_t *W, int M, int K, const uint8_t *img, float *out, const float *resid, const bnk::Q2Next &next, bool swiglu = false) {
+        bnk::Q2GemmArgs a = {};
+        a.W = W; a.M = M; a.K = K; a.swiglu = swiglu; a.image = img; a.ncol = ncol; a.out = out; a.out_stride = AS;
+        a.resid = resid; a.resid_stride = AS; a.next = next; a.err = m->ctx->err_dev;
+        cudaError_t e = bnk::launch_q2_gemm(st, m->ctx->sm_count, a, m->use_pdl);
         if (e != cudaSuccess && m->launch_err == cudaSuccess) m->launch_err = e;
     };
     if (m->b0 == 0) {
@@ -594,19 +549,18 @@ void enqueue_batch(bn_model *m, int ncol, bool one_sequence = false) {
     }
     for (int b = m->b0; b < m->b1; ++b) {
         const bn_model::Layer &L = m->layers[b];
-        const bn_model::TiledLayer &T = m->tl[b];
         if (L.attn) {
             const bnk::AttnDims ad = attn_dims(m);
             const bnk::KvLayer kv = kv_layer(m, L.idx);
             prep(bnk::PREP_NORM, m->RES, L.attn_norm, m->signs, h.hidden, m->IMG_H, nullptr);
-            gemm(T.in, 2 * QD + 2 * KD, h.hidden, m->IMG_H, m->QKV, nullptr);
+            gemm(L.q2_in, 2 * QD + 2 * KD, h.hidden, m->IMG_H, m->QKV, nullptr, q2_next(L.q2_out, h.hidden, QD, nullptr));
             bnk::attn_prep(st, ad, m->QKV, m->KBUF, m->VBUF, L.q_norm, L.k_norm, m->POS, kv, m->Q16F, m->GATEB, cols);
             bnk::attn_decode(st, ad, m->Q16F, m->GATEB, m->POS, kv, m->SCORE, m->P16F, m->ESUM, m->PVPART, m->pv_splits, nullptr, m->GOUT, true, cols);
             prep(bnk::PREP_PLAIN, m->GOUT, nullptr, m->signs, QD, m->IMG_H, nullptr);
-            gemm(T.out, h.hidden, QD, m->IMG_H, m->RES, m->RES);
+            gemm(L.q2_out, h.hidden, QD, m->IMG_H, m->RES, m->RES, q2_next(L.q2_ffn, 2 * h.ffn, h.hidden, L.post_norm));
         } else {
             prep(bnk::PREP_NORM, m->RES, L.attn_norm, m->signs, h.hidden, m->IMG_H, m->G + 48);
-            gemm(T.in, C + IN, h.hidden, m->IMG_H, m->QKV, nullptr);
+            gemm(L.q2_in, C + IN, h.hidden, m->IMG_H, m->QKV, nullptr, q2_next(L.q2_out, h.hidden, IN, nullptr));
             const bnk::GdnDims gd{NH, NQ, D};
             if (one_sequence) {
                 // position after position on the one recurrent state. The kernel requests its state and conv taps before
@@ -625,17 +579,16 @@ void enqueue_batch(bn_model *m, int ncol, bool one_sequence = false) {
             bnk::gdn_core_fused(st, gd, h.hidden, m->QKV, L.conv_w, conv_of(m, 0, L.idx), conv_of(m, 1, L.idx), m->POS, m->RES, m->G + 48,
                                 L.attn_norm, L.alpha_w, L.beta_w, L.dt_bias, L.ssm_a, gdn_state_of(m, L.idx), m->Z, L.ssm_norm, h.rms_eps, m->X1, cols);
             prep(bnk::PREP_PLAIN, m->X1, nullptr, m->signs, IN, m->IMG_H, nullptr);
-            gemm(T.out, h.hidden, IN, m->IMG_H, m->RES, m->RES);
+            gemm(L.q2_out, h.hidden, IN, m->IMG_H, m->RES, m->RES, q2_next(L.q2_ffn, 2 * h.ffn, h.hidden, L.post_norm));
         }
         prep(bnk::PREP_NORM, m->RES, L.post_norm, m->signs, h.hidden, m->IMG_H, nullptr);
-        gemm(T.ffn_in, 2 * h.ffn, h.hidden, m->IMG_H, m->FG, nullptr);
-        bnk::swiglu(st, m->FG, m->FU, h.ffn, m->FS, cols);
+        gemm(L.q2_ffn, 2 * h.ffn, h.hidden, m->IMG_H, m->FS, nullptr, q2_next(L.q2_down, h.hidden, h.ffn, nullptr), true);
         prep(bnk::PREP_PLAIN, m->FS, nullptr, m->signs + h.hidden, h.ffn, m->IMG_F, nullptr);
-        gemm(T.ffn_down, h.hidden, h.ffn, m->IMG_F, m->RES, m->RES);
+        gemm(L.q2_down, h.hidden, h.ffn, m->IMG_F, m->RES, m->RES, m->head_sharded && b + 1 == m->b1 ? bnk::Q2Next() : next_after(m, b));
     }
     if (m->b1 != h.n_layer || m->head_sharded || one_sequence) return;      // (a prefill block picks from its last column only)
     prep(bnk::PREP_NORM, m->RES, m->out_norm, m->signs, h.hidden, m->IMG_H, nullptr);
-    gemm(m->t_head, h.vocab, h.hidden, m->IMG_H, m->LOGITS, nullptr);
+    gemm(m->q2_head, h.vocab, h.hidden, m->IMG_H, m->LOGITS, nullptr, next_after(m, m->b0 - 1));
     bnk::argmax_first(st, m->LOGITS, h.vocab, m->NEXT, m->AMV, m->AMI, cols);
 }
 
@@ -864,7 +817,9 @@ int bn_model_finalize(bn_model *m) {
         m->kv_layer_bytes = o;
         BN_CUDA(cudaMalloc(&m->kv, m->kv_layer_bytes * m->n_attn * S));
     }
-    if (m->fused) {
+    if (m->fused || h.batch_cols > 0) {
+        BN_REQUIRE(bnk::q2_gemv_supported(h.hidden, h.hat_block) && bnk::q2_gemv_supported(h.ffn, h.hat_block), BN_ERR_ARG,
+                   "bn_model_finalize: the multi-sequence pass needs hidden and ffn to be multiples of 512 up to 16384");
         rc = build_q2(m);
         if (rc != BN_OK) return rc;
     }
@@ -925,13 +880,11 @@ void bn_model_destroy(bn_model *m) {
     if (m->token_graph) cudaGraphExecDestroy(m->token_graph);
     for (cudaGraphExec_t g : m->stage_graphs) if (g) cudaGraphExecDestroy(g);
     for (auto &kv : m->batch_graphs) cudaGraphExecDestroy(kv.second);
-    if (m->tiled) cudaFree(m->tiled);
     if (m->tok_bar) cudaFree(m->tok_bar);
     if (m->tok_stamps) cudaFree(m->tok_stamps);
     if (m->IMG_H) cudaFree(m->IMG_H);
     if (m->IMG_HD) cudaFree(m->IMG_HD);
     if (m->IMG_F) cudaFree(m->IMG_F);
-    if (m->GROUPS) cudaFree(m->GROUPS);
     if (m->q2) cudaFree(m->q2);
     if (m->SGN) cudaFree(m->SGN);
     if (m->CAND) cudaFree(m->CAND);
@@ -1221,9 +1174,9 @@ int bn_model_head_batch(bn_model *m, int ncol, const bn_buf *in, size_t in_off, 
     p.image = m->IMG_HD; p.inv_stride = AS; p.mode = bnk::PREP_NORM;
     bnk::prep_cols(st, p);
     const int rows = m->head_r1 - m->head_r0;
-    bnk::GemmArgs a = {};
-    a.W = m->t_head; a.M = rows; a.K = h.hidden; a.tiled = 1; a.image = m->IMG_HD; a.ncol = ncol; a.out = m->LOGITS; a.out_stride = AS; a.err = m->ctx->err_dev;
-    cudaError_t e = bnk::launch_gemm(st, m->ctx->sm_count, a, m->use_pdl);
+    bnk::Q2GemmArgs a = {};
+    a.W = m->q2_shard; a.M = rows; a.K = h.hidden; a.image = m->IMG_HD; a.ncol = ncol; a.out = m->LOGITS; a.out_stride = AS; a.err = m->ctx->err_dev;
+    cudaError_t e = bnk::launch_q2_gemm(st, m->ctx->sm_count, a, m->use_pdl);
     if (e != cudaSuccess) return bn_cuda_fail(e, "bn_model_head_batch");
     bnk::argmax_first(st, m->LOGITS, rows, m->NEXT, m->AMV, m->AMI, cols, m->CAND, m->head_r0);
     BN_CUDA(cudaMemcpyAsync(bn_ptr<char>(out, out_off), m->CAND, size_t(ncol) * 8, cudaMemcpyDeviceToDevice, st));

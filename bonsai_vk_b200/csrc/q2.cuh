@@ -66,7 +66,32 @@ struct Q2Args {
 bool q2_gemv_supported(int K, int hat_block);
 cudaError_t launch_q2_gemv(cudaStream_t st, int sm_count, const Q2Args &a, bool pdl);
 
+struct Q2GemmArgs {
+    const uint8_t *W;            // two-bit tiles
+    int M, K;                    // valid rows; K % 512 == 0
+    int swiglu;                  // as in Q2Args
+    const uint8_t *image;        // activation image (gemm_tc.cuh), ncol columns padded to 8, 16 or 32
+    int ncol;
+    float *out; size_t out_stride;                 // column c at out + c * out_stride
+    const float *resid; size_t resid_stride;       // optional: out = sum + resid (may alias out)
+    Q2Next next;
+    int *err;
+    Q2Share share; int kc, tiles;                  // filled in by the launch
+};
+cudaError_t launch_q2_gemm(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl);
+
 #ifdef __CUDACC__
+__device__ __forceinline__ void q2_prefetch(const uint8_t *p, int bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+// one thread: the share of the next projection's weights that CTA `cta`'s successor reads, and its norm weights, towards L2
+__device__ __forceinline__ void q2_prefetch_next(const Q2Next &n, int cta) {
+    if (!n.W) return;
+    const uint8_t *src = n.W + size_t(cta * n.share.q + min(cta, n.share.r)) * n.unit_bytes;
+    const int bytes = min((n.share.q + (cta < n.share.r)) * n.unit_bytes, n.max_bytes);
+    for (int o = 0; o < bytes; o += 16384) q2_prefetch(src + o, min(16384, bytes - o));
+    if (cta == 0 && n.w) for (int o = 0; o < n.w_bytes; o += 16384) q2_prefetch(reinterpret_cast<const uint8_t *>(n.w) + o, min(16384, n.w_bytes - o));
+}
 constexpr int Q2_MAGIC = 0x4B400000;           // bits of 12582912.0f: adding an int |i| < 2^22 gives the bits of 12582912 + i
 
 // D = A (u8) x B (s8) + C; the first instruction of a chain takes its C from constants

@@ -1,0 +1,246 @@
+// q2_gemm.cu - the projection of several activation columns (prefill tokens, concurrent sequences) over the two-bit weight
+// tiles of q2.cuh: integer tensor-core dots per (row, column, sub-block), combined in fp32 in the single-column kernel's order,
+//     t_sb = fma(d, I, -s); v = d_w ((t0 + t1) + (t2 + t3)); p_g = (v0 + v1) + (v2 + v3); out = p_0 + p_1 + ...
+// so a column is bit-identical to the single-column projection of its vector.
+//
+// What bounds it: memory at 8 columns; beyond, the fp32 combination, which the contract fixes at 26 packed operations per
+// (16 rows, 8 columns, 128 weights) - 13 cycles of the SM's FMA pipes - against 4 mma (8 cycles of the tensor cores) and 16
+// ANDs per 16 rows. The accumulators of mma.sync are registers, in the layout the combination wants; tcgen05 would bring them
+// through tensor memory and hand-offs between warps (18 944 x 4096: 20.8 / 25.4 / 36.7 us for 8 / 16 / 32 columns that way,
+// where an instruction of 128 rows costs 190 cycles whatever its column count, and the tensor pipe is idle either way).
+//
+// Work split. A CTA of 8 warps owns a run of row tiles over all of K. K is walked in waves of `kc` groups (512 weights each);
+// a wave's piece of the activation image is double-buffered in shared memory. A wave's units (MT row tiles, one group, up to 16
+// columns) are dealt to the warps; a unit keeps everything in registers and leaves its group sums p_g in shared memory, where
+// after a barrier every thread adds its own (row, column)s' in ascending order. MT = 3 row tiles share a group's operands and
+// scales: with one, shared-memory reads (24 wavefronts per 16 rows x 8 columns x 128 weights) would bound the loop.
+#include "q2.cuh"
+#include "rotate_quant.cuh"
+
+#include <algorithm>
+
+namespace {
+using namespace bnk;
+
+constexpr int NT = 256, NW = NT / 32, SMEM_MAX = 227 << 10;
+constexpr int IMG_COL = 160;                   // image bytes per column and block (gemm_tc.cuh)
+constexpr int MAX_TILES = 12;                  // row tiles per pass over K (a thread keeps their running sums in registers)
+
+__device__ __forceinline__ bool full_wait(uint32_t bar, uint32_t parity, int *err) {
+    for (int it = 0; it < (1 << 22); ++it) {
+        uint32_t ok;
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (__builtin_expect(ok != 0u, 1)) return true;
+    }
+    atomicExch(err, 2);
+    return false;
+}
+
+template <int NCP, int MT>
+__global__ void __launch_bounds__(NT, 1) k_q2_gemm(const Q2GemmArgs a) {
+    constexpr int NG = NCP / 8, NGW = NG >= 2 ? 2 : 1, H = NG / NGW;      // column groups: all, per unit; units across the columns
+    constexpr int ITEMS = (MAX_TILES * 16 * NCP + NT - 1) / NT;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tig = lane & 3, cta = blockIdx.x;
+    const int ng = a.K >> 9, kc = a.kc, nw = (ng + kc - 1) / kc;
+    const int t0 = cta * a.share.q + min(cta, a.share.r), nt = a.share.q + (cta < a.share.r);
+    const int npass = (nt + a.tiles - 1) / a.tiles, nchunks = nw == 1 ? 1 : npass * nw;
+    const uint32_t gbytes = 4 * NCP * IMG_COL;                            // image bytes of a group
+    const uint32_t bars = uint32_t(__cvta_generic_to_shared(smem));
+    unsigned char *img = smem + 128;
+    float *sums = reinterpret_cast<float *>(img + (nchunks > 1 ? 2 : 1) * kc * gbytes);
+    auto request = [&](int q) {                                            // image piece of chunk q (wave q % nw) into buffer q & 1
+        const int g0 = (q % nw) * kc, n = min(kc, ng - g0);
+        const uint32_t bytes = uint32_t(n) * gbytes, bar = bars + (q & 1) * 8;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     ::"r"(uint32_t(__cvta_generic_to_shared(img)) + (q & 1) * kc * gbytes), "l"(a.image + size_t(g0) * gbytes), "r"(bytes), "r"(bar) : "memory");
+    };
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        // this CTA's weights (as far as the previous projection has not fetched them) and the next projection's towards L2
+        const uint8_t *own = a.W + size_t(t0) * ng * Q2_PIECE;
+        const int bytes = min(nt * ng * Q2_PIECE, Q2_NEXT_BYTES);
+        for (int o = 0; o < bytes; o += 16384) q2_prefetch(own + o, min(16384, bytes - o));
+        q2_prefetch_next(a.next, cta);
+    }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    __syncthreads();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (tid == 0) for (int q = 0; q < min(2, nchunks); ++q) request(q);
+
+    const f32pair magic2 = pair_of(__int_as_float(Q2_MAGIC), __int_as_float(Q2_MAGIC));
+    bool alive = true;
+    int q = 0;
+    for (int pass = 0; pass < npass; ++pass) {
+        const int tb = pass * a.tiles, n = min(a.tiles, nt - tb), nur = (n + MT - 1) / MT;      // this pass's tiles, units of rows
+        const uint8_t *W = a.W + size_t(t0 + tb) * ng * Q2_PIECE;
+        float acc[ITEMS];
+        for (int w = 0; w < nw; ++w) {
+            const int g0 = w * kc, gn = min(kc, ng - g0);
+            const int buf = nchunks > 1 ? q & 1 : 0;
+            if (alive && (nchunks > 1 || pass == 0)) alive = full_wait(bars + buf * 8, (q >> 1) & 1, a.err);
+            const unsigned char *chunk = img + buf * kc * gbytes;
+            for (int u = warp; u < gn * nur * H; u += NW) {
+                const int h = u % H, ur = (u / H) % nur, gl = u / (H * nur);
+                const uint8_t *src = W + (size_t(ur * MT) * ng + g0 + gl) * Q2_PIECE;
+                uint4 c[MT][4], dw[MT];
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    const uint8_t *p = src + size_t(min(m, n - 1 - ur * MT)) * ng * Q2_PIECE;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) c[m][k] = __ldg(reinterpret_cast<const uint4 *>(p + k * 512 + lane * 16));
+                    dw[m] = __ldg(reinterpret_cast<const uint4 *>(p + Q2_SCALES + g * 16));
+                }
+                f32pair us[MT][NGW][2], ve[MT][NGW][2];                   // v0 + v1; v0 or v2 (rows g, g + 8)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const unsigned char *blk = chunk + (gl * 4 + j) * (NCP * IMG_COL);
+                    uint2 B[NGW][4];
+                    f32pair sd[NGW][4], sn[NGW][4];
+#pragma unroll
+                    for (int cg = 0; cg < NGW; ++cg) {
+                        const int c8 = h * NGW + cg;
+#pragma unroll
+                        for (int s = 0; s < 4; ++s) {
+                            B[cg][s] = *reinterpret_cast<const uint2 *>(blk + c8 * 1024 + s * 256 + (tig >> 1) * 128 + g * 16 + (tig & 1) * 8);
+                            const ulonglong2 sc = *reinterpret_cast<const ulonglong2 *>(blk + NCP * 128 + c8 * 256 + (s * 4 + tig) * 16);
+                            // the dot of sub-block s comes as 4^s I
+                            const float sh = s == 0 ? 1.0f : (s == 1 ? 0.25f : (s == 2 ? 0.0625f : 0.015625f));
+                            sd[cg][s] = s ? pair_mul(sc.x, pair_of(sh, sh)) : sc.x;
+                            sn[cg][s] = sc.y;
+                        }
+                    }
+#pragma unroll
+                    for (int m = 0; m < MT; ++m) {
+                        const uint4 &lo = c[m][j >> 1], &hi = c[m][2 + (j >> 1)];
+                        const uint32_t l0 = (j & 1) ? lo.z : lo.x, l1 = (j & 1) ? lo.w : lo.y, h0 = (j & 1) ? hi.z : hi.x, h1 = (j & 1) ? hi.w : hi.y;
+                        const uint32_t dwj = j == 0 ? dw[m].x : (j == 1 ? dw[m].y : (j == 2 ? dw[m].z : dw[m].w));
+                        const float dlo = half_bits_to_float(dwj), dhi = half_bits_to_float(dwj >> 16);
+                        uint32_t A[4][4];
+#pragma unroll
+                        for (int s = 0; s < 4; ++s) {
+                            const uint32_t mask = 0x03030303u << (2 * s);
+                            A[s][0] = l0 & mask; A[s][1] = h0 & mask; A[s][2] = l1 & mask; A[s][3] = h1 & mask;
+                        }
+#pragma unroll
+                        for (int cg = 0; cg < NGW; ++cg) {
+                            f32pair tl[4], th[4];
+#pragma unroll
+                            for (int s = 0; s < 4; ++s) {
+                                int d[4];
+                                q2_mma_first(d, A[s][0], A[s][1], A[s][2], A[s][3], B[cg][s].x, B[cg][s].y);
+                                tl[s] = pair_fma(sd[cg][s], pair_sub(pair_of(__int_as_float(d[0]), __int_as_float(d[1])), magic2), sn[cg][s]);
+                                th[s] = pair_fma(sd[cg][s], pair_sub(pair_of(__int_as_float(d[2]), __int_as_float(d[3])), magic2), sn[cg][s]);
+                            }
+                            float x, y;
+                            split_pair(pair_add(pair_add(tl[0], tl[1]), pair_add(tl[2], tl[3])), x, y);
+                            const f32pair vl = pair_of(__fmul_rn(dlo, x), __fmul_rn(dlo, y));
+                            split_pair(pair_add(pair_add(th[0], th[1]), pair_add(th[2], th[3])), x, y);
+                            const f32pair vh = pair_of(__fmul_rn(dhi, x), __fmul_rn(dhi, y));
+                            if (j == 0 || j == 2) { ve[m][cg][0] = vl; ve[m][cg][1] = vh; }
+                            else if (j == 1) { us[m][cg][0] = pair_add(ve[m][cg][0], vl); us[m][cg][1] = pair_add(ve[m][cg][1], vh); }
+                            else {
+                                const f32pair pl = pair_add(us[m][cg][0], pair_add(ve[m][cg][0], vl)), ph = pair_add(us[m][cg][1], pair_add(ve[m][cg][1], vh));
+                                if (ur * MT + m < n) {                    // [group][tile][column group][16 rows][8 columns]
+                                    float *dst = sums + (size_t(gl * n + ur * MT + m) * NG + h * NGW + cg) * 128 + g * 8 + 2 * tig;
+                                    *reinterpret_cast<f32pair *>(dst) = pl;
+                                    *reinterpret_cast<f32pair *>(dst + 64) = ph;
+                                }
+                            }
+                        }
+                    }
+                }
+            }
+            __syncthreads();                       // the wave's group sums are there, its image piece is no longer read
+            if (nchunks > 1) {
+                if (tid == 0 && q + 2 < nchunks) request(q + 2);
+                ++q;
+            }
+            const int items = n * NG * 128;
+#pragma unroll
+            for (int k = 0; k < ITEMS; ++k) {
+                const int i = tid + k * NT;
+                if (i < items) {
+                    const float *p = sums + i;
+                    float s = w == 0 ? p[0] : __fadd_rn(acc[k], p[0]);
+                    for (int gi = 1; gi < gn; ++gi) s = __fadd_rn(s, p[gi * items]);
+                    acc[k] = s;
+                }
+            }
+            if (w + 1 < nw) __syncthreads();
+        }
+        const int items = n * NG * 128;
+        if (a.swiglu) {                            // rows r and r + 8 of a tile: gate and up of one FFN row
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < ITEMS; ++k) if (tid + k * NT < items) sums[tid + k * NT] = acc[k];
+            __syncthreads();
+            for (int i = tid; i < items / 2; i += NT) {
+                const int tc = i >> 6, r = (i >> 3) & 7, col = (tc % NG) * 8 + (i & 7);
+                if (col < a.ncol)
+                    a.out[size_t(col) * a.out_stride + (t0 + tb + tc / NG) * 8 + r] = __fmul_rn(silu_f(sums[tc * 128 + r * 8 + (i & 7)]), sums[tc * 128 + 64 + r * 8 + (i & 7)]);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < ITEMS; ++k) {
+                const int i = tid + k * NT, tc = i >> 7, row = (t0 + tb + tc / NG) * 16 + ((i >> 3) & 15), col = (tc % NG) * 8 + (i & 7);
+                if (i < items && row < a.M && col < a.ncol) {
+                    float r = acc[k];
+                    if (a.resid) r = __fadd_rn(r, a.resid[size_t(col) * a.resid_stride + row]);
+                    a.out[size_t(col) * a.out_stride + row] = r;
+                }
+            }
+        }
+        if (pass + 1 < npass) __syncthreads();
+    }
+}
+
+template <int NCP, int MT>
+cudaError_t launch_t(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl) {
+    static bool attr_set = false;
+    if (!attr_set) {
+        cudaError_t e = cudaFuncSetAttribute(k_q2_gemm<NCP, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
+        if (e != cudaSuccess) return e;
+        attr_set = true;
+    }
+    const int ng = a.K / 512, tiles = (a.M + 15) / 16, grid = std::min(tiles, sm_count);
+    a.share = {tiles / grid, tiles % grid};
+    a.tiles = std::min(a.share.q + (a.share.r > 0), MAX_TILES);
+    // groups per wave: as many as fit with their image piece twice (once when one wave is all of K) and their group sums
+    const int gimg = 4 * NCP * IMG_COL, gsum = a.tiles * 16 * NCP * 4;
+    auto bytes = [&](int kc) { return 128 + kc * ((kc >= ng ? 1 : 2) * gimg + gsum); };
+    a.kc = std::min(ng, 8);
+    while (a.kc > 1 && bytes(a.kc) > SMEM_MAX) a.kc = (a.kc + 1) / 2;
+    if (a.next.W) a.next.share = {a.next.units / grid, a.next.units % grid};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = std::max(bytes(a.kc), 116 << 10);             // one CTA per SM, as in q2_gemv.cu
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl ? 1 : 0;
+    BN_COUNT(1);
+    return cudaLaunchKernelEx(&cfg, k_q2_gemm<NCP, MT>, a);
+}
+
+}  // namespace
+
+namespace bnk {
+
+cudaError_t launch_q2_gemm(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl) {
+    const int ncp = a.ncol <= 8 ? 8 : (a.ncol <= 16 ? 16 : 32), tiles = (a.M + 15) / 16;
+    // two row tiles per unit where a CTA has no more (the 4096-row projections), else three
+    const bool two = tiles <= 2 * sm_count;
+    if (ncp == 8) return two ? launch_t<8, 2>(st, sm_count, a, pdl) : launch_t<8, 3>(st, sm_count, a, pdl);
+    if (ncp == 16) return two ? launch_t<16, 2>(st, sm_count, a, pdl) : launch_t<16, 3>(st, sm_count, a, pdl);
+    return two ? launch_t<32, 2>(st, sm_count, a, pdl) : launch_t<32, 3>(st, sm_count, a, pdl);
+}
+
+}  // namespace bnk

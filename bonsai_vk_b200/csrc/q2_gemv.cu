@@ -65,9 +65,6 @@ __device__ __forceinline__ bool slot_wait(uint32_t bar, uint32_t parity, int *er
     atomicExch(err, 1);
     return false;
 }
-__device__ __forceinline__ void prefetch_l2(const uint8_t *p, int bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
 // sign bits 2k and 2k + 1 of a byte as a pair of sign masks
 __device__ __forceinline__ f32pair sign_pair(uint32_t sg, int k) {
     return (unsigned long long)((sg << (31 - 2 * k)) & 0x80000000u) | (unsigned long long)((sg << (30 - 2 * k)) & 0x80000000u) << 32;
@@ -108,13 +105,7 @@ __global__ void __launch_bounds__(NT + 32, 1) k_q2_gemv(const Q2Args a) {
             }
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             for (int i = 0; i < min(EARLY, slots); ++i) request(i, i);
-            if (a.next.W) {
-                const Q2Next &n = a.next;
-                const uint8_t *src = n.W + size_t(cta * n.share.q + min(cta, n.share.r)) * n.unit_bytes;
-                const int bytes = min((n.share.q + (cta < n.share.r)) * n.unit_bytes, n.max_bytes);
-                for (int o = 0; o < bytes; o += 16384) prefetch_l2(src + o, min(16384, bytes - o));
-                if (cta == 0 && n.w) for (int o = 0; o < n.w_bytes; o += 16384) prefetch_l2(reinterpret_cast<const uint8_t *>(n.w) + o, min(16384, n.w_bytes - o));
-            }
+            q2_prefetch_next(a.next, cta);
         }
         __syncwarp();
         asm volatile("bar.arrive 2, %0;" ::"n"(NT + 32) : "memory");

@@ -127,8 +127,8 @@ size_t bn_gemm_image_bytes(int K, int ncol);
 int bn_gemm_act_quant(bn_ctx *ctx, const bn_buf *x, size_t x_off, size_t x_stride, int K, int ncol, const bn_buf *signs,
                       size_t signs_off, int hat_block, bn_buf *image, size_t image_off);
 /* Optional second copy of a weight matrix for this kernel (reference: the engine also repacks its weights once at load,
- * bonsai_weights.h:502-558): per tile of 128 rows and 8 blocks of K one contiguous piece, so that a pipeline stage is a
- * single bulk copy. Same bytes, other order; rows beyond M are zero. */
+ * bonsai_weights.h:502-558): two bits per weight, laid out as the tensor cores' operand fragments, per tile of 16 rows and
+ * 512 weights of K one contiguous piece; rows beyond M are zero. About a fifth larger than the matrix itself. */
 size_t bn_gemm_tiled_bytes(int M, int K);
 int bn_gemm_repack(bn_ctx *ctx, const bn_buf *w, size_t w_off, int M, int K, bn_buf *tiled, size_t tiled_off);
 /* w_tiled = 0: w is the native row-major matrix; 1: w is the copy made by bn_gemm_repack.
