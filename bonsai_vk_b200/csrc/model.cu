@@ -517,7 +517,7 @@ __global__ void k_set_cols(int *tok, int *pos, size_t arena, int n, ColInit ci, 
 // the token schedule for ncol sequences at once; m->cur = first sequence.
 // one_sequence (batched prefill): the columns are ncol consecutive positions of ONE sequence (m->cur). Projections,
 // norms, the embedding and the FFN treat them like independent sequences; the recurrent mixer walks the columns in
-// order on the one state (a launch per position: the delta rule is sequential in time); attention inserts every
+// order on the one state (gdn_seq.cu); attention inserts every
 // column's K/V row first and then lets column c attend to the prefix that ends at its own position (causal), all
 // columns at once against the one cache. Every column's result is bit-identical to the token-serial schedule.
 void enqueue_batch(bn_model *m, int ncol, bool one_sequence = false) {
@@ -563,18 +563,12 @@ void enqueue_batch(bn_model *m, int ncol, bool one_sequence = false) {
             gemm(L.q2_in, C + IN, h.hidden, m->IMG_H, m->QKV, nullptr, q2_next(L.q2_out, h.hidden, IN, nullptr));
             const bnk::GdnDims gd{NH, NQ, D};
             if (one_sequence) {
-                // position after position on the one recurrent state. The kernel requests its state and conv taps before
-                // its dependency wait (in the decode schedule its predecessor never writes them); here the predecessor is
-                // the previous position's kernel, which does - so from the second position on the launch is a plain,
-                // fully serialised one.
-                const bool pdl_was = bnk::g_pdl;
-                for (int c = 0; c < ncol; ++c) {
-                    if (c == 1) bnk::g_pdl = false;
-                    bnk::gdn_core_fused(st, gd, h.hidden, m->QKV + c * AS, L.conv_w, conv_of(m, 0, L.idx), conv_of(m, 1, L.idx), m->POS + c * AS,
-                                        m->RES + c * AS, m->G + 48 + c * AS, L.attn_norm, L.alpha_w, L.beta_w, L.dt_bias, L.ssm_a,
-                                        gdn_state_of(m, L.idx), m->Z + c * AS, L.ssm_norm, h.rms_eps, m->X1 + c * AS, bnk::Cols());
-                }
-                bnk::g_pdl = pdl_was;
+                bnk::GdnSeq s = {};
+                s.heads = NH; s.qk_heads = NQ; s.hidden = h.hidden; s.qkv = m->QKV; s.conv_w = L.conv_w; s.hist0 = conv_of(m, 0, L.idx); s.hist1 = conv_of(m, 1, L.idx);
+                s.pos = m->POS; s.x = m->RES; s.inv = m->G + 48; s.norm_w = L.attn_norm; s.alpha_w = L.alpha_w; s.beta_w = L.beta_w; s.dt_bias = L.dt_bias; s.ssm_a = L.ssm_a;
+                s.state = gdn_state_of(m, L.idx); s.qk = m->L2; s.v = m->CONV; s.eg = m->ALPHA; s.bt = m->BETA; s.o = m->O;
+                s.scale = 1.0f / sqrtf(float(D)); s.stride = m->arena_bytes;
+                bnk::gdn_sequence(st, s, ncol, m->Z, L.ssm_norm, h.rms_eps, m->X1);
             } else
             bnk::gdn_core_fused(st, gd, h.hidden, m->QKV, L.conv_w, conv_of(m, 0, L.idx), conv_of(m, 1, L.idx), m->POS, m->RES, m->G + 48,
                                 L.attn_norm, L.alpha_w, L.beta_w, L.dt_bias, L.ssm_a, gdn_state_of(m, L.idx), m->Z, L.ssm_norm, h.rms_eps, m->X1, cols);

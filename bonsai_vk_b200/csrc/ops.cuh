@@ -86,6 +86,19 @@ void gdn_core_split(cudaStream_t st, GdnDims d, int hidden, const float *qkv, co
                     const int *pos_ptr, const float *x, const float *inv_ptr, const float *norm_w, const float *alpha_w,
                     const float *beta_w, const float *dt_bias, const float *ssm_a, float *state, const float *z,
                     const float *ssm_norm, float eps, float *y);
+// the mixer for n <= 32 consecutive positions of one sequence (gdn_seq.cu): column c's activations at + c * stride bytes
+struct GdnSeq {
+    int heads, qk_heads, hidden;
+    const float *qkv, *conv_w;
+    float *hist0, *hist1;                  // conv taps by position parity
+    const int *pos;                        // position of the first column
+    const float *x, *inv, *norm_w, *alpha_w, *beta_w, *dt_bias, *ssm_a;
+    float *state;
+    float *qk, *v, *eg, *bt, *o;           // working memory per column: normed q and k heads, v, decay, beta, delta-rule output
+    float scale;
+    size_t stride;
+};
+void gdn_sequence(cudaStream_t st, const GdnSeq &a, int n, const float *z, const float *ssm_norm, float eps, float *y);
 // per-head RMS (no weight) * ssm_norm, swiglu(z, .), v-grouped permutation -> y[heads*dim]
 void gdn_out(cudaStream_t st, GdnDims d, const float *o, const float *z, const float *ssm_norm, float eps, float *y);
 
