@@ -1,0 +1,507 @@
+// attn.cu - decode attention over the quantised KV cache: prep (head norm, rope, cache insert), scores, softmax numerators,
+// PV over splits of the keys, combine. The order of every floating-point sum is part of the contract with the CPU checker (the
+// file is compiled without fused-multiply-add contraction; fmaf is written where one is meant).
+//
+// One query token reads every key and value once: 71 MB at 32 768 keys, 11 us of memory. What bounds the kernels is CUDA-core
+// work, because the contract fixes one fused multiply-add per (key, head, dim) for the scores and a rounded product and a
+// rounded sum per (key, head, dim), keys ascending, for PV; and below a few thousand keys the five launches' latency.
+#include "ops.cuh"
+#include "rotate_quant.cuh"
+
+namespace {
+using namespace bnk;
+
+__device__ __forceinline__ void pdl_early() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// order-preserving image of a float, for atomicMax (0 = below every float)
+__device__ __forceinline__ unsigned ord(float f) { const unsigned b = __float_as_uint(f); return (b & 0x80000000u) ? ~b : b | 0x80000000u; }
+__device__ __forceinline__ float unord(unsigned k) { return __uint_as_float((k & 0x80000000u) ? k & 0x7FFFFFFFu : ~k); }
+
+// q8_0 of one 32-element block held one value per lane (recipe: attn_norm_rope2.comp:39-49,184-217)
+__device__ __forceinline__ void q80_store(float v, int lane, int8_t *codes, uint16_t *scale) {
+    float amax = fabsf(v);
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, s));
+    const float d = amax > 1e-35f ? __fdiv_rn(amax, 127.0f) : 0.0f;
+    const float id = d != 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
+    float r = roundf(__fmul_rn(v, id));
+    r = fminf(fmaxf(r, -127.0f), 127.0f);
+    codes[lane] = int8_t(int(r));
+    if (lane == 0) *scale = (uint16_t)float_to_half_bits(d);
+}
+
+// one CTA per head row (n_head query rows, then n_kv key rows) and column or token; blockDim = head_dim = 256.
+// Query rows: RMS norm * weight, NeoX rope on the first n_rot dims, fp16 rounding, gate split; the row's softmax maximum is
+// cleared. Key rows: the same norm / rope, then cache insert (fp16 or q8_0) of K and of the raw V row.
+// Columns (cols.n > 0) are sequences; tokens (the op-level insert) are consecutive positions whose rows follow each other, and
+// only the last one's query is kept. The rope factors need the position only (written a token ago) and are worked out before
+// the wait: a double-precision power, sine and cosine are most of this kernel's chain.
+__global__ void __launch_bounds__(256) k_attn_prep(AttnDims a, AttnPos where, const float *__restrict__ qg, const float *__restrict__ kin,
+                                                   const float *__restrict__ vin, const float *__restrict__ qn_w, const float *__restrict__ kn_w,
+                                                   KvLayer kv, float *__restrict__ q16f, float *__restrict__ gate, unsigned *__restrict__ mx, Cols cols) {
+    const int tok = cols.n > 0 ? 0 : blockIdx.z;
+    if (cols.n > 0) { const size_t col = blockIdx.z; qg = colp(qg, col * cols.arena); kin = colp(kin, col * cols.arena); vin = colp(vin, col * cols.arena); where.ptr = colp(where.ptr, col * cols.arena); kv.k_data = colp(kv.k_data, col * cols.kv); kv.k_scale = colp(kv.k_scale, col * cols.kv); kv.v_data = colp(kv.v_data, col * cols.kv); kv.v_scale = colp(kv.v_scale, col * cols.kv); q16f = colp(q16f, col * cols.arena); gate = colp(gate, col * cols.arena); mx = colp(mx, col * cols.arena); }
+    __shared__ __align__(16) float part[256];
+    __shared__ float sx[256];
+    __shared__ float ssum;
+    const int d = threadIdx.x, hd = a.head_dim, w = blockIdx.x;
+    const bool is_q = w < a.n_head;
+    const int h = is_q ? w : w - a.n_head;
+    if (is_q && tok + 1 < int(gridDim.z) && cols.n == 0) return;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int pos = where.get() + tok;
+    const float *nwp = is_q ? qn_w : kn_w;
+    const int half = a.n_rot >> 1, p = d < half ? d : d - half, pd = d < half ? d + half : d - half;
+    const float nw = nwp[d];
+    float c = 1.0f, s = 0.0f, nwr = 0.0f;
+    if (d < a.n_rot) {
+        const float ex = __fdiv_rn(__fmul_rn(-2.0f, float(p)), float(a.n_rot));
+        const float th = float(pow(double(a.rope_base), double(ex)));
+        const float ang = __fmul_rn(float(pos), th);
+        c = float(cos(double(ang))); s = float(sin(double(ang)));
+        nwr = nwp[pd];
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const float *src = is_q ? qg + size_t(h) * 2 * hd : kin + (size_t(tok) * a.n_kv + h) * hd;
+    const float x = src[d], vr = is_q ? src[hd + d] : vin[(size_t(tok) * a.n_kv + h) * hd + d];
+    sx[d] = x;
+    part[d] = __fmul_rn(x, x);
+    __syncthreads();
+    // the 256 squares are added serially in ascending order, as the reference's CPU mirror adds them
+    // (attn_vk.h:102-108), so that the fp16 operands below are the mirror's bit for bit
+    if (d == 0) {
+        float acc = 0.0f;
+        const float4 *p4 = reinterpret_cast<const float4 *>(part);
+#pragma unroll 8
+        for (int i = 0; i < 64; ++i) {
+            const float4 v = p4[i];
+            acc = __fadd_rn(acc, v.x); acc = __fadd_rn(acc, v.y); acc = __fadd_rn(acc, v.z); acc = __fadd_rn(acc, v.w);
+        }
+        ssum = acc;
+    }
+    __syncthreads();
+    const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ssum, float(hd)), a.eps)));
+    float y = __fmul_rn(__fmul_rn(x, inv), nw);
+    if (d < a.n_rot) {
+        const float xp = __fmul_rn(__fmul_rn(sx[pd], inv), nwr);
+        y = d < half ? __fsub_rn(__fmul_rn(y, c), __fmul_rn(xp, s)) : __fadd_rn(__fmul_rn(y, c), __fmul_rn(xp, s));
+    }
+    if (is_q) {
+        q16f[size_t(h) * hd + d] = __half2float(__float2half_rn(y));
+        gate[size_t(h) * hd + d] = vr;
+        if (d == 0) mx[h] = 0u;
+        return;
+    }
+    const size_t row = (size_t(pos) * a.n_kv + h) * hd;
+    const int lane = d & 31, blk = d >> 5;
+    if (a.k_mode == 1) reinterpret_cast<__half *>(kv.k_data)[row + d] = __float2half_rn(y);
+    else q80_store(y, lane, reinterpret_cast<int8_t *>(kv.k_data) + row + blk * 32, kv.k_scale + row / 32 + blk);
+    if (a.v_mode == 1) reinterpret_cast<__half *>(kv.v_data)[row + d] = __float2half_rn(vr);
+    else q80_store(vr, lane, reinterpret_cast<int8_t *>(kv.v_data) + row + blk * 32, kv.v_scale + row / 32 + blk);
+}
+
+// int8 code -> float without the conversion unit: the word's bytes are biased by 128 (one xor for four codes), a byte
+// is dropped into the mantissa of 2^23 and 2^23 + 128 is subtracted: exact for every code
+constexpr float CODE_MAGIC = 8388736.0f;       // 2^23 + 128
+template <int BYTE> __device__ __forceinline__ float code_f(uint32_t biased_word) {
+    return __uint_as_float(__byte_perm(biased_word, 0x4B000000u, 0x7440u + BYTE));   // 2^23 + (code + 128), magic still to subtract
+}
+
+// Scores: a warp takes octets of consecutive keys of one kv head, the next octet's rows in flight while it works on one; the
+// gqa query heads of the kv head share every K row (merge idea: attn_qk_softmax_gqa.glslh:15-24). Per key and head: lane l
+// covers dims 8l..8l+7 with an fmaf chain, then the 32 lane sums meet in the xor-butterfly tree (16, 8, 4, 2, 1). Two keys
+// travel in the halves of packed registers (the duplicated query values stay in registers for all octets), and the 32 trees of
+// an octet x 4 heads run as one transposed butterfly - every lane ends up with one total - which forms the same pair sums in
+// the same order. The maximum of the scaled scores of each head goes to mx with one atomic per CTA (a maximum has no order).
+// Measured at 32 768 keys: 21 us with one octet per warp (its query loads and latency were most of it), 18 us so.
+template <int KMODE>
+__global__ void __launch_bounds__(256, 2) k_attn_scores4(AttnDims a, AttnPos where, const float *__restrict__ q16f, KvLayer kv,
+                                                         float *__restrict__ score, float scale, unsigned *__restrict__ mx, Cols cols) {
+    { const size_t col = blockIdx.z; q16f = colp(q16f, col * cols.arena); where.ptr = colp(where.ptr, col * cols.arena); kv.k_data = colp(kv.k_data, col * cols.kv); kv.k_scale = colp(kv.k_scale, col * cols.kv); score = colp(score, col * cols.arena); mx = colp(mx, col * cols.arena); }
+    __shared__ unsigned smx[4];
+    if (threadIdx.x < 4) smx[threadIdx.x] = 0u;
+    const int kvh = blockIdx.y, lane = threadIdx.x & 31, hd = a.head_dim;
+    pdl_early();
+    const int nfill = where.get() + 1, step = gridDim.x * 64;
+    int jb = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 8;
+    if (blockIdx.x * 64 >= nfill) return;          // (the whole CTA)
+    uint4 raw16[KMODE == 1 ? 8 : 1];
+    uint2 raw8[KMODE == 1 ? 1 : 8];
+    uint16_t sc[8];
+    auto fetch = [&](int jo) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const size_t row = (size_t(min(jo + u, nfill - 1)) * a.n_kv + kvh) * hd;
+            if (KMODE == 1) raw16[u] = *reinterpret_cast<const uint4 *>(reinterpret_cast<const __half *>(kv.k_data) + row + lane * 8);
+            else {
+                raw8[u] = *reinterpret_cast<const uint2 *>(reinterpret_cast<const int8_t *>(kv.k_data) + row + lane * 8);
+                sc[u] = kv.k_scale[row / 32 + (lane >> 2)];
+            }
+        }
+    };
+    if (jb < nfill) fetch(jb);
+    f32pair qd[4][8];                              // (q, q): both keys of a pair meet the same query value
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        const float4 *qv = reinterpret_cast<const float4 *>(q16f + size_t(kvh * 4 + g) * hd + lane * 8);
+        const float4 q0 = qv[0], q1 = qv[1];
+        qd[g][0] = pair_of(q0.x, q0.x); qd[g][1] = pair_of(q0.y, q0.y); qd[g][2] = pair_of(q0.z, q0.z); qd[g][3] = pair_of(q0.w, q0.w);
+        qd[g][4] = pair_of(q1.x, q1.x); qd[g][5] = pair_of(q1.y, q1.y); qd[g][6] = pair_of(q1.z, q1.z); qd[g][7] = pair_of(q1.w, q1.w);
+    }
+    const f32pair magic2 = pair_of(CODE_MAGIC, CODE_MAGIC);
+    float best = -INFINITY;                        // of head lane & 3
+    for (; jb < nfill; jb += step) {
+        float v[32];                               // v[4u + g]: this lane's part of (key jb+u, head g)
+#pragma unroll
+        for (int up = 0; up < 4; ++up) {           // keys jb+2up, jb+2up+1
+            f32pair kf[8];
+            if (KMODE == 1) {
+                const __half2 *ha = reinterpret_cast<const __half2 *>(&raw16[2 * up]), *hb = reinterpret_cast<const __half2 *>(&raw16[2 * up + 1]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 fa = __half22float2(ha[e]), fb = __half22float2(hb[e]);
+                    kf[2 * e] = pair_of(fa.x, fb.x); kf[2 * e + 1] = pair_of(fa.y, fb.y);
+                }
+            } else {
+                const uint32_t a0 = raw8[2 * up].x ^ 0x80808080u, a1 = raw8[2 * up].y ^ 0x80808080u;
+                const uint32_t b0 = raw8[2 * up + 1].x ^ 0x80808080u, b1 = raw8[2 * up + 1].y ^ 0x80808080u;
+                const f32pair sc2 = pair_of(half_bits_to_float(sc[2 * up]), half_bits_to_float(sc[2 * up + 1]));
+                kf[0] = pair_mul(sc2, pair_sub(pair_of(code_f<0>(a0), code_f<0>(b0)), magic2)); kf[1] = pair_mul(sc2, pair_sub(pair_of(code_f<1>(a0), code_f<1>(b0)), magic2));
+                kf[2] = pair_mul(sc2, pair_sub(pair_of(code_f<2>(a0), code_f<2>(b0)), magic2)); kf[3] = pair_mul(sc2, pair_sub(pair_of(code_f<3>(a0), code_f<3>(b0)), magic2));
+                kf[4] = pair_mul(sc2, pair_sub(pair_of(code_f<0>(a1), code_f<0>(b1)), magic2)); kf[5] = pair_mul(sc2, pair_sub(pair_of(code_f<1>(a1), code_f<1>(b1)), magic2));
+                kf[6] = pair_mul(sc2, pair_sub(pair_of(code_f<2>(a1), code_f<2>(b1)), magic2)); kf[7] = pair_mul(sc2, pair_sub(pair_of(code_f<3>(a1), code_f<3>(b1)), magic2));
+            }
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                f32pair acc = 0ull;
+#pragma unroll
+                for (int e = 0; e < 8; ++e) acc = pair_fma(qd[g][e], kf[e], acc);
+                split_pair(acc, v[8 * up + g], v[8 * up + 4 + g]);
+            }
+        }
+        if (jb + step < nfill) fetch(jb + step);
+        // transposed butterfly: at distance `off` a lane keeps the half of its values that its bit selects and adds the
+        // partner's copy of the same values; lane l ends with the total of value l
+#pragma unroll
+        for (int off = 16, n = 32; off >= 1; off >>= 1, n >>= 1) {
+            const bool upper = lane & off;
+#pragma unroll
+            for (int i = 0; i < n / 2; ++i) {
+                const float send = upper ? v[i] : v[i + n / 2];
+                const float keep = upper ? v[i + n / 2] : v[i];
+                v[i] = __fadd_rn(keep, __shfl_xor_sync(0xFFFFFFFFu, send, off));
+            }
+        }
+        const int j = jb + (lane >> 2);
+        if (j < nfill) {
+            score[size_t(kvh * 4 + (lane & 3)) * a.cap + j] = v[0];
+            best = fmaxf(best, __fmul_rn(v[0], scale));
+        }
+    }
+#pragma unroll
+    for (int s = 4; s < 32; s <<= 1) best = fmaxf(best, __shfl_xor_sync(0xFFFFFFFFu, best, s));
+    __syncthreads();                               // smx is cleared
+    if (lane < 4) atomicMax(smx + lane, ord(best));
+    __syncthreads();
+    if (threadIdx.x < 4) atomicMax(mx + kvh * 4 + threadIdx.x, smx[threadIdx.x]);
+}
+
+// The same scores for any number of query heads per kv head: a warp takes 8 consecutive keys of one kv head and walks the query
+// heads one after the other - per (key, head) the same fmaf chain over the lane's 8 dims and the same xor-butterfly tree.
+template <int KMODE>
+__global__ void __launch_bounds__(256) k_attn_scores_any(AttnDims a, int gqa, AttnPos where, const float *__restrict__ q16f, KvLayer kv,
+                                                         float *__restrict__ score, float scale, unsigned *__restrict__ mx, Cols cols) {
+    { const size_t col = blockIdx.z; q16f = colp(q16f, col * cols.arena); where.ptr = colp(where.ptr, col * cols.arena); kv.k_data = colp(kv.k_data, col * cols.kv); kv.k_scale = colp(kv.k_scale, col * cols.kv); score = colp(score, col * cols.arena); mx = colp(mx, col * cols.arena); }
+    pdl_early();
+    const int kvh = blockIdx.y, lane = threadIdx.x & 31, hd = a.head_dim;
+    const int nfill = where.get() + 1;
+    const int jb = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 8;
+    if (jb >= nfill) return;
+    float kf[8][8];                              // this lane's 8 dims of the 8 keys
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        const int j = min(jb + u, nfill - 1);
+        const size_t row = (size_t(j) * a.n_kv + kvh) * hd;
+        if (KMODE == 1) {
+            const uint4 raw = *reinterpret_cast<const uint4 *>(reinterpret_cast<const __half *>(kv.k_data) + row + lane * 8);
+            const __half2 *h2 = reinterpret_cast<const __half2 *>(&raw);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { const float2 f = __half22float2(h2[e]); kf[u][2 * e] = f.x; kf[u][2 * e + 1] = f.y; }
+        } else {
+            const uint2 raw = *reinterpret_cast<const uint2 *>(reinterpret_cast<const int8_t *>(kv.k_data) + row + lane * 8);
+            const float sc = half_bits_to_float(kv.k_scale[row / 32 + (lane >> 2)]);
+            const int8_t *c8 = reinterpret_cast<const int8_t *>(&raw);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) kf[u][e] = __fmul_rn(sc, float(int(c8[e])));
+        }
+    }
+    for (int g = 0; g < gqa; ++g) {
+        const float4 *qv = reinterpret_cast<const float4 *>(q16f + size_t(kvh * gqa + g) * hd + lane * 8);
+        const float4 q0 = qv[0], q1 = qv[1];
+        const float qe[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+        float best = -INFINITY;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            float acc = 0.0f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc = fmaf(qe[e], kf[u][e], acc);
+#pragma unroll
+            for (int off = 16; off >= 1; off >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(0xFFFFFFFFu, acc, off));
+            if (jb + u < nfill) {
+                if (lane == u) score[size_t(kvh * gqa + g) * a.cap + jb + u] = acc;
+                best = fmaxf(best, __fmul_rn(acc, scale));
+            }
+        }
+        if (lane == 0) atomicMax(mx + kvh * gqa + g, ord(best));
+    }
+}
+
+// Softmax numerators and their sums, spread over 8 CTAs per head with the summation order of one 1024-thread CTA: "virtual
+// thread" vt adds the keys vt, vt+1024, ... ascending, and the 1024 partial sums are combined by the fixed tree p[i] += p[i + s],
+// s = 512 .. 1. A CTA owns 16 residues modulo 128 and all eight virtual threads of each, so the tree's first three steps stay
+// inside it; the last seven, over 128 sums per head, are evaluated by every warp that needs the total (k_attn_pv): no barrier
+// between CTAs (a cluster barrier or an arrival counter here cost 1.5 us). The exponentials of a virtual thread's next eight
+// keys are evaluated by eight real threads and added in order from shared memory.
+constexpr int EXPSUM_PARTS = 8;
+__global__ void __launch_bounds__(1024) k_attn_expsum(AttnDims a, AttnPos where, const float *__restrict__ score, float scale, float *__restrict__ pe,
+                                                      float *__restrict__ partial, const unsigned *__restrict__ mxp, Cols cols) {
+    { const size_t col = blockIdx.z; where.ptr = colp(where.ptr, col * cols.arena); score = colp(score, col * cols.arena); pe = colp(pe, col * cols.arena); partial = colp(partial, col * cols.arena); mxp = colp(mxp, col * cols.arena); }
+    __shared__ float ex[2][1024];
+    __shared__ float sums[128];
+    const int h = blockIdx.x, t = threadIdx.x, i = t & 127, vt = (i >> 4) * 128 + blockIdx.y * 16 + (i & 15), sub = t >> 7;
+    pdl_early();
+    const int nfill = where.get() + 1;
+    const float mx = unord(mxp[h]);
+    const float *sr = score + size_t(h) * a.cap;
+    float *pr = pe + size_t(h) * a.cap;
+    float sum = 0.0f;
+    int buf = 0;
+    for (int j0 = 0; j0 < nfill; j0 += 8192, buf ^= 1) {
+        const int j = j0 + vt + 1024 * sub;
+        float e = 0.0f;
+        if (j < nfill) { e = exp_f(__fsub_rn(__fmul_rn(sr[j], scale), mx)); pr[j] = e; }
+        ex[buf][t] = e;
+        __syncthreads();
+        if (sub == 0) {
+#pragma unroll
+            for (int s = 0; s < 8; ++s) if (j0 + vt + 1024 * s < nfill) sum = __fadd_rn(sum, ex[buf][128 * s + t]);
+        }
+    }
+    if (sub == 0) sums[t] = sum;
+    __syncthreads();
+    if (t < 16) {
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = sums[16 * k + t];
+        partial[size_t(h) * 128 + blockIdx.y * 16 + t] = __fadd_rn(__fadd_rn(__fadd_rn(v[0], v[4]), __fadd_rn(v[2], v[6])), __fadd_rn(__fadd_rn(v[1], v[5]), __fadd_rn(v[3], v[7])));
+    }
+}
+// the rest of the tree: s = 64 .. 1 over a head's 128 sums
+__device__ __forceinline__ float tree128(float e0, float e1, float e2, float e3) {
+    float v = __fadd_rn(__fadd_rn(e0, e2), __fadd_rn(e1, e3));
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xFFFFFFFFu, v, s));
+    return v;
+}
+
+// PV: grid (n_kv, splits, columns); a thread owns DPT output dims of all GQA heads of the kv head and walks the split's keys
+// ascending: acc = acc + p*v with p = fp16(e / total), product and sum rounded (attn_pv_q8v.comp:85-112). V comes through a
+// ring of two 32-key tiles in shared memory (cp.async; small enough that the 1024 CTAs of a long context are all resident),
+// probabilities are staged as one [key][head] row, so a key costs a thread three shared-memory loads whatever the number of
+// dims. The rounded products of two dims are one fma.f32x2 with -0 (x * y - 0 is the rounded product; the -0 is an
+// argument `nz`, because the assembler contracts a packed multiply, or one with a constant -0, with the packed add behind it). DPT = 4 where splits and columns fill the GPU with 64-thread CTAs,
+// else 1 (short caches: the keys' serial chain is what takes the time).
+constexpr int PV_TILE = 32;
+template <int GQA, int DPT, int VMODE>
+__global__ void __launch_bounds__(256 / DPT) k_attn_pv(AttnDims a, AttnPos where, const float *__restrict__ pe, const float *__restrict__ partial,
+                                                       KvLayer kv, int splits, float *__restrict__ part, float nz, Cols cols) {
+    constexpr int T = 256 / DPT, ROW = VMODE == 0 ? 256 : 512, VB = PV_TILE * ROW, TILE_BYTES = VB + (VMODE == 0 ? PV_TILE * 16 : 0);
+    extern __shared__ __align__(16) unsigned char dyn[];
+    { const size_t col = blockIdx.z; pe = colp(pe, col * cols.arena); partial = colp(partial, col * cols.arena); where.ptr = colp(where.ptr, col * cols.arena); kv.v_data = colp(kv.v_data, col * cols.kv); kv.v_scale = colp(kv.v_scale, col * cols.kv); part = colp(part, col * cols.arena); }
+    float *ps = reinterpret_cast<float *>(dyn + 2 * TILE_BYTES);           // [key][GQA]
+    const int kvh = blockIdx.x, sp = blockIdx.y, tid = threadIdx.x, hd = a.head_dim;
+    pdl_early();
+    const int nfill = where.get() + 1, per = (nfill + splits - 1) / splits, j0 = sp * per, n = max(0, min(nfill, j0 + per) - j0);
+    if (n == 0) return;                            // k_attn_combine leaves empty splits out (the first is never empty)
+    auto fetch = [&](int jb, int buf) {            // a tile of keys from jb of the split on
+        const uint32_t dst = uint32_t(__cvta_generic_to_shared(dyn)) + buf * TILE_BYTES;
+        const int m = min(PV_TILE, n - jb);
+        const unsigned char *vd = reinterpret_cast<const unsigned char *>(kv.v_data) + (size_t(j0 + jb) * a.n_kv + kvh) * ROW;
+        for (int i = tid; i < m * (ROW / 16); i += T) {
+            const int k = i / (ROW / 16), b = (i % (ROW / 16)) * 16;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + k * ROW + b), "l"(vd + size_t(k) * a.n_kv * ROW + b) : "memory");
+        }
+        if (VMODE == 0)
+            for (int k = tid; k < m; k += T)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + VB + k * 16), "l"(kv.v_scale + (size_t(j0 + jb + k) * a.n_kv + kvh) * (hd / 32)) : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0, 0);
+    if (n > PV_TILE) fetch(PV_TILE, 1);
+    float tot[GQA], pt[GQA][4];
+#pragma unroll
+    for (int g = 0; g < GQA; ++g)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) pt[g][k] = partial[size_t(kvh * GQA + g) * 128 + (tid & 31) + 32 * k];
+#pragma unroll
+    for (int g = 0; g < GQA; ++g) tot[g] = tree128(pt[g][0], pt[g][1], pt[g][2], pt[g][3]);
+    for (int k = tid; k < n; k += T) {
+        const float *e = pe + size_t(kvh * GQA) * a.cap + j0 + k;
+        float x[GQA];
+#pragma unroll
+        for (int g = 0; g < GQA; ++g) x[g] = e[size_t(g) * a.cap];
+#pragma unroll
+        for (int g = 0; g < GQA; ++g) ps[k * GQA + g] = __half2float(__float2half_rn(__fdiv_rn(x[g], tot[g])));
+    }
+    f32pair acc2[GQA][2];
+    float acc[GQA];
+#pragma unroll
+    for (int g = 0; g < GQA; ++g) { acc2[g][0] = acc2[g][1] = 0ull; acc[g] = 0.0f; }
+    const f32pair nzero = pair_of(nz, nz);
+    const f32pair magic2 = pair_of(CODE_MAGIC, CODE_MAGIC);
+    int buf = 0;
+    for (int jb = 0; jb < n; jb += PV_TILE, buf ^= 1) {
+        if (jb + PV_TILE < n) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        const unsigned char *tile = dyn + buf * TILE_BYTES;
+        const int lim = min(PV_TILE, n - jb);
+        const float *pk = ps + jb * GQA;
+#pragma unroll 4
+        for (int k = 0; k < lim; ++k) {
+            float p[GQA];
+            if (GQA % 4 == 0) {
+#pragma unroll
+                for (int g = 0; g < GQA / 4; ++g) {
+                    const float4 f = *reinterpret_cast<const float4 *>(pk + k * GQA + 4 * g);
+                    p[(4 * g) % GQA] = f.x; p[(4 * g + 1) % GQA] = f.y; p[(4 * g + 2) % GQA] = f.z; p[(4 * g + 3) % GQA] = f.w;
+                }
+            } else {
+#pragma unroll
+                for (int g = 0; g < GQA; ++g) p[g] = pk[k * GQA + g];
+            }
+            if (DPT == 4) {
+                f32pair v01, v23;
+                if (VMODE == 0) {
+                    const float s = half_bits_to_float(*reinterpret_cast<const uint16_t *>(tile + VB + k * 16 + (tid >> 3) * 2));
+                    const uint32_t c = *reinterpret_cast<const uint32_t *>(tile + k * 256 + tid * 4) ^ 0x80808080u;
+                    v01 = pair_mul(pair_of(s, s), pair_sub(pair_of(code_f<0>(c), code_f<1>(c)), magic2));
+                    v23 = pair_mul(pair_of(s, s), pair_sub(pair_of(code_f<2>(c), code_f<3>(c)), magic2));
+                } else {
+                    const uint2 c = *reinterpret_cast<const uint2 *>(tile + k * 512 + tid * 8);
+                    v01 = pair_of(half_bits_to_float(c.x), half_bits_to_float(c.x >> 16));
+                    v23 = pair_of(half_bits_to_float(c.y), half_bits_to_float(c.y >> 16));
+                }
+#pragma unroll
+                for (int g = 0; g < GQA; ++g) {
+                    const f32pair pp = pair_of(p[g], p[g]);
+                    acc2[g][0] = pair_add(acc2[g][0], pair_fma(pp, v01, nzero));
+                    acc2[g][1] = pair_add(acc2[g][1], pair_fma(pp, v23, nzero));
+                }
+            } else {
+                float v;
+                if (VMODE == 0) {
+                    const float s = half_bits_to_float(*reinterpret_cast<const uint16_t *>(tile + VB + k * 16 + (tid >> 5) * 2));
+                    v = __fmul_rn(s, __fsub_rn(__uint_as_float(0x4B000000u | (uint32_t(tile[k * 256 + tid]) ^ 0x80u)), CODE_MAGIC));
+                } else v = half_bits_to_float(*reinterpret_cast<const uint16_t *>(tile + k * 512 + tid * 2));
+#pragma unroll
+                for (int g = 0; g < GQA; ++g) acc[g] = __fadd_rn(acc[g], __fmul_rn(p[g], v));
+            }
+        }
+        if (jb + 2 * PV_TILE < n) { __syncthreads(); fetch(jb + 2 * PV_TILE, buf); }
+    }
+#pragma unroll
+    for (int g = 0; g < GQA; ++g) {
+        float *o = part + (size_t(sp) * a.n_head + kvh * GQA + g) * hd + tid * DPT;
+        if (DPT == 4) *reinterpret_cast<ulonglong2 *>(o) = make_ulonglong2(acc2[g][0], acc2[g][1]);
+        else o[0] = acc[g];
+    }
+}
+
+// combine the splits ascending, then the sigmoid gate: 32 outputs per CTA, whose partials come in with all threads at once and
+// are added in order from shared memory (16 CTAs walking them in batches of 64 loads took 9 us for 64 splits, 24 us for 256).
+// Clears the row maxima again: the kept query may attend once more, over other positions.
+__global__ void __launch_bounds__(256) k_attn_combine(AttnDims a, AttnPos where, const float *__restrict__ part, int splits,
+                                                      const float *__restrict__ gate, float *__restrict__ pregate, float *__restrict__ gated,
+                                                      unsigned *__restrict__ mx, Cols cols) {
+    { const size_t col = blockIdx.z; part = colp(part, col * cols.arena); where.ptr = colp(where.ptr, col * cols.arena); gate = colp(gate, col * cols.arena); pregate = colp(pregate, col * cols.arena); gated = colp(gated, col * cols.arena); mx = colp(mx, col * cols.arena); }
+    __shared__ float sp[256][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = blockIdx.x * 32 + lane, n = a.n_head * a.head_dim;
+    pdl_early();
+    const int nfill = where.get() + 1, per = (nfill + splits - 1) / splits, used = (nfill + per - 1) / per;      // splits with keys
+    for (int s = warp; s < used; s += 8) sp[s][lane] = part[size_t(s) * n + i];
+    float gt = 0.0f;
+    if (warp == 0) gt = __fdiv_rn(1.0f, __fadd_rn(1.0f, exp_f(-gate[i])));
+    __syncthreads();
+    if (warp) return;
+    float acc = sp[0][lane];
+    int s = 1;
+    for (; s + 8 <= used; s += 8) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = sp[s + u][lane];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) acc = __fadd_rn(acc, v[u]);
+    }
+    for (; s < used; ++s) acc = __fadd_rn(acc, sp[s][lane]);
+    if (pregate) pregate[i] = acc;
+    gated[i] = __fmul_rn(acc, gt);
+    if (i % a.head_dim == 0) mx[i / a.head_dim] = 0u;
+}
+
+template <int GQA, int DPT, int VMODE>
+void pv(cudaStream_t st, AttnDims a, AttnPos where, const float *pe, const float *partial, KvLayer kv, int splits, float *part, Cols cols) {
+    constexpr int TILE_BYTES = PV_TILE * (VMODE == 0 ? 256 + 16 : 512);
+    const size_t smem = 2 * TILE_BYTES + size_t(GQA) * ((a.cap + splits - 1) / splits) * 4;
+    static size_t set = 48 << 10;
+    if (smem > set) { cudaFuncSetAttribute(k_attn_pv<GQA, DPT, VMODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)); set = smem; }
+    launch(k_attn_pv<GQA, DPT, VMODE>, dim3(a.n_kv, splits, cols.z()), dim3(256 / DPT), smem, st, a, where, pe, partial, kv, splits, part, -0.0f, cols);
+}
+template <int GQA>
+void pv_any(cudaStream_t st, AttnDims a, AttnPos where, const float *pe, const float *partial, KvLayer kv, int splits, float *part, Cols cols) {
+    // four dims per thread from three 64-thread CTAs per SM on
+    const bool wide = size_t(a.n_kv) * splits * cols.z() >= 444;
+    if (a.v_mode == 0) { if (wide) pv<GQA, 4, 0>(st, a, where, pe, partial, kv, splits, part, cols); else pv<GQA, 1, 0>(st, a, where, pe, partial, kv, splits, part, cols); }
+    else { if (wide) pv<GQA, 4, 1>(st, a, where, pe, partial, kv, splits, part, cols); else pv<GQA, 1, 1>(st, a, where, pe, partial, kv, splits, part, cols); }
+}
+
+}  // namespace
+
+namespace bnk {
+
+void attn_prep(cudaStream_t st, AttnDims a, const float *qg, const float *kin, const float *vin, const float *qn_w,
+               const float *kn_w, AttnPos where, KvLayer kv, float *q16f, float *gate, float *esum, Cols cols, int tokens) {
+    unsigned *mx = reinterpret_cast<unsigned *>(esum + size_t(a.n_head) * 128);
+    launch(k_attn_prep, dim3(a.n_head + a.n_kv, 1, cols.n > 0 ? cols.z() : tokens), dim3(256), 0, st, a, where, qg, kin, vin, qn_w, kn_w, kv, q16f, gate, mx, cols);
+}
+void attn_decode(cudaStream_t st, AttnDims a, const float *q16f, const float *gate, AttnPos where, KvLayer kv,
+                 float *score, float *p16f, float *esum, float *pv_part, int splits, float *pregate, float *gated, Cols cols) {
+    // grids are sized for the cache capacity; CTAs beyond the filled prefix return at once.
+    // esum: [n_head][128] partial softmax sums, then n_head row maxima (cleared by attn_prep and again by the combine kernel)
+    unsigned *mx = reinterpret_cast<unsigned *>(esum + size_t(a.n_head) * 128);
+    const float scale = 1.0f / sqrtf(float(a.head_dim));
+    const int gqa = a.n_head / a.n_kv;            // 1, 2, 4 or 8 (checked where the dimensions enter: bn_model_create, the attention ABI)
+    if (gqa == 4) {
+        // octets per warp: as many as leave two CTAs per SM, at most 8
+        const size_t ctas = size_t((a.cap + 63) / 64) * a.n_kv * cols.z();
+        int rounds = int((ctas + 295) / 296);
+        rounds = rounds < 1 ? 1 : (rounds > 8 ? 8 : rounds);
+        const dim3 sg(((a.cap + 63) / 64 + rounds - 1) / rounds, a.n_kv, cols.z());
+        if (a.k_mode == 1) launch(k_attn_scores4<1>, sg, dim3(256), 0, st, a, where, q16f, kv, score, scale, mx, cols);
+        else launch(k_attn_scores4<0>, sg, dim3(256), 0, st, a, where, q16f, kv, score, scale, mx, cols);
+    } else {
+        const dim3 sg((a.cap + 63) / 64, a.n_kv, cols.z());
+        if (a.k_mode == 1) launch(k_attn_scores_any<1>, sg, dim3(256), 0, st, a, gqa, where, q16f, kv, score, scale, mx, cols);
+        else launch(k_attn_scores_any<0>, sg, dim3(256), 0, st, a, gqa, where, q16f, kv, score, scale, mx, cols);
+    }
+    launch(k_attn_expsum, dim3(a.n_head, EXPSUM_PARTS, cols.z()), dim3(1024), 0, st, a, where, score, scale, p16f, esum, mx, cols);
+    if (gqa == 4) pv_any<4>(st, a, where, p16f, esum, kv, splits, pv_part, cols);
+    else if (gqa == 1) pv_any<1>(st, a, where, p16f, esum, kv, splits, pv_part, cols);
+    else if (gqa == 2) pv_any<2>(st, a, where, p16f, esum, kv, splits, pv_part, cols);
+    else pv_any<8>(st, a, where, p16f, esum, kv, splits, pv_part, cols);
+    launch(k_attn_combine, dim3(a.n_head * a.head_dim / 32, 1, cols.z()), dim3(256), 0, st, a, where, pv_part, splits, gate, pregate, gated, mx, cols);
+}
+
+}  // namespace bnk

@@ -52,11 +52,6 @@ bnk::KvLayer kv_of(const bn_attn_dims &d, const bn_buf *kv, size_t off) {
     k.v_scale = d.v_mode == 0 ? reinterpret_cast<uint16_t *>(base + L.v_scale) : nullptr;
     return k;
 }
-__global__ void k_iota(int *p, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = i;
-}
-
 }  // namespace
 
 extern "C" {
@@ -81,15 +76,15 @@ int bn_attn_insert(bn_ctx *ctx, const bn_attn_dims *d, bn_buf *kv, size_t kv_off
     const Scr S = scratch_layout(*d);
     BN_RANGE(scratch, scratch_off, S.bytes, 256, "bn_attn_insert scratch");
     char *sb = bn_ptr<char>(scratch, scratch_off);
-    int *pos = reinterpret_cast<int *>(sb + S.pos);
-    k_iota<<<(d->cap + 255) / 256, 256, 0, ctx->stream>>>(pos, d->cap);
-    BN_COUNT(1);
     const bnk::AttnDims a = to_dims(*d);
     const bnk::KvLayer K = kv_of(*d, kv, kv_off);
-    for (int t = 0; t < n; ++t)
+    for (int t = 0; t < n; t += 32768) {           // (a launch takes up to 65535 tokens)
+        const int m = n - t < 32768 ? n - t : 32768;
         bnk::attn_prep(ctx->stream, a, bn_ptr<float>(qg, qg_off), bn_ptr<float>(k_rows, k_off) + size_t(t) * KD,
                        bn_ptr<float>(v_rows, v_off) + size_t(t) * KD, bn_ptr<float>(q_norm, qn_off), bn_ptr<float>(k_norm, kn_off),
-                       pos + pos0 + t, K, reinterpret_cast<float *>(sb + S.q16f), reinterpret_cast<float *>(sb + S.gate));
+                       {nullptr, pos0 + t}, K, reinterpret_cast<float *>(sb + S.q16f), reinterpret_cast<float *>(sb + S.gate),
+                       reinterpret_cast<float *>(sb + S.esum), {}, m);
+    }
     return bn_launch_check(ctx, "bn_attn_insert");
 }
 
@@ -107,9 +102,9 @@ int bn_attn_attend(bn_ctx *ctx, const bn_attn_dims *d, const bn_buf *kv, size_t 
     BN_RANGE(gated, g_off, QD * 4, 4, "bn_attn_attend gated");
     char *sb = bn_ptr<char>(scratch, scratch_off);
     bnk::attn_decode(ctx->stream, to_dims(*d), reinterpret_cast<float *>(sb + S.q16f), reinterpret_cast<float *>(sb + S.gate),
-                     reinterpret_cast<int *>(sb + S.pos) + pos, kv_of(*d, kv, kv_off), reinterpret_cast<float *>(sb + S.score),
+                     {nullptr, pos}, kv_of(*d, kv, kv_off), reinterpret_cast<float *>(sb + S.score),
                      reinterpret_cast<float *>(sb + S.pe), reinterpret_cast<float *>(sb + S.esum), reinterpret_cast<float *>(sb + S.pv),
-                     splits_for(d->cap), pregate ? bn_ptr<float>(pregate, pg_off) : nullptr, bn_ptr<float>(gated, g_off), true);
+                     splits_for(d->cap), pregate ? bn_ptr<float>(pregate, pg_off) : nullptr, bn_ptr<float>(gated, g_off));
     return bn_launch_check(ctx, "bn_attn_attend");
 }
 

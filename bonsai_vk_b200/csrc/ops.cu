@@ -516,372 +516,6 @@ __global__ void k_gdn_out(int heads, int qk_heads, const float *__restrict__ o, 
     }
 }
 
-// ---- attention ------------------------------------------------------------------------------------
-// q8_0 of one 32-element block held one value per lane (recipe: attn_norm_rope2.comp:39-49,184-217)
-__device__ __forceinline__ void q80_store(float v, int lane, int8_t *codes, uint16_t *scale) {
-    float amax = fabsf(v);
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, s));
-    const float d = amax > 1e-35f ? __fdiv_rn(amax, 127.0f) : 0.0f;
-    const float id = d != 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
-    float r = roundf(__fmul_rn(v, id));
-    r = fminf(fmaxf(r, -127.0f), 127.0f);
-    codes[lane] = int8_t(int(r));
-    if (lane == 0) *scale = (uint16_t)float_to_half_bits(d);
-}
-
-// one CTA per head row (n_head query rows, then n_kv key rows); blockDim = head_dim = 256.
-// Query rows: RMS norm * weight, NeoX rope on the first n_rot dims, fp16 rounding, gate split.
-// Key rows: the same norm/rope, then cache insert (fp16 or q8_0) of K and of the raw V row.
-__global__ void __launch_bounds__(256) k_attn_prep(bnk::AttnDims a, const float *__restrict__ qg,
-                                                   const float *__restrict__ kin, const float *__restrict__ vin,
-                                                   const float *__restrict__ qn_w, const float *__restrict__ kn_w,
-                                                   const int *__restrict__ pos_ptr, bnk::KvLayer kv,
-                                                   float *__restrict__ q16f, float *__restrict__ gate, bnk::Cols cols) {
-    bnk::pdl_sync();
-    { const size_t col = blockIdx.z; qg = bnk::colp(qg, col * cols.arena); kin = bnk::colp(kin, col * cols.arena); vin = bnk::colp(vin, col * cols.arena); pos_ptr = bnk::colp(pos_ptr, col * cols.arena); kv.k_data = bnk::colp(kv.k_data, col * cols.kv); kv.k_scale = bnk::colp(kv.k_scale, col * cols.kv); kv.v_data = bnk::colp(kv.v_data, col * cols.kv); kv.v_scale = bnk::colp(kv.v_scale, col * cols.kv); q16f = bnk::colp(q16f, col * cols.arena); gate = bnk::colp(gate, col * cols.arena); }
-    __shared__ __align__(16) float part[256];
-    __shared__ float sx[256];
-    const int d = threadIdx.x, hd = a.head_dim, w = blockIdx.x;
-    const bool is_q = w < a.n_head;
-    const int h = is_q ? w : w - a.n_head;
-    const int pos = pos_ptr[0];
-    const float *src = is_q ? qg + size_t(h) * 2 * hd : kin + size_t(h) * hd;
-    const float *nw = is_q ? qn_w : kn_w;
-    const float x = src[d];
-    sx[d] = x;
-    part[d] = __fmul_rn(x, x);
-    __syncthreads();
-    // the 256 squares are added serially in ascending order, as the reference's CPU mirror adds them
-    // (attn_vk.h:102-108), so that the fp16 operands below are the mirror's bit for bit
-    __shared__ float ssum;
-    if (d == 0) {
-        float acc = 0.0f;
-        const float4 *p4 = reinterpret_cast<const float4 *>(part);
-#pragma unroll 8
-        for (int i = 0; i < 64; ++i) {
-            const float4 v = p4[i];
-            acc = __fadd_rn(acc, v.x); acc = __fadd_rn(acc, v.y); acc = __fadd_rn(acc, v.z); acc = __fadd_rn(acc, v.w);
-        }
-        ssum = acc;
-    }
-    __syncthreads();
-    const float ss = ssum;
-    const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, float(hd)), a.eps)));
-    float y = __fmul_rn(__fmul_rn(x, inv), nw[d]);
-    if (d < a.n_rot) {
-        const int half = a.n_rot >> 1;
-        const bool low = d < half;
-        const int p = low ? d : d - half, pd = low ? d + half : d - half;
-        const float ex = __fdiv_rn(__fmul_rn(-2.0f, float(p)), float(a.n_rot));
-        const float th = float(pow(double(a.rope_base), double(ex)));
-        const float ang = __fmul_rn(float(pos), th);
-        const float c = float(cos(double(ang))), s = float(sin(double(ang)));
-        const float xp = __fmul_rn(__fmul_rn(sx[pd], inv), nw[pd]);
-        y = low ? __fsub_rn(__fmul_rn(y, c), __fmul_rn(xp, s)) : __fadd_rn(__fmul_rn(y, c), __fmul_rn(xp, s));
-    }
-    if (is_q) {
-        q16f[size_t(h) * hd + d] = __half2float(__float2half_rn(y));
-        gate[size_t(h) * hd + d] = src[hd + d];
-        return;
-    }
-    const size_t row = (size_t(pos) * a.n_kv + h) * hd;
-    const int lane = d & 31, blk = d >> 5;
-    if (a.k_mode == 1) reinterpret_cast<__half *>(kv.k_data)[row + d] = __float2half_rn(y);
-    else q80_store(y, lane, reinterpret_cast<int8_t *>(kv.k_data) + row + blk * 32, kv.k_scale + row / 32 + blk);
-    const float v = vin[size_t(h) * hd + d];
-    if (a.v_mode == 1) reinterpret_cast<__half *>(kv.v_data)[row + d] = __float2half_rn(v);
-    else q80_store(v, lane, reinterpret_cast<int8_t *>(kv.v_data) + row + blk * 32, kv.v_scale + row / 32 + blk);
-}
-
-// ---- packed fp32 pairs: two IEEE single operations per instruction, each half rounded as the scalar instruction ----
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pk2(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
-__device__ __forceinline__ void unpk2(f32x2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { f32x2 d; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-// int8 code -> float without the conversion unit: the word's bytes are biased by 128 (one xor for four codes), a byte
-// is dropped into the mantissa of 2^23 and 2^23 + 128 is subtracted: exact for every code
-constexpr float CODE_MAGIC = 8388736.0f;       // 2^23 + 128
-__device__ __forceinline__ float code_f(uint32_t biased_word, int byte) {
-    const uint32_t sel = byte == 0 ? 0x7440u : (byte == 1 ? 0x7441u : (byte == 2 ? 0x7442u : 0x7443u));
-    return __uint_as_float(__byte_perm(biased_word, 0x4B000000u, sel));   // 2^23 + (code + 128), magic still to subtract
-}
-
-// scores: each warp takes 8 consecutive keys of one kv head; the gqa query heads of that kv head share every K row
-// (merge idea: attn_qk_softmax_gqa.glslh:15-24). Per key and head: lane l covers dims 8l..8l+7 with an fmaf chain,
-// then the 32 lane sums meet in the xor-butterfly tree (16, 8, 4, 2, 1). Two keys travel in the halves of packed
-// registers (the duplicated query values are loop constants), and the 32 trees of a warp (8 keys x 4 heads) run as
-// one transposed butterfly - every lane ends up with one total - which forms the same pair sums in the same order.
-template <int GQA, int KMODE>
-__global__ void __launch_bounds__(256) k_attn_scores(bnk::AttnDims a, const float *__restrict__ q16f,
-                                                     const int *__restrict__ pos_ptr, bnk::KvLayer kv,
-                                                     float *__restrict__ score, unsigned *__restrict__ counters, bnk::Cols cols) {
-    static_assert(GQA == 4, "the transposed reduction is laid out for 8 keys x 4 heads");
-    bnk::pdl_sync();
-    { const size_t col = blockIdx.z; q16f = bnk::colp(q16f, col * cols.arena); pos_ptr = bnk::colp(pos_ptr, col * cols.arena); kv.k_data = bnk::colp(kv.k_data, col * cols.kv); kv.k_scale = bnk::colp(kv.k_scale, col * cols.kv); score = bnk::colp(score, col * cols.arena); counters = bnk::colp(counters, col * cols.arena); }
-    const int kvh = blockIdx.y, lane = threadIdx.x & 31, hd = a.head_dim;
-    // arrival counters of the softmax-sum kernel that follows: zero before it starts
-    if (blockIdx.x == 0 && kvh == 0 && int(threadIdx.x) < a.n_head) counters[threadIdx.x] = 0u;
-    const int nfill = pos_ptr[0] + 1;
-    const int jb = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 8;
-    if (jb >= nfill) return;
-    f32x2 qd[GQA][8];                            // (q, q): both keys of a pair meet the same query value
-#pragma unroll
-    for (int g = 0; g < GQA; ++g) {
-        const float4 *qv = reinterpret_cast<const float4 *>(q16f + size_t(kvh * GQA + g) * hd + lane * 8);
-        const float4 q0 = qv[0], q1 = qv[1];
-        const float qe[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-#pragma unroll
-        for (int e = 0; e < 8; ++e) qd[g][e] = pk2(qe[e], qe[e]);
-    }
-    uint4 raw16[KMODE == 1 ? 8 : 1];
-    uint2 raw8[KMODE == 1 ? 1 : 8];
-    float sc[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-        const int j = min(jb + u, nfill - 1);
-        const size_t row = (size_t(j) * a.n_kv + kvh) * hd;
-        if (KMODE == 1) raw16[u] = *reinterpret_cast<const uint4 *>(reinterpret_cast<const __half *>(kv.k_data) + row + lane * 8);
-        else {
-            raw8[u] = *reinterpret_cast<const uint2 *>(reinterpret_cast<const int8_t *>(kv.k_data) + row + lane * 8);
-            sc[u] = half_bits_to_float(kv.k_scale[row / 32 + (lane >> 2)]);
-        }
-    }
-    float v[32];                                 // v[4u + g]: this lane's part of (key jb+u, head g)
-    const f32x2 magic2 = pk2(CODE_MAGIC, CODE_MAGIC);
-#pragma unroll
-    for (int up = 0; up < 4; ++up) {             // keys jb+2up, jb+2up+1
-        f32x2 kf[8];
-        if (KMODE == 1) {
-            const __half2 *ha = reinterpret_cast<const __half2 *>(&raw16[2 * up]), *hb = reinterpret_cast<const __half2 *>(&raw16[2 * up + 1]);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float2 fa = __half22float2(ha[e]), fb = __half22float2(hb[e]);
-                kf[2 * e] = pk2(fa.x, fb.x); kf[2 * e + 1] = pk2(fa.y, fb.y);
-            }
-        } else {
-            const uint32_t a0 = raw8[2 * up].x ^ 0x80808080u, a1 = raw8[2 * up].y ^ 0x80808080u;
-            const uint32_t b0 = raw8[2 * up + 1].x ^ 0x80808080u, b1 = raw8[2 * up + 1].y ^ 0x80808080u;
-            const f32x2 sc2 = pk2(sc[2 * up], sc[2 * up + 1]);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const f32x2 c = sub2(pk2(code_f(e < 4 ? a0 : a1, e & 3), code_f(e < 4 ? b0 : b1, e & 3)), magic2);
-                kf[e] = mul2(sc2, c);
-            }
-        }
-#pragma unroll
-        for (int g = 0; g < GQA; ++g) {
-            f32x2 acc = 0ull;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) acc = fma2(qd[g][e], kf[e], acc);
-            unpk2(acc, v[8 * up + g], v[8 * up + 4 + g]);
-        }
-    }
-    // transposed butterfly: at distance `off` a lane keeps the half of its values that its bit selects and adds the
-    // partner's copy of the same values; lane l ends with the total of value l
-#pragma unroll
-    for (int off = 16, n = 32; off >= 1; off >>= 1, n >>= 1) {
-        const bool upper = lane & off;
-#pragma unroll
-        for (int i = 0; i < n / 2; ++i) {
-            const float send = upper ? v[i] : v[i + n / 2];
-            const float keep = upper ? v[i + n / 2] : v[i];
-            v[i] = __fadd_rn(keep, __shfl_xor_sync(0xFFFFFFFFu, send, off));
-        }
-    }
-    const int u = lane >> 2, g = lane & 3, j = jb + u;
-    if (j < nfill) score[size_t(kvh * GQA + g) * a.cap + j] = v[0];
-}
-
-// The same scores for any number of query heads per kv head (the kernel above is laid out for four): a warp takes 8
-// consecutive keys of one kv head and walks the query heads one after the other - per (key, head) the same fmaf chain over
-// the lane's 8 dims and the same xor-butterfly tree, so the same floats.
-template <int KMODE>
-__global__ void __launch_bounds__(256) k_attn_scores_any(bnk::AttnDims a, int gqa, const float *__restrict__ q16f,
-                                                         const int *__restrict__ pos_ptr, bnk::KvLayer kv,
-                                                         float *__restrict__ score, unsigned *__restrict__ counters, bnk::Cols cols) {
-    bnk::pdl_sync();
-    { const size_t col = blockIdx.z; q16f = bnk::colp(q16f, col * cols.arena); pos_ptr = bnk::colp(pos_ptr, col * cols.arena); kv.k_data = bnk::colp(kv.k_data, col * cols.kv); kv.k_scale = bnk::colp(kv.k_scale, col * cols.kv); score = bnk::colp(score, col * cols.arena); counters = bnk::colp(counters, col * cols.arena); }
-    const int kvh = blockIdx.y, lane = threadIdx.x & 31, hd = a.head_dim;
-    if (blockIdx.x == 0 && kvh == 0) for (int i = threadIdx.x; i < a.n_head; i += 256) counters[i] = 0u;
-    const int nfill = pos_ptr[0] + 1;
-    const int jb = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 8;
-    if (jb >= nfill) return;
-    float kf[8][8];                              // this lane's 8 dims of the 8 keys
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-        const int j = min(jb + u, nfill - 1);
-        const size_t row = (size_t(j) * a.n_kv + kvh) * hd;
-        if (KMODE == 1) {
-            const uint4 raw = *reinterpret_cast<const uint4 *>(reinterpret_cast<const __half *>(kv.k_data) + row + lane * 8);
-            const __half2 *h2 = reinterpret_cast<const __half2 *>(&raw);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) { const float2 f = __half22float2(h2[e]); kf[u][2 * e] = f.x; kf[u][2 * e + 1] = f.y; }
-        } else {
-            const uint2 raw = *reinterpret_cast<const uint2 *>(reinterpret_cast<const int8_t *>(kv.k_data) + row + lane * 8);
-            const float sc = half_bits_to_float(kv.k_scale[row / 32 + (lane >> 2)]);
-            const int8_t *c8 = reinterpret_cast<const int8_t *>(&raw);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) kf[u][e] = __fmul_rn(sc, float(int(c8[e])));
-        }
-    }
-    for (int g = 0; g < gqa; ++g) {
-        const float4 *qv = reinterpret_cast<const float4 *>(q16f + size_t(kvh * gqa + g) * hd + lane * 8);
-        const float4 q0 = qv[0], q1 = qv[1];
-        const float qe[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            float acc = 0.0f;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) acc = fmaf(qe[e], kf[u][e], acc);
-#pragma unroll
-            for (int off = 16; off >= 1; off >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(0xFFFFFFFFu, acc, off));
-            if (lane == u && jb + u < nfill) score[size_t(kvh * gqa + g) * a.cap + jb + u] = acc;
-        }
-    }
-}
-
-// Softmax numerators and their sum, spread over EXPSUM_PARTS CTAs per head with the summation order of one
-// 1024-thread CTA: "virtual thread" vt adds the keys vt, vt+1024, ... ascending, and the 1024 partial sums are
-// then combined by the fixed tree (attn_qk_softmax.comp / attn_vk.h:175-190 in the regrouped order the CPU
-// checker also carries). Every CTA recomputes the row maximum (a maximum does not depend on order); the
-// exponentials of one virtual thread are evaluated by 8 real threads, then its owner adds them in order. The CTA of
-// a head that finishes last (arrival counter, no waiting) runs the tree and leaves the head's total.
-constexpr int EXPSUM_PARTS = 8;
-__global__ void __launch_bounds__(1024) k_attn_expsum(bnk::AttnDims a, const int *__restrict__ pos_ptr,
-                                                      const float *__restrict__ score, float scale,
-                                                      float *__restrict__ pe, float *__restrict__ partial, bnk::Cols cols) {
-    bnk::pdl_sync();
-    { const size_t col = blockIdx.z; pos_ptr = bnk::colp(pos_ptr, col * cols.arena); score = bnk::colp(score, col * cols.arena); pe = bnk::colp(pe, col * cols.arena); partial = bnk::colp(partial, col * cols.arena); }
-    __shared__ float red[1024];
-    __shared__ unsigned arrived;
-    const int h = blockIdx.x, c = blockIdx.y, t = threadIdx.x, nfill = pos_ptr[0] + 1;
-    float *total = partial + size_t(a.n_head) * 1024;
-    unsigned *counters = reinterpret_cast<unsigned *>(total + a.n_head);
-    const float *sr = score + size_t(h) * a.cap;
-    float mx = -INFINITY;
-    for (int j = t; j < nfill; j += 1024) mx = fmaxf(mx, __fmul_rn(sr[j], scale));
-    red[t] = mx;
-    for (int s = 512; s > 0; s >>= 1) { __syncthreads(); if (t < s) red[t] = fmaxf(red[t], red[t + s]); }
-    __syncthreads();
-    mx = red[0];
-    float *pr = pe + size_t(h) * a.cap;
-    const int vt = c * 128 + (t & 127), sub = t >> 7;
-    for (int j = vt + 1024 * sub; j < nfill; j += 1024 * 8) pr[j] = exp_f(__fsub_rn(__fmul_rn(sr[j], scale), mx));
-    __syncthreads();
-    if (sub == 0) {
-        float sum = 0.0f;
-        for (int j = vt; j < nfill; j += 1024) sum = __fadd_rn(sum, pr[j]);
-        partial[size_t(h) * 1024 + vt] = sum;
-        __threadfence();
-    }
-    __syncthreads();
-    if (t == 0) arrived = atomicAdd(counters + h, 1u);
-    __syncthreads();
-    if (arrived != EXPSUM_PARTS - 1) return;
-    __threadfence();
-    red[t] = __ldcg(partial + size_t(h) * 1024 + t);
-    const float tot = block_tree_sum(red, 1024);
-    if (t == 0) total[h] = tot;
-}
-
-// PV: grid (n_kv, splits); thread d = output dim; keys of the split ascending; acc = acc + p*v with p = fp16(e / total)
-// formed while the split's numerators are staged in shared memory
-// (no fused multiply-add, runtime_vk/shaders/attn_pv_q8v.comp:85-112). The split's probabilities are staged in
-// shared memory and the V bytes of 8 keys are requested before the 8 dependent adds run.
-template <int GQA>
-__global__ void __launch_bounds__(256) k_attn_pv(bnk::AttnDims a, const float *__restrict__ p16f, const float *__restrict__ total,
-                                                 const int *__restrict__ pos_ptr, bnk::KvLayer kv, int splits,
-                                                 float *__restrict__ part, bnk::Cols cols) {
-    bnk::pdl_sync();
-    { const size_t col = blockIdx.z; p16f = bnk::colp(p16f, col * cols.arena); total = bnk::colp(total, col * cols.arena); pos_ptr = bnk::colp(pos_ptr, col * cols.arena); kv.k_data = bnk::colp(kv.k_data, col * cols.kv); kv.k_scale = bnk::colp(kv.k_scale, col * cols.kv); kv.v_data = bnk::colp(kv.v_data, col * cols.kv); kv.v_scale = bnk::colp(kv.v_scale, col * cols.kv); part = bnk::colp(part, col * cols.arena); }
-    extern __shared__ float ps[];                     // [GQA][per]
-    const int kvh = blockIdx.x, sp = blockIdx.y, d = threadIdx.x, hd = a.head_dim;
-    const int nfill = pos_ptr[0] + 1;
-    const int per = (nfill + splits - 1) / splits;
-    const int j0 = sp * per, j1 = min(nfill, j0 + per);
-    const int n = max(0, j1 - j0);
-    for (int i = d; i < GQA * n; i += 256) {
-        const int g = i / n, jj = i - g * n;
-        ps[g * per + jj] = __half2float(__float2half_rn(__fdiv_rn(p16f[size_t(kvh * GQA + g) * a.cap + j0 + jj], total[kvh * GQA + g])));
-    }
-    __syncthreads();
-    float acc[GQA];
-#pragma unroll
-    for (int g = 0; g < GQA; ++g) acc[g] = 0.0f;
-    if (a.v_mode == 0) {
-        // q8_0 V: tiles of 32 keys x 256 bytes come in with 16-byte loads (the next tile is in flight while this one
-        // is consumed) and are walked from shared memory, key by key in ascending order as before
-        __shared__ uint4 vt[2][32 * 16];
-        __shared__ uint16_t vsc[2][32 * 8];
-        const int8_t *vd = reinterpret_cast<const int8_t *>(kv.v_data);
-        uint4 r0, r1;
-        uint16_t rs;
-        auto fetch = [&](int jb) {
-            const int k0 = min(jb + (d >> 4), n - 1), k1 = min(jb + 16 + (d >> 4), n - 1), ks = min(jb + (d >> 3), n - 1);
-            r0 = *reinterpret_cast<const uint4 *>(vd + (size_t(j0 + k0) * a.n_kv + kvh) * hd + (d & 15) * 16);
-            r1 = *reinterpret_cast<const uint4 *>(vd + (size_t(j0 + k1) * a.n_kv + kvh) * hd + (d & 15) * 16);
-            rs = kv.v_scale[(size_t(j0 + ks) * a.n_kv + kvh) * (hd / 32) + (d & 7)];
-        };
-        if (n > 0) fetch(0);
-        int buf = 0;
-        for (int jb = 0; jb < n; jb += 32, buf ^= 1) {
-            vt[buf][d] = r0; vt[buf][256 + d] = r1; vsc[buf][d] = rs;
-            __syncthreads();
-            if (jb + 32 < n) fetch(jb + 32);
-            const int8_t *tile = reinterpret_cast<const int8_t *>(vt[buf]);
-            const int lim = min(32, n - jb);
-            for (int u = 0; u < lim; ++u) {
-                const float v = __fmul_rn(half_bits_to_float(vsc[buf][u * 8 + (d >> 5)]), float(tile[u * 256 + d]));
-#pragma unroll
-                for (int g = 0; g < GQA; ++g) acc[g] = __fadd_rn(acc[g], __fmul_rn(ps[g * per + jb + u], v));
-            }
-        }
-    } else
-    for (int jb = 0; jb < n; jb += 8) {            // fp16 V
-        float v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int jj = min(jb + u, n - 1);
-            const size_t idx = (size_t(j0 + jj) * a.n_kv + kvh) * hd + d;
-            v[u] = __half2float(reinterpret_cast<const __half *>(kv.v_data)[idx]);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            if (jb + u < n) {
-#pragma unroll
-                for (int g = 0; g < GQA; ++g) acc[g] = __fadd_rn(acc[g], __fmul_rn(ps[g * per + jb + u], v[u]));
-            }
-        }
-    }
-#pragma unroll
-    for (int g = 0; g < GQA; ++g) part[(size_t(sp) * a.n_head + kvh * GQA + g) * hd + d] = acc[g];
-}
-
-// combine the splits ascending, then the sigmoid gate
-__global__ void k_attn_combine(bnk::AttnDims a, const float *__restrict__ part, int splits, const int *pos_ptr,
-                               const float *__restrict__ gate, float *__restrict__ pregate, float *__restrict__ gated, bnk::Cols cols) {
-    bnk::pdl_sync();
-    { const size_t col = blockIdx.z; part = bnk::colp(part, col * cols.arena); pos_ptr = bnk::colp(pos_ptr, col * cols.arena); gate = bnk::colp(gate, col * cols.arena); pregate = bnk::colp(pregate, col * cols.arena); gated = bnk::colp(gated, col * cols.arena); }
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, n = a.n_head * a.head_dim;
-    if (i >= n) return;
-    const int nfill = pos_ptr[0] + 1;
-    const int per = (nfill + splits - 1) / splits;
-    float acc = part[i];
-    for (int sb = 1; sb < splits; sb += 64) {          // 64 partials in flight, added in ascending order
-        float v[64];
-#pragma unroll
-        for (int u = 0; u < 64; ++u) v[u] = (sb + u < splits && (sb + u) * per < nfill) ? part[size_t(sb + u) * n + i] : 0.0f;
-#pragma unroll
-        for (int u = 0; u < 64; ++u) if (sb + u < splits && (sb + u) * per < nfill) acc = __fadd_rn(acc, v[u]);
-    }
-    if (pregate) pregate[i] = acc;
-    gated[i] = __fmul_rn(acc, __fdiv_rn(1.0f, __fadd_rn(1.0f, exp_f(-gate[i]))));
-}
-
 // ---- greedy pick: first maximum (Sampler::pick, runtime_vk/bonsai_forward.h:2568-2570) ----------
 __global__ void __launch_bounds__(1024) k_argmax_part(const float *__restrict__ x, int n, float *__restrict__ bv,
                                                       int *__restrict__ bi, bnk::Cols cols) {
@@ -1006,42 +640,6 @@ void gdn_core_split(cudaStream_t st, GdnDims d, int hidden, const float *qkv, co
 }
 void gdn_out(cudaStream_t st, GdnDims d, const float *o, const float *z, const float *ssm_norm, float eps, float *y) {
     launch(k_gdn_out, dim3((d.heads + 7) / 8), dim3(256), 0, st, d.heads, d.qk_heads, o, z, ssm_norm, eps, y); 
-}
-void attn_prep(cudaStream_t st, AttnDims a, const float *qg, const float *kin, const float *vin, const float *qn_w,
-               const float *kn_w, const int *pos_ptr, KvLayer kv, float *q16f, float *gate, Cols cols) {
-    launch(k_attn_prep, dim3(a.n_head + a.n_kv, 1, cols.z()), dim3(256), 0, st, a, qg, kin, vin, qn_w, kn_w, pos_ptr, kv, q16f, gate, cols); 
-}
-void attn_decode(cudaStream_t st, AttnDims a, const float *q16f, const float *gate, const int *pos_ptr, KvLayer kv,
-                 float *score, float *p16f, float *esum, float *pv_part, int splits, float *pregate, float *gated, bool combine,
-                 Cols cols) {
-    // grids are sized for the cache capacity; warps beyond the filled prefix return at once.
-    // esum: [n_head][1024] partial sums, then n_head totals, then n_head arrival counters
-    float *total = esum + size_t(a.n_head) * 1024;
-    unsigned *counters = reinterpret_cast<unsigned *>(total + a.n_head);
-    const dim3 sg((a.cap + 63) / 64, a.n_kv, cols.z());
-    const int gqa = a.n_head / a.n_kv;            // 1, 2, 4 or 8 (checked where the dimensions enter: bn_model_create, the attention ABI)
-    if (gqa == 4) {
-        if (a.k_mode == 1) launch(k_attn_scores<4, 1>, sg, dim3(256), 0, st, a, q16f, pos_ptr, kv, score, counters, cols);
-        else launch(k_attn_scores<4, 0>, sg, dim3(256), 0, st, a, q16f, pos_ptr, kv, score, counters, cols);
-    } else {
-        if (a.k_mode == 1) launch(k_attn_scores_any<1>, sg, dim3(256), 0, st, a, gqa, q16f, pos_ptr, kv, score, counters, cols);
-        else launch(k_attn_scores_any<0>, sg, dim3(256), 0, st, a, gqa, q16f, pos_ptr, kv, score, counters, cols);
-    }
-    launch(k_attn_expsum, dim3(a.n_head, EXPSUM_PARTS, cols.z()), dim3(1024), 0, st, a, pos_ptr, score, 1.0f / sqrtf(float(a.head_dim)), p16f, esum, cols);
-    const dim3 pg(a.n_kv, splits, cols.z());
-    const size_t ps_bytes = size_t(gqa) * ((a.cap + splits - 1) / splits) * 4;
-    const float *pe = static_cast<const float *>(p16f), *tot = static_cast<const float *>(total);
-    if (gqa == 4) launch(k_attn_pv<4>, pg, dim3(256), ps_bytes, st, a, pe, tot, pos_ptr, kv, splits, pv_part, cols);
-    else if (gqa == 1) launch(k_attn_pv<1>, pg, dim3(256), ps_bytes, st, a, pe, tot, pos_ptr, kv, splits, pv_part, cols);
-    else if (gqa == 2) launch(k_attn_pv<2>, pg, dim3(256), ps_bytes, st, a, pe, tot, pos_ptr, kv, splits, pv_part, cols);
-    else {
-        static bool attr = false;
-        if (!attr) { cudaFuncSetAttribute(k_attn_pv<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024); attr = true; }
-        launch(k_attn_pv<8>, pg, dim3(256), ps_bytes, st, a, pe, tot, pos_ptr, kv, splits, pv_part, cols);
-    }
-    if (!combine) return;
-    const int n = a.n_head * a.head_dim;
-    launch(k_attn_combine, dim3((n + 255) / 256, 1, cols.z()), dim3(256), 0, st, a, pv_part, splits, pos_ptr, gate, pregate, gated, cols); 
 }
 void argmax_first(cudaStream_t st, const float *x, int n, int *out_idx, float *scratch_val, int *scratch_idx, Cols cols, float *cand, int row0) {
     const int parts = 64;

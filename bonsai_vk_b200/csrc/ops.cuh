@@ -104,14 +104,23 @@ void gdn_out(cudaStream_t st, GdnDims d, const float *o, const float *z, const f
 
 struct AttnDims { int n_head, n_kv, head_dim, n_rot, cap; float eps, rope_base; int k_mode, v_mode; };
 struct KvLayer { void *k_data; uint16_t *k_scale; void *v_data; uint16_t *v_scale; };   // scales null in fp16 mode
-// norm + rope + fp16 rounding of q, gate split, K/V quantise + insert at *pos_ptr
+// where a query token stands: at ptr[0] (a device word; one per column) or, with ptr null, at `imm`
+struct AttnPos {
+    const int *ptr;
+    int imm;
+#ifdef __CUDACC__
+    __device__ __forceinline__ int get() const { return ptr ? ptr[0] : imm; }
+#endif
+};
+// norm + rope + fp16 rounding of q, gate split, K/V quantise + insert at the position; tokens > 1 (no columns): that many
+// consecutive K / V rows from there, the query at the last of them
 void attn_prep(cudaStream_t st, AttnDims a, const float *qg, const float *kin, const float *vin, const float *qn_w,
-               const float *kn_w, const int *pos_ptr, KvLayer kv, float *q16f, float *gate, Cols cols = {});
+               const float *kn_w, AttnPos where, KvLayer kv, float *q16f, float *gate, float *esum, Cols cols = {}, int tokens = 1);
 // scores -> softmax (fp16-rounded probabilities) -> PV -> sigmoid gate. Scratch buffers sized by cap.
-void attn_decode(cudaStream_t st, AttnDims a, const float *q16f, const float *gate, const int *pos_ptr, KvLayer kv,
-                 float *score /*[nh][cap]*/, float *p16f /*[nh][cap]*/, float *esum /*[nh][1024] partial sums + [nh] totals + [nh] counters*/,
+void attn_decode(cudaStream_t st, AttnDims a, const float *q16f, const float *gate, AttnPos where, KvLayer kv,
+                 float *score /*[nh][cap]*/, float *p16f /*[nh][cap]*/, float *esum /*[nh][128] partial softmax sums + [nh] row maxima*/,
                  float *pv_part /*[splits][nh][hd]*/, int splits,
-                 float *pregate /*[nh][hd] or null*/, float *gated, bool combine /*false: leave the split partials*/, Cols cols = {});
+                 float *pregate /*[nh][hd] or null*/, float *gated, Cols cols = {});
 // cand (optional): per column (value, row0 + index) of the maximum, for an output head whose rows are sharded
 void argmax_first(cudaStream_t st, const float *x, int n, int *out_idx, float *scratch_val, int *scratch_idx, Cols cols = {},
                   float *cand = nullptr, int row0 = 0);
