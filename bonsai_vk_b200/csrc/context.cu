@@ -76,12 +76,10 @@ int bn_init(int device, bn_ctx **out) {
     e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) { delete c; return bn_cuda_fail(e, "cudaStreamCreate"); }
     c->own_stream = true;
-    c->counters = nullptr;
     c->err_dev = nullptr;
-    e = cudaMalloc(&c->counters, size_t(BN_MAX_TILES) * 4 + 256);
-    if (e != cudaSuccess) { delete c; return bn_cuda_fail(e, "cudaMalloc(counters)"); }
-    cudaMemset(c->counters, 0, size_t(BN_MAX_TILES) * 4 + 256);
-    c->err_dev = reinterpret_cast<int *>(c->counters + BN_MAX_TILES);
+    e = cudaMalloc(&c->err_dev, 256);
+    if (e != cudaSuccess) { delete c; return bn_cuda_fail(e, "cudaMalloc(error word)"); }
+    cudaMemset(c->err_dev, 0, 256);
     *out = c;
     g_err[0] = 0;
     return BN_OK;
@@ -92,7 +90,7 @@ void bn_destroy(bn_ctx *ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     if (ctx->scratch) cudaFree(ctx->scratch);
-    if (ctx->counters) cudaFree(ctx->counters);
+    if (ctx->err_dev) cudaFree(ctx->err_dev);
     if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }

@@ -52,6 +52,9 @@ inline size_t act_pack_bytes(int K) { return size_t(K / 128) * (Q81_DWORDS + BF_
 void gemv_q81(cudaStream_t st, int sm_count, const uint32_t *W, int M, int K, const uint32_t *pack, float *out,
               float *scratch, int32_t *dots);
 void act_quant_q81(cudaStream_t st, const float *x, int K, uint32_t *pack);
+// the same projection streamed from the native rows without scratch (ptq_stream.cu); W 4-byte aligned
+bool ptq_stream_supported(int K);
+cudaError_t ptq_stream(cudaStream_t st, int sm_count, const void *W, int M, int K, const uint32_t *pack, float *out);
 
 // y = H(s . x) per `block`-wide chunk, then q8_1 + operand table into pack (pack may be null: rotate only,
 // y may be null when only the pack is wanted). n % block == 0, block = power of two in [128, 4096].

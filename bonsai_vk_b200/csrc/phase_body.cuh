@@ -1,8 +1,7 @@
 // phase_body.cuh - device-side body of the fused projection "phase": [prologue that rebuilds the rotated, q8_1-quantised
 // input of a projection from the previous phase's outputs] + [PTQ1_0 x q8_1 GEMV streamed through a bulk-copy ring] +
-// [epilogue: residual add, swiglu of a gate/up row pair, silu of a row range, or a first-maximum pick]. Two kernels are
-// built from it: k_phase_gemv (one launch per projection, phase_gemv.cu) and k_token (one launch per token or per run of
-// tokens, token_kernel.cu), which walks a list of phases with grid-wide barriers between them.
+// [epilogue: residual add, swiglu of a gate/up row pair, silu of a row range, or a first-maximum pick]. k_token (one
+// launch per token or per run of tokens, token_kernel.cu) walks a list of such phases with grid-wide barriers between them.
 //
 // Work split. A CTA (16 compute warps + 1 copy warp) owns a contiguous run of 16-row tiles and computes those rows over
 // ALL of K, so no partial sums ever leave the CTA (no atomics, no fences). K is walked in chunks of up to 32 blocks (4096
@@ -357,13 +356,6 @@ __device__ __forceinline__ void prologue(const PhaseArgs &a, const Smem &s, cons
     int8_t *codes = s.codes;
     uint32_t *dsw = s.dsw;
     float *red = s.red, *hinv = s.hinv, *xs = s.xs;
-    if (a.pro == PRO_PACKED) {
-        BN_STAMP(3); BN_STAMP(4);
-        for (int i = tid; i < nb * 32; i += NT) reinterpret_cast<uint32_t *>(codes)[i] = a.pack[size_t(i >> 5) * Q81_DWORDS + 4 + (i & 31)];
-        for (int i = tid; i < nb * 4; i += NT) dsw[i] = a.pack[size_t(i >> 2) * Q81_DWORDS + (i & 3)];
-        csync();
-        return;
-    }
     float inv = 1.0f;
     float xe[8];
     const bool merged = a.pro == PRO_NORM && K == 4096 && a.hat_block == 4096;   // one pass over x0: norm and input
@@ -555,15 +547,10 @@ __device__ __forceinline__ void prologue(const PhaseArgs &a, const Smem &s, cons
 }
 
 // ---- main loop: consume this phase's items from the ring, starting at running item number git0 (compute warps only) ----
-// Who refills the ring. The per-projection kernel has a 17th warp that only issues copies (NoFeed here). The whole-token
-// kernel has no such warp: at the iteration of running item g the compute warp g % 16 refills the stage of item g - FEED_LAG
+// Who refills the ring: at the iteration of running item g the compute warp g % 16 refills the stage of item g - FEED_LAG
 // (every warp has taken that item's rows into registers by then, or will within a few hundred cycles) with item
 // g - FEED_LAG + STAGES, whatever projection of whatever token that item belongs to.
 constexpr int FEED_LAG = 2;
-struct NoFeed {
-    static constexpr bool on = false;
-    __device__ __forceinline__ void operator()(uint32_t) const {}
-};
 // EPI >= 0: the epilogue is fixed at compile time (the per-projection kernel only ever needs EPI_PLAIN and keeps its lean
 // loop); EPI < 0: taken from the phase record at run time (whole-token kernel: one copy of the loop for all phases).
 template <int EPI, class Feed>

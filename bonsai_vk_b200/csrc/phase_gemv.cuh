@@ -1,13 +1,12 @@
-// phase_gemv.cuh - the fused "phase" kernel: [prologue that rebuilds the rotated, quantised input of a
-// projection from the previous phase's outputs] + [PTQ1_0 x q8_1 GEMV streamed through a bulk-copy ring]
-// + [split-K finalisation and residual add by the last CTA to touch a row tile].
+// phase_gemv.cuh - the projection "phase" of the whole-token kernel (token_kernel.cu): [prologue that rebuilds the rotated,
+// quantised input of a projection from the previous phase's outputs] + [PTQ1_0 x q8_1 GEMV streamed through a bulk-copy ring]
+// + [epilogue].
 #pragma once
 #include "ops.cuh"
 
 namespace bnk {
 
 enum Prologue {
-    PRO_PACKED = 0,   // activation pack already in global memory (op-level entry point)
     PRO_PLAIN = 1,    // x0 is the plain fp32 input: rotate + quantise
     PRO_NORM = 2,     // x = rms_norm(x0) * w                                   (pre_norm, bonsai_forward.h:480)
     PRO_SWIGLU = 3,   // x = silu(x0) * x1                                       (ffn_block :498)
@@ -31,8 +30,6 @@ struct PhaseArgs {
     float *out;              // [M] final sums (may be null when resid_out is set)
     const float *resid_in;   // optional [M]
     float *resid_out;        // optional [M]: resid_out = out + resid_in
-    float *part;             // unused by the streamed kernel (kept for the op-level callers)
-    unsigned *counters;
     int epi, epi_arg;        // Epilogue
     float *out2;             // EPI_SWIGLU: [M/2]
     float *cand_val;         // EPI_ARGMAX: per-CTA candidate
@@ -40,7 +37,6 @@ struct PhaseArgs {
     // prologue
     int pro;
     const float *x0, *x1, *w;
-    const uint32_t *pack;    // PRO_PACKED
     const int32_t *signs;    // K sign values
     int hat_block;
     float hat_inv, eps;
@@ -55,8 +51,6 @@ struct PhaseArgs {
 
 constexpr int PHASE_THREADS = 512;
 size_t phase_smem_bytes(int hat_block);
-// launches with programmatic dependent launch when pdl is true
-cudaError_t launch_phase(cudaStream_t st, int sm_count, const PhaseArgs &a, bool pdl);
 bool phase_supported(int M, int K, int hat_block);
 // one tiny kernel whose only wait can never complete and gives up after ~1000 tries: sets *err = 1 and returns
 cudaError_t launch_wait_selftest_ring(cudaStream_t st, int *err);

@@ -138,6 +138,8 @@ __global__ void __launch_bounds__(128) k_act_quant_q81(const float *__restrict__
                                                        uint32_t *__restrict__ bf) {
     __shared__ int8_t qs[128];
     const int b = blockIdx.x, i = threadIdx.x;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     bnk::quant_block_128(x[size_t(b) * 128 + i], i, qs, q81 + size_t(b) * Q81_DWORDS, bf + size_t(b) * BF_WORDS, 1);
 }
 
@@ -147,8 +149,7 @@ namespace bnk {
 
 void act_quant_q81(cudaStream_t st, const float *x, int K, uint32_t *pack) {
     const int nb = K / 128;
-    k_act_quant_q81<<<nb, 128, 0, st>>>(x, pack, pack + size_t(nb) * Q81_DWORDS);
-    BN_COUNT(1);
+    launch(k_act_quant_q81, dim3(nb), dim3(128), 0, st, x, pack, pack + size_t(nb) * Q81_DWORDS);
 }
 
 void gemv_q81(cudaStream_t st, int sm_count, const uint32_t *W, int M, int K, const uint32_t *pack, float *out,
@@ -196,23 +197,13 @@ int bn_gemv_q81(bn_ctx *ctx, const bn_buf *w, size_t w_off, int M, int K, const 
     BN_RANGE(pack, pack_off, bn_act_pack_bytes(K), 16, "bn_gemv_q81 pack");
     BN_RANGE(out, out_off, size_t(M) * 4, 4, "bn_gemv_q81 out");
     if (dots) BN_RANGE(dots, dots_off, size_t(M) * nb * 16, 4, "bn_gemv_q81 dots");
+    if (!dots && bnk::ptq_stream_supported(K)) {
+        cudaError_t e = bnk::ptq_stream(ctx->stream, ctx->sm_count, bn_ptr<void>(w, w_off), M, K, bn_ptr<uint32_t>(pack, pack_off), bn_ptr<float>(out, out_off));
+        if (e != cudaSuccess) return bn_cuda_fail(e, "k_ptq_stream");
+        return bn_launch_check(ctx, "k_ptq_stream");
+    }
     int rc = bn_scratch_reserve(ctx, size_t(ngroups) * M * 4);
     if (rc != BN_OK) return rc;
-    // the streamed kernel moves rows with bulk copies, which need a 16-byte aligned source; any other 4-byte aligned
-    // placement goes through the kernel that reads with plain 4-byte loads (same results)
-    const bool w16 = (reinterpret_cast<uintptr_t>(bn_ptr<uint8_t>(w, w_off)) & 15u) == 0;
-    if (!dots && w16 && bnk::phase_supported(M, K, 512) && (M + 15) / 16 <= BN_MAX_TILES) {
-        // streamed kernel; the op-level call hands it a ready-made activation pack
-        bnk::PhaseArgs a = {};
-        a.W = bn_ptr<uint8_t>(w, w_off); a.M = M; a.K = K;
-        a.out = bn_ptr<float>(out, out_off);
-        a.part = ctx->scratch; a.counters = ctx->counters;
-        a.pro = bnk::PRO_PACKED; a.pack = bn_ptr<uint32_t>(pack, pack_off);
-        a.hat_block = 512; a.err = ctx->err_dev;
-        cudaError_t e = bnk::launch_phase(ctx->stream, ctx->sm_count, a, false);
-        if (e != cudaSuccess) return bn_cuda_fail(e, "k_phase_gemv");
-        return bn_launch_check(ctx, "k_phase_gemv");
-    }
     bnk::gemv_q81(ctx->stream, ctx->sm_count, bn_ptr<uint32_t>(w, w_off), M, K, bn_ptr<uint32_t>(pack, pack_off),
                   bn_ptr<float>(out, out_off), ctx->scratch, dots ? bn_ptr<int32_t>(dots, dots_off) : nullptr);
     return bn_launch_check(ctx, "gemv_q81");
