@@ -40,7 +40,7 @@ PTQ_BYTES_PER_TOKEN = 1_734_541_312                        # their PTQ1_0 bytes
 ALGO_BYTES_PER_TOKEN = 1_734_541_312 + 29_411_328 + 2 * 50_331_648 + 2 * 2_359_296 + 896   # + f32, GDN state r/w, conv
 
 
-NCU_TRAFFIC_RATIO = 1.023      # dram read+write / PTQ1_0 bytes of the launch (ncu, head projection 248320 x 4096)
+TRAFFIC_RATIO = 34 / 28      # bytes the projection kernels read per PTQ1_0 byte: their two-bit tiles hold 34 bytes per 128 weights
 
 
 def peaks():
@@ -453,11 +453,9 @@ def main():
         ms_g = m.gemv_sweep_ms(reps=reps)
         n_l = (ctx.launches - l1) // (reps + 1)
         ach = PTQ_BYTES_PER_TOKEN / (ms_g / 1000.0) / 1e9
-        # DRAM bytes per algorithmic byte of k_phase_gemv, from the ncu capture summarised under profiles/
-        # (head projection: 227.7 MB moved for 222.5 MB of weights); the sweep's launches move the same ratio
         line["roofline"] = {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
-                            "traffic": NCU_TRAFFIC_RATIO * PTQ_BYTES_PER_TOKEN / n_l, "peak_source": which,
-                            "kernel": f"k_phase_gemv: the {n_l} fused projection launches of one token (201 projections, "
+                            "traffic": TRAFFIC_RATIO * PTQ_BYTES_PER_TOKEN / n_l, "peak_source": which,
+                            "kernel": f"k_q2_gemv: the {n_l} fused projection launches of one token (201 projections, "
                                       "grouped where they share an input), with their prologues, back to back",
                             "algorithmic_bytes_per_launch": PTQ_BYTES_PER_TOKEN / n_l,
                             "avg_launch_us": ms_g * 1000.0 / n_l,
@@ -499,7 +497,7 @@ def main():
                                "algorithmic_bytes": nb, "us": ms_a * 1e3, "achieved": nb / ms_a / 1e6, "frac": nb / ms_a / 1e6 / peak})
             for ncol in (8, 32):
                 ms_g2, nb = kernel_lab.gemm_lab(["18944", "4096", str(ncol), "3"], ctx=ctx, quiet=True)
-                others.append({"kernel": f"k_ptq_gemm_tc: 18944 x 4096 projection, {ncol} sequences per pass (tcgen05 kind::i8)",
+                others.append({"kernel": f"k_q2_gemm: 18944 x 4096 projection, {ncol} sequences per pass (two-bit tiles, int8 tensor cores)",
                                "algorithmic_bytes": nb, "us": ms_g2 * 1e3, "achieved": nb / ms_g2 / 1e6, "frac": nb / ms_g2 / 1e6 / peak})
         except Exception as exc:
             others.append({"error": str(exc)[:200]})

@@ -1,10 +1,9 @@
 // gemm_abi.cu - C entry points of the multi-column tensor-core projection (declared in include/bonsai_cuda.h).
-#include "gemm_tc.cuh"
+#include "act_image.cuh"
 #include "q2.cuh"
 #include "phase_gemv.cuh"
 
-#include <cstdio>
-#include <cstdlib>
+#include <algorithm>
 
 extern "C" {
 
@@ -58,66 +57,36 @@ int bn_gemm_q81(bn_ctx *ctx, const bn_buf *w, size_t w_off, int w_tiled, int M, 
     else BN_RANGE(w, w_off, size_t(M) * (K / 128) * 28, 16, "bn_gemm_q81 W");
     BN_RANGE(image, image_off, bnk::gemm_image_bytes(K, ncol), 128, "bn_gemm_q81 image");
     BN_RANGE(out, out_off, (size_t(ncol - 1) * out_stride + M) * 4, 4, "bn_gemm_q81 out");
-    if (w_tiled) {
+    auto project = [&](const uint8_t *tiles, int r0, int rows) {
         bnk::Q2GemmArgs q = {};
-        q.W = bn_ptr<uint8_t>(w, w_off); q.M = M; q.K = K; q.image = bn_ptr<uint8_t>(image, image_off); q.ncol = ncol;
-        q.out = bn_ptr<float>(out, out_off); q.out_stride = out_stride; q.err = ctx->err_dev;
-        cudaError_t e = bnk::launch_q2_gemm(ctx->stream, ctx->sm_count, q, bnk::g_pdl);
-        if (e != cudaSuccess) return bn_cuda_fail(e, "k_q2_gemm");
-        return bn_launch_check(ctx, "k_q2_gemm");
-    }
-    bnk::GemmArgs a = {};
-    a.W = bn_ptr<uint8_t>(w, w_off); a.M = M; a.K = K; a.tiled = 0;
-    a.image = bn_ptr<uint8_t>(image, image_off); a.ncol = ncol;
-    a.out = bn_ptr<float>(out, out_off); a.out_stride = out_stride;
-    a.err = ctx->err_dev;
-    if (bnk::gemm_wants_split(ctx->sm_count, M, K, ncol)) {
-        int rc = bn_scratch_reserve(ctx, bnk::gemm_group_floats(M, K, ncol) * 4);
+        q.W = tiles; q.M = rows; q.K = K; q.image = bn_ptr<uint8_t>(image, image_off); q.ncol = ncol;
+        q.out = bn_ptr<float>(out, out_off) + r0; q.out_stride = out_stride; q.err = ctx->err_dev;
+        return bnk::launch_q2_gemm(ctx->stream, ctx->sm_count, q, bnk::g_pdl);
+    };
+    cudaError_t e = cudaSuccess;
+    if (w_tiled) e = project(bn_ptr<uint8_t>(w, w_off), 0, M);
+    else {
+        // native rows: unpacked into two-bit tiles and projected, in chunks of at most 48 MB of scratch, which stay in L2 (24 576 x
+        // 4096: 27 / 32 / 55 us for 8 / 16 / 32 columns; decoding inside a tcgen05 pipeline took 51 / 56 / 74 us)
+        const int step = int(std::max<size_t>(1, (size_t(48) << 20) / (size_t(K / 512) * bnk::Q2_PIECE))) * 16;
+        int rc = bn_scratch_reserve(ctx, bnk::q2_bytes(std::min(M, step), K));
         if (rc != BN_OK) return rc;
-        a.groups = ctx->scratch;
-    }
-    // profiling aid (library built with -DGEMM_PROF): BONSAI_GEMM_PROF=1 prints where the roles of CTA 0 spent their
-    // cycles (waiting vs working); without that build flag the counters stay zero
-    static const bool want_prof = getenv("BONSAI_GEMM_PROF") != nullptr;
-    long long *prof = nullptr;
-    if (want_prof) {
-        BN_CUDA(cudaMalloc(&prof, 128 * sizeof(long long)));
-        BN_CUDA(cudaMemsetAsync(prof, 0, 128 * sizeof(long long), ctx->stream));
-        a.prof = prof;
-    }
-    cudaError_t e = bnk::launch_gemm(ctx->stream, ctx->sm_count, a, false);
-    if (e != cudaSuccess) return bn_cuda_fail(e, "k_ptq_gemm_tc");
-    // timing aid: BONSAI_GEMM_REPS=n repeats the launch n-1 more times (same result) so that a host loop in an
-    // interpreted language does not become the bottleneck when small shapes are timed
-    static const int reps = getenv("BONSAI_GEMM_REPS") ? atoi(getenv("BONSAI_GEMM_REPS")) : 1;
-    for (int r = 1; r < reps; ++r) bnk::launch_gemm(ctx->stream, ctx->sm_count, a, false);
-    if (want_prof) {
-        long long h[128];
-        BN_CUDA(cudaStreamSynchronize(ctx->stream));
-        BN_CUDA(cudaMemcpy(h, prof, sizeof h, cudaMemcpyDeviceToHost));
-        cudaFree(prof);
-        fprintf(stderr, "gemm prof (cycles, CTA 0): decode[wait full %lld, unpack %lld, publish %lld, wait slot %lld] "
-                        "mma[wait full %lld, wait A %lld, wait D %lld] epilogue[wait D %lld, wait ld %lld, combine %lld]; CTA 0 set-up %lld ns, "
-                        "whole CTA %lld ns; last CTA after set-up %lld ns\n",
-                h[0], h[1], h[2], h[3], h[4], h[5], h[6], h[8], h[9], h[10], h[12], h[14], h[13]);
-        if (getenv("BONSAI_GEMM_PROF_EVENTS")) {
-            static const char *names[7] = {"decode start", "decode stored", "mma has A", "mma has D", "mma committed", "epilogue has D", "epilogue done"};
-            long long t0 = h[16];
-            for (int ev = 0; ev < 7; ++ev) {
-                fprintf(stderr, "%-16s", names[ev]);
-                for (int g = 0; g < 16; ++g) fprintf(stderr, " %6lld", h[16 + ev * 16 + g] - t0);
-                fprintf(stderr, "\n");
-            }
+        uint8_t *tiles = reinterpret_cast<uint8_t *>(ctx->scratch);
+        for (int r0 = 0; r0 < M && e == cudaSuccess; r0 += step) {
+            const int n = std::min(step, M - r0);
+            bnk::q2_repack(ctx->stream, bn_ptr<uint32_t>(w, w_off) + size_t(r0) * (K / 128) * 7, n, K, tiles);
+            e = project(tiles, r0, n);
         }
     }
-    return bn_launch_check(ctx, "k_ptq_gemm_tc");
+    if (e != cudaSuccess) return bn_cuda_fail(e, "k_q2_gemm");
+    return bn_launch_check(ctx, "k_q2_gemm");
 }
 
 int bn_selftest_wait(bn_ctx *ctx, int which) {
     BN_REQUIRE(ctx, BN_ERR_ARG, "bn_selftest_wait: null context");
     BN_REQUIRE(which == 0 || which == 1, BN_ERR_ARG, "bn_selftest_wait: which=%d (0 = copy-ring wait, 1 = tensor-core pipeline wait)", which);
     cudaError_t e = which == 0 ? bnk::launch_wait_selftest_ring(ctx->stream, ctx->err_dev)
-                               : bnk::launch_wait_selftest_tc(ctx->stream, ctx->err_dev);
+                               : bnk::launch_wait_selftest_gemm(ctx->stream, ctx->err_dev);
     if (e != cudaSuccess) return bn_cuda_fail(e, "bn_selftest_wait");
     return BN_OK;
 }

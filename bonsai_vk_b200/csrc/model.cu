@@ -4,7 +4,7 @@
 
 #include "phase_gemv.cuh"
 #include "q2.cuh"
-#include "gemm_tc.cuh"
+#include "act_image.cuh"
 #include "token_kernel.cuh"
 
 #include <algorithm>
@@ -449,12 +449,12 @@ int build_q2(bn_model *m) {
     const bn_hparams &h = m->hp;
     const int NH = h.gdn_heads, NQ = h.gdn_qk_heads, D = h.gdn_dim, C = 2 * NQ * D + NH * D, IN = NH * D;
     const int QD = h.n_head * h.head_dim, KD = h.n_kv * h.head_dim;
-    struct Part { const uint32_t *w; int M, K; size_t off; int half; };
+    struct Part { const uint32_t *w, *second; int M, K; size_t off; };
     std::vector<Part> parts;
     size_t total = 0;
     std::vector<std::pair<const uint8_t **, size_t>> where;
     auto matrix = [&](const uint8_t **dst) { where.push_back({dst, total}); };
-    auto part = [&](const uint32_t *w, int M, int K) { parts.push_back({w, M, K, total, -1}); total += bnk::q2_bytes(M, K); };   // (heights are multiples of 16)
+    auto part = [&](const uint32_t *w, int M, int K) { parts.push_back({w, nullptr, M, K, total}); total += bnk::q2_bytes(M, K); };   // (heights are multiples of 16)
     for (int b = m->b0; b < m->b1; ++b) {
         bn_model::Layer &L = m->layers[b];
         matrix(&L.q2_in);
@@ -463,8 +463,7 @@ int build_q2(bn_model *m) {
         matrix(&L.q2_out);
         part(L.attn ? L.o_w : L.ssm_out, h.hidden, h.hidden);
         matrix(&L.q2_ffn);
-        parts.push_back({L.ffn_gate, h.ffn, h.hidden, total, 0});
-        parts.push_back({L.ffn_up, h.ffn, h.hidden, total, 1});
+        parts.push_back({L.ffn_gate, L.ffn_up, h.ffn, h.hidden, total});
         total += 2 * bnk::q2_bytes(h.ffn, h.hidden);
         matrix(&L.q2_down);
         part(L.ffn_down, h.hidden, h.ffn);
@@ -475,7 +474,10 @@ int build_q2(bn_model *m) {
     BN_CUDA(cudaMalloc(&m->SGN, size_t(h.hidden + h.ffn) / 8));
     for (auto &w : where) *w.first = m->q2 + w.second;
     if (m->q2_head) m->q2_shard = m->q2_head + size_t(m->head_sharded ? m->head_r0 / 16 : 0) * (h.hidden / 512) * bnk::Q2_PIECE;
-    for (const Part &p : parts) bnk::q2_repack(m->ctx->stream, p.w, p.M, p.K, m->q2 + p.off, p.half);
+    for (const Part &p : parts) {
+        if (p.second) bnk::q2_repack_pair(m->ctx->stream, p.w, p.second, p.M, p.K, m->q2 + p.off);
+        else bnk::q2_repack(m->ctx->stream, p.w, p.M, p.K, m->q2 + p.off);
+    }
     bnk::pack_sign_bits(m->ctx->stream, m->signs, h.hidden + h.ffn, m->SGN);
     return bn_launch_check(m->ctx, "two-bit tiles");
 }

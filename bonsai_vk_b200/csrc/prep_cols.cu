@@ -1,8 +1,8 @@
-// prep_cols.cu - the activation image of the multi-column projection (layout: gemm_tc.cuh): per column [rms norm] -> signs ->
+// prep_cols.cu - the activation image of the multi-column projection (layout: act_image.cuh): per column [rms norm] -> signs ->
 // Hadamard -> q8_1 codes and scales. One CTA of 512 threads per column and span of 4096 values, eight values per thread, on the
 // helpers of the single-sequence prologue (rotate_quant.cuh), so the same bits. Bound by that chain's latency (2.5 us for a
 // normed 4096-wide input; 5 us with the transform split into shuffles and shared-memory passes of two stages each).
-#include "gemm_tc.cuh"
+#include "act_image.cuh"
 #include "rotate_quant.cuh"
 
 namespace {

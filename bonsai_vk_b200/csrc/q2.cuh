@@ -24,9 +24,10 @@ namespace bnk {
 constexpr int Q2_PIECE = 2176, Q2_SCALES = 2048;
 
 inline size_t q2_bytes(int M, int K) { return size_t((M + 15) / 16) * size_t(K / 512) * Q2_PIECE; }
-// native row-major PTQ1_0 -> two-bit tiles. half = 0 / 1: the matrix is the first / second of a pair whose rows share tiles
-// (rows 0..7 of a tile from the first, 8..15 from the second: gate and up of an FFN). K % 512 == 0; pairs: M % 8 == 0.
-void q2_repack(cudaStream_t st, const uint32_t *W, int M, int K, uint8_t *out, int half = -1);
+// native row-major PTQ1_0 -> two-bit tiles; the pair: rows 0..7 of a tile from the first matrix, 8..15 from the second (gate and
+// up of an FFN; M rows each, M % 8 == 0). K % 512 == 0.
+void q2_repack(cudaStream_t st, const uint32_t *W, int M, int K, uint8_t *out);
+void q2_repack_pair(cudaStream_t st, const uint32_t *Wa, const uint32_t *Wb, int M, int K, uint8_t *out);
 // sign values -> one bit per value (set = -1), 8 values per byte
 void pack_sign_bits(cudaStream_t st, const int32_t *signs, int n, uint8_t *bits);
 
@@ -70,7 +71,7 @@ struct Q2GemmArgs {
     const uint8_t *W;            // two-bit tiles
     int M, K;                    // valid rows; K % 512 == 0
     int swiglu;                  // as in Q2Args
-    const uint8_t *image;        // activation image (gemm_tc.cuh), ncol columns padded to 8, 16 or 32
+    const uint8_t *image;        // activation image (act_image.cuh), ncol columns padded to 8, 16 or 32
     int ncol;
     float *out; size_t out_stride;                 // column c at out + c * out_stride
     const float *resid; size_t resid_stride;       // optional: out = sum + resid (may alias out)

@@ -6,13 +6,14 @@
 // What bounds it: memory at 8 columns; beyond, the fp32 combination, which the contract fixes at 26 packed operations per
 // (16 rows, 8 columns, 128 weights) - 13 cycles of the SM's FMA pipes - against 4 mma (8 cycles of the tensor cores) and 16
 // ANDs per 16 rows. The accumulators of mma.sync are registers, in the layout the combination wants; tcgen05 would bring them
-// through tensor memory and hand-offs between warps (18 944 x 4096: 20.8 / 25.4 / 36.7 us for 8 / 16 / 32 columns that way,
-// where an instruction of 128 rows costs 190 cycles whatever its column count, and the tensor pipe is idle either way).
+// through tensor memory and hand-offs between warps: the kernel that did so, with the operand decoded into tensor memory, took
+// 28 / 33 / 48 us for 24 576 x 4096 at 8 / 16 / 32 columns against 15 / 21 / 43 here (a tcgen05.mma of 128 rows costs 190 cycles
+// whatever its column count, and the tensor pipe is idle either way).
 //
-// Work split. A CTA of 8 warps owns a run of row tiles over all of K. K is walked in waves of `kc` groups (512 weights each);
+// Work split. A CTA of 12 or 16 warps owns a run of row tiles over all of K. K is walked in waves of `kc` groups (512 weights each);
 // a wave's piece of the activation image is double-buffered in shared memory. A wave's units (MT row tiles, one group, up to 16
 // columns) are dealt to the warps; a unit keeps everything in registers and leaves its group sums p_g in shared memory, where
-// after a barrier every thread adds its own (row, column)s' in ascending order. MT = 3 row tiles share a group's operands and
+// after a barrier every thread adds its own (row, column)s' in ascending order. MT = 2 or 3 row tiles share a group's operands and
 // scales: with one, shared-memory reads (24 wavefronts per 16 rows x 8 columns x 128 weights) would bound the loop.
 #include "q2.cuh"
 #include "rotate_quant.cuh"
@@ -22,12 +23,17 @@
 namespace {
 using namespace bnk;
 
-constexpr int NT = 256, NW = NT / 32, SMEM_MAX = 227 << 10;
-constexpr int IMG_COL = 160;                   // image bytes per column and block (gemm_tc.cuh)
+// Threads and row tiles per unit, by measurement (24 576 x 4096, and 4096 x 12 288 in brackets): 8 columns 384 threads x 3 tiles
+// 15.3 us (256 x 3: 16.2, 512 x 2: 16.3); 16 columns 512 x 2 21.0 us (256 x 3: 22.3); 32 columns 512 x 2 43.3 (28.8) us (256 x 3: 48.7
+// (32.6)). Requesting a warp's next unit before the present one (weights in 60 more registers) changed nothing: the other warps
+// hide the loads.
+template <int NCP> __host__ __device__ constexpr int threads() { return NCP == 8 ? 384 : 512; }
+constexpr int SMEM_MAX = 227 << 10;
+constexpr int IMG_COL = 160;                   // image bytes per column and block (act_image.cuh)
 constexpr int MAX_TILES = 12;                  // row tiles per pass over K (a thread keeps their running sums in registers)
 
-__device__ __forceinline__ bool full_wait(uint32_t bar, uint32_t parity, int *err) {
-    for (int it = 0; it < (1 << 22); ++it) {
+__device__ __forceinline__ bool full_wait(uint32_t bar, uint32_t parity, int *err, int limit = 1 << 22) {
+    for (int it = 0; it < limit; ++it) {
         uint32_t ok;
         asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
                      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
@@ -38,7 +44,8 @@ __device__ __forceinline__ bool full_wait(uint32_t bar, uint32_t parity, int *er
 }
 
 template <int NCP, int MT>
-__global__ void __launch_bounds__(NT, 1) k_q2_gemm(const Q2GemmArgs a) {
+__global__ void __launch_bounds__(threads<NCP>(), 1) k_q2_gemm(const Q2GemmArgs a) {
+    constexpr int NT = threads<NCP>(), NW = NT / 32;
     constexpr int NG = NCP / 8, NGW = NG >= 2 ? 2 : 1, H = NG / NGW;      // column groups: all, per unit; units across the columns
     constexpr int ITEMS = (MAX_TILES * 16 * NCP + NT - 1) / NT;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -199,6 +206,16 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm(const Q2GemmArgs a) {
     }
 }
 
+// A wait that nothing will ever satisfy, with a short limit: the give-up path of full_wait (error word = 2, kernel returns)
+__global__ void k_wait_selftest_gemm(int *err) {
+    __shared__ uint64_t bar;
+    const uint32_t b = uint32_t(__cvta_generic_to_shared(&bar));
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\nfence.mbarrier_init.release.cluster;" ::"r"(b) : "memory");
+        full_wait(b, 0, err, 1 << 10);
+    }
+}
+
 template <int NCP, int MT>
 cudaError_t launch_t(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl) {
     static bool attr_set = false;
@@ -210,15 +227,16 @@ cudaError_t launch_t(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl) {
     const int ng = a.K / 512, tiles = (a.M + 15) / 16, grid = std::min(tiles, sm_count);
     a.share = {tiles / grid, tiles % grid};
     a.tiles = std::min(a.share.q + (a.share.r > 0), MAX_TILES);
-    // groups per wave: as many as fit with their image piece twice (once when one wave is all of K) and their group sums
+    // groups per wave: all of K where its image piece fits beside its group sums (one wave: no barrier in between, and the units
+    // spread over more warps), else as many as fit with the image piece twice
     const int gimg = 4 * NCP * IMG_COL, gsum = a.tiles * 16 * NCP * 4;
     auto bytes = [&](int kc) { return 128 + kc * ((kc >= ng ? 1 : 2) * gimg + gsum); };
-    a.kc = std::min(ng, 8);
-    while (a.kc > 1 && bytes(a.kc) > SMEM_MAX) a.kc = (a.kc + 1) / 2;
+    a.kc = ng;
+    if (bytes(ng) > SMEM_MAX) for (a.kc = std::min(ng - 1, 8); a.kc > 1 && bytes(a.kc) > SMEM_MAX;) a.kc = (a.kc + 1) / 2;
     if (a.next.W) a.next.share = {a.next.units / grid, a.next.units % grid};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(NT);
+    cfg.blockDim = dim3(threads<NCP>());
     cfg.dynamicSmemBytes = std::max(bytes(a.kc), 116 << 10);             // one CTA per SM, as in q2_gemv.cu
     cfg.stream = st;
     cudaLaunchAttribute at[1];
@@ -236,11 +254,19 @@ namespace bnk {
 
 cudaError_t launch_q2_gemm(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl) {
     const int ncp = a.ncol <= 8 ? 8 : (a.ncol <= 16 ? 16 : 32), tiles = (a.M + 15) / 16;
-    // two row tiles per unit where a CTA has no more (the 4096-row projections), else three
-    const bool two = tiles <= 2 * sm_count;
-    if (ncp == 8) return two ? launch_t<8, 2>(st, sm_count, a, pdl) : launch_t<8, 3>(st, sm_count, a, pdl);
-    if (ncp == 16) return two ? launch_t<16, 2>(st, sm_count, a, pdl) : launch_t<16, 3>(st, sm_count, a, pdl);
-    return two ? launch_t<32, 2>(st, sm_count, a, pdl) : launch_t<32, 3>(st, sm_count, a, pdl);
+    // row tiles per unit: where a CTA has two tiles at most (the 4096-row projections) one, so that a wave has a unit for every
+    // warp (4096 x 12 288: 12.6 against 15.5 us at 8 columns); at 32 columns there are units enough and two are better (28.7
+    // against 31.8 us)
+    const bool few = tiles <= 2 * sm_count;
+    if (ncp == 8) return few ? launch_t<8, 1>(st, sm_count, a, pdl) : launch_t<8, 3>(st, sm_count, a, pdl);
+    if (ncp == 16) return few ? launch_t<16, 1>(st, sm_count, a, pdl) : launch_t<16, 2>(st, sm_count, a, pdl);
+    return launch_t<32, 2>(st, sm_count, a, pdl);
+}
+
+cudaError_t launch_wait_selftest_gemm(cudaStream_t st, int *err) {
+    BN_COUNT(1);
+    k_wait_selftest_gemm<<<1, 32, 0, st>>>(err);
+    return cudaGetLastError();
 }
 
 }  // namespace bnk

@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(NT + 32, 1) k_q2_gemv(const Q2Args a) {
     Q2_STAMP(7);
 }
 
-// one thread per (row, block): five base-3 digits per byte -> the four two-bit fields of the piece (unpacking as in the
+// four packed bytes: five base-3 digits per byte -> the four two-bit fields of the piece (unpacking as in the
 // multi-column kernel: T_t = (b * 3^(t+1)) >> 8 is the base-3 prefix of byte b, digit t = T_t - 3 T_(t-1))
 __device__ __forceinline__ void unpack4(uint32_t w, uint32_t *o, int stride) {
     const uint32_t e = __byte_perm(w, 0u, 0x4240u), d = __byte_perm(w, 0u, 0x4341u);
@@ -349,35 +349,54 @@ __device__ __forceinline__ void unpack4(uint32_t w, uint32_t *o, int stride) {
         prev = T;
     }
 }
-__global__ void __launch_bounds__(256) k_q2_repack(const uint32_t *__restrict__ W, int M, int nb, uint8_t *__restrict__ out, int half) {
-    pdl_sync();
-    const int ng = nb >> 2, ntiles = (M + 15) >> 4;
-    const size_t total = size_t(ntiles) * 16 * nb;
-    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
-        const int b = int(i % nb), row = int(i / nb), r = half < 0 ? row & 15 : (row & 7) + 8 * half, tile = half < 0 ? row >> 4 : row >> 3, j = b & 3;
-        uint32_t o[32], w[7] = {0, 0, 0, 0, 0, 0, 0};
-        if (row < M) {
+// A warp per piece: lane (row, block) unpacks 28 bytes into shared memory, eight rows at a time, and the finished piece leaves
+// as 16-byte stores (stored straight from the lanes, 8 bytes of every 16, it ran at a third of the rate). Rows 0..7 of a tile
+// come from Wa and 8..15 from Wb, `half` rows apart in each (Wb = Wa + 8 rows and half = 16 for a single matrix).
+__global__ void __launch_bounds__(256) k_q2_repack(const uint32_t *__restrict__ Wa, const uint32_t *__restrict__ Wb, int half, int Ma, int Mb, int nb,
+                                                   size_t pieces, uint8_t *__restrict__ out) {
+    __shared__ __align__(16) uint8_t stage[8][Q2_PIECE];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ng = nb >> 2, r = lane >> 2, j = lane & 3;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    uint8_t *piece = stage[warp];
+    for (size_t p = size_t(blockIdx.x) * 8 + warp; p < pieces; p += size_t(gridDim.x) * 8) {
+        const int tile = int(p / ng), gr = int(p - size_t(tile) * ng), row = tile * half + r;
+        uint32_t w[2][7];
 #pragma unroll
-            for (int k = 0; k < 7; ++k) w[k] = W[(size_t(row) * nb + b) * 7 + k];
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t *src = (h ? Wb : Wa) + (size_t(row) * nb + gr * 4 + j) * 7;
+            const bool on = row < (h ? Mb : Ma);
+#pragma unroll
+            for (int k = 0; k < 7; ++k) w[h][k] = on ? src[k] : 0u;
         }
+        __syncwarp();                          // the previous piece has left
 #pragma unroll
-        for (int k = 0; k < 4; ++k) unpack4(w[k], o + k, 4);
-        unpack4(w[4], o + 20, 2);
-        unpack4(w[5], o + 21, 2);
-        const uint32_t v = __byte_perm(w[6], 0u, 0x4140u);
-        const uint32_t ta = __byte_perm(v * 3u, v * 9u, 0x7531u), tb = __byte_perm(v * 27u, v * 81u, 0x7531u);
-        o[30] = ta - 3u * (ta << 16);
-        o[31] = tb - 3u * __byte_perm(ta, tb, 0x5432u);
-        uint8_t *piece = out + (size_t(tile) * ng + (b >> 2)) * Q2_PIECE;
-        uint8_t *dst = piece + ((r >> 3) * 2 + (j >> 1)) * 512 + (r & 7) * 64 + (j & 1) * 8;
+        for (int h = 0; h < 2; ++h) {
+            uint32_t o[32];
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            uint2 p;
-            p.x = o[2 * t] | o[8 + 2 * t] << 2 | o[16 + 2 * t] << 4 | o[24 + 2 * t] << 6;
-            p.y = o[2 * t + 1] | o[9 + 2 * t] << 2 | o[17 + 2 * t] << 4 | o[25 + 2 * t] << 6;
-            *reinterpret_cast<uint2 *>(dst + t * 16) = p;
+            for (int k = 0; k < 4; ++k) unpack4(w[h][k], o + k, 4);
+            unpack4(w[h][4], o + 20, 2);
+            unpack4(w[h][5], o + 21, 2);
+            const uint32_t v = __byte_perm(w[h][6], 0u, 0x4140u);
+            const uint32_t ta = __byte_perm(v * 3u, v * 9u, 0x7531u), tb = __byte_perm(v * 27u, v * 81u, 0x7531u);
+            o[30] = ta - 3u * (ta << 16);
+            o[31] = tb - 3u * __byte_perm(ta, tb, 0x5432u);
+            uint8_t *dst = piece + (h * 2 + (j >> 1)) * 512 + r * 64 + (j & 1) * 8;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                uint2 q;
+                q.x = o[2 * t] | o[8 + 2 * t] << 2 | o[16 + 2 * t] << 4 | o[24 + 2 * t] << 6;
+                q.y = o[2 * t + 1] | o[9 + 2 * t] << 2 | o[17 + 2 * t] << 4 | o[25 + 2 * t] << 6;
+                *reinterpret_cast<uint2 *>(dst + t * 16) = q;
+            }
+            *reinterpret_cast<uint16_t *>(piece + Q2_SCALES + (r * 4 + j) * 4 + h * 2) = uint16_t(w[h][6] >> 16);
         }
-        *reinterpret_cast<uint16_t *>(piece + Q2_SCALES + ((r & 7) * 4 + j) * 4 + (r >> 3) * 2) = uint16_t(w[6] >> 16);
+        __syncwarp();
+        uint4 *d = reinterpret_cast<uint4 *>(out + p * Q2_PIECE);
+        const uint4 *s = reinterpret_cast<const uint4 *>(piece);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[i * 32 + lane] = s[i * 32 + lane];
+        if (lane < 8) d[128 + lane] = s[128 + lane];
     }
 }
 __global__ void k_sign_bits(const int32_t *__restrict__ signs, int nwords, uint8_t *__restrict__ bits) {
@@ -432,10 +451,14 @@ cudaError_t launch_q2_gemv(cudaStream_t st, int sm_count, const Q2Args &a, bool 
     return a.K <= 4096 ? launch_spans<1>(st, sm_count, a, pdl) : launch_spans<4>(st, sm_count, a, pdl);
 }
 
-void q2_repack(cudaStream_t st, const uint32_t *W, int M, int K, uint8_t *out, int half) {
-    const size_t total = size_t((M + 15) / 16) * 16 * (K / 128);
-    launch(k_q2_repack, dim3(unsigned(std::min<size_t>((total + 255) / 256, 148 * 16))), dim3(256), 0, st, W, M, K / 128, out, half);
+static void repack(cudaStream_t st, const uint32_t *Wa, const uint32_t *Wb, int half, int Ma, int Mb, int tiles, int K, uint8_t *out) {
+    const size_t pieces = size_t(tiles) * (K / 512);
+    launch(k_q2_repack, dim3(unsigned(std::min<size_t>((pieces + 7) / 8, 148 * 8))), dim3(256), 0, st, Wa, Wb, half, Ma, Mb, K / 128, pieces, out);
 }
+void q2_repack(cudaStream_t st, const uint32_t *W, int M, int K, uint8_t *out) {
+    repack(st, W, W + size_t(8) * (K / 128) * 7, 16, M, M - 8, (M + 15) / 16, K, out);
+}
+void q2_repack_pair(cudaStream_t st, const uint32_t *Wa, const uint32_t *Wb, int M, int K, uint8_t *out) { repack(st, Wa, Wb, 8, M, M, M / 8, K, out); }
 void pack_sign_bits(cudaStream_t st, const int32_t *signs, int n, uint8_t *bits) {
     BN_COUNT(1);
     k_sign_bits<<<(n / 8 + 255) / 256, 256, 0, st>>>(signs, n / 8, bits);

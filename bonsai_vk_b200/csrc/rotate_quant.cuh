@@ -1,8 +1,8 @@
-// rotate_quant.cuh - the pieces of "rotate, then quantise" that the single-sequence prologue (phase_body.cuh), the
-// packed swiglu kernel (phase_gemv.cu) and the multi-column activation image (gemm_tc.cu) share, so that all three
-// produce the same bits: the mean of a power-of-two count, the sign flip, the register / shuffle butterflies of the
-// Sylvester-Walsh-Hadamard transform (reference network: runtime_vk/shaders/hat4096.comp:41-60) and the q8_1 quantiser
-// of eight values (recipe: runtime_vk/shaders/attn_norm_rope2.comp:39-49).
+// rotate_quant.cuh - the pieces of "rotate, then quantise" that the projection kernels' input preparation (q2_gemv.cu), the
+// multi-column activation image (prep_cols.cu) and the whole-token kernel (phase_body.cuh) share, so that all of them produce
+// the same bits: the mean of a power-of-two count, the sign flip, the butterflies of the Sylvester-Walsh-Hadamard transform
+// (reference network: runtime_vk/shaders/hat4096.comp:41-60) and the q8_1 quantiser (recipe:
+// runtime_vk/shaders/attn_norm_rope2.comp:39-49).
 #pragma once
 #include "common.cuh"
 

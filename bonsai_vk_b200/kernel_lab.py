@@ -3,7 +3,7 @@
 
   python -m bonsai_vk_b200.kernel_lab M K [ITER]
   python -m bonsai_vk_b200.kernel_lab attn CTX [ITER]      one decode-attention layer (16/4 heads x 256, q8_0 K and V)
-  python -m bonsai_vk_b200.kernel_lab gemm M K NCOL [ITER]  the multi-column tensor-core projection (tcgen05), timed
+  python -m bonsai_vk_b200.kernel_lab gemm M K NCOL [ITER]  the multi-column tensor-core projection, timed
   python -m bonsai_vk_b200.kernel_lab stage NBLOCKS NCOL CTX [ITER]   one pipeline stage (first NBLOCKS blocks of the 9B
                                             shape) for NCOL sequences per pass at context CTX, timed per pass
   python -m bonsai_vk_b200.kernel_lab stamps [TOKENS]       where one B=1 token of the 9B shape spends its time: device time

@@ -116,7 +116,7 @@ int bn_gemv_f32act(bn_ctx *ctx, const bn_buf *w, size_t w_off, int M, int K, con
                    bn_buf *out, size_t out_off);
 
 /* ---- the same projection for several activation columns at once (prefill tokens, concurrent sequences) on the
- *      tcgen05 tensor cores. Reference: the multi-column path of _mul_mat_vecq_ptq1_0.comp:204-347 (<= 8 columns;
+ *      int8 tensor cores. Reference: the multi-column path of _mul_mat_vecq_ptq1_0.comp:204-347 (<= 8 columns;
  *      beyond that the reference falls back to dequantise + f16 matmul, _ggml-vulkan.cpp:2195-2197, which has no
  *      integer block dots). Every column of the result is bit-identical to bn_gemv_q81 on that column's vector. -----
  * The activations are handed over as one "image" for all columns: int8 codes in the tensor-core operand layout plus
@@ -233,7 +233,7 @@ int bn_model_stage_prepare(bn_model *m, int stream0, int ncol);
  * replaced by 0 and reported by the next bn_sync (BN_ERR_ARG). */
 int bn_model_stage(bn_model *m, int stream, int tok, int pos, const bn_buf *in, size_t in_off, bn_buf *out, size_t out_off);
 /* The same stage for ncol consecutive sequences stream0 .. stream0+ncol-1 in one pass (the micro-batch of the layer
- * pipeline): every projection reads its weights once for all of them (tcgen05 kernel, bn_gemm_q81), the other
+ * pipeline): every projection reads its weights once for all of them (the kernel of bn_gemm_q81), the other
  * kernels run one grid slice per sequence. pos[c] is the position of sequence stream0+c. First stage: tok != NULL gives
  * the token ids, tok == NULL reads ncol ints from (in, in_off). Other stages: (in, in_off) holds ncol x hidden fp32,
  * sequence-major. Output: ncol x hidden fp32, or ncol ints (the greedy picks) on the last stage. Each sequence's result
