@@ -245,9 +245,9 @@ bnk::Q2Next next_after(const bn_model *m, int b) {
     return m->b1 == h.n_layer ? q2_next(m->q2_head, h.vocab, h.hidden, m->out_norm) : bnk::Q2Next();
 }
 // x = rms_norm(RES) * w through one projection group
-void norm_project(bn_model *m, const uint8_t *W, int M, const float *w, float *out, const bnk::Q2Next &next, float *inv_out = nullptr, bool swiglu = false) {
+void norm_project(bn_model *m, const uint8_t *W, int M, const float *w, float *out, const bnk::Q2Next &next, float *inv_out = nullptr, bool swiglu = false, bool mixer = false) {
     bnk::Q2Args a = phase_base(m, W, M, m->hp.hidden);
-    a.next = next;
+    a.next = next; a.lean = mixer; a.late = inv_out != nullptr;
     a.pro = bnk::Q2_NORM; a.x0 = m->RES; a.w = w; a.out = out; a.inv_out = inv_out; a.swiglu = swiglu;
     launch(m, a);
 }
@@ -271,14 +271,18 @@ void ffn_fused(bn_model *m, const bn_model::Layer &L) {
 void gdn_fused(bn_model *m, const bn_model::Layer &L) {
     const bn_hparams &h = m->hp;
     const int NH = h.gdn_heads, NQ = h.gdn_qk_heads, D = h.gdn_dim, C = 2 * NQ * D + NH * D, IN = NH * D;
-    norm_project(m, L.q2_in, C + IN, L.attn_norm, m->QKV, q2_next(L.q2_out, h.hidden, IN, nullptr), m->G + 48);      // (the norm factor also goes to the layer core's two small projections)
+    norm_project(m, L.q2_in, C + IN, L.attn_norm, m->QKV, q2_next(L.q2_out, h.hidden, IN, nullptr), m->G + 48, false, true);      // (the norm factor also goes to the layer core's two small projections)
     if (!m->phases_only) {
         const bnk::GdnDims gd{NH, NQ, D};
         float *h0 = conv_of(m, 0, L.idx), *h1 = conv_of(m, 1, L.idx);
         // one sequence: heads x 4 CTAs in clusters of 4 (fills the GPU); several sequences: one CTA per head and sequence
-        if (D == 128 && getenv("BONSAI_GDN_ONE_CTA_PER_HEAD") == nullptr)
-            bnk::gdn_core_split(m->ctx->stream, gd, h.hidden, m->QKV, L.conv_w, h0, h1, m->POS, m->RES, m->G + 48, L.attn_norm, L.alpha_w,
-                                L.beta_w, L.dt_bias, L.ssm_a, gdn_state_of(m, L.idx), m->Z, L.ssm_norm, h.rms_eps, m->X1);
+        if (D == 128 && getenv("BONSAI_GDN_ONE_CTA_PER_HEAD") == nullptr) {
+            bnk::GdnStep s = {};
+            s.heads = NH; s.qk_heads = NQ; s.hidden = h.hidden; s.qkv = m->QKV; s.z = m->Z; s.conv_w = L.conv_w; s.hist0 = h0; s.hist1 = h1; s.pos = m->POS;
+            s.x = m->RES; s.norm_w = L.attn_norm; s.alpha_w = L.alpha_w; s.beta_w = L.beta_w; s.dt_bias = L.dt_bias; s.ssm_a = L.ssm_a;
+            s.state = gdn_state_of(m, L.idx); s.ssm_norm = L.ssm_norm; s.eps = h.rms_eps; s.scale = 1.0f / sqrtf(float(D)); s.y = m->X1;
+            bnk::gdn_step(m->ctx->stream, s);
+        }
         else
             bnk::gdn_core_fused(m->ctx->stream, gd, h.hidden, m->QKV, L.conv_w, h0, h1, m->POS, m->RES, m->G + 48, L.attn_norm,
                                 L.alpha_w, L.beta_w, L.dt_bias, L.ssm_a, gdn_state_of(m, L.idx), m->Z, L.ssm_norm, h.rms_eps, m->X1);
@@ -292,7 +296,7 @@ void attn_fused(bn_model *m, const bn_model::Layer &L) {
     const int QD = h.n_head * h.head_dim, KD = h.n_kv * h.head_dim;
     const bnk::AttnDims ad = attn_dims(m);
     const bnk::KvLayer kv = kv_layer(m, L.idx);
-    norm_project(m, L.q2_in, 2 * QD + 2 * KD, L.attn_norm, m->QKV, q2_next(L.q2_out, h.hidden, QD, nullptr));
+    norm_project(m, L.q2_in, 2 * QD + 2 * KD, L.attn_norm, m->QKV, q2_next(L.q2_out, h.hidden, QD, nullptr), nullptr, false, true);
     if (!m->phases_only) {
         bnk::attn_prep(st, ad, m->QKV, m->KBUF, m->VBUF, L.q_norm, L.k_norm, {m->POS, 0}, kv, m->Q16F, m->GATEB, m->ESUM);
         bnk::attn_decode(st, ad, m->Q16F, m->GATEB, {m->POS, 0}, kv, m->SCORE, m->P16F, m->ESUM, m->PVPART, m->pv_splits, nullptr, m->GOUT);

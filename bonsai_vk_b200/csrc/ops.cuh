@@ -83,12 +83,20 @@ void gdn_core_fused(cudaStream_t st, GdnDims d, int hidden, const float *qkv, co
                     float *hist1, const int *pos_ptr, const float *x, const float *inv_ptr, const float *norm_w, const float *alpha_w,
                     const float *beta_w, const float *dt_bias, const float *ssm_a, float *state, const float *z,
                     const float *ssm_norm, float eps, float *y, Cols cols = {});
-// the same fused mixer for one sequence on heads x 4 CTAs (clusters of 4, 32 state rows per CTA, the head norm through
-// distributed shared memory): same arguments and results as gdn_core_fused
-void gdn_core_split(cudaStream_t st, GdnDims d, int hidden, const float *qkv, const float *conv_w, float *hist0, float *hist1,
-                    const int *pos_ptr, const float *x, const float *inv_ptr, const float *norm_w, const float *alpha_w,
-                    const float *beta_w, const float *dt_bias, const float *ssm_a, float *state, const float *z,
-                    const float *ssm_norm, float eps, float *y);
+// the same fused mixer for one token of one sequence on heads x 4 CTAs (gdn_step.cu). The kernel reads the residual before its
+// dependency wait: the launch in front of it must be one that releases its dependents behind its own wait (Q2Args::late).
+struct GdnStep {
+    int heads, qk_heads, hidden;
+    const float *qkv, *z, *conv_w;
+    float *hist0, *hist1;
+    const int *pos;
+    const float *x, *norm_w, *alpha_w, *beta_w, *dt_bias, *ssm_a;
+    float *state;
+    const float *ssm_norm;
+    float eps, scale;
+    float *y;
+};
+void gdn_step(cudaStream_t st, const GdnStep &a);
 // the mixer for n <= 32 consecutive positions of one sequence (gdn_seq.cu): column c's activations at + c * stride bytes
 struct GdnSeq {
     int heads, qk_heads, hidden;

@@ -60,6 +60,8 @@ struct Q2Args {
     Q2Share share;               // the CTAs' shares of the row tiles;
     int slots;                   // ring slots
     float *inv_out;              // Q2_NORM, optional: 1/sqrt(mean(x0^2) + eps)
+    int late;                    // release the dependent launch behind this kernel's own dependency wait (see GdnStep)
+    int lean;                    // leave room for the next kernel's CTA on the SM (a mixer follows)
     Q2Next next;
     int *err;                    // device error word (bounded waits)
     unsigned long long *stamps;  // optional, 8 device time stamps of CTA 0 (see PhaseArgs)

@@ -71,8 +71,12 @@ __device__ __forceinline__ f32pair sign_pair(uint32_t sg, int k) {
 }
 
 // SPANS: spans of 4096 values whose inputs a thread holds at once (1: K <= 4096; 4: up to 16384)
-template <int SPANS>
-__global__ void __launch_bounds__(NT + 32, 1) k_q2_gemv(const Q2Args a) {
+// LEAN: 80 registers instead of 94, so that beside the 17 warps (five of them on one of the SM's four schedulers, each with
+// 16 384 registers) the CTA of a latency-bound mixer kernel fits, and a shared-memory carve-out that leaves room for it: the
+// kernel behind the projections of a layer's input. It costs 0.6 us here (12 288 x 4096: 3.0 -> 3.6 us in the loop) and takes
+// 3.5 us off what follows.
+template <int SPANS, bool LEAN>
+__global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Args a) {
     extern __shared__ __align__(128) unsigned char smem[];
     const Lay L = layout(a.K);
     unsigned char *codes = smem + L.codes;
@@ -109,7 +113,7 @@ __global__ void __launch_bounds__(NT + 32, 1) k_q2_gemv(const Q2Args a) {
         }
         __syncwarp();
         asm volatile("bar.arrive 2, %0;" ::"n"(NT + 32) : "memory");
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        if (!a.late) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         asm volatile("bar.sync 3, %0;" ::"n"(NT + 32) : "memory");
         if (lane == 0) for (int i = EARLY; i < min(slots, nchunks); ++i) request(i, i);
         for (int i = slots, s = 0, ph = 0; i < nchunks; ++i) {
@@ -130,13 +134,14 @@ __global__ void __launch_bounds__(NT + 32, 1) k_q2_gemv(const Q2Args a) {
     if (SPANS == 1 && a.pro == Q2_NORM && base < a.K) load8(a.w + base, nw);
     Q2_STAMP(1);
     // The next kernel may start now: whatever it does before its own wait touches constants only.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (!a.late) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (SPANS == 1) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) nw[k] ^= sign_pair(sg[0], k);
     }
     asm volatile("bar.sync 2, %0;" ::"n"(NT + 32) : "memory");          // the ring's barriers are initialised
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (a.late) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     Q2_STAMP(2);
 
     // ---- input preparation -------------------------------------------------------------------------------------------
@@ -407,7 +412,7 @@ __global__ void k_sign_bits(const int32_t *__restrict__ signs, int nwords, uint8
     bits[i] = uint8_t(b);
 }
 
-template <int SPANS>
+template <int SPANS, bool LEAN>
 cudaError_t launch_spans(cudaStream_t st, int sm_count, Q2Args a, bool pdl) {
     static int smem_set = 0;
     // as many chunks of weights as fit beside the rest, and at least half of an SM's shared memory in all, so that two CTAs of a
@@ -418,8 +423,10 @@ cudaError_t launch_spans(cudaStream_t st, int sm_count, Q2Args a, bool pdl) {
     a.slots = std::min({chunks, MAX_SLOTS, (SMEM_MAX - layout(a.K).ring) / CHUNK});
     const int smem = std::max(layout(a.K).ring + a.slots * CHUNK, 116 << 10);
     if (smem > smem_set) {
-        cudaError_t e = cudaFuncSetAttribute(k_q2_gemv<SPANS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t e = cudaFuncSetAttribute(k_q2_gemv<SPANS, LEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
+        // (an SM changes its carve-out only when it is empty, so every projection asks for the largest one)
+        cudaFuncSetAttribute(k_q2_gemv<SPANS, LEAN>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         smem_set = smem;
     }
     a.inv_k = (a.K & (a.K - 1)) == 0 ? 1.0f / float(a.K) : 0.0f;
@@ -436,7 +443,7 @@ cudaError_t launch_spans(cudaStream_t st, int sm_count, Q2Args a, bool pdl) {
     cfg.attrs = at;
     cfg.numAttrs = pdl ? 1 : 0;
     BN_COUNT(1);
-    return cudaLaunchKernelEx(&cfg, k_q2_gemv<SPANS>, a);
+    return cudaLaunchKernelEx(&cfg, k_q2_gemv<SPANS, LEAN>, a);
 }
 
 }  // namespace
@@ -448,7 +455,8 @@ bool q2_gemv_supported(int K, int hat_block) {
 }
 
 cudaError_t launch_q2_gemv(cudaStream_t st, int sm_count, const Q2Args &a, bool pdl) {
-    return a.K <= 4096 ? launch_spans<1>(st, sm_count, a, pdl) : launch_spans<4>(st, sm_count, a, pdl);
+    if (a.K > 4096) return launch_spans<4, false>(st, sm_count, a, pdl);
+    return a.lean ? launch_spans<1, true>(st, sm_count, a, pdl) : launch_spans<1, false>(st, sm_count, a, pdl);
 }
 
 static void repack(cudaStream_t st, const uint32_t *Wa, const uint32_t *Wb, int half, int Ma, int Mb, int tiles, int K, uint8_t *out) {
