@@ -15,42 +15,24 @@ __device__ __forceinline__ float tree128(float e0, float e1, float e2, float e3)
     return a;
 }
 
-// grid (heads, positions / 4), 512 threads: four positions of one value head (and of q / k head h, where h is one).
+// grid (2 x heads, positions / 4), 256 threads. Even CTAs: conv + silu + L2 norms of four positions of one value head (and of q / k
+// head h, where h is one). Odd CTAs: alpha and beta of one value head for the same positions, one warp per dot: as a second task of
+// the even CTAs' warps the dots took 18 us with the rest; side by side, 4 us.
 constexpr int PP = 4;
-__global__ void __launch_bounds__(512) k_gdn_seq_pre(bnk::GdnSeq a, int n) {
+__global__ void __launch_bounds__(256) k_gdn_seq_pre(bnk::GdnSeq a, int n) {
     __shared__ float sq[PP][256];                  // q and k channels of the positions
-    const int h = blockIdx.x, c0 = blockIdx.y * PP, np = min(PP, n - c0), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int h = blockIdx.x >> 1, c0 = blockIdx.y * PP, np = min(PP, n - c0), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const bool own_qk = h < a.qk_heads;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const float *hist = (a.pos[0] & 1) ? a.hist1 : a.hist0;
-    // input of channel ch at position c of the block; positions before it are the history taps
-    auto in = [&](int ch, int c) { return c < 0 ? hist[3 * size_t(ch) + 3 + c] : bnk::colp(a.qkv, c * a.stride)[ch]; };
-    auto conv = [&](int ch, int c) {
-        const float *wc = a.conv_w + 4 * size_t(ch);
-        float acc = __fmul_rn(wc[0], in(ch, c - 3));
-        acc = __fadd_rn(acc, __fmul_rn(wc[1], in(ch, c - 2)));
-        acc = __fadd_rn(acc, __fmul_rn(wc[2], in(ch, c - 1)));
-        acc = __fadd_rn(acc, __fmul_rn(wc[3], in(ch, c)));
-        return silu_f(acc);
-    };
-    if (tid < 128 * np) {
-        const int p = tid >> 7, d = tid & 127;
-        bnk::colp(a.v, (c0 + p) * a.stride)[h * 128 + d] = conv(2 * a.qk_heads * 128 + h * 128 + d, c0 + p);
-    }
-    if (own_qk)
-        for (int i = tid; i < 256 * np; i += 512) {
-            const int p = i >> 8, d = i & 255;
-            sq[p][d] = conv((d < 128 ? 0 : a.qk_heads * 128) + h * 128 + (d & 127), c0 + p);
-        }
-    // two small projections of the normed residual and their gate functions: warp = (position, alpha / beta)
-    if (warp >= 8 && warp < 8 + 2 * np) {
-        const int p = (warp - 8) >> 1, beta = warp & 1, n4 = a.hidden / 4;
+    if (blockIdx.x & 1) {
+        const int p = warp >> 1, beta = warp & 1, n4 = a.hidden / 4;
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (p >= np) return;
         const float inv = bnk::colp(a.inv, (c0 + p) * a.stride)[0];
         const float4 *xv = reinterpret_cast<const float4 *>(bnk::colp(a.x, (c0 + p) * a.stride)), *nw = reinterpret_cast<const float4 *>(a.norm_w);
         const float4 *wr = reinterpret_cast<const float4 *>((beta ? a.beta_w : a.alpha_w) + size_t(h) * a.hidden);
         float acc = 0.0f;
-#pragma unroll 4
+#pragma unroll 8
         for (int i = lane; i < n4; i += 32) {
             const float4 x4 = xv[i], w4 = nw[i], r4 = wr[i];
             acc = fmaf(r4.x, __fmul_rn(__fmul_rn(x4.x, inv), w4.x), acc); acc = fmaf(r4.y, __fmul_rn(__fmul_rn(x4.y, inv), w4.y), acc);
@@ -66,7 +48,28 @@ __global__ void __launch_bounds__(512) k_gdn_seq_pre(bnk::GdnSeq a, int n) {
                 bnk::colp(a.eg, (c0 + p) * a.stride)[h] = exp_f(__fmul_rn(sp, a.ssm_a[h]));
             }
         }
+        return;
     }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const float *hist = (a.pos[0] & 1) ? a.hist1 : a.hist0;
+    // input of channel ch at position c of the block; positions before it are the history taps
+    auto in = [&](int ch, int c) { return c < 0 ? hist[3 * size_t(ch) + 3 + c] : bnk::colp(a.qkv, c * a.stride)[ch]; };
+    auto conv = [&](int ch, int c) {
+        const float *wc = a.conv_w + 4 * size_t(ch);
+        float acc = __fmul_rn(wc[0], in(ch, c - 3));
+        acc = __fadd_rn(acc, __fmul_rn(wc[1], in(ch, c - 2)));
+        acc = __fadd_rn(acc, __fmul_rn(wc[2], in(ch, c - 1)));
+        acc = __fadd_rn(acc, __fmul_rn(wc[3], in(ch, c)));
+        return silu_f(acc);
+    };
+    for (int i = tid; i < 128 * np; i += 256) {
+        const int p = i >> 7, d = i & 127;
+        bnk::colp(a.v, (c0 + p) * a.stride)[h * 128 + d] = conv(2 * a.qk_heads * 128 + h * 128 + d, c0 + p);
+    }
+    if (own_qk)
+#pragma unroll 4
+        for (int p = 0; p < np; ++p) sq[p][tid] = conv((tid < 128 ? 0 : a.qk_heads * 128) + h * 128 + (tid & 127), c0 + p);
     __syncthreads();
     if (own_qk && warp < 2 * np) {                 // L2 norms: warp = (position, q / k)
         const int p = warp >> 1, k = warp & 1;
@@ -78,27 +81,34 @@ __global__ void __launch_bounds__(512) k_gdn_seq_pre(bnk::GdnSeq a, int n) {
     }
 }
 
-// grid heads x 4: 32 state rows of a head, two per warp, in registers for all positions. The head's q and k of every position
+// grid heads x 4: 32 state rows of a head, four per warp, in registers for all positions. The head's q and k of every position
 // are staged in shared memory first. Per position a row's chain is two 128-value trees (prediction, output) with the update
-// between; the output tree of one position runs beside the prediction tree of the next.
-__global__ void __launch_bounds__(512) k_gdn_seq(bnk::GdnSeq a, int n) {
+// between; the output trees of one position run beside the prediction trees of the next, eight trees on nine shuffles: a level's
+// two values change hands between the lanes that go on with one and those that go on with the other (the shuffles' throughput
+// bounds the loop: with five per tree and two rows per warp 1000 cycles a position, now 400).
+// One CTA per SM (its shared memory): launched early, beside the CTAs of the kernel in front, several landed on one SM while
+// others stayed idle (37 against 19 us in the 9B shape's schedule of 32 positions).
+__device__ __forceinline__ float fold(float a, float b, int s, bool up) {    // lanes with bit s clear: a + a', set: b + b' (a', b' of lane ^ s)
+    return __fadd_rn(up ? b : a, __shfl_xor_sync(0xFFFFFFFFu, up ? a : b, s));
+}
+__global__ void __launch_bounds__(256) k_gdn_seq(bnk::GdnSeq a, int n) {
     extern __shared__ float dyn[];                 // [n][256]: q then k; [n][32] v; [n][2] gates
     float *sv = dyn + n * 256, *sg = sv + n * 32;
     const int h = blockIdx.x >> 2, q4 = blockIdx.x & 3, hq = h % a.qk_heads, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    float S[4][4];                                 // (the kernel in front writes no state)
+    float *Sr = a.state + (size_t(h) * 128 + q4 * 32 + warp * 4) * 128 + lane;
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    float S[2][4];
-    float *Sr = a.state + (size_t(h) * 128 + q4 * 32 + warp * 2) * 128 + lane;
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
+    for (int r = 0; r < 4; ++r)
 #pragma unroll
         for (int e = 0; e < 4; ++e) S[r][e] = Sr[r * 128 + 32 * e];
-    for (int i = tid; i < n * 64; i += 512) {
+    for (int i = tid; i < n * 64; i += 256) {
         const int c = i >> 6, d = (i & 63) * 4;
         const float *src = bnk::colp(a.qk, c * a.stride) + ((d < 128 ? 0 : a.qk_heads) + hq) * 128 + (d & 127);
         *reinterpret_cast<float4 *>(dyn + c * 256 + d) = *reinterpret_cast<const float4 *>(src);
     }
-    for (int i = tid; i < n * 32; i += 512) sv[i] = bnk::colp(a.v, (i >> 5) * a.stride)[h * 128 + q4 * 32 + (i & 31)];
+    for (int i = tid; i < n * 32; i += 256) sv[i] = bnk::colp(a.v, (i >> 5) * a.stride)[h * 128 + q4 * 32 + (i & 31)];
     if (tid < n) { sg[2 * tid] = bnk::colp(a.eg, tid * a.stride)[h]; sg[2 * tid + 1] = bnk::colp(a.bt, tid * a.stride)[h]; }
     // the taps the next token reads: the last three inputs of every channel, into the buffer of its position's parity (one
     // writer per channel; the kernel before this one has read the old ones)
@@ -107,8 +117,8 @@ __global__ void __launch_bounds__(512) k_gdn_seq(bnk::GdnSeq a, int n) {
         const float *rd = (p0 & 1) ? a.hist1 : a.hist0;
         float *wr = ((p0 + n) & 1) ? a.hist1 : a.hist0;
         const int cnt = 32 + (h < a.qk_heads && q4 == 0 ? 256 : 0);
-        if (tid < cnt) {
-            const int ch = tid < 32 ? 2 * a.qk_heads * 128 + h * 128 + q4 * 32 + tid : (tid - 32 < 128 ? h * 128 + tid - 32 : a.qk_heads * 128 + h * 128 + tid - 160);
+        for (int j = tid; j < cnt; j += 256) {
+            const int ch = j < 32 ? 2 * a.qk_heads * 128 + h * 128 + q4 * 32 + j : (j - 32 < 128 ? h * 128 + j - 32 : a.qk_heads * 128 + h * 128 + j - 160);
             float t[3];
 #pragma unroll
             for (int i = 0; i < 3; ++i) { const int c = n - 3 + i; t[i] = c < 0 ? rd[3 * size_t(ch) + 3 + c] : bnk::colp(a.qkv, c * a.stride)[ch]; }
@@ -117,35 +127,35 @@ __global__ void __launch_bounds__(512) k_gdn_seq(bnk::GdnSeq a, int n) {
         }
     }
     __syncthreads();
-    float ov[2] = {0.0f, 0.0f};                    // this lane's part of the previous position's outputs
+    float ov[4] = {0.0f, 0.0f, 0.0f, 0.0f};        // this lane's part of the previous position's outputs
+    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
     for (int c = 0; c <= n; ++c) {
-        float k[4], q[4], pr[2] = {0.0f, 0.0f};
+        float k[4], q[4], pr[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         if (c < n) {
             const float *qk = dyn + c * 256 + lane;
             const float eg = sg[2 * c];
 #pragma unroll
             for (int e = 0; e < 4; ++e) { q[e] = qk[32 * e]; k[e] = qk[128 + 32 * e]; }
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
+            for (int r = 0; r < 4; ++r) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) S[r][e] = __fmul_rn(S[r][e], eg);
                 pr[r] = __fadd_rn(__fadd_rn(__fmul_rn(S[r][0], k[0]), __fmul_rn(S[r][2], k[2])), __fadd_rn(__fmul_rn(S[r][1], k[1]), __fmul_rn(S[r][3], k[3])));
             }
         }
+        // lanes 0..15: predictions, 16..31: outputs; within them bit 3 and bit 2 name the row
+        float x[4];
 #pragma unroll
-        for (int s = 16; s > 0; s >>= 1) {         // four trees side by side
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                ov[r] = __fadd_rn(ov[r], __shfl_xor_sync(0xFFFFFFFFu, ov[r], s));
-                pr[r] = __fadd_rn(pr[r], __shfl_xor_sync(0xFFFFFFFFu, pr[r], s));
-            }
-        }
-        if (c && lane < 2) bnk::colp(a.o, (c - 1) * a.stride)[h * 128 + q4 * 32 + warp * 2 + lane] = __fmul_rn(lane ? ov[1] : ov[0], a.scale);
+        for (int r = 0; r < 4; ++r) x[r] = fold(pr[r], ov[r], 16, b4);
+        float t = fold(fold(x[0], x[1], 8, b3), fold(x[2], x[3], 8, b3), 4, b2);
+        t = __fadd_rn(t, __shfl_xor_sync(0xFFFFFFFFu, t, 2));
+        t = __fadd_rn(t, __shfl_xor_sync(0xFFFFFFFFu, t, 1));
+        if (c && (lane & 19) == 16) bnk::colp(a.o, (c - 1) * a.stride)[h * 128 + q4 * 32 + warp * 4 + ((lane >> 3) & 1) + ((lane >> 1) & 2)] = __fmul_rn(t, a.scale);
         if (c < n) {
             const float bt = sg[2 * c + 1];
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                const float u = __fmul_rn(bt, __fsub_rn(sv[c * 32 + warp * 2 + r], pr[r]));
+            for (int r = 0; r < 4; ++r) {
+                const float u = __fmul_rn(bt, __fsub_rn(sv[c * 32 + warp * 4 + r], __shfl_sync(0xFFFFFFFFu, t, (r & 1) * 8 + (r >> 1) * 4)));
 #pragma unroll
                 for (int e = 0; e < 4; ++e) S[r][e] = fmaf(k[e], u, S[r][e]);
                 ov[r] = __fadd_rn(__fadd_rn(__fmul_rn(S[r][0], q[0]), __fmul_rn(S[r][2], q[2])), __fadd_rn(__fmul_rn(S[r][1], q[1]), __fmul_rn(S[r][3], q[3])));
@@ -153,7 +163,7 @@ __global__ void __launch_bounds__(512) k_gdn_seq(bnk::GdnSeq a, int n) {
         }
     }
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
+    for (int r = 0; r < 4; ++r)
 #pragma unroll
         for (int e = 0; e < 4; ++e) Sr[r * 128 + 32 * e] = S[r][e];
 }
@@ -184,8 +194,10 @@ __global__ void __launch_bounds__(256) k_gdn_seq_post(bnk::GdnSeq a, const float
 namespace bnk {
 
 void gdn_sequence(cudaStream_t st, const GdnSeq &a, int n, const float *z, const float *ssm_norm, float eps, float *y) {
-    launch(k_gdn_seq_pre, dim3(a.heads, (n + PP - 1) / PP), dim3(512), 0, st, a, n);
-    launch(k_gdn_seq, dim3(a.heads * 4), dim3(512), size_t(n) * 290 * 4, st, a, n);       // at most 32 positions: 37 KB
+    static bool attr = false;
+    if (!attr) { cudaFuncSetAttribute(k_gdn_seq, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 << 10); attr = true; }
+    launch(k_gdn_seq_pre, dim3(a.heads * 2, (n + PP - 1) / PP), dim3(256), 0, st, a, n);
+    launch(k_gdn_seq, dim3(a.heads * 4), dim3(256), 116 << 10, st, a, n);                 // at most 32 positions: 37 KB; 116: one CTA per SM
     launch(k_gdn_seq_post, dim3((a.heads + 7) / 8, n), dim3(256), 0, st, a, z, ssm_norm, eps, y);
 }
 
