@@ -79,9 +79,12 @@ struct Q2GemmArgs {
     const float *resid; size_t resid_stride;       // optional: out = sum + resid (may alias out)
     Q2Next next;
     int *err;
-    Q2Share share; int kc, tiles;                  // filled in by the launch
+    int kc, tiles;                                 // filled in by the launch;
+    int early;                                     // the weights are constant: they may be read before the launch in front ends
+    Q2Share share;                                 // filled in by the launch: the CTAs' shares of the row tiles
 };
 cudaError_t launch_q2_gemm(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl);
+cudaError_t launch_q2_gemm_wide(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl);      // 17 to 32 columns (q2_gemm_wide.cu)
 
 #ifdef __CUDACC__
 __device__ __forceinline__ void q2_prefetch(const uint8_t *p, int bytes) {
