@@ -264,10 +264,38 @@ __global__ void __launch_bounds__(256) k_attn_scores_any(AttnDims a, int gqa, At
 // inside it; the last seven, over 128 sums per head, are evaluated by every warp that needs the total (k_attn_pv): no barrier
 // between CTAs (a cluster barrier or an arrival counter here cost 1.5 us). The exponentials of a virtual thread's next eight
 // keys are evaluated by eight real threads and added in order from shared memory.
+// With several columns one CTA per head and column is enough to fill the GPU, and a virtual thread is a real one (PARTS = 1):
+// 32 columns of a short cache are 512 CTAs then instead of 4096 with a few keys each (21 -> 6 us).
 constexpr int EXPSUM_PARTS = 8;
+template <int PARTS>
 __global__ void __launch_bounds__(1024) k_attn_expsum(AttnDims a, AttnPos where, const float *__restrict__ score, float scale, float *__restrict__ pe,
                                                       float *__restrict__ partial, const unsigned *__restrict__ mxp, Cols cols) {
     { const size_t col = blockIdx.z; where.ptr = colp(where.ptr, col * cols.arena); score = colp(score, col * cols.arena); pe = colp(pe, col * cols.arena); partial = colp(partial, col * cols.arena); mxp = colp(mxp, col * cols.arena); }
+    if (PARTS == 1) {
+        __shared__ float all[1024];
+        const int h = blockIdx.x, t = threadIdx.x;
+        pdl_early();
+        const int nfill = where.get() + 1;
+        const float mx = unord(mxp[h]);
+        const float *sr = score + size_t(h) * a.cap;
+        float *pr = pe + size_t(h) * a.cap;
+        float sum = 0.0f;
+#pragma unroll 2
+        for (int j = t; j < nfill; j += 1024) {
+            const float e = exp_f(__fsub_rn(__fmul_rn(sr[j], scale), mx));
+            pr[j] = e;
+            sum = __fadd_rn(sum, e);
+        }
+        all[t] = sum;
+        __syncthreads();
+        if (t < 128) {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = all[128 * k + t];
+            partial[size_t(h) * 128 + t] = __fadd_rn(__fadd_rn(__fadd_rn(v[0], v[4]), __fadd_rn(v[2], v[6])), __fadd_rn(__fadd_rn(v[1], v[5]), __fadd_rn(v[3], v[7])));
+        }
+        return;
+    }
     __shared__ float ex[2][1024];
     __shared__ float sums[128];
     const int h = blockIdx.x, t = threadIdx.x, i = t & 127, vt = (i >> 4) * 128 + blockIdx.y * 16 + (i & 15), sub = t >> 7;
@@ -420,6 +448,7 @@ __global__ void __launch_bounds__(256 / DPT) k_attn_pv(AttnDims a, AttnPos where
     }
 }
 
+constexpr int COMBINE_FEW = 8;
 // combine the splits ascending, then the sigmoid gate: 32 outputs per CTA, whose partials come in with all threads at once and
 // are added in order from shared memory (16 CTAs walking them in batches of 64 loads took 9 us for 64 splits, 24 us for 256).
 // Clears the row maxima again: the kept query may attend once more, over other positions.
@@ -446,6 +475,27 @@ __global__ void __launch_bounds__(256) k_attn_combine(AttnDims a, AttnPos where,
         for (int u = 0; u < 8; ++u) acc = __fadd_rn(acc, v[u]);
     }
     for (; s < used; ++s) acc = __fadd_rn(acc, sp[s][lane]);
+    if (pregate) pregate[i] = acc;
+    gated[i] = __fmul_rn(acc, gt);
+    if (i % a.head_dim == 0) mx[i / a.head_dim] = 0u;
+}
+
+// the same for few splits and several columns: a thread per output (32 columns x 8 splits: 512 CTAs instead of 4096, 8 -> 4 us)
+__global__ void __launch_bounds__(256) k_attn_combine_few(AttnDims a, AttnPos where, const float *__restrict__ part, int splits,
+                                                          const float *__restrict__ gate, float *__restrict__ pregate, float *__restrict__ gated,
+                                                          unsigned *__restrict__ mx, Cols cols) {
+    { const size_t col = blockIdx.z; part = colp(part, col * cols.arena); where.ptr = colp(where.ptr, col * cols.arena); gate = colp(gate, col * cols.arena); pregate = colp(pregate, col * cols.arena); gated = colp(gated, col * cols.arena); mx = colp(mx, col * cols.arena); }
+    const int i = blockIdx.x * 256 + threadIdx.x, n = a.n_head * a.head_dim;
+    pdl_early();
+    if (i >= n) return;
+    const int nfill = where.get() + 1, per = (nfill + splits - 1) / splits, used = (nfill + per - 1) / per;      // splits with keys
+    const float gt = __fdiv_rn(1.0f, __fadd_rn(1.0f, exp_f(-gate[i])));
+    float v[COMBINE_FEW];
+#pragma unroll
+    for (int s = 0; s < COMBINE_FEW; ++s) v[s] = s < used ? part[size_t(s) * n + i] : 0.0f;
+    float acc = v[0];
+#pragma unroll
+    for (int s = 1; s < COMBINE_FEW; ++s) if (s < used) acc = __fadd_rn(acc, v[s]);
     if (pregate) pregate[i] = acc;
     gated[i] = __fmul_rn(acc, gt);
     if (i % a.head_dim == 0) mx[i / a.head_dim] = 0u;
@@ -499,12 +549,17 @@ void attn_decode(cudaStream_t st, AttnDims a, const float *q16f, const float *ga
         if (a.k_mode == 1) launch(k_attn_scores_any<1>, sg, dim3(256), 0, st, a, gqa, where, q16f, kv, score, scale, mx, cols);
         else launch(k_attn_scores_any<0>, sg, dim3(256), 0, st, a, gqa, where, q16f, kv, score, scale, mx, cols);
     }
-    launch(k_attn_expsum, dim3(a.n_head, EXPSUM_PARTS, cols.z()), dim3(1024), 0, st, a, where, score, scale, p16f, esum, mx, cols);
+    // eight CTAs per head while all of them are resident at once (two per SM)
+    if (a.n_head * EXPSUM_PARTS * cols.z() <= 296) launch(k_attn_expsum<EXPSUM_PARTS>, dim3(a.n_head, EXPSUM_PARTS, cols.z()), dim3(1024), 0, st, a, where, score, scale, p16f, esum, mx, cols);
+    else launch(k_attn_expsum<1>, dim3(a.n_head, 1, cols.z()), dim3(1024), 0, st, a, where, score, scale, p16f, esum, mx, cols);
     if (gqa == 4) pv_any<4>(st, a, where, p16f, esum, kv, splits, pv_part, cols);
     else if (gqa == 1) pv_any<1>(st, a, where, p16f, esum, kv, splits, pv_part, cols);
     else if (gqa == 2) pv_any<2>(st, a, where, p16f, esum, kv, splits, pv_part, cols);
     else pv_any<8>(st, a, where, p16f, esum, kv, splits, pv_part, cols);
-    launch(k_attn_combine, dim3(a.n_head * a.head_dim / 32, 1, cols.z()), dim3(256), 0, st, a, where, pv_part, splits, gate, pregate, gated, mx, cols);
+    if (splits <= COMBINE_FEW && cols.z() > 1)
+        launch(k_attn_combine_few, dim3((a.n_head * a.head_dim + 255) / 256, 1, cols.z()), dim3(256), 0, st, a, where, pv_part, splits, gate, pregate, gated, mx, cols);
+    else
+        launch(k_attn_combine, dim3(a.n_head * a.head_dim / 32, 1, cols.z()), dim3(256), 0, st, a, where, pv_part, splits, gate, pregate, gated, mx, cols);
 }
 
 }  // namespace bnk
