@@ -545,7 +545,7 @@ void enqueue_batch(bn_model *m, int ncol, bool one_sequence = false) {
     auto gemm = [&](const uint8_t *W, int M, int K, const uint8_t *img, float *out, const float *resid, const bnk::Q2Next &next, bool swiglu = false) {
         bnk::Q2GemmArgs a = {};
         a.W = W; a.M = M; a.K = K; a.swiglu = swiglu; a.image = img; a.ncol = ncol; a.out = out; a.out_stride = AS;
-        a.resid = resid; a.resid_stride = AS; a.next = next; a.err = m->ctx->err_dev; a.early = 1;
+        a.resid = resid; a.resid_stride = AS; a.next = next; a.err = m->ctx->err_dev;
         cudaError_t e = bnk::launch_q2_gemm(st, m->ctx->sm_count, a, m->use_pdl);
         if (e != cudaSuccess && m->launch_err == cudaSuccess) m->launch_err = e;
     };
@@ -1175,7 +1175,7 @@ int bn_model_head_batch(bn_model *m, int ncol, const bn_buf *in, size_t in_off, 
     bnk::prep_cols(st, p);
     const int rows = m->head_r1 - m->head_r0;
     bnk::Q2GemmArgs a = {};
-    a.W = m->q2_shard; a.M = rows; a.K = h.hidden; a.image = m->IMG_HD; a.ncol = ncol; a.out = m->LOGITS; a.out_stride = AS; a.err = m->ctx->err_dev; a.early = 1;
+    a.W = m->q2_shard; a.M = rows; a.K = h.hidden; a.image = m->IMG_HD; a.ncol = ncol; a.out = m->LOGITS; a.out_stride = AS; a.err = m->ctx->err_dev;
     cudaError_t e = bnk::launch_q2_gemm(st, m->ctx->sm_count, a, m->use_pdl);
     if (e != cudaSuccess) return bn_cuda_fail(e, "bn_model_head_batch");
     bnk::argmax_first(st, m->LOGITS, rows, m->NEXT, m->AMV, m->AMI, cols, m->CAND, m->head_r0);

@@ -80,7 +80,6 @@ struct Q2GemmArgs {
     Q2Next next;
     int *err;
     int kc, tiles;                                 // filled in by the launch;
-    int early;                                     // the weights are constant: they may be read before the launch in front ends
     Q2Share share;                                 // filled in by the launch: the CTAs' shares of the row tiles
 };
 cudaError_t launch_q2_gemm(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl);

@@ -107,7 +107,6 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm_wide(const Q2GemmArgs a, cons
             if (++w_slot == sp.wslots) { w_slot = 0; w_phase ^= 1; }
             if (++w_i == gs) { w_i = 0; ++w_pass; }
         };
-        if (a.early) for (int u = 0; u < min(sp.wslots, groups); ++u) weights();
         asm volatile("griddepcontrol.wait;" ::: "memory");
         int slot = 0, phase = 1;
         for (int u = 0, i = 0; u < groups; ++u) {
