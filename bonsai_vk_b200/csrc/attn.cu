@@ -505,9 +505,7 @@ template <int GQA, int DPT, int VMODE>
 void pv(cudaStream_t st, AttnDims a, AttnPos where, const float *pe, const float *partial, KvLayer kv, int splits, float *part, Cols cols) {
     constexpr int TILE_BYTES = PV_TILE * (VMODE == 0 ? 256 + 16 : 512);
     const size_t smem = 2 * TILE_BYTES + size_t(GQA) * ((a.cap + splits - 1) / splits) * 4;
-    static size_t set = 48 << 10;
-    if (smem > set) { cudaFuncSetAttribute(k_attn_pv<GQA, DPT, VMODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)); set = smem; }
-    launch(k_attn_pv<GQA, DPT, VMODE>, dim3(a.n_kv, splits, cols.z()), dim3(256 / DPT), smem, st, a, where, pe, partial, kv, splits, part, -0.0f, cols);
+    launch_spread<k_attn_pv<GQA, DPT, VMODE>>(dim3(a.n_kv, splits, cols.z()), dim3(256 / DPT), smem, st, a, where, pe, partial, kv, splits, part, -0.0f, cols);
 }
 template <int GQA>
 void pv_any(cudaStream_t st, AttnDims a, AttnPos where, const float *pe, const float *partial, KvLayer kv, int splits, float *part, Cols cols) {
@@ -524,7 +522,10 @@ namespace bnk {
 void attn_prep(cudaStream_t st, AttnDims a, const float *qg, const float *kin, const float *vin, const float *qn_w,
                const float *kn_w, AttnPos where, KvLayer kv, float *q16f, float *gate, float *esum, Cols cols, int tokens) {
     unsigned *mx = reinterpret_cast<unsigned *>(esum + size_t(a.n_head) * 128);
-    launch(k_attn_prep, dim3(a.n_head + a.n_kv, 1, cols.n > 0 ? cols.z() : tokens), dim3(256), 0, st, a, where, qg, kin, vin, qn_w, kn_w, kv, q16f, gate, mx, cols);
+    const dim3 grid(a.n_head + a.n_kv, 1, cols.n > 0 ? cols.z() : tokens);
+    // (one token's few CTAs run beside the projection in front of them)
+    if (grid.z == 1) launch(k_attn_prep, grid, dim3(256), 0, st, a, where, qg, kin, vin, qn_w, kn_w, kv, q16f, gate, mx, cols);
+    else launch_spread<k_attn_prep>(grid, dim3(256), 0, st, a, where, qg, kin, vin, qn_w, kn_w, kv, q16f, gate, mx, cols);
 }
 void attn_decode(cudaStream_t st, AttnDims a, const float *q16f, const float *gate, AttnPos where, KvLayer kv,
                  float *score, float *p16f, float *esum, float *pv_part, int splits, float *pregate, float *gated, Cols cols) {
@@ -542,24 +543,24 @@ void attn_decode(cudaStream_t st, AttnDims a, const float *q16f, const float *ga
         int rounds = int((ctas + 295) / 296);
         rounds = rounds < 1 ? 1 : (rounds > 8 ? 8 : rounds);
         const dim3 sg(((a.cap + 63) / 64 + rounds - 1) / rounds, a.n_kv, cols.z());
-        if (a.k_mode == 1) launch(k_attn_scores4<1>, sg, dim3(256), 0, st, a, where, q16f, kv, score, scale, mx, cols);
-        else launch(k_attn_scores4<0>, sg, dim3(256), 0, st, a, where, q16f, kv, score, scale, mx, cols);
+        if (a.k_mode == 1) launch_spread<k_attn_scores4<1>>(sg, dim3(256), 0, st, a, where, q16f, kv, score, scale, mx, cols);
+        else launch_spread<k_attn_scores4<0>>(sg, dim3(256), 0, st, a, where, q16f, kv, score, scale, mx, cols);
     } else {
         const dim3 sg((a.cap + 63) / 64, a.n_kv, cols.z());
-        if (a.k_mode == 1) launch(k_attn_scores_any<1>, sg, dim3(256), 0, st, a, gqa, where, q16f, kv, score, scale, mx, cols);
-        else launch(k_attn_scores_any<0>, sg, dim3(256), 0, st, a, gqa, where, q16f, kv, score, scale, mx, cols);
+        if (a.k_mode == 1) launch_spread<k_attn_scores_any<1>>(sg, dim3(256), 0, st, a, gqa, where, q16f, kv, score, scale, mx, cols);
+        else launch_spread<k_attn_scores_any<0>>(sg, dim3(256), 0, st, a, gqa, where, q16f, kv, score, scale, mx, cols);
     }
     // eight CTAs per head while all of them are resident at once (two per SM)
-    if (a.n_head * EXPSUM_PARTS * cols.z() <= 296) launch(k_attn_expsum<EXPSUM_PARTS>, dim3(a.n_head, EXPSUM_PARTS, cols.z()), dim3(1024), 0, st, a, where, score, scale, p16f, esum, mx, cols);
-    else launch(k_attn_expsum<1>, dim3(a.n_head, 1, cols.z()), dim3(1024), 0, st, a, where, score, scale, p16f, esum, mx, cols);
+    if (a.n_head * EXPSUM_PARTS * cols.z() <= 296) launch_spread<k_attn_expsum<EXPSUM_PARTS>>(dim3(a.n_head, EXPSUM_PARTS, cols.z()), dim3(1024), 0, st, a, where, score, scale, p16f, esum, mx, cols);
+    else launch_spread<k_attn_expsum<1>>(dim3(a.n_head, 1, cols.z()), dim3(1024), 0, st, a, where, score, scale, p16f, esum, mx, cols);
     if (gqa == 4) pv_any<4>(st, a, where, p16f, esum, kv, splits, pv_part, cols);
     else if (gqa == 1) pv_any<1>(st, a, where, p16f, esum, kv, splits, pv_part, cols);
     else if (gqa == 2) pv_any<2>(st, a, where, p16f, esum, kv, splits, pv_part, cols);
     else pv_any<8>(st, a, where, p16f, esum, kv, splits, pv_part, cols);
     if (splits <= COMBINE_FEW && cols.z() > 1)
-        launch(k_attn_combine_few, dim3((a.n_head * a.head_dim + 255) / 256, 1, cols.z()), dim3(256), 0, st, a, where, pv_part, splits, gate, pregate, gated, mx, cols);
+        launch_spread<k_attn_combine_few>(dim3((a.n_head * a.head_dim + 255) / 256, 1, cols.z()), dim3(256), 0, st, a, where, pv_part, splits, gate, pregate, gated, mx, cols);
     else
-        launch(k_attn_combine, dim3(a.n_head * a.head_dim / 32, 1, cols.z()), dim3(256), 0, st, a, where, pv_part, splits, gate, pregate, gated, mx, cols);
+        launch_spread<k_attn_combine>(dim3(a.n_head * a.head_dim / 32, 1, cols.z()), dim3(256), 0, st, a, where, pv_part, splits, gate, pregate, gated, mx, cols);
 }
 
 }  // namespace bnk

@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(256) k_gdn_seq_pre(bnk::GdnSeq a, int n) {
 // between; the output trees of one position run beside the prediction trees of the next, eight trees on nine shuffles: a level's
 // two values change hands between the lanes that go on with one and those that go on with the other (the shuffles' throughput
 // bounds the loop: with five per tree and two rows per warp 1000 cycles a position, now 400).
-// One CTA per SM (its shared memory): launched early, beside the CTAs of the kernel in front, several landed on one SM while
+// One CTA per SM (launch_spread): launched early, beside the CTAs of the kernel in front, several landed on one SM while
 // others stayed idle (37 against 19 us in the 9B shape's schedule of 32 positions).
 __device__ __forceinline__ float fold(float a, float b, int s, bool up) {    // lanes with bit s clear: a + a', set: b + b' (a', b' of lane ^ s)
     return __fadd_rn(up ? b : a, __shfl_xor_sync(0xFFFFFFFFu, up ? a : b, s));
@@ -194,11 +194,9 @@ __global__ void __launch_bounds__(256) k_gdn_seq_post(bnk::GdnSeq a, const float
 namespace bnk {
 
 void gdn_sequence(cudaStream_t st, const GdnSeq &a, int n, const float *z, const float *ssm_norm, float eps, float *y) {
-    static bool attr = false;
-    if (!attr) { cudaFuncSetAttribute(k_gdn_seq, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 << 10); attr = true; }
-    launch(k_gdn_seq_pre, dim3(a.heads * 2, (n + PP - 1) / PP), dim3(256), 0, st, a, n);
-    launch(k_gdn_seq, dim3(a.heads * 4), dim3(256), 116 << 10, st, a, n);                 // at most 32 positions: 37 KB; 116: one CTA per SM
-    launch(k_gdn_seq_post, dim3((a.heads + 7) / 8, n), dim3(256), 0, st, a, z, ssm_norm, eps, y);
+    launch_spread<k_gdn_seq_pre>(dim3(a.heads * 2, (n + PP - 1) / PP), dim3(256), 0, st, a, n);
+    launch_spread<k_gdn_seq>(dim3(a.heads * 4), dim3(256), size_t(n) * 290 * 4, st, a, n);       // at most 32 positions: 37 KB
+    launch_spread<k_gdn_seq_post>(dim3((a.heads + 7) / 8, n), dim3(256), 0, st, a, z, ssm_norm, eps, y);
 }
 
 }  // namespace bnk

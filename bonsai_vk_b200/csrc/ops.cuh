@@ -1,5 +1,6 @@
 // ops.cuh - internal launch helpers shared between the op-level entry points and the token schedule.
 #pragma once
+#include <algorithm>
 #include "common.cuh"
 
 #include <type_traits>
@@ -22,6 +23,21 @@ inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
     cfg.numAttrs = g_pdl ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
     BN_COUNT(1);
+}
+// The same for a grid of at most a few CTAs per SM: as much unused shared memory as keeps them evenly spread. Launched while the
+// kernel in front is finishing, small CTAs would otherwise crowd on the first SMs that become free while others stay idle.
+template <auto K, typename... Args>
+inline void launch_spread(dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+    constexpr int SM = 233472, RESERVED = 1024, MAX_CTA = 232448;         // shared memory of an SM, of it per CTA, a CTA's most
+    static const int fixed = [] {                                          // the kernel's static shared memory
+        cudaFuncAttributes fa;
+        if (cudaFuncGetAttributes(&fa, K) != cudaSuccess) return MAX_CTA;
+        cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_CTA - int(fa.sharedSizeBytes));
+        return int(fa.sharedSizeBytes);
+    }();
+    const int per = int((size_t(grid.x) * grid.y * grid.z + 147) / 148), apart = SM / (per + 1) - RESERVED - fixed + 256;
+    if (per <= 4 && apart > int(smem)) smem = size_t(apart);
+    launch(K, grid, block, smem, st, args...);
 }
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_sync() {

@@ -8,9 +8,6 @@
 namespace {
 using namespace bnk;
 constexpr int NT = 512;
-// Unused shared memory that keeps a second CTA off the SM: launched while the projection in front of it is finishing, several
-// CTAs would share the first SMs that become free.
-constexpr int ONE_PER_SM = 100 << 10;
 constexpr int IMG_COL = 160;                   // image bytes per column and block: 128 int8 codes + 4 x (fp32 d, fp32 -s)
 
 __device__ __forceinline__ void load8(const float *p, f32pair (&v)[4]) {
@@ -124,9 +121,7 @@ namespace bnk {
 
 void prep_cols(cudaStream_t st, const PrepArgs &a) {
     const int hb = a.signs ? a.hat_block : 16;
-    static bool attr = false;
-    if (!attr) { cudaFuncSetAttribute(k_prep_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, ONE_PER_SM); attr = true; }
-    launch(k_prep_cols, dim3((a.K + 4095) / 4096, gemm_padded_cols(a.ncol)), dim3(NT), ONE_PER_SM, st, a, 31 - __builtin_clz(unsigned(hb)), 1.0f / sqrtf(float(hb)),
+    launch_spread<k_prep_cols>(dim3((a.K + 4095) / 4096, gemm_padded_cols(a.ncol)), dim3(NT), 0, st, a, 31 - __builtin_clz(unsigned(hb)), 1.0f / sqrtf(float(hb)),
            (a.K & (a.K - 1)) == 0 ? 1.0f / float(a.K) : 0.0f, gemm_padded_cols(a.ncol));
 }
 
