@@ -566,7 +566,9 @@ void enqueue_batch(bn_model *m, int ncol, bool one_sequence = false) {
             gemm(L.q2_out, h.hidden, QD, m->IMG_H, m->RES, m->RES, q2_next(L.q2_ffn, 2 * h.ffn, h.hidden, L.post_norm));
         } else {
             prep(bnk::PREP_NORM, m->RES, L.attn_norm, m->signs, h.hidden, m->IMG_H, m->G + 48);
-            gemm(L.q2_in, C + IN, h.hidden, m->IMG_H, m->QKV, nullptr, q2_next(L.q2_out, h.hidden, IN, nullptr));
+            bnk::Q2Next next = q2_next(L.q2_out, h.hidden, IN, nullptr);
+            next.state = gdn_state_of(m, L.idx); next.cols = one_sequence ? 1 : ncol; next.col_bytes = NH * D * D * 4; next.col_stride = cols.gdn;
+            gemm(L.q2_in, C + IN, h.hidden, m->IMG_H, m->QKV, nullptr, next);
             const bnk::GdnDims gd{NH, NQ, D};
             if (one_sequence) {
                 bnk::GdnSeq s = {};

@@ -326,19 +326,40 @@ __global__ void __launch_bounds__(512, MINB) k_gdn_core(int heads, int qk_heads,
     }
     __syncthreads();
     const float eg = exp_f(sgb[0]), bt = sgb[1];
+    // four rows at a time; their trees share six shuffles (a level's two values change hands between the lanes that go on with
+    // one and those that go on with the other), as the shuffles' throughput bounds this part
+    const bool b4 = lane & 16, b3 = lane & 8;
+    auto trees4 = [&](const float (&v)[4]) {           // lane l: the sum of row (l >> 4) + 2 * (l >> 3 & 1)
+        const float x = __fadd_rn(b4 ? v[1] : v[0], __shfl_xor_sync(0xFFFFFFFFu, b4 ? v[0] : v[1], 16));
+        const float y = __fadd_rn(b4 ? v[3] : v[2], __shfl_xor_sync(0xFFFFFFFFu, b4 ? v[2] : v[3], 16));
+        float s = __fadd_rn(b3 ? y : x, __shfl_xor_sync(0xFFFFFFFFu, b3 ? x : y, 8));
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const int j = warp * 8 + r;
-        float *Sr = state + (size_t(h) * 128 + j) * 128;
-        float s[4];
+        for (int d = 4; d > 0; d >>= 1) s = __fadd_rn(s, __shfl_xor_sync(0xFFFFFFFFu, s, d));
+        return s;
+    };
 #pragma unroll
-        for (int e = 0; e < 4; ++e) s[e] = __fmul_rn(S[r][e], eg);
-        const float pred = warp_tree128(__fmul_rn(s[0], kk[0]), __fmul_rn(s[1], kk[1]), __fmul_rn(s[2], kk[2]), __fmul_rn(s[3], kk[3]));
-        const float u = __fmul_rn(bt, __fsub_rn(sv[j], pred));
+    for (int r0 = 0; r0 < 8; r0 += 4) {
+        float p[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) { s[e] = fmaf(kk[e], u, s[e]); Sr[lane + 32 * e] = s[e]; }
-        const float ov = warp_tree128(__fmul_rn(s[0], qq[0]), __fmul_rn(s[1], qq[1]), __fmul_rn(s[2], qq[2]), __fmul_rn(s[3], qq[3]));
-        if (lane == 0) so[j] = __fmul_rn(ov, scale);
+        for (int r = 0; r < 4; ++r) {
+            float (&s)[4] = S[r0 + r];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[e] = __fmul_rn(s[e], eg);
+            p[r] = __fadd_rn(__fadd_rn(__fmul_rn(s[0], kk[0]), __fmul_rn(s[2], kk[2])), __fadd_rn(__fmul_rn(s[1], kk[1]), __fmul_rn(s[3], kk[3])));
+        }
+        const float pred = trees4(p);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int j = warp * 8 + r0 + r;
+            float *Sr = state + (size_t(h) * 128 + j) * 128;
+            float (&s)[4] = S[r0 + r];
+            const float u = __fmul_rn(bt, __fsub_rn(sv[j], __shfl_sync(0xFFFFFFFFu, pred, (r & 1) * 16 + (r >> 1) * 8)));
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { s[e] = fmaf(kk[e], u, s[e]); Sr[lane + 32 * e] = s[e]; }
+            p[r] = __fadd_rn(__fadd_rn(__fmul_rn(s[0], qq[0]), __fmul_rn(s[2], qq[2])), __fadd_rn(__fmul_rn(s[1], qq[1]), __fmul_rn(s[3], qq[3])));
+        }
+        const float ov = trees4(p);
+        if (!(lane & 7)) so[warp * 8 + r0 + (lane >> 4) + ((lane >> 3) & 1) * 2] = __fmul_rn(ov, scale);
     }
     __syncthreads();
     if (warp == 0) {

@@ -42,6 +42,10 @@ struct Q2Next {
     const float *w = nullptr;
     int w_bytes = 0;
     Q2Share share = {0, 0};               // filled in by the launch
+    // recurrent state that the mixer behind this projection reads: `cols` pieces, any CTA any part of them
+    const float *state = nullptr;
+    int cols = 0, col_bytes = 0;
+    size_t col_stride = 0;                // bytes
 };
 struct Q2Args {
     const uint8_t *W;            // two-bit tiles
@@ -89,13 +93,18 @@ cudaError_t launch_q2_gemm_wide(cudaStream_t st, int sm_count, Q2GemmArgs a, boo
 __device__ __forceinline__ void q2_prefetch(const uint8_t *p, int bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
-// one thread: the share of the next projection's weights that CTA `cta`'s successor reads, and its norm weights, towards L2
-__device__ __forceinline__ void q2_prefetch_next(const Q2Next &n, int cta) {
+// thread `part` of `parts`: the share of the next projection's weights that CTA `cta`'s successor reads, and its norm weights, and
+// this CTA's part of the state, towards L2 (several threads, because a prefetch costs the one that asks for it some 70 cycles)
+__device__ __forceinline__ void q2_prefetch_next(const Q2Next &n, int cta, int part, int parts) {
+    for (int k = cta + part * int(gridDim.x), per = (n.col_bytes + 16383) >> 14; k < n.cols * per; k += parts * int(gridDim.x)) {
+        const int o = k % per * 16384;
+        q2_prefetch(reinterpret_cast<const uint8_t *>(n.state) + size_t(k / per) * n.col_stride + o, min(16384, n.col_bytes - o));
+    }
     if (!n.W) return;
     const uint8_t *src = n.W + size_t(cta * n.share.q + min(cta, n.share.r)) * n.unit_bytes;
     const int bytes = min((n.share.q + (cta < n.share.r)) * n.unit_bytes, n.max_bytes);
-    for (int o = 0; o < bytes; o += 16384) q2_prefetch(src + o, min(16384, bytes - o));
-    if (cta == 0 && n.w) for (int o = 0; o < n.w_bytes; o += 16384) q2_prefetch(reinterpret_cast<const uint8_t *>(n.w) + o, min(16384, n.w_bytes - o));
+    for (int o = part * 16384; o < bytes; o += parts * 16384) q2_prefetch(src + o, min(16384, bytes - o));
+    if (cta == 0 && n.w) for (int o = part * 16384; o < n.w_bytes; o += parts * 16384) q2_prefetch(reinterpret_cast<const uint8_t *>(n.w) + o, min(16384, n.w_bytes - o));
 }
 constexpr int Q2_MAGIC = 0x4B400000;           // bits of 12582912.0f: adding an int |i| < 2^22 gives the bits of 12582912 + i
 

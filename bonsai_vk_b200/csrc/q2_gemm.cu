@@ -68,11 +68,13 @@ __global__ void __launch_bounds__(threads<NCP>(), 1) k_q2_gemm(const Q2GemmArgs 
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars));
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (lane == 0) {
         // this CTA's weights (as far as the previous projection has not fetched them) and the next projection's towards L2
         const uint8_t *own = a.W + size_t(t0) * ng * Q2_PIECE;
         const int bytes = min(nt * ng * Q2_PIECE, Q2_NEXT_BYTES);
-        for (int o = 0; o < bytes; o += 16384) q2_prefetch(own + o, min(16384, bytes - o));
-        q2_prefetch_next(a.next, cta);
+        for (int o = warp * 16384; o < bytes; o += NW * 16384) q2_prefetch(own + o, min(16384, bytes - o));
+        q2_prefetch_next(a.next, cta, warp, NW);
     }
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __syncthreads();

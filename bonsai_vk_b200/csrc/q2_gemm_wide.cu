@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm_wide(const Q2GemmArgs a, cons
             const uint8_t *own = a.W + size_t(t0) * ng * Q2_PIECE;
             const int bytes = min(nt * ng * Q2_PIECE, Q2_NEXT_BYTES);
             for (int o = lane * 16384; o < bytes; o += 32 * 16384) q2_prefetch(own + o, min(16384, bytes - o));
-            if (lane == 0) q2_prefetch_next(a.next, blockIdx.x);
+            if (lane == 0) q2_prefetch_next(a.next, blockIdx.x, 0, 1);
         }
         if (warp != NW || lane) return;
         int w_u = 0, w_i = 0, w_pass = 0, w_slot = 0, w_phase = 1;        // the next group of weights

@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Arg
             }
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             for (int i = 0; i < min(EARLY, slots); ++i) request(i, i);
-            q2_prefetch_next(a.next, cta);
+            q2_prefetch_next(a.next, cta, 0, 1);
         }
         __syncwarp();
         asm volatile("bar.arrive 2, %0;" ::"n"(NT + 32) : "memory");
