@@ -309,8 +309,7 @@ void enqueue_token(bn_model *m, int stop_after, bool want_logits) {
     const bn_hparams &h = m->hp;
     cudaStream_t st = m->ctx->stream;
     if (m->b0 == 0) {
-        bnk::embed_row(st, m->embd, h.hidden, m->TOK, m->X1);
-        bnk::rotate_inv(st, m->X1, m->signs, h.hidden, h.hat_block, m->RES);
+        bnk::embed_rotate(st, m->embd, h.hidden, m->TOK, m->signs, h.hat_block, m->RES);
     }
     for (int b = m->b0; b < m->b1; ++b) {
         const bn_model::Layer &L = m->layers[b];
@@ -550,8 +549,7 @@ void enqueue_batch(bn_model *m, int ncol, bool one_sequence = false) {
         if (e != cudaSuccess && m->launch_err == cudaSuccess) m->launch_err = e;
     };
     if (m->b0 == 0) {
-        bnk::embed_row(st, m->embd, h.hidden, m->TOK, m->X1, cols);
-        bnk::rotate_inv(st, m->X1, m->signs, h.hidden, h.hat_block, m->RES, cols);
+        bnk::embed_rotate(st, m->embd, h.hidden, m->TOK, m->signs, h.hat_block, m->RES, cols);
     }
     for (int b = m->b0; b < m->b1; ++b) {
         const bn_model::Layer &L = m->layers[b];

@@ -6,6 +6,7 @@
 // file is compiled without fused-multiply-add contraction (fmaf is written where one is meant).
 #include "ops.cuh"
 #include "quant.cuh"
+#include "rotate_quant.cuh"
 
 namespace {
 
@@ -61,35 +62,51 @@ __global__ void __launch_bounds__(512) k_rotate_quant(const float *__restrict__ 
     }
 }
 
-__global__ void __launch_bounds__(512) k_rotate_inv(const float *__restrict__ x, const int32_t *__restrict__ signs,
-                                                    int block, float inv, float *__restrict__ y, bnk::Cols cols) {
+// ---- embedding gather (reference addressing: runtime_vk/shaders/gather_rows.comp:12-16) and its inverse rotation ----------------
+// y = s . H(row): one CTA per span of 4096 values and column, eight values per thread, on the transform of the projections'
+// prologue (rotate_quant.cuh). A kernel each, the rotation on one pair of values per thread and stage, took 13 us; this one 3 us.
+__global__ void __launch_bounds__(512) k_embed_rotate(const uint32_t *__restrict__ W, int K, const int *__restrict__ tok_ptr, const int32_t *__restrict__ signs,
+                                                      int log_hb, float inv, float *__restrict__ y, bnk::Cols cols) {
+    __shared__ __align__(16) float xs[bnk::XS8_SPAN];
+    const int t = threadIdx.x, at = blockIdx.x * 4096 + t * 8;
+    int sg[8] = {};
+    if (at < K) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) sg[k] = signs[at + k];
+    }
     bnk::pdl_sync();
-    { const size_t col = blockIdx.z; x = bnk::colp(x, col * cols.arena); y = bnk::colp(y, col * cols.arena); }
-    extern __shared__ float s[];
-    const size_t base = size_t(blockIdx.x) * block;
-    for (int i = threadIdx.x; i < block; i += blockDim.x) s[i] = x[base + i];
-    fwht_smem(s, block, block, inv);
-    for (int i = threadIdx.x; i < block; i += blockDim.x) y[base + i] = __fmul_rn(s[i], float(signs[base + i]));
-}
-
-// ---- embedding gather (reference addressing: runtime_vk/shaders/gather_rows.comp:12-16) ----------
-__global__ void k_embed_row(const uint32_t *__restrict__ W, int K, const int *__restrict__ tok_ptr,
-                            float *__restrict__ out, bnk::Cols cols) {
-    bnk::pdl_sync();
-    { const size_t col = blockIdx.z; tok_ptr = bnk::colp(tok_ptr, col * cols.arena); out = bnk::colp(out, col * cols.arena); }
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= K) return;
-    const int tok = tok_ptr[0];
-    const uint32_t *blk = W + (size_t(tok) * (K / 128) + e / 128) * 7;
-    const int el = e & 127;
-    int byte, t;
-    if (el < 80) { byte = el & 15; t = el >> 4; }
-    else if (el < 120) { byte = 16 + ((el - 80) & 7); t = (el - 80) >> 3; }
-    else { byte = 24 + ((el - 120) & 1); t = (el - 120) >> 1; }
-    uint32_t v = (blk[byte >> 2] >> ((byte & 3) * 8)) & 0xFFu;
-    for (int i = 0; i < t; ++i) v = (v * 3u) & 0xFFu;
-    const int trit = int((v * 3u) >> 8);
-    out[e] = __fmul_rn(float(trit) - 1.0f, half_bits_to_float(blk[6] >> 16));
+    { const size_t col = blockIdx.z; tok_ptr = bnk::colp(tok_ptr, col * cols.arena); y = bnk::colp(y, col * cols.arena); }
+    float e[8] = {};
+    if (at < K) {
+        const uint32_t *blk = W + (size_t(tok_ptr[0]) * (K / 128) + at / 128) * 7;
+        const float d = half_bits_to_float(blk[6] >> 16);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int el = (at & 127) + k;
+            int byte, r;
+            if (el < 80) { byte = el & 15; r = el >> 4; }
+            else if (el < 120) { byte = 16 + ((el - 80) & 7); r = (el - 80) >> 3; }
+            else { byte = 24 + ((el - 120) & 1); r = (el - 120) >> 1; }
+            uint32_t v = (blk[byte >> 2] >> ((byte & 3) * 8)) & 0xFFu;
+            for (int i = 0; i < r; ++i) v = (v * 3u) & 0xFFu;
+            e[k] = __fmul_rn(float(int((v * 3u) >> 8)) - 1.0f, d);
+        }
+    }
+    bnk::f32pair v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = bnk::pair_of(e[2 * k], e[2 * k + 1]);
+    bnk::fwht_pairs8(v, 3);
+    bnk::span_store8(xs, t, v);
+    bnk::fwht_spans(xs, t, 1, log_hb, [] { __syncthreads(); });
+    bnk::span_load8(xs, t, v);
+    if (at < K) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            bnk::split_pair(v[k], e[0], e[1]);
+            y[at + 2 * k] = __fmul_rn(__fmul_rn(e[0], inv), float(sg[2 * k]));
+            y[at + 2 * k + 1] = __fmul_rn(__fmul_rn(e[1], inv), float(sg[2 * k + 1]));
+        }
+    }
 }
 
 // ---- RMS norm (reference: runtime_vk/shaders/rms_norm.comp:60-103) --------------------------------
@@ -404,27 +421,39 @@ __global__ void k_gdn_out(int heads, int qk_heads, const float *__restrict__ o, 
 }
 
 // ---- greedy pick: first maximum (Sampler::pick, runtime_vk/bonsai_forward.h:2568-2570) ----------
+// the warp's largest value, of equal ones the smallest index (any order of comparisons gives the same)
+__device__ __forceinline__ void better_of_warp(float &v, int &i) {
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+        const float w = __shfl_xor_sync(0xFFFFFFFFu, v, s);
+        const int k = __shfl_xor_sync(0xFFFFFFFFu, i, s);
+        if (w > v || (w == v && k < i)) { v = w; i = k; }
+    }
+}
 __global__ void __launch_bounds__(1024) k_argmax_part(const float *__restrict__ x, int n, float *__restrict__ bv,
                                                       int *__restrict__ bi, bnk::Cols cols) {
     bnk::pdl_sync();
     { const size_t col = blockIdx.z; x = bnk::colp(x, col * cols.arena); bv = bnk::colp(bv, col * cols.arena); bi = bnk::colp(bi, col * cols.arena); }
-    __shared__ float sv[1024];
-    __shared__ int si[1024];
+    __shared__ float sv[32];
+    __shared__ int si[32];
     const int t = threadIdx.x;
     float best = -INFINITY; int idx = 0x7FFFFFFF;
-    for (int i = blockIdx.x * 1024 + t; i < n; i += gridDim.x * 1024) {
-        const float v = x[i];
-        if (v > best || (v == best && i < idx)) { best = v; idx = i; }
+    const int step = gridDim.x * 1024;
+    for (int i = blockIdx.x * 1024 + t; i < n; i += 4 * step) {        // four loads at a time
+        float v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = i + k * step < n ? x[i + k * step] : -INFINITY;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) if (i + k * step < n && (v[k] > best || (v[k] == best && i + k * step < idx))) { best = v[k]; idx = i + k * step; }
     }
-    sv[t] = best; si[t] = idx;
-    for (int s = 512; s > 0; s >>= 1) {
-        __syncthreads();
-        if (t < s) {
-            const float v = sv[t + s]; const int i = si[t + s];
-            if (v > sv[t] || (v == sv[t] && i < si[t])) { sv[t] = v; si[t] = i; }
-        }
+    better_of_warp(best, idx);
+    if (!(t & 31)) { sv[t >> 5] = best; si[t >> 5] = idx; }
+    __syncthreads();
+    if (t < 32) {
+        best = sv[t]; idx = si[t];
+        better_of_warp(best, idx);
+        if (t == 0) { bv[blockIdx.x] = best; bi[blockIdx.x] = idx; }
     }
-    if (t == 0) { bv[blockIdx.x] = sv[0]; bi[blockIdx.x] = si[0]; }
 }
 // cand != null (the rows are one shard of the output head, starting at row0): the column's candidate (value, global
 // row or 0x7FFFFFFF when no row qualified) also goes to cand[2 * column], for the pick over all shards
@@ -432,9 +461,14 @@ __global__ void k_argmax_final(const float *__restrict__ bv, const int *__restri
                                float *__restrict__ cand, int row0) {
     bnk::pdl_sync();
     { const size_t col = blockIdx.z; bv = bnk::colp(bv, col * cols.arena); bi = bnk::colp(bi, col * cols.arena); out = bnk::colp(out, col * cols.arena); }
+    float best = -INFINITY; int idx = 0x7FFFFFFF;
+    for (int p = threadIdx.x; p < nparts; p += 32) {
+        const float v = bv[p];
+        const int k = bi[p];
+        if (v > best || (v == best && k < idx)) { best = v; idx = k; }
+    }
+    better_of_warp(best, idx);
     if (threadIdx.x != 0) return;
-    float best = bv[0]; int idx = bi[0];
-    for (int p = 1; p < nparts; ++p) if (bv[p] > best || (bv[p] == best && bi[p] < idx)) { best = bv[p]; idx = bi[p]; }
     // a row of NaN or -inf never satisfies v > best: fall back to index 0 as the scalar loop does
     out[0] = idx == 0x7FFFFFFF ? 0 : idx;
     if (cand) {
@@ -468,11 +502,8 @@ void rotate_quant(cudaStream_t st, const float *x, const int32_t *signs, int n, 
     const int span = block < 128 ? 128 : block;
     launch(k_rotate_quant, dim3(n / span), dim3(512), size_t(span) * 4 + 512, st, x, signs, span, block, inv, y, q81, table);
 }
-void rotate_inv(cudaStream_t st, const float *x, const int32_t *signs, int n, int block, float *y, Cols cols) {
-    launch(k_rotate_inv, dim3(n / block, 1, cols.z()), dim3(512), size_t(block) * 4, st, x, signs, block, 1.0f / sqrtf(float(block)), y, cols); 
-}
-void embed_row(cudaStream_t st, const uint32_t *W, int K, const int *tok_ptr, float *out, Cols cols) {
-    launch(k_embed_row, dim3((K + 255) / 256, 1, cols.z()), dim3(256), 0, st, W, K, tok_ptr, out, cols); 
+void embed_rotate(cudaStream_t st, const uint32_t *W, int K, const int *tok_ptr, const int32_t *signs, int block, float *y, Cols cols) {
+    launch_spread<k_embed_rotate>(dim3((K + 4095) / 4096, 1, cols.z()), dim3(512), 0, st, W, K, tok_ptr, signs, 31 - __builtin_clz(unsigned(block)), 1.0f / sqrtf(float(block)), y, cols);
 }
 void rms_norm(cudaStream_t st, const float *x, const float *w, int rows, int cols, float eps, float *y) {
     launch(k_rms_norm, dim3(rows), dim3(256), 0, st, x, w, cols, eps, y); 

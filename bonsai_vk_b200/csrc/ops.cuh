@@ -76,9 +76,9 @@ cudaError_t ptq_stream(cudaStream_t st, int sm_count, const void *W, int M, int 
 // y may be null when only the pack is wanted). n % block == 0, block = power of two in [128, 4096].
 void rotate_quant(cudaStream_t st, const float *x, const int32_t *signs, int n, int block, float *y, uint32_t *pack);
 // embedding side: y = s . H(x)
-void rotate_inv(cudaStream_t st, const float *x, const int32_t *signs, int n, int block, float *y, Cols cols = {});
 // PTQ1_0 row gather: out[K] = dequantised row `tok` (tok read from tok_ptr[0])
-void embed_row(cudaStream_t st, const uint32_t *W, int K, const int *tok_ptr, float *out, Cols cols = {});
+// y = signs . H(row tok_ptr[0] of the embedding), Hadamard blocks of `block` values
+void embed_rotate(cudaStream_t st, const uint32_t *W, int K, const int *tok_ptr, const int32_t *signs, int block, float *y, Cols cols = {});
 
 void rms_norm(cudaStream_t st, const float *x, const float *w, int rows, int cols, float eps, float *y);
 void add_inplace(cudaStream_t st, float *res, const float *d, int n);       // res = d + res
