@@ -505,7 +505,8 @@ template <int GQA, int DPT, int VMODE>
 void pv(cudaStream_t st, AttnDims a, AttnPos where, const float *pe, const float *partial, KvLayer kv, int splits, float *part, Cols cols) {
     constexpr int TILE_BYTES = PV_TILE * (VMODE == 0 ? 256 + 16 : 512);
     const size_t smem = 2 * TILE_BYTES + size_t(GQA) * ((a.cap + splits - 1) / splits) * 4;
-    launch_spread<k_attn_pv<GQA, DPT, VMODE>>(dim3(a.n_kv, splits, cols.z()), dim3(256 / DPT), smem, st, a, where, pe, partial, kv, splits, part, -0.0f, cols);
+    // (1024 CTAs of two warps at 32 768 positions: seven per SM everywhere instead of up to eleven, 57 -> 49 us a layer)
+    launch_spread<k_attn_pv<GQA, DPT, VMODE>, 8>(dim3(a.n_kv, splits, cols.z()), dim3(256 / DPT), smem, st, a, where, pe, partial, kv, splits, part, -0.0f, cols);
 }
 template <int GQA>
 void pv_any(cudaStream_t st, AttnDims a, AttnPos where, const float *pe, const float *partial, KvLayer kv, int splits, float *part, Cols cols) {

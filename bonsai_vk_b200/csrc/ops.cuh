@@ -26,7 +26,8 @@ inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
 }
 // The same for a grid of at most a few CTAs per SM: as much unused shared memory as keeps them evenly spread. Launched while the
 // kernel in front is finishing, small CTAs would otherwise crowd on the first SMs that become free while others stay idle.
-template <auto K, typename... Args>
+// MOST: CTAs per SM up to which it is done.
+template <auto K, int MOST = 4, typename... Args>
 inline void launch_spread(dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     constexpr int SM = 233472, RESERVED = 1024, MAX_CTA = 232448;         // shared memory of an SM, of it per CTA, a CTA's most
     static const int fixed = [] {                                          // the kernel's static shared memory
@@ -36,7 +37,7 @@ inline void launch_spread(dim3 grid, dim3 block, size_t smem, cudaStream_t st, A
         return int(fa.sharedSizeBytes);
     }();
     const int per = int((size_t(grid.x) * grid.y * grid.z + 147) / 148), apart = SM / (per + 1) - RESERVED - fixed + 256;
-    if (per <= 4 && apart > int(smem)) smem = size_t(apart);
+    if (per <= MOST && apart > int(smem)) smem = size_t(apart);
     launch(K, grid, block, smem, st, args...);
 }
 #ifdef __CUDACC__
