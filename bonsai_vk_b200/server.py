@@ -49,6 +49,7 @@ class Conversation:
         self.events: "queue.Queue" = queue.Queue()     # ("tok", id) ... ("end", finish_reason)
         self.finish: Optional[str] = None
         self.slot = -1
+        self.started = False               # the slot has been cleared for it
 
     def next_feed(self) -> int:
         return self.prompt[self.pos] if self.pos < len(self.prompt) else self.out[self.pos - len(self.prompt)]
@@ -91,7 +92,6 @@ class Batcher:
             live_groups = {s // self.G for s in range(self.S) if self.conv[s] is not None}
             free.sort(key=lambda s: (s // self.G not in live_groups, s))
             c.slot = free[0]
-            self.e.reset_slot(c.slot)
             self.conv[c.slot] = c
             self.lock.notify_all()
         return c
@@ -103,6 +103,11 @@ class Batcher:
                     self.lock.wait()
                 if self.stop_flag:
                     return
+                # cleared here, between two steps: a step under way still feeds the slot's idle column
+                for s, c in enumerate(self.conv):
+                    if c is not None and not c.started:
+                        self.e.reset_slot(s)
+                        c.started = True
                 plan = []
                 for g in range(self.S // self.G):
                     cs = self.conv[g * self.G:(g + 1) * self.G]
