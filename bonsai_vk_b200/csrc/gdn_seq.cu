@@ -110,20 +110,25 @@ __global__ void __launch_bounds__(256) k_gdn_seq(bnk::GdnSeq a, int n) {
     }
     for (int i = tid; i < n * 32; i += 256) sv[i] = bnk::colp(a.v, (i >> 5) * a.stride)[h * 128 + q4 * 32 + (i & 31)];
     if (tid < n) { sg[2 * tid] = bnk::colp(a.eg, tid * a.stride)[h]; sg[2 * tid + 1] = bnk::colp(a.bt, tid * a.stride)[h]; }
-    // the taps the next token reads: the last three inputs of every channel, into the buffer of its position's parity (one
-    // writer per channel; the kernel before this one has read the old ones)
+    // Both tap buffers end as position after position leaves them: the last three inputs of every channel in the buffer of the next
+    // position's parity, the three in front of the last position in the other one (which a single position does not touch). Any
+    // pass over one of these positions again reads what a token-serial prompt would have left it. One thread per channel, all
+    // reads before the stores: with an odd n the second buffer is the one being read (the kernel before this one has read it).
     {
         const int p0 = a.pos[0];
         const float *rd = (p0 & 1) ? a.hist1 : a.hist0;
-        float *wr = ((p0 + n) & 1) ? a.hist1 : a.hist0;
+        float *wr = ((p0 + n) & 1) ? a.hist1 : a.hist0, *wr2 = ((p0 + n) & 1) ? a.hist0 : a.hist1;
         const int cnt = 32 + (h < a.qk_heads && q4 == 0 ? 256 : 0);
         for (int j = tid; j < cnt; j += 256) {
             const int ch = j < 32 ? 2 * a.qk_heads * 128 + h * 128 + q4 * 32 + j : (j - 32 < 128 ? h * 128 + j - 32 : a.qk_heads * 128 + h * 128 + j - 160);
-            float t[3];
+            float t[4];                            // inputs n - 4 .. n - 1 (the first one only for n > 1)
 #pragma unroll
-            for (int i = 0; i < 3; ++i) { const int c = n - 3 + i; t[i] = c < 0 ? rd[3 * size_t(ch) + 3 + c] : bnk::colp(a.qkv, c * a.stride)[ch]; }
+            for (int i = 0; i < 4; ++i) { const int c = n - 4 + i; t[i] = c < -3 ? 0.0f : (c < 0 ? rd[3 * size_t(ch) + 3 + c] : bnk::colp(a.qkv, c * a.stride)[ch]); }
 #pragma unroll
-            for (int i = 0; i < 3; ++i) wr[3 * size_t(ch) + i] = t[i];
+            for (int i = 0; i < 3; ++i) {
+                wr[3 * size_t(ch) + i] = t[i + 1];
+                if (n > 1) wr2[3 * size_t(ch) + i] = t[i];
+            }
         }
     }
     __syncthreads();
