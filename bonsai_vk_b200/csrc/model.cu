@@ -817,14 +817,13 @@ int bn_model_finalize(bn_model *m) {
         m->kv_layer_bytes = o;
         BN_CUDA(cudaMalloc(&m->kv, m->kv_layer_bytes * m->n_attn * S));
     }
-    if (m->fused || h.batch_cols > 0) {
-        BN_REQUIRE(bnk::q2_gemv_supported(h.hidden, h.hat_block) && bnk::q2_gemv_supported(h.ffn, h.hat_block), BN_ERR_ARG,
-                   "bn_model_finalize: the multi-sequence pass needs hidden and ffn to be multiples of 512 up to 16384");
-        rc = build_q2(m);
-        if (rc != BN_OK) return rc;
-    }
     if (h.batch_cols > 0) {
         rc = build_batch_side(m);
+        if (rc != BN_OK) return rc;
+    }
+    // (a model whose FFN is too wide for the fused kernels may still have columns: the sharded output head is one projection)
+    if (m->fused || h.batch_cols > 0) {
+        rc = build_q2(m);
         if (rc != BN_OK) return rc;
     }
     if (m->ctx->sm_count <= 1024) {
