@@ -15,6 +15,8 @@
 #include "ops.cuh"
 #include "rotate_quant.cuh"
 
+#include <cstdlib>
+
 namespace {
 using namespace bnk;
 
@@ -359,11 +361,6 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
 template <int GQA, int KMODE, int VMODE>
 bool launch_c(cudaStream_t st, const Args &g, size_t smem) {
     auto kernel = k_attn_cluster<GQA, KMODE, VMODE>;
-    static int ok = -1;
-    static size_t set = 0;
-    if (ok < 0) ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-    if (!ok) return false;
-    if (smem > set) { if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return false; set = smem; }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(CL, g.a.n_kv, g.cols.z()); cfg.blockDim = dim3(T); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute at[2];
@@ -372,9 +369,24 @@ bool launch_c(cudaStream_t st, const Args &g, size_t smem) {
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
+    cfg.numAttrs = 1;
+    // asked once, before the first launch, for the largest CTA: 16 CTAs are beyond the portable cluster size, and a launch that
+    // does not fit would leave an error behind, or an invalid capture
+    static const bool fits = [&] {
+        cudaLaunchConfig_t most = cfg;
+        most.dynamicSmemBytes = SMEM_MAX;
+        int clusters = 0;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX) == cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&clusters, kernel, &most) == cudaSuccess && clusters > 0) return true;
+        cudaGetLastError();                    // (a refusal is an answer, not a failed call)
+        return false;
+    }();
+    if (!fits) return false;
     cfg.numAttrs = g_pdl ? 2 : 1;
     BN_COUNT(1);
-    return cudaLaunchKernelEx(&cfg, kernel, g) == cudaSuccess;
+    cudaLaunchKernelEx(&cfg, kernel, g);       // (a failure now is one of the caller's, who asks for the last error)
+    return true;
 }
 template <int GQA>
 bool launch_g(cudaStream_t st, const Args &g) {
@@ -391,6 +403,7 @@ namespace bnk {
 
 bool attn_cluster(cudaStream_t st, AttnDims a, const float *q16f, const float *gate, AttnPos where, KvLayer kv, int splits, float *pregate, float *gated, Cols cols) {
     if (a.cap > 8192 || (splits != 1 && splits != 8 && splits != 64)) return false;
+    if (getenv("BONSAI_ATTN_CHAIN")) return false;                         // the answer "does not fit", for comparisons
     const Args g = {a, where, q16f, gate, kv, splits, 1.0f / sqrtf(float(a.head_dim)), -0.0f, pregate, gated, cols};
     switch (a.n_head / a.n_kv) {
         case 1: return launch_g<1>(st, g);
