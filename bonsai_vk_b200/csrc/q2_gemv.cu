@@ -414,7 +414,6 @@ __global__ void k_sign_bits(const int32_t *__restrict__ signs, int nwords, uint8
 
 template <int SPANS, bool LEAN>
 cudaError_t launch_spans(cudaStream_t st, int sm_count, Q2Args a, bool pdl) {
-    static int smem_set = 0;
     // as many chunks of weights as fit beside the rest, and at least half of an SM's shared memory in all, so that two CTAs of a
     // launch never share an SM (see above)
     const int ng = a.K / 512, tiles = (a.M + 15) / 16, grid = tiles < sm_count ? tiles : sm_count;
@@ -422,13 +421,13 @@ cudaError_t launch_spans(cudaStream_t st, int sm_count, Q2Args a, bool pdl) {
     const int chunks = ((a.share.q + (a.share.r > 0)) * ng + NW - 1) / NW;
     a.slots = std::min({chunks, MAX_SLOTS, (SMEM_MAX - layout(a.K).ring) / CHUNK});
     const int smem = std::max(layout(a.K).ring + a.slots * CHUNK, 116 << 10);
-    if (smem > smem_set) {
-        cudaError_t e = cudaFuncSetAttribute(k_q2_gemv<SPANS, LEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return e;
-        // (an SM changes its carve-out only when it is empty, so every projection asks for the largest one)
-        cudaFuncSetAttribute(k_q2_gemv<SPANS, LEAN>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        smem_set = smem;
-    }
+    // once, to the largest value, whatever this launch needs: with a limit that grows from call to call a second thread could lower
+    // it again under the first (an SM changes its carve-out only when it is empty, so every projection asks for the largest one)
+    static const cudaError_t limits = [] {
+        cudaError_t e = cudaFuncSetAttribute(k_q2_gemv<SPANS, LEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(k_q2_gemv<SPANS, LEAN>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    }();
+    if (limits != cudaSuccess) return limits;
     a.inv_k = (a.K & (a.K - 1)) == 0 ? 1.0f / float(a.K) : 0.0f;
     a.log_hat = 31 - __builtin_clz(unsigned(a.hat_block));
     if (a.next.W) a.next.share = {a.next.units / grid, a.next.units % grid};
