@@ -468,7 +468,7 @@ def main():
         # projection through the op-level C ABI on buffers larger than L2
         us_gdn, _ = m.mixer_sweep_us(reps=5)
         others = [{"kernel": "k_gdn_step: gated-delta-net core of one layer (2 MiB state read + written, the layer's state of the "
-                             "previous token is still in L2)", "algorithmic_bytes": 4_194_304 + 98_304, "us": us_gdn,
+                             "previous token is still in L2; one core behind the other's end, launch gap included)", "algorithmic_bytes": 4_194_304 + 98_304, "us": us_gdn,
                    "achieved": (4_194_304 + 98_304) / us_gdn / 1e3, "frac": (4_194_304 + 98_304) / us_gdn / 1e3 / peak}]
         line["cpu_baseline"] = cpu_gemv_tokens_per_s(seconds=12.0)
         # the end-to-end CPU point: whole decode tokens of this workload through the CPU checker's forward (integer

@@ -199,14 +199,14 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(T, 5) k_gdn_step(con
 
 namespace bnk {
 
-void gdn_step(cudaStream_t st, const GdnStep &a) {
+void gdn_step(cudaStream_t st, const GdnStep &a, bool alone) {
     static bool attr = false;
     if (!attr) {
         cudaFuncSetAttribute(k_gdn_step, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 16384 * 4);
         cudaFuncSetAttribute(k_gdn_step, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         attr = true;
     }
-    launch(k_gdn_step, dim3(a.heads * 4), dim3(T), size_t(a.hidden) * 8, st, a);
+    launch_as(g_pdl && !alone, k_gdn_step, dim3(a.heads * 4), dim3(T), size_t(a.hidden) * 8, st, a);
 }
 
 }  // namespace bnk

@@ -281,11 +281,11 @@ void gdn_fused(bn_model *m, const bn_model::Layer &L) {
             s.heads = NH; s.qk_heads = NQ; s.hidden = h.hidden; s.qkv = m->QKV; s.z = m->Z; s.conv_w = L.conv_w; s.hist0 = h0; s.hist1 = h1; s.pos = m->POS;
             s.x = m->RES; s.norm_w = L.attn_norm; s.alpha_w = L.alpha_w; s.beta_w = L.beta_w; s.dt_bias = L.dt_bias; s.ssm_a = L.ssm_a;
             s.state = gdn_state_of(m, L.idx); s.ssm_norm = L.ssm_norm; s.eps = h.rms_eps; s.scale = 1.0f / sqrtf(float(D)); s.y = m->X1;
-            bnk::gdn_step(m->ctx->stream, s);
+            bnk::gdn_step(m->ctx->stream, s, m->mixers_only);
         }
         else
             bnk::gdn_core_fused(m->ctx->stream, gd, h.hidden, m->QKV, L.conv_w, h0, h1, m->POS, m->RES, m->G + 48, L.attn_norm,
-                                L.alpha_w, L.beta_w, L.dt_bias, L.ssm_a, gdn_state_of(m, L.idx), m->Z, L.ssm_norm, h.rms_eps, m->X1);
+                                L.alpha_w, L.beta_w, L.dt_bias, L.ssm_a, gdn_state_of(m, L.idx), m->Z, L.ssm_norm, h.rms_eps, m->X1, bnk::Cols(), m->mixers_only);
     }
     project_add(m, L.q2_out, IN, m->X1, q2_next(L.q2_ffn, 2 * h.ffn, h.hidden, L.post_norm));
 }

@@ -533,17 +533,17 @@ void gdn_delta(cudaStream_t st, GdnDims d, const float *q, const float *k, const
 void gdn_core_fused(cudaStream_t st, GdnDims d, int hidden, const float *qkv, const float *conv_w, float *hist0,
                     float *hist1, const int *pos_ptr, const float *x, const float *inv_ptr, const float *norm_w, const float *alpha_w,
                     const float *beta_w, const float *dt_bias, const float *ssm_a, float *state, const float *z,
-                    const float *ssm_norm, float eps, float *y, Cols cols) {
+                    const float *ssm_norm, float eps, float *y, Cols cols, bool alone) {
     static bool attr = false;
     if (!attr) {
         cudaFuncSetAttribute(k_gdn_core<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * 16384 * 4);
         cudaFuncSetAttribute(k_gdn_core<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * 16384 * 4);
         attr = true;
     }
-    if (cols.z() > 1) launch(k_gdn_core<2>, dim3(d.heads, 1, cols.z()), dim3(512), size_t(hidden) * 12, st, d.heads, d.qk_heads, hidden, qkv, conv_w, hist0, hist1, pos_ptr, x, inv_ptr,
+    if (cols.z() > 1) launch_as(g_pdl && !alone, k_gdn_core<2>, dim3(d.heads, 1, cols.z()), dim3(512), size_t(hidden) * 12, st, d.heads, d.qk_heads, hidden, qkv, conv_w, hist0, hist1, pos_ptr, x, inv_ptr,
                                                          norm_w, alpha_w, beta_w, dt_bias, ssm_a, state, z, ssm_norm, eps, y,
                                                          1.0f / sqrtf(float(d.dim)), cols);
-    else launch(k_gdn_core<1>, dim3(d.heads, 1, cols.z()), dim3(512), size_t(hidden) * 12, st, d.heads, d.qk_heads, hidden, qkv, conv_w, hist0, hist1, pos_ptr, x, inv_ptr,
+    else launch_as(g_pdl && !alone, k_gdn_core<1>, dim3(d.heads, 1, cols.z()), dim3(512), size_t(hidden) * 12, st, d.heads, d.qk_heads, hidden, qkv, conv_w, hist0, hist1, pos_ptr, x, inv_ptr,
                                                          norm_w, alpha_w, beta_w, dt_bias, ssm_a, state, z, ssm_norm, eps, y,
                                                          1.0f / sqrtf(float(d.dim)), cols); 
 }

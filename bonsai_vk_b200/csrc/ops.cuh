@@ -13,16 +13,20 @@ namespace bnk {
 // memory is visible. Hides the launch latency between the ~230 small kernels of a token.
 extern bool g_pdl;
 template <class... KArgs, class... Args>
-inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+inline void launch_as(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = g_pdl ? 1 : 0;
+    cfg.numAttrs = pdl ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
     BN_COUNT(1);
+}
+template <class... KArgs, class... Args>
+inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+    launch_as(g_pdl, kernel, grid, block, smem, st, args...);
 }
 // The same for a grid of at most a few CTAs per SM: as much unused shared memory as keeps them evenly spread. Launched while the
 // kernel in front is finishing, small CTAs would otherwise crowd on the first SMs that become free while others stay idle.
@@ -99,9 +103,11 @@ void gdn_delta(cudaStream_t st, GdnDims d, const float *q, const float *k, const
 void gdn_core_fused(cudaStream_t st, GdnDims d, int hidden, const float *qkv, const float *conv_w, float *hist0,
                     float *hist1, const int *pos_ptr, const float *x, const float *inv_ptr, const float *norm_w, const float *alpha_w,
                     const float *beta_w, const float *dt_bias, const float *ssm_a, float *state, const float *z,
-                    const float *ssm_norm, float eps, float *y, Cols cols = {});
+                    const float *ssm_norm, float eps, float *y, Cols cols = {}, bool alone = false);
 // the same fused mixer for one token of one sequence on heads x 4 CTAs (gdn_step.cu). The kernel reads the residual before its
 // dependency wait: the launch in front of it must be one that releases its dependents behind its own wait (Q2Args::late).
+// alone (both): a plain launch, for a sweep of cores without the projections between them - a core reads the layer's state before
+// its wait, and the core in front may be the one that writes it.
 struct GdnStep {
     int heads, qk_heads, hidden;
     const float *qkv, *z, *conv_w;
@@ -113,7 +119,7 @@ struct GdnStep {
     float eps, scale;
     float *y;
 };
-void gdn_step(cudaStream_t st, const GdnStep &a);
+void gdn_step(cudaStream_t st, const GdnStep &a, bool alone = false);
 // the mixer for n <= 32 consecutive positions of one sequence (gdn_seq.cu): column c's activations at + c * stride bytes
 struct GdnSeq {
     int heads, qk_heads, hidden;
