@@ -74,6 +74,8 @@ static inline T *bn_ptr(const bn_buf *b, size_t off) {
 }
 
 int bn_scratch_reserve(bn_ctx *ctx, size_t bytes);
+// the same for an op that can do without: false (and no error) while the stream is capturing or when the memory is not to be had
+bool bn_scratch_available(bn_ctx *ctx, size_t bytes);
 // every kernel launch of this library is counted here (one process drives one GPU)
 extern unsigned long long g_bn_launches;
 #define BN_COUNT(n) (g_bn_launches += (n))

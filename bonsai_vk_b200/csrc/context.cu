@@ -42,6 +42,14 @@ int bn_scratch_reserve(bn_ctx *ctx, size_t bytes) {
     return BN_OK;
 }
 
+bool bn_scratch_available(bn_ctx *ctx, size_t bytes) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) return false;
+    if (bn_scratch_reserve(ctx, bytes) == BN_OK) return true;
+    cudaGetLastError();
+    return false;
+}
+
 extern "C" {
 
 const char *bn_last_error(void) { return g_err; }

@@ -57,25 +57,26 @@ int bn_gemm_q81(bn_ctx *ctx, const bn_buf *w, size_t w_off, int w_tiled, int M, 
     else BN_RANGE(w, w_off, size_t(M) * (K / 128) * 28, 16, "bn_gemm_q81 W");
     BN_RANGE(image, image_off, bnk::gemm_image_bytes(K, ncol), 128, "bn_gemm_q81 image");
     BN_RANGE(out, out_off, (size_t(ncol - 1) * out_stride + M) * 4, 4, "bn_gemm_q81 out");
-    auto project = [&](const uint8_t *tiles, int r0, int rows) {
+    auto args = [&](const uint8_t *W, int r0, int rows) {
         bnk::Q2GemmArgs q = {};
-        q.W = tiles; q.M = rows; q.K = K; q.image = bn_ptr<uint8_t>(image, image_off); q.ncol = ncol;
+        q.W = W; q.M = rows; q.K = K; q.image = bn_ptr<uint8_t>(image, image_off); q.ncol = ncol;
         q.out = bn_ptr<float>(out, out_off) + r0; q.out_stride = out_stride; q.err = ctx->err_dev;
-        return bnk::launch_q2_gemm(ctx->stream, ctx->sm_count, q, bnk::g_pdl);
+        return q;
     };
+    // native rows: unpacked into two-bit tiles and projected, in chunks of at most 48 MB of scratch, which stay in L2 (24 576 x
+    // 4096: 25 / 30 / 41 us for 8 / 16 / 32 columns; decoding inside a tcgen05 pipeline took 51 / 56 / 74 us). Inside a capture (a
+    // graph may outlive the scratch), or with no memory left for it, the warps unpack the pieces that they use (22 / 28 / 59 us).
+    const int step = int(std::max<size_t>(1, (size_t(48) << 20) / (size_t(K / 512) * bnk::Q2_PIECE))) * 16;
     cudaError_t e = cudaSuccess;
-    if (w_tiled) e = project(bn_ptr<uint8_t>(w, w_off), 0, M);
+    if (w_tiled) e = bnk::launch_q2_gemm(ctx->stream, ctx->sm_count, args(bn_ptr<uint8_t>(w, w_off), 0, M), bnk::g_pdl);
+    else if (!bn_scratch_available(ctx, bnk::q2_bytes(std::min(M, step), K)))
+        e = bnk::launch_q2_gemm_native(ctx->stream, ctx->sm_count, args(bn_ptr<uint8_t>(w, w_off), 0, M), bnk::g_pdl);
     else {
-        // native rows: unpacked into two-bit tiles and projected, in chunks of at most 48 MB of scratch, which stay in L2 (24 576 x
-        // 4096: 27 / 32 / 55 us for 8 / 16 / 32 columns; decoding inside a tcgen05 pipeline took 51 / 56 / 74 us)
-        const int step = int(std::max<size_t>(1, (size_t(48) << 20) / (size_t(K / 512) * bnk::Q2_PIECE))) * 16;
-        int rc = bn_scratch_reserve(ctx, bnk::q2_bytes(std::min(M, step), K));
-        if (rc != BN_OK) return rc;
         uint8_t *tiles = reinterpret_cast<uint8_t *>(ctx->scratch);
         for (int r0 = 0; r0 < M && e == cudaSuccess; r0 += step) {
             const int n = std::min(step, M - r0);
             bnk::q2_repack(ctx->stream, bn_ptr<uint32_t>(w, w_off) + size_t(r0) * (K / 128) * 7, n, K, tiles);
-            e = project(tiles, r0, n);
+            e = bnk::launch_q2_gemm(ctx->stream, ctx->sm_count, args(tiles, r0, n), bnk::g_pdl);
         }
     }
     if (e != cudaSuccess) return bn_cuda_fail(e, "k_q2_gemm");

@@ -87,6 +87,8 @@ struct Q2GemmArgs {
     Q2Share share;                                 // filled in by the launch: the CTAs' shares of the row tiles
 };
 cudaError_t launch_q2_gemm(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl);
+// the same with W in the file's native rows (16-byte aligned, K % 1024 == 0): each warp unpacks its pieces itself, no scratch
+cudaError_t launch_q2_gemm_native(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl);
 cudaError_t launch_q2_gemm_wide(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl);      // 17 to 32 columns (q2_gemm_wide.cu)
 
 #ifdef __CUDACC__
@@ -116,6 +118,40 @@ __device__ __forceinline__ void q2_mma_first(int (&d)[4], uint32_t a0, uint32_t 
 __device__ __forceinline__ void q2_mma(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
         : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// four packed bytes: five base-3 digits per byte, each in a byte of its own word (T_t = (b * 3^(t+1)) >> 8 is the base-3 prefix of
+// byte b, digit t = T_t - 3 T_(t-1))
+__device__ __forceinline__ void q2_unpack4(uint32_t w, uint32_t *o, int stride) {
+    const uint32_t e = __byte_perm(w, 0u, 0x4240u), d = __byte_perm(w, 0u, 0x4341u);
+    uint32_t prev = 0u, p = 3u;
+#pragma unroll
+    for (int t = 0; t < 5; ++t, p *= 3u) {
+        const uint32_t T = __byte_perm(e * p, d * p, 0x7351u);
+        o[t * stride] = T - 3u * prev;
+        prev = T;
+    }
+}
+// one native block (row 8 * h + r, block j of a piece) into its places in the piece
+__device__ __forceinline__ void q2_unpack_block(const uint32_t (&w)[7], uint8_t *piece, int h, int r, int j) {
+    uint32_t o[32];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) q2_unpack4(w[k], o + k, 4);
+    q2_unpack4(w[4], o + 20, 2);
+    q2_unpack4(w[5], o + 21, 2);
+    const uint32_t v = __byte_perm(w[6], 0u, 0x4140u);
+    const uint32_t ta = __byte_perm(v * 3u, v * 9u, 0x7531u), tb = __byte_perm(v * 27u, v * 81u, 0x7531u);
+    o[30] = ta - 3u * (ta << 16);
+    o[31] = tb - 3u * __byte_perm(ta, tb, 0x5432u);
+    uint8_t *dst = piece + (h * 2 + (j >> 1)) * 512 + r * 64 + (j & 1) * 8;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        uint2 q;
+        q.x = o[2 * t] | o[8 + 2 * t] << 2 | o[16 + 2 * t] << 4 | o[24 + 2 * t] << 6;
+        q.y = o[2 * t + 1] | o[9 + 2 * t] << 2 | o[17 + 2 * t] << 4 | o[25 + 2 * t] << 6;
+        *reinterpret_cast<uint2 *>(dst + t * 16) = q;
+    }
+    *reinterpret_cast<uint16_t *>(piece + Q2_SCALES + (r * 4 + j) * 4 + h * 2) = uint16_t(w[6] >> 16);
 }
 #endif
 

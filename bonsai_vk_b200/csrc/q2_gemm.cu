@@ -43,7 +43,8 @@ __device__ __forceinline__ bool full_wait(uint32_t bar, uint32_t parity, int *er
     return false;
 }
 
-template <int NCP, int MT>
+// NATIVE: W holds the file's rows; a warp unpacks each of its pieces in a corner of shared memory of its own first
+template <int NCP, int MT, bool NATIVE>
 __global__ void __launch_bounds__(threads<NCP>(), 1) k_q2_gemm(const Q2GemmArgs a) {
     constexpr int NT = threads<NCP>(), NW = NT / 32;
     constexpr int NG = NCP / 8, NGW = NG >= 2 ? 2 : 1, H = NG / NGW;      // column groups: all, per unit; units across the columns
@@ -57,6 +58,8 @@ __global__ void __launch_bounds__(threads<NCP>(), 1) k_q2_gemm(const Q2GemmArgs 
     const uint32_t bars = uint32_t(__cvta_generic_to_shared(smem));
     unsigned char *img = smem + 128;
     float *sums = reinterpret_cast<float *>(img + (nchunks > 1 ? 2 : 1) * kc * gbytes);
+    unsigned char *stage = reinterpret_cast<unsigned char *>(sums + size_t(kc) * a.tiles * 16 * NCP) + warp * Q2_PIECE;       // NATIVE only
+    const size_t rowbytes = size_t(a.K >> 7) * 28;
     auto request = [&](int q) {                                            // image piece of chunk q (wave q % nw) into buffer q & 1
         const int g0 = (q % nw) * kc, n = min(kc, ng - g0);
         const uint32_t bytes = uint32_t(n) * gbytes, bar = bars + (q & 1) * 8;
@@ -71,8 +74,8 @@ __global__ void __launch_bounds__(threads<NCP>(), 1) k_q2_gemm(const Q2GemmArgs 
     }
     if (lane == 0) {
         // this CTA's weights (as far as the previous projection has not fetched them) and the next projection's towards L2
-        const uint8_t *own = a.W + size_t(t0) * ng * Q2_PIECE;
-        const int bytes = min(nt * ng * Q2_PIECE, Q2_NEXT_BYTES);
+        const uint8_t *own = a.W + (NATIVE ? size_t(t0) * 16 * rowbytes : size_t(t0) * ng * Q2_PIECE);
+        const int bytes = int(min(NATIVE ? size_t(min(nt * 16, a.M - t0 * 16)) * rowbytes : size_t(nt) * ng * Q2_PIECE, size_t(Q2_NEXT_BYTES)));
         for (int o = warp * 16384; o < bytes; o += NW * 16384) q2_prefetch(own + o, min(16384, bytes - o));
         q2_prefetch_next(a.next, cta, warp, NW);
     }
@@ -100,9 +103,24 @@ __global__ void __launch_bounds__(threads<NCP>(), 1) k_q2_gemm(const Q2GemmArgs 
 #pragma unroll
                 for (int m = 0; m < MT; ++m) {
                     const uint8_t *p = src + size_t(min(m, n - 1 - ur * MT)) * ng * Q2_PIECE;
+                    if (NATIVE) {                  // lane (row g or g + 8, block tig); rows beyond M are zero
+                        const int r0 = (t0 + tb + ur * MT + min(m, n - 1 - ur * MT)) * 16 + g;
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) c[m][k] = __ldg(reinterpret_cast<const uint4 *>(p + k * 512 + lane * 16));
-                    dw[m] = __ldg(reinterpret_cast<const uint4 *>(p + Q2_SCALES + g * 16));
+                        for (int hf = 0; hf < 2; ++hf) {
+                            const int r = r0 + 8 * hf;
+                            const uint32_t *wp = reinterpret_cast<const uint32_t *>(a.W + size_t(r) * rowbytes) + ((g0 + gl) * 4 + tig) * 7;
+                            uint32_t w[7];
+#pragma unroll
+                            for (int k = 0; k < 7; ++k) w[k] = r < a.M ? wp[k] : 0u;
+                            q2_unpack_block(w, stage, hf, g, tig);
+                        }
+                        __syncwarp();
+                        p = stage;
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) c[m][k] = NATIVE ? *reinterpret_cast<const uint4 *>(p + k * 512 + lane * 16) : __ldg(reinterpret_cast<const uint4 *>(p + k * 512 + lane * 16));
+                    dw[m] = NATIVE ? *reinterpret_cast<const uint4 *>(p + Q2_SCALES + g * 16) : __ldg(reinterpret_cast<const uint4 *>(p + Q2_SCALES + g * 16));
+                    if (NATIVE) __syncwarp();      // every lane has its part before the next piece is unpacked
                 }
                 f32pair us[MT][NGW][2], ve[MT][NGW][2];                   // v0 + v1; v0 or v2 (rows g, g + 8)
 #pragma unroll
@@ -218,11 +236,11 @@ __global__ void k_wait_selftest_gemm(int *err) {
     }
 }
 
-template <int NCP, int MT>
+template <int NCP, int MT, bool NATIVE = false>
 cudaError_t launch_t(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl) {
     static bool attr_set = false;
     if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(k_q2_gemm<NCP, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
+        cudaError_t e = cudaFuncSetAttribute(k_q2_gemm<NCP, MT, NATIVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
@@ -231,8 +249,8 @@ cudaError_t launch_t(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl) {
     a.tiles = std::min(a.share.q + (a.share.r > 0), MAX_TILES);
     // groups per wave: all of K where its image piece fits beside its group sums (one wave: no barrier in between, and the units
     // spread over more warps), else as many as fit with the image piece twice
-    const int gimg = 4 * NCP * IMG_COL, gsum = a.tiles * 16 * NCP * 4;
-    auto bytes = [&](int kc) { return 128 + kc * ((kc >= ng ? 1 : 2) * gimg + gsum); };
+    const int gimg = 4 * NCP * IMG_COL, gsum = a.tiles * 16 * NCP * 4, stages = NATIVE ? threads<NCP>() / 32 * Q2_PIECE : 0;
+    auto bytes = [&](int kc) { return 128 + kc * ((kc >= ng ? 1 : 2) * gimg + gsum) + stages; };
     a.kc = ng;
     if (bytes(ng) > SMEM_MAX) for (a.kc = std::min(ng - 1, 8); a.kc > 1 && bytes(a.kc) > SMEM_MAX;) a.kc = (a.kc + 1) / 2;
     if (a.next.W) a.next.share = {a.next.units / grid, a.next.units % grid};
@@ -247,7 +265,7 @@ cudaError_t launch_t(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl) {
     cfg.attrs = at;
     cfg.numAttrs = pdl ? 1 : 0;
     BN_COUNT(1);
-    return cudaLaunchKernelEx(&cfg, k_q2_gemm<NCP, MT>, a);
+    return cudaLaunchKernelEx(&cfg, k_q2_gemm<NCP, MT, NATIVE>, a);
 }
 
 }  // namespace
@@ -265,6 +283,12 @@ cudaError_t launch_q2_gemm(cudaStream_t st, int sm_count, const Q2GemmArgs &a, b
     // 32 columns: a wave of all of K fits only the smallest matrices, where this kernel's units fill more warps (4096 x 4096, with the
     // preparation of the columns: 12.6 against 13.6 us); beyond, q2_gemm_wide.cu
     return few && a.K <= 4096 ? launch_t<32, 2>(st, sm_count, a, pdl) : launch_q2_gemm_wide(st, sm_count, a, pdl);
+}
+
+cudaError_t launch_q2_gemm_native(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl) {
+    if (a.ncol <= 8) return launch_t<8, 1, true>(st, sm_count, a, pdl);
+    if (a.ncol <= 16) return launch_t<16, 1, true>(st, sm_count, a, pdl);
+    return launch_t<32, 1, true>(st, sm_count, a, pdl);
 }
 
 cudaError_t launch_wait_selftest_gemm(cudaStream_t st, int *err) {

@@ -342,18 +342,6 @@ __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Arg
     Q2_STAMP(7);
 }
 
-// four packed bytes: five base-3 digits per byte -> the four two-bit fields of the piece (unpacking as in the
-// multi-column kernel: T_t = (b * 3^(t+1)) >> 8 is the base-3 prefix of byte b, digit t = T_t - 3 T_(t-1))
-__device__ __forceinline__ void unpack4(uint32_t w, uint32_t *o, int stride) {
-    const uint32_t e = __byte_perm(w, 0u, 0x4240u), d = __byte_perm(w, 0u, 0x4341u);
-    uint32_t prev = 0u, p = 3u;
-#pragma unroll
-    for (int t = 0; t < 5; ++t, p *= 3u) {
-        const uint32_t T = __byte_perm(e * p, d * p, 0x7351u);
-        o[t * stride] = T - 3u * prev;
-        prev = T;
-    }
-}
 // A warp per piece: lane (row, block) unpacks 28 bytes into shared memory, eight rows at a time, and the finished piece leaves
 // as 16-byte stores (stored straight from the lanes, 8 bytes of every 16, it ran at a third of the rate). Rows 0..7 of a tile
 // come from Wa and 8..15 from Wb, `half` rows apart in each (Wb = Wa + 8 rows and half = 16 for a single matrix).
@@ -376,26 +364,7 @@ __global__ void __launch_bounds__(256) k_q2_repack(const uint32_t *__restrict__ 
         }
         __syncwarp();                          // the previous piece has left
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            uint32_t o[32];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) unpack4(w[h][k], o + k, 4);
-            unpack4(w[h][4], o + 20, 2);
-            unpack4(w[h][5], o + 21, 2);
-            const uint32_t v = __byte_perm(w[h][6], 0u, 0x4140u);
-            const uint32_t ta = __byte_perm(v * 3u, v * 9u, 0x7531u), tb = __byte_perm(v * 27u, v * 81u, 0x7531u);
-            o[30] = ta - 3u * (ta << 16);
-            o[31] = tb - 3u * __byte_perm(ta, tb, 0x5432u);
-            uint8_t *dst = piece + (h * 2 + (j >> 1)) * 512 + r * 64 + (j & 1) * 8;
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                uint2 q;
-                q.x = o[2 * t] | o[8 + 2 * t] << 2 | o[16 + 2 * t] << 4 | o[24 + 2 * t] << 6;
-                q.y = o[2 * t + 1] | o[9 + 2 * t] << 2 | o[17 + 2 * t] << 4 | o[25 + 2 * t] << 6;
-                *reinterpret_cast<uint2 *>(dst + t * 16) = q;
-            }
-            *reinterpret_cast<uint16_t *>(piece + Q2_SCALES + (r * 4 + j) * 4 + h * 2) = uint16_t(w[h][6] >> 16);
-        }
+        for (int h = 0; h < 2; ++h) q2_unpack_block(w[h], piece, h, r, j);
         __syncwarp();
         uint4 *d = reinterpret_cast<uint4 *>(out + p * Q2_PIECE);
         const uint4 *s = reinterpret_cast<const uint4 *>(piece);
