@@ -29,6 +29,7 @@ struct PrepArgs {
     uint8_t *image;
     float *inv_out; size_t inv_stride;    // PREP_NORM, optional: the norm factor of column c at inv_out + c * inv_stride
     int mode;
+    bool unit_signs;                      // the signs are known to be +-1 (a model's, checked when they are set); else any integers, PREP_PLAIN
 };
 void prep_cols(cudaStream_t st, const PrepArgs &a);
 

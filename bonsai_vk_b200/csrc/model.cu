@@ -538,7 +538,7 @@ void enqueue_batch(bn_model *m, int ncol, bool one_sequence = false) {
     auto prep = [&](int mode, const float *x, const float *w, const int32_t *sg, int K, uint8_t *img, float *inv_out) {
         bnk::PrepArgs a = {};
         a.x = x; a.x_stride = AS; a.w = w; a.signs = sg; a.K = K; a.hat_block = h.hat_block; a.eps = h.rms_eps; a.ncol = ncol;
-        a.image = img; a.inv_out = inv_out; a.inv_stride = AS; a.mode = mode;
+        a.image = img; a.inv_out = inv_out; a.inv_stride = AS; a.mode = mode; a.unit_signs = true;
         bnk::prep_cols(st, a);
     };
     auto gemm = [&](const uint8_t *W, int M, int K, const uint8_t *img, float *out, const float *resid, const bnk::Q2Next &next, bool swiglu = false) {
@@ -1170,7 +1170,7 @@ int bn_model_head_batch(bn_model *m, int ncol, const bn_buf *in, size_t in_off, 
     cols.n = ncol; cols.arena = m->arena_bytes; cols.gdn = 0; cols.conv = 0; cols.kv = 0;
     bnk::PrepArgs p = {};
     p.x = bn_ptr<float>(in, in_off); p.x_stride = size_t(h.hidden); p.w = m->out_norm; p.signs = m->signs; p.K = h.hidden; p.hat_block = h.hat_block; p.eps = h.rms_eps; p.ncol = ncol;
-    p.image = m->IMG_HD; p.inv_stride = AS; p.mode = bnk::PREP_NORM;
+    p.image = m->IMG_HD; p.inv_stride = AS; p.mode = bnk::PREP_NORM; p.unit_signs = true;
     bnk::prep_cols(st, p);
     const int rows = m->head_r1 - m->head_r0;
     bnk::Q2GemmArgs a = {};

@@ -34,9 +34,14 @@ __global__ void __launch_bounds__(NT) k_prep_cols(const PrepArgs a, int log_hb, 
 #pragma unroll
                 for (int k = 0; k < 8; ++k) sg[k] = a.signs[at + k];
             }
+            if (a.unit_signs) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-                nw[k] ^= (unsigned long long)(uint32_t(sg[2 * k]) & 0x80000000u) | (unsigned long long)(uint32_t(sg[2 * k + 1]) & 0x80000000u) << 32;
+                for (int k = 0; k < 4; ++k)
+                    nw[k] ^= (unsigned long long)(uint32_t(sg[2 * k]) & 0x80000000u) | (unsigned long long)(uint32_t(sg[2 * k + 1]) & 0x80000000u) << 32;
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) nw[k] = pair_of(float(sg[2 * k]), float(sg[2 * k + 1]));
+            }
         }
     }
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -91,7 +96,7 @@ __global__ void __launch_bounds__(NT) k_prep_cols(const PrepArgs a, int log_hb, 
         for (int k = 0; k < 4; ++k) v[k] = pair_mul(pair_mul(v[k], pair_of(inv, inv)), nw[k]);
     } else {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] ^= nw[k];
+        for (int k = 0; k < 4; ++k) v[k] = a.unit_signs || !a.signs ? v[k] ^ nw[k] : pair_mul(v[k], nw[k]);
     }
     if (!on) {
 #pragma unroll
