@@ -110,27 +110,6 @@ __global__ void __launch_bounds__(256) k_gdn_seq(bnk::GdnSeq a, int n) {
     }
     for (int i = tid; i < n * 32; i += 256) sv[i] = bnk::colp(a.v, (i >> 5) * a.stride)[h * 128 + q4 * 32 + (i & 31)];
     if (tid < n) { sg[2 * tid] = bnk::colp(a.eg, tid * a.stride)[h]; sg[2 * tid + 1] = bnk::colp(a.bt, tid * a.stride)[h]; }
-    // Both tap buffers end as position after position leaves them: the last three inputs of every channel in the buffer of the next
-    // position's parity, the three in front of the last position in the other one (which a single position does not touch). Any
-    // pass over one of these positions again reads what a token-serial prompt would have left it. One thread per channel, all
-    // reads before the stores: with an odd n the second buffer is the one being read (the kernel before this one has read it).
-    {
-        const int p0 = a.pos[0];
-        const float *rd = (p0 & 1) ? a.hist1 : a.hist0;
-        float *wr = ((p0 + n) & 1) ? a.hist1 : a.hist0, *wr2 = ((p0 + n) & 1) ? a.hist0 : a.hist1;
-        const int cnt = 32 + (h < a.qk_heads && q4 == 0 ? 256 : 0);
-        for (int j = tid; j < cnt; j += 256) {
-            const int ch = j < 32 ? 2 * a.qk_heads * 128 + h * 128 + q4 * 32 + j : (j - 32 < 128 ? h * 128 + j - 32 : a.qk_heads * 128 + h * 128 + j - 160);
-            float t[4];                            // inputs n - 4 .. n - 1 (the first one only for n > 1)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) { const int c = n - 4 + i; t[i] = c < -3 ? 0.0f : (c < 0 ? rd[3 * size_t(ch) + 3 + c] : bnk::colp(a.qkv, c * a.stride)[ch]); }
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                wr[3 * size_t(ch) + i] = t[i + 1];
-                if (n > 1) wr2[3 * size_t(ch) + i] = t[i];
-            }
-        }
-    }
     __syncthreads();
     float ov[4] = {0.0f, 0.0f, 0.0f, 0.0f};        // this lane's part of the previous position's outputs
     const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
@@ -173,12 +152,37 @@ __global__ void __launch_bounds__(256) k_gdn_seq(bnk::GdnSeq a, int n) {
         for (int e = 0; e < 4; ++e) Sr[r * 128 + 32 * e] = S[r][e];
 }
 
-// one warp per (source head, position): per-head RMS, * ssm_norm, swiglu(z, .), v-grouped permutation (k_gdn_out, ops.cu)
+// Both tap buffers end as position after position leaves them: the last three inputs of every channel in the buffer of the next
+// position's parity, the three in front of the last position in the other one (which a single position does not touch). Any pass
+// over one of these positions again reads what a token-serial prompt would have left it. All reads of a channel come before its
+// stores: with an odd n the second buffer is the one being read.
+__device__ __forceinline__ void seq_taps(const bnk::GdnSeq &a, int n, int ch) {
+    const int p0 = a.pos[0];
+    const float *rd = ((p0 & 1) ? a.hist1 : a.hist0) + 3 * size_t(ch);
+    float *wr = (((p0 + n) & 1) ? a.hist1 : a.hist0) + 3 * size_t(ch), *wr2 = (((p0 + n) & 1) ? a.hist0 : a.hist1) + 3 * size_t(ch);
+    float t[4];                                    // inputs n - 4 .. n - 1 (the first one only for n > 1)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { const int c = n - 4 + i; t[i] = c < -3 ? 0.0f : (c < 0 ? rd[3 + c] : bnk::colp(a.qkv, c * a.stride)[ch]); }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        wr[i] = t[i + 1];
+        if (n > 1) wr2[i] = t[i];
+    }
+}
+// one warp per (source head, position): per-head RMS, * ssm_norm, swiglu(z, .), v-grouped permutation (k_gdn_out, ops.cu). The CTAs
+// behind those of the heads bring the conv taps up to date, a channel per thread (in k_gdn_seq, whose chain is the longer one, the
+// second buffer's stores cost 0.6 us a launch, 0.4 % of a 100-token prompt; here nothing).
 __global__ void __launch_bounds__(256) k_gdn_seq_post(bnk::GdnSeq a, const float *__restrict__ z, const float *__restrict__ ssm_norm, float eps, float *__restrict__ y) {
     const int hs = blockIdx.x * 8 + (threadIdx.x >> 5), l = threadIdx.x & 31;
     const size_t off = blockIdx.y * a.stride;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int own = (a.heads + 7) / 8;
+    if (int(blockIdx.x) >= own) {
+        const int ch = ((blockIdx.x - own) * gridDim.y + blockIdx.y) * 256 + threadIdx.x;
+        if (ch < (2 * a.qk_heads + a.heads) * 128) seq_taps(a, gridDim.y, ch);
+        return;
+    }
     if (hs >= a.heads) return;
     const float *o = bnk::colp(a.o, off) + hs * 128;
     float e[4];
@@ -201,7 +205,8 @@ namespace bnk {
 void gdn_sequence(cudaStream_t st, const GdnSeq &a, int n, const float *z, const float *ssm_norm, float eps, float *y) {
     launch_spread<k_gdn_seq_pre>(dim3(a.heads * 2, (n + PP - 1) / PP), dim3(256), 0, st, a, n);
     launch_spread<k_gdn_seq>(dim3(a.heads * 4), dim3(256), size_t(n) * 290 * 4, st, a, n);       // at most 32 positions: 37 KB
-    launch_spread<k_gdn_seq_post>(dim3((a.heads + 7) / 8, n), dim3(256), 0, st, a, z, ssm_norm, eps, y);
+    const int taps = ((2 * a.qk_heads + a.heads + 1) / 2 + n - 1) / n;     // CTAs of 256 channels, over n rows
+    launch_spread<k_gdn_seq_post>(dim3((a.heads + 7) / 8 + taps, n), dim3(256), 0, st, a, z, ssm_norm, eps, y);
 }
 
 }  // namespace bnk
