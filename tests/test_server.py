@@ -67,6 +67,41 @@ def test_scheduler_continuous_batching():
     b.close()
 
 
+def test_a_slot_is_cleared_between_steps():
+    """A conversation that arrives while a step is under way takes a slot whose idle column that step still feeds: the slot is
+    cleared after the step, not beside it, and before the conversation's first token."""
+    class Watched(FakeEngine):
+        def __init__(self):
+            super().__init__()
+            self.entered, self.go, self.stepping, self.log = threading.Event(), threading.Event(), False, []
+
+        def reset_slot(self, s):
+            self.log.append(("reset", s, self.stepping))
+
+        def step(self, g, toks, pos):
+            self.stepping = True
+            self.log.append(("step", g, list(toks)))
+            self.entered.set()
+            self.go.wait(10)
+            out = super().step(g, toks, pos)
+            self.stepping = False
+            return out
+
+    e = Watched()
+    b = server.Batcher(e)
+    a = b.submit([5, 6, 7], 2)
+    assert e.entered.wait(10)
+    c = b.submit([9], 2)                       # same group, while a's first step is held
+    e.go.set()
+    _drain(a); _drain(c)
+    b.close()
+    resets = [x for x in e.log if x[0] == "reset"]
+    assert [s for _, s, _ in resets] == [a.slot, c.slot] and not any(during for _, _, during in resets)
+    first = next(i for i, x in enumerate(e.log) if x[0] == "step" and x[2][c.slot % e.group] == 9)
+    assert e.log.index(resets[1]) < first
+    assert a.out == _serial([5, 6, 7], 2) and c.out == _serial([9], 2)
+
+
 def test_scheduler_samples_on_the_host_when_asked():
     """A conversation with a sampler picks from its own column's logits over its own generation; its neighbour in the
     same group keeps the engine's greedy pick."""
