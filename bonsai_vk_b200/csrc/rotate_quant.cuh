@@ -172,8 +172,10 @@ __device__ __forceinline__ void fwht_spans(float *xs, int t, int spans, int log_
         bar();
     }
 }
-// amax / 127 rounded to nearest in three operations: quotient by the rounded reciprocal, its exact remainder, one correction
-// (checked against the division for every mantissa; amax above 1e-35 keeps the remainder exact)
+// amax / 127 rounded to nearest in three operations: quotient by the rounded reciprocal, its exact remainder by a fused
+// multiply-add, one correction - division by a constant known in advance (Brisebarre, Muller, Raina: Accelerating correctly
+// rounded floating-point division when the divisor is known in advance, IEEE Trans. Computers 53, 2004). amax above 1e-35 keeps
+// the remainder exact. tests/test_gpu_quantiser.py compares every mantissa with the division, and every code below.
 __device__ __forceinline__ float div127(float amax) {
     const float q = __fmul_rn(amax, 1.0f / 127.0f);
     const float d = fmaf(fmaf(-127.0f, q, amax), 1.0f / 127.0f, q);
