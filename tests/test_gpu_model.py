@@ -305,8 +305,9 @@ def test_batched_prefill_equals_the_token_serial_prompt(ctx):
     assert np.array_equal(blocked.logits().view(np.uint32), logits_s.view(np.uint32))
     n_kv = len(prompt) * hp.n_kv * hp.head_dim
     for what, dt, n in [(L.READ_K_DATA, np.int8, n_kv), (L.READ_K_SCALE, np.uint16, n_kv // 32), (L.READ_V_DATA, np.int8, n_kv),
-                        (L.READ_V_SCALE, np.uint16, n_kv // 32), (L.READ_GDN_STATE, np.float32, hp.gdn_heads * hp.gdn_dim ** 2)]:
-        for idx in range(hp.n_layer // hp.attn_interval if what != L.READ_GDN_STATE else hp.n_layer - hp.n_layer // hp.attn_interval):
+                        (L.READ_V_SCALE, np.uint16, n_kv // 32), (L.READ_GDN_STATE, np.float32, hp.gdn_heads * hp.gdn_dim ** 2),
+                        (L.READ_CONV_HIST, np.float32, hp.qkv_dim * 3)]:
+        for idx in range(hp.n_layer // hp.attn_interval if what not in (L.READ_GDN_STATE, L.READ_CONV_HIST) else hp.n_layer - hp.n_layer // hp.attn_interval):
             a, b = serial.read(what, dt, n, idx), blocked.read(what, dt, n, idx)
             assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), f"read {what} layer {idx} differs"
     assert blocked.decode(nxt_b, len(prompt), 16) == serial.decode(nxt_s, len(prompt), 16)
