@@ -352,7 +352,7 @@ __device__ __forceinline__ void q81_pass(const float *xs, int8_t *codes, uint32_
 template <bool CG>
 __device__ __forceinline__ void prologue(const PhaseArgs &a, const Smem &s, const Preload &pl, int cta) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int K = a.K, nb = K >> 7;
+    const int K = a.K;
     int8_t *codes = s.codes;
     uint32_t *dsw = s.dsw;
     float *red = s.red, *hinv = s.hinv, *xs = s.xs;
@@ -388,10 +388,7 @@ __device__ __forceinline__ void prologue(const PhaseArgs &a, const Smem &s, cons
 #pragma unroll
             for (int s2 = 16; s2 > 0; s2 >>= 1) t = __fadd_rn(t, __shfl_xor_sync(0xFFFFFFFFu, t, s2));
             inv = __frcp_rn(__fsqrt_rn(__fadd_rn(mean_of(t, K), a.eps)));
-            if (tid == 0) {
-                hinv[0] = inv;
-                if (a.inv_out && cta == 0) a.inv_out[0] = inv;
-            }
+            if (tid == 0) hinv[0] = inv;
         }
     } else if (a.pro == PRO_NORM) {
         // rms_norm.comp order: 256 lane slices of `per` consecutive elements summed ascending, then the
@@ -421,17 +418,13 @@ __device__ __forceinline__ void prologue(const PhaseArgs &a, const Smem &s, cons
                                 __fadd_rn(__fadd_rn(v[1], v[5]), __fadd_rn(v[3], v[7])));
 #pragma unroll
             for (int s2 = 16; s2 > 0; s2 >>= 1) t = __fadd_rn(t, __shfl_xor_sync(0xFFFFFFFFu, t, s2));
-            if (lane == 0) {
-                const float r = __frcp_rn(__fsqrt_rn(__fadd_rn(mean_of(t, K), a.eps)));
-                hinv[0] = r;
-                if (a.inv_out && cta == 0) a.inv_out[0] = r;
-            }
+            if (lane == 0) hinv[0] = __frcp_rn(__fsqrt_rn(__fadd_rn(mean_of(t, K), a.eps)));
         }
         csync();
         inv = hinv[0];
     }
     BN_STAMP(3);
-    if (a.pro == PRO_GDN_OUT || a.pro == PRO_GDN_OUT_SZ) {
+    if (a.pro == PRO_GDN_OUT_SZ) {
         // per-head RMS factor of the delta-rule output (no weight; 128 squares, tree)
         for (int h = warp; h < a.gdn_heads; h += NWARP) {
             const float *o = a.x0 + h * 128;
@@ -452,18 +445,10 @@ __device__ __forceinline__ void prologue(const PhaseArgs &a, const Smem &s, cons
         auto input = [&](int t) -> float {
             if (a.pro == PRO_PLAIN) return ldf<CG>(a.x0 + t);
             if (a.pro == PRO_NORM) return __fmul_rn(__fmul_rn(ldf<CG>(a.x0 + t), inv), a.w[t]);
-            if (a.pro == PRO_SWIGLU) return __fmul_rn(silu_f(ldf<CG>(a.x0 + t)), ldf<CG>(a.x1 + t));
-            if (a.pro == PRO_GDN_OUT || a.pro == PRO_GDN_OUT_SZ) {
-                const int hd = t >> 7, d = t & 127, sub = a.gdn_heads / a.gdn_qk_heads;
-                const int hs = hd / sub + a.gdn_qk_heads * (hd % sub);
-                const float nrm = __fmul_rn(__fmul_rn(ldf<CG>(a.x0 + hs * 128 + d), hinv[1 + hs]), a.w[d]);
-                const float z = ldf<CG>(a.x1 + hs * 128 + d);          // PRO_GDN_OUT_SZ: silu already applied by the producer
-                return __fmul_rn(a.pro == PRO_GDN_OUT ? silu_f(z) : z, nrm);
-            }
-            const int nfill = a.pos_ptr[0] + 1, per = (nfill + a.pv_splits - 1) / a.pv_splits;   // PRO_ATTN_OUT
-            float acc = ldf<CG>(a.x0 + t);
-            for (int s2 = 1; s2 < a.pv_splits; ++s2) if (s2 * per < nfill) acc = __fadd_rn(acc, ldf<CG>(a.x0 + size_t(s2) * K + t));
-            return __fmul_rn(acc, __fdiv_rn(1.0f, __fadd_rn(1.0f, exp_f(-ldf<CG>(a.x1 + t)))));
+            const int hd = t >> 7, d = t & 127, sub = a.gdn_heads / a.gdn_qk_heads;              // PRO_GDN_OUT_SZ
+            const int hs = hd / sub + a.gdn_qk_heads * (hd % sub);
+            const float nrm = __fmul_rn(__fmul_rn(ldf<CG>(a.x0 + hs * 128 + d), hinv[1 + hs]), a.w[d]);
+            return __fmul_rn(ldf<CG>(a.x1 + hs * 128 + d), nrm);
         };
         if (fast) {
             // butterflies h = 1, 2, 4 inside a thread's 8 consecutive elements, h = 8..128 across lanes
@@ -494,7 +479,7 @@ __device__ __forceinline__ void prologue(const PhaseArgs &a, const Smem &s, cons
 #pragma unroll
                         for (int r = 0; r < 8; ++r) v[r] = apply_sign(xv[r], sg[r]);
                     }
-                } else if (a.pro == PRO_GDN_OUT || a.pro == PRO_GDN_OUT_SZ) {
+                } else {
                     // 8 consecutive values lie in one destination head: one source head, three 32-byte loads
                     const int hd = tb >> 7, d0 = tb & 127, sub = a.gdn_heads / a.gdn_qk_heads;
                     const int hs = hd / sub + a.gdn_qk_heads * (hd % sub);
@@ -508,12 +493,8 @@ __device__ __forceinline__ void prologue(const PhaseArgs &a, const Smem &s, cons
 #pragma unroll
                     for (int r = 0; r < 8; ++r) {
                         const float nrm = __fmul_rn(__fmul_rn(ov[r], hi), nv[r]);
-                        const float zz = a.pro == PRO_GDN_OUT ? silu_f(zv[r]) : zv[r];
-                        v[r] = apply_sign(__fmul_rn(zz, nrm), sg[r]);
+                        v[r] = apply_sign(__fmul_rn(zv[r], nrm), sg[r]);
                     }
-                } else {
-#pragma unroll
-                    for (int r = 0; r < 8; ++r) v[r] = apply_sign(input(tb + r), sg[r]);
                 }
                 fwht_regs_lanes(v, lane);
                 float4 *dst = reinterpret_cast<float4 *>(xs + tid * 8);
@@ -551,11 +532,10 @@ __device__ __forceinline__ void prologue(const PhaseArgs &a, const Smem &s, cons
 // (every warp has taken that item's rows into registers by then, or will within a few hundred cycles) with item
 // g - FEED_LAG + STAGES, whatever projection of whatever token that item belongs to.
 constexpr int FEED_LAG = 2;
-// EPI >= 0: the epilogue is fixed at compile time (the per-projection kernel only ever needs EPI_PLAIN and keeps its lean
-// loop); EPI < 0: taken from the phase record at run time (whole-token kernel: one copy of the loop for all phases).
-template <int EPI, class Feed>
+// The epilogue is taken from the phase record at run time: one copy of the loop for all phases.
+template <class Feed>
 __device__ __forceinline__ void main_loop(const PhaseArgs &a, const Work &w, const Smem &s, uint32_t git0, int cta, Feed &feed) {
-    const int epi = EPI >= 0 ? EPI : a.epi;
+    const int epi = a.epi;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tig = lane & 3;
     const int CH = w.CH, nt = w.nt, items = w.items, gpitch = w.gpitch;
     float *sv = s.sv, *accs = s.accs;

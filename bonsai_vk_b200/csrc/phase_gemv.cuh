@@ -9,10 +9,7 @@ namespace bnk {
 enum Prologue {
     PRO_PLAIN = 1,    // x0 is the plain fp32 input: rotate + quantise
     PRO_NORM = 2,     // x = rms_norm(x0) * w                                   (pre_norm, bonsai_forward.h:480)
-    PRO_SWIGLU = 3,   // x = silu(x0) * x1                                       (ffn_block :498)
-    PRO_GDN_OUT = 4,  // x = permute(silu(z = x1) * (rms_head(o = x0) * w))      (gdn_block :559-567)
-    PRO_ATTN_OUT = 5, // x = (sum_s pv[s]) * sigmoid(gate = x1)                  (attn_pv_q8v.comp tail)
-    PRO_GDN_OUT_SZ = 6 // as PRO_GDN_OUT with x1 = silu(z) already applied by the producing phase's epilogue
+    PRO_GDN_OUT_SZ = 3 // x = permute(x1 * (rms_head(o = x0) * w)), x1 = silu(z) from the producing phase's epilogue   (gdn_block :559-567)
 };
 
 enum Epilogue {
@@ -40,10 +37,7 @@ struct PhaseArgs {
     const int32_t *signs;    // K sign values
     int hat_block;
     float hat_inv, eps;
-    int gdn_heads, gdn_qk_heads;   // PRO_GDN_OUT
-    int pv_splits;                 // PRO_ATTN_OUT: x0 = pv partials [splits][K]
-    const int *pos_ptr;            // PRO_ATTN_OUT: number of filled keys = pos + 1
-    float *inv_out;                // PRO_NORM: optional, receives 1/sqrt(mean(x0^2) + eps) for a later consumer
+    int gdn_heads, gdn_qk_heads;   // PRO_GDN_OUT_SZ
     int *err;                      // device error word (bounded waits)
     unsigned long long *stamps;    // optional: 8 nanosecond time stamps of CTA 0 (start, copies issued, previous grid
                                    // done, norm, input built, quantised, operands built, end) for profiling

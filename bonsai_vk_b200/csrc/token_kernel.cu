@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(NT, 1) k_token(const TokenArgs ta) {
                 if (stamps) { stamps[i * 8 + 2] = gtime(); stamps[i * 8 + 6] = stamps[i * 8 + 2]; }
             }
             TokFeed feed;
-            main_loop<-1>(a, w, s, ls->git, cta, feed);
+            main_loop(a, w, s, ls->git, cta, feed);
             items = unsigned(w.items);
         } else if (kind == TOP_GDN) {
             gdn_phase(c_ops[i].gdn, s, bar, c_ops[i].wait != 0, cta, ncta, pos);

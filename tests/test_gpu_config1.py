@@ -34,7 +34,7 @@ def test_ffn_block_batch1_and_16_tokens(ctx):
         assert np.array_equal(m1.logits().view(np.uint32), want_logits[i].view(np.uint32)), f"token {i}: logits differ"
     m1.close()
 
-    # 16 tokens in one pass (16 independent sequences of one token each): the tcgen05 projection kernel
+    # 16 tokens in one pass (16 independent sequences of one token each): the multi-column projection kernel
     hb = synth.HParams(n_layer=1, vocab=2048, cap=32, n_streams=16, batch_cols=16)
     mb = Model(ctx, hb, tensors, signs)
     out = ctx.alloc(16 * 4)

@@ -1,4 +1,4 @@
-"""GPU parity of the multi-column tensor-core projection (tcgen05, through the C ABI).
+"""GPU parity of the multi-column tensor-core projection (through the C ABI).
 
 The reference has no integer-dot GEMM beyond 8 columns (it falls back to dequantise + f16 matmul), so the pin is
 column-wise: every column must equal the single-column projection of the same vector - the CPU oracle's
