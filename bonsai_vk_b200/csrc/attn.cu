@@ -36,8 +36,8 @@ __device__ __forceinline__ void q80_store(float v, int lane, int8_t *codes, uint
 // Query rows: RMS norm * weight, NeoX rope on the first n_rot dims, fp16 rounding, gate split; the row's softmax maximum is
 // cleared. Key rows: the same norm / rope, then cache insert (fp16 or q8_0) of K and of the raw V row.
 // Columns (cols.n > 0) are sequences; tokens (the op-level insert) are consecutive positions whose rows follow each other, and
-// only the last one's query is kept. The rope factors need the position only (written a token ago) and are worked out before
-// the wait: a double-precision power, sine and cosine are most of this kernel's chain.
+// only the last one's query is kept. The rope factors need the position only (set before the pass: the rule at bnk::launch)
+// and are worked out before the wait: a double-precision power, sine and cosine are most of this kernel's chain.
 __global__ void __launch_bounds__(256) k_attn_prep(AttnDims a, AttnPos where, const float *__restrict__ qg, const float *__restrict__ kin,
                                                    const float *__restrict__ vin, const float *__restrict__ qn_w, const float *__restrict__ kn_w,
                                                    KvLayer kv, float *__restrict__ q16f, float *__restrict__ gate, unsigned *__restrict__ mx, Cols cols) {

@@ -244,10 +244,13 @@ bnk::Q2Next next_after(const bn_model *m, int b) {
     }
     return m->b1 == h.n_layer ? q2_next(m->q2_head, h.vocab, h.hidden, m->out_norm) : bnk::Q2Next();
 }
-// x = rms_norm(RES) * w through one projection group
-void norm_project(bn_model *m, const uint8_t *W, int M, const float *w, float *out, const bnk::Q2Next &next, float *inv_out = nullptr, bool swiglu = false, bool mixer = false) {
+// x = rms_norm(RES) * w through one projection group. before: what runs behind it - a mixer beside which it leaves room on the SM, and
+// for the recurrent one the dependent launch is released late, because that core reads the residual before its wait (GdnStep)
+enum Before { BEFORE_PROJECTION, BEFORE_ATTENTION, BEFORE_RECURRENCE };
+void norm_project(bn_model *m, const uint8_t *W, int M, const float *w, float *out, const bnk::Q2Next &next, Before before = BEFORE_PROJECTION,
+                  bool swiglu = false, float *inv_out = nullptr) {
     bnk::Q2Args a = phase_base(m, W, M, m->hp.hidden);
-    a.next = next; a.lean = mixer; a.late = inv_out != nullptr;
+    a.next = next; a.lean = before != BEFORE_PROJECTION; a.late = before == BEFORE_RECURRENCE;
     a.pro = bnk::Q2_NORM; a.x0 = m->RES; a.w = w; a.out = out; a.inv_out = inv_out; a.swiglu = swiglu;
     launch(m, a);
 }
@@ -264,19 +267,21 @@ void ffn_fused(bn_model *m, const bn_model::Layer &L) {
     const bn_hparams &h = m->hp;
     // gate and up rows share tiles, so the CTA that has a row's two sums writes silu(gate) * up; the down projection walks the
     // FFN width's Hadamard blocks in its preparation
-    norm_project(m, L.q2_ffn, 2 * h.ffn, L.post_norm, m->FS, q2_next(L.q2_down, h.hidden, h.ffn, nullptr), nullptr, true);
+    norm_project(m, L.q2_ffn, 2 * h.ffn, L.post_norm, m->FS, q2_next(L.q2_down, h.hidden, h.ffn, nullptr), BEFORE_PROJECTION, true);
     project_add(m, L.q2_down, h.ffn, m->FS, next_after(m, int(&L - m->layers.data())));
 }
 
 void gdn_fused(bn_model *m, const bn_model::Layer &L) {
     const bn_hparams &h = m->hp;
     const int NH = h.gdn_heads, NQ = h.gdn_qk_heads, D = h.gdn_dim, C = 2 * NQ * D + NH * D, IN = NH * D;
-    norm_project(m, L.q2_in, C + IN, L.attn_norm, m->QKV, q2_next(L.q2_out, h.hidden, IN, nullptr), m->G + 48, false, true);      // (the norm factor also goes to the layer core's two small projections)
+    // (k_gdn_step works out the norm factor itself, while this projection runs; k_gdn_core takes it from here)
+    const bool one_cta = getenv("BONSAI_GDN_ONE_CTA_PER_HEAD") != nullptr;
+    norm_project(m, L.q2_in, C + IN, L.attn_norm, m->QKV, q2_next(L.q2_out, h.hidden, IN, nullptr), BEFORE_RECURRENCE, false, one_cta ? m->G + 48 : nullptr);
     if (!m->phases_only) {
         const bnk::GdnDims gd{NH, NQ, D};
         float *h0 = conv_of(m, 0, L.idx), *h1 = conv_of(m, 1, L.idx);
         // one sequence: heads x 4 CTAs in clusters of 4 (fills the GPU); several sequences: one CTA per head and sequence
-        if (D == 128 && getenv("BONSAI_GDN_ONE_CTA_PER_HEAD") == nullptr) {
+        if (!one_cta) {
             bnk::GdnStep s = {};
             s.heads = NH; s.qk_heads = NQ; s.hidden = h.hidden; s.qkv = m->QKV; s.z = m->Z; s.conv_w = L.conv_w; s.hist0 = h0; s.hist1 = h1; s.pos = m->POS;
             s.x = m->RES; s.norm_w = L.attn_norm; s.alpha_w = L.alpha_w; s.beta_w = L.beta_w; s.dt_bias = L.dt_bias; s.ssm_a = L.ssm_a;
@@ -296,7 +301,7 @@ void attn_fused(bn_model *m, const bn_model::Layer &L) {
     const int QD = h.n_head * h.head_dim, KD = h.n_kv * h.head_dim;
     const bnk::AttnDims ad = attn_dims(m);
     const bnk::KvLayer kv = kv_layer(m, L.idx);
-    norm_project(m, L.q2_in, 2 * QD + 2 * KD, L.attn_norm, m->QKV, q2_next(L.q2_out, h.hidden, QD, nullptr), nullptr, false, true);
+    norm_project(m, L.q2_in, 2 * QD + 2 * KD, L.attn_norm, m->QKV, q2_next(L.q2_out, h.hidden, QD, nullptr), BEFORE_ATTENTION);
     if (!m->phases_only) {
         bnk::attn_prep(st, ad, m->QKV, m->KBUF, m->VBUF, L.q_norm, L.k_norm, {m->POS, 0}, kv, m->Q16F, m->GATEB, m->ESUM);
         bnk::attn_decode(st, ad, m->Q16F, m->GATEB, {m->POS, 0}, kv, m->SCORE, m->P16F, m->ESUM, m->PVPART, m->pv_splits, nullptr, m->GOUT);
@@ -512,6 +517,7 @@ __device__ __forceinline__ int checked_tok(int t, int vocab, int *err) {
     atomicExch(err, 3);
     return 0;
 }
+// (Launched plainly, like k_set_tok_pos: see the rule at bnk::launch.)
 __global__ void k_set_cols(int *tok, int *pos, size_t arena, int n, ColInit ci, const int *tok_src, int vocab, int *err) {
     const int c = threadIdx.x;
     if (c >= n) return;

@@ -266,9 +266,9 @@ __global__ void __launch_bounds__(512, MINB) k_gdn_core(int heads, int qk_heads,
     const int h = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int hq = h % qk_heads, n4 = hidden / 4;
     // ---- before the dependency wait: everything that the preceding kernel (the qkv / gate projection) does not write.
-    // Constants, this layer's recurrent state and conv taps (last written one token ago) and the position (written at
-    // the end of the previous token) are requested while the projection's last CTAs are still running; every kernel of
-    // the schedule waits for its predecessor before it releases its successor, so all older kernels are complete here.
+    // Constants, this layer's recurrent state and conv taps (last written one token ago) and the position (set before
+    // the pass) are requested while the projection's last CTAs are still running; nothing else may be, older kernels of
+    // the pass may be unfinished too (the rule at bnk::launch).
     const bool odd = pos_ptr[0] & 1;               // a token at position p reads taps from buffer p & 1, writes the other
     const float *hist_rd = odd ? hist1 : hist0;
     float *hist_wr = odd ? hist0 : hist1;

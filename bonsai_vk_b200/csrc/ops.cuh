@@ -8,9 +8,17 @@
 // All helpers enqueue on `st` and return cudaGetLastError() state through bn_launch_check by the caller.
 namespace bnk {
 
-// Programmatic dependent launch for every kernel of the token schedule: a kernel may be scheduled while its
-// predecessor drains; it blocks in pdl_sync() (first statement of every kernel) until the predecessor's
-// memory is visible. Hides the launch latency between the ~230 small kernels of a token.
+// Programmatic dependent launch for every kernel of the token schedule: a kernel may be scheduled while its predecessor
+// drains, which hides the launch latency, and blocks in its dependency wait (griddepcontrol.wait) until the predecessor is
+// complete and its memory visible. Most kernels release their successor before that wait, so a chain of unfinished kernels may
+// stand in front of one that has just started. What a kernel may read before its wait is therefore
+//   * constants (weights, signs, norm weights), and
+//   * words that no kernel of the same pass writes in front of it: the position, and the layer's recurrent state and conv taps,
+//     which one kernel of a pass updates, behind its own wait. They were written in an earlier pass, or by the kernel that sets
+//     token and position (k_set_cols, k_set_tok_pos), and every pass begins behind a plain launch, a copy or a graph launch,
+//     which waits for all that was enqueued before it. Those must stay plain: with this attribute they would be part of the chain.
+//     (In a pass whose first launch follows k_set_cols directly that launch is embed_rotate, which waits before it releases.)
+//   * the residual, in gdn_step alone: the projection in front of it releases it late (Q2Args::late).
 extern bool g_pdl;
 template <class... KArgs, class... Args>
 inline void launch_as(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {

@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Arg
     for (int s = 0; s < SPANS; ++s) sg[s] = base + s * 4096 < a.K ? a.sgn[(base >> 3) + s * 512] : 0u;
     if (SPANS == 1 && a.pro == Q2_NORM && base < a.K) load8(a.w + base, nw);
     Q2_STAMP(1);
-    // The next kernel may start now: whatever it does before its own wait touches constants only.
+    // The next kernel may start now: before its own wait it reads constants and words set before the pass (the rule at bnk::launch).
     if (!a.late) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (SPANS == 1) {
 #pragma unroll
