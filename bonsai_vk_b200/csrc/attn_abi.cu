@@ -19,6 +19,7 @@ Lay kv_layout(const bn_attn_dims &d) {
 }
 int splits_for(int cap) { return cap >= 16384 ? 256 : (cap >= 4096 ? 64 : (cap >= 512 ? 8 : 1)); }
 
+// (pos is unused: positions are launch arguments. It keeps the size and layout that callers have allocated)
 struct Scr { size_t pos, q16f, gate, score, pe, esum, pv, bytes; };
 Scr scratch_layout(const bn_attn_dims &d) {
     const size_t QD = size_t(d.n_head) * d.head_dim;

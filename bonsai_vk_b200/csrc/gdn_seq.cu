@@ -2,7 +2,7 @@
 // Only the delta rule itself is sequential in time. Everything in front of it (alpha / beta projections and gates, conv + silu,
 // L2 norms) and behind it (head norm, ssm_norm, swiglu(z, .), permutation) is done for all positions side by side, and the
 // delta rule walks the positions inside one kernel with its state rows in registers. Before, the fused single-position core
-// was launched once per position, about 12 us each: more than half of the 43 ms of a 100-token prompt, which now takes 21 ms.
+// was launched once per position, about 12 us each: more than half of the 43 ms of a 100-token prompt, which now takes 14 ms.
 // Arithmetic and its order are those of k_gdn_core (ops.cu).
 #include "ops.cuh"
 

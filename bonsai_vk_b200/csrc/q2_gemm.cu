@@ -7,8 +7,9 @@
 // (16 rows, 8 columns, 128 weights) - 13 cycles of the SM's FMA pipes - against 4 mma (8 cycles of the tensor cores) and 16
 // ANDs per 16 rows. The accumulators of mma.sync are registers, in the layout the combination wants; tcgen05 would bring them
 // through tensor memory and hand-offs between warps: the kernel that did so, with the operand decoded into tensor memory, took
-// 28 / 33 / 48 us for 24 576 x 4096 at 8 / 16 / 32 columns against 15 / 21 / 43 here (a tcgen05.mma of 128 rows costs 190 cycles
-// whatever its column count, and the tensor pipe is idle either way).
+// 28 / 33 us for 24 576 x 4096 at 8 / 16 columns (a tcgen05.mma of 128 rows costs 190 cycles whatever its column count, and the
+// tensor pipe is idle either way). Here, weights from DRAM, back to back, without the preparation of the columns: 11.1 / 15.5 us;
+// 4096 x 12 288: 7.2 / 12.9 us.
 //
 // Work split. A CTA of 12 or 16 warps owns a run of row tiles over all of K. K is walked in waves of `kc` groups (512 weights each);
 // a wave's piece of the activation image is double-buffered in shared memory. A wave's units (MT row tiles, one group, up to 16
@@ -23,10 +24,10 @@
 namespace {
 using namespace bnk;
 
-// Threads and row tiles per unit, by measurement (24 576 x 4096, and 4096 x 12 288 in brackets): 8 columns 384 threads x 3 tiles
-// 15.3 us (256 x 3: 16.2, 512 x 2: 16.3); 16 columns 512 x 2 21.0 us (256 x 3: 22.3); 32 columns 512 x 2 43.3 (28.8) us (256 x 3: 48.7
-// (32.6)). Requesting a warp's next unit before the present one (weights in 60 more registers) changed nothing: the other warps
-// hide the loads.
+// Threads and row tiles per unit, by measurement (24 576 x 4096, with the preparation of the columns as it was then): 8 columns 384
+// threads x 3 tiles 15.3 us (256 x 3: 16.2, 512 x 2: 16.3); 16 columns 512 x 2 21.0 us (256 x 3: 22.3). 32 columns, small matrices
+// only (see the launch): 512 x 2. Requesting a warp's next unit before the present one (weights in 60 more registers) changed
+// nothing: the other warps hide the loads.
 template <int NCP> __host__ __device__ constexpr int threads() { return NCP == 8 ? 384 : 512; }
 constexpr int SMEM_MAX = 227 << 10;
 constexpr int IMG_COL = 160;                   // image bytes per column and block (act_image.cuh)

@@ -4,8 +4,9 @@
 // What bounds it: the instruction rate. Blackwell's integer and fp32 instructions share their lanes, and a packed fp32 instruction
 // takes two turns, so the work of (16 rows, 8 columns, 128 weights) - 4 mma, 8 ANDs, 16 conversions, 22 packed fp32 operations,
 // 4 multiplications - costs a scheduler about 90 cycles with two or three warps at it, and removing every shared-memory read from
-// the loop changes nothing. That is 19 us for 24 576 x 4096 x 32; the kernel takes 22 us (the wave-by-wave one of q2_gemm.cu,
-// which loses to its barriers and to weights loaded on demand, 32 us; 4096 x 12 288: 17 against 20 us).
+// the loop changes nothing. That is 19 us for 24 576 x 4096 x 32; the kernel takes 27 us with weights from DRAM, back
+// to back and without the preparation of the columns (under ncu with cold caches 32.5, where the wave-by-wave kernel of q2_gemm.cu,
+// which loses to its barriers and to weights loaded on demand, took 45.4); 4096 x 12 288: 20.2 us.
 //
 // Work split. 12 compute warps of 160 registers: a warp has two row tiles, 16 of the columns and a segment of K, and walks the
 // segment group by group with everything in registers (two tiles x 16 columns share the operands: half the ANDs and half the

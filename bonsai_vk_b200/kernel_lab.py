@@ -179,8 +179,8 @@ def stamps_lab(argv):
     nxt = 0
     for pos in range(20):                                   # warm-up: state, cache and clocks
         nxt = m.token(int(nxt) % hp.vocab, pos)
-    names = ["launch -> first copies issued", "waiting for the previous grid", "norm", "signs + Hadamard (+ q8_1 of earlier blocks)", "q8_1 (last Hadamard block)",
-             "operand registers", "main loop + epilogue", "gap after the previous launch's CTA 0", "in kernel"]
+    names = ["launch -> constants requested", "waiting for the previous grid", "norm", "signs + Hadamard (+ q8_1 of earlier blocks)", "q8_1 (last Hadamard block)",
+             "operands set up", "main loop + epilogue", "gap after the previous launch's CTA 0", "in kernel"]
     acc, span = None, 0.0
     for rep in range(reps):
         st = m.profile_token(int(nxt) % hp.vocab, 20 + rep).astype(np.int64)

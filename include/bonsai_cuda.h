@@ -195,7 +195,11 @@ int bn_model_create(bn_ctx *ctx, const bn_hparams *hp, bn_model **out);
 int bn_model_set_tensor(bn_model *m, const char *name, const bn_buf *buf, size_t off, size_t bytes);
 int bn_model_set_signs(bn_model *m, const bn_buf *buf, size_t off, int count);
 /* resolves every tensor the architecture needs (refuses with the missing name), allocates the
- * activation arena, the KV cache and the recurrent state (reference: fwd_init, bonsai_forward.h:1490) */
+ * activation arena, the KV cache and the recurrent state (reference: fwd_init, bonsai_forward.h:1490). Lays the local
+ * projections out a second time, at two bits per weight and about a fifth larger than the native blocks (9B shape: 2.1 GB beside
+ * 1.7 GB), and packs the signs: every tensor's bytes must be in place by then, or queued on the context's stream, and later changes
+ * to projection weights or signs have no effect. The buffers stay the caller's and must outlive the model: the embedding, the f32
+ * tensors and the schedules that are not fused are read from them. */
 int bn_model_finalize(bn_model *m);
 /* zero KV, recurrent state and scratch (reference: fwd_reset_state, bonsai_forward.h:2624-2643) */
 int bn_model_reset(bn_model *m);
@@ -288,8 +292,8 @@ int bn_model_gemv_sweep(bn_model *m, int reps, float *ms_per_sweep);
  * discarded afterwards. */
 int bn_model_mixer_sweep(bn_model *m, int reps, float *us_per_gdn_layer, float *us_per_attn_layer);
 /* profiling aid (reference: BONSAI_PROFILE per-token ledger, bonsai_forward.h:650-662): run one token with
- * every fused projection kernel recording 8 device time stamps in ns (CTA 0: start, first copies issued,
- * previous kernel done, norm done, rotated input built, quantised, first weights awaited, end).
+ * every fused projection kernel recording 8 device time stamps in ns (CTA 0: start, constants requested, previous kernel
+ * done, norm done, input transformed, quantised, operands set up, end).
  * stamps_out receives [n_phases][8]. */
 int bn_model_profile_token(bn_model *m, int tok, int pos, unsigned long long *stamps_out, int max_phases, int *n_phases);
 /* copy a device-side result or state region to the host (reference: act_rd / kv_dump). index = the recurrent or
