@@ -5,8 +5,7 @@
 // One query token reads every key and value once: 71 MB at 32 768 keys, 11 us of memory. What bounds the kernels is CUDA-core
 // work, because the contract fixes one fused multiply-add per (key, head, dim) for the scores and a rounded product and a
 // rounded sum per (key, head, dim), keys ascending, for PV; and below a few thousand keys the five launches' latency.
-#include "ops.cuh"
-#include "rotate_quant.cuh"
+#include "attn_octet.cuh"
 
 namespace {
 using namespace bnk;
@@ -15,9 +14,6 @@ __device__ __forceinline__ void pdl_early() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-// order-preserving image of a float, for atomicMax (0 = below every float)
-__device__ __forceinline__ unsigned ord(float f) { const unsigned b = __float_as_uint(f); return (b & 0x80000000u) ? ~b : b | 0x80000000u; }
-__device__ __forceinline__ float unord(unsigned k) { return __uint_as_float((k & 0x80000000u) ? k & 0x7FFFFFFFu : ~k); }
 
 // q8_0 of one 32-element block held one value per lane (recipe: attn_norm_rope2.comp:39-49,184-217)
 __device__ __forceinline__ void q80_store(float v, int lane, int8_t *codes, uint16_t *scale) {
@@ -102,19 +98,9 @@ __global__ void __launch_bounds__(256) k_attn_prep(AttnDims a, AttnPos where, co
     else q80_store(vr, lane, reinterpret_cast<int8_t *>(kv.v_data) + row + blk * 32, kv.v_scale + row / 32 + blk);
 }
 
-// int8 code -> float without the conversion unit: the word's bytes are biased by 128 (one xor for four codes), a byte
-// is dropped into the mantissa of 2^23 and 2^23 + 128 is subtracted: exact for every code
-constexpr float CODE_MAGIC = 8388736.0f;       // 2^23 + 128
-template <int BYTE> __device__ __forceinline__ float code_f(uint32_t biased_word) {
-    return __uint_as_float(__byte_perm(biased_word, 0x4B000000u, 0x7440u + BYTE));   // 2^23 + (code + 128), magic still to subtract
-}
-
-// Scores: a warp takes octets of consecutive keys of one kv head, the next octet's rows in flight while it works on one; the
-// gqa query heads of the kv head share every K row (merge idea: attn_qk_softmax_gqa.glslh:15-24). Per key and head: lane l
-// covers dims 8l..8l+7 with an fmaf chain, then the 32 lane sums meet in the xor-butterfly tree (16, 8, 4, 2, 1). Two keys
-// travel in the halves of packed registers (the duplicated query values stay in registers for all octets), and the 32 trees of
-// an octet x 4 heads run as one transposed butterfly - every lane ends up with one total - which forms the same pair sums in
-// the same order. The maximum of the scaled scores of each head goes to mx with one atomic per CTA (a maximum has no order).
+// Scores: a warp takes octets of consecutive keys of one kv head (attn_octet.cuh), the next octet's rows in flight while it works
+// on one; the gqa query heads of the kv head share every K row (merge idea: attn_qk_softmax_gqa.glslh:15-24). The maximum of the
+// scaled scores of each head goes to mx with one atomic per CTA (a maximum has no order).
 // Measured at 32 768 keys: 21 us with one octet per warp (its query loads and latency were most of it), 18 us so.
 template <int KMODE>
 __global__ void __launch_bounds__(256, 2) k_attn_scores4(AttnDims a, AttnPos where, const float *__restrict__ q16f, KvLayer kv,
@@ -127,73 +113,17 @@ __global__ void __launch_bounds__(256, 2) k_attn_scores4(AttnDims a, AttnPos whe
     const int nfill = where.get() + 1, step = gridDim.x * 64;
     int jb = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 8;
     if (blockIdx.x * 64 >= nfill) return;          // (the whole CTA)
-    uint4 raw16[KMODE == 1 ? 8 : 1];
-    uint2 raw8[KMODE == 1 ? 1 : 8];
-    uint16_t sc[8];
-    auto fetch = [&](int jo) {
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const size_t row = (size_t(min(jo + u, nfill - 1)) * a.n_kv + kvh) * hd;
-            if (KMODE == 1) raw16[u] = *reinterpret_cast<const uint4 *>(reinterpret_cast<const __half *>(kv.k_data) + row + lane * 8);
-            else {
-                raw8[u] = *reinterpret_cast<const uint2 *>(reinterpret_cast<const int8_t *>(kv.k_data) + row + lane * 8);
-                sc[u] = kv.k_scale[row / 32 + (lane >> 2)];
-            }
-        }
-    };
-    if (jb < nfill) fetch(jb);
-    f32pair qd[4][8];                              // (q, q): both keys of a pair meet the same query value
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-        const float4 *qv = reinterpret_cast<const float4 *>(q16f + size_t(kvh * 4 + g) * hd + lane * 8);
-        const float4 q0 = qv[0], q1 = qv[1];
-        qd[g][0] = pair_of(q0.x, q0.x); qd[g][1] = pair_of(q0.y, q0.y); qd[g][2] = pair_of(q0.z, q0.z); qd[g][3] = pair_of(q0.w, q0.w);
-        qd[g][4] = pair_of(q1.x, q1.x); qd[g][5] = pair_of(q1.y, q1.y); qd[g][6] = pair_of(q1.z, q1.z); qd[g][7] = pair_of(q1.w, q1.w);
-    }
+    KeyOctet<KMODE> keys;
+    if (jb < nfill) keys.fetch(kv, a.n_kv, kvh, hd, lane, jb, nfill - 1);
+    f32pair qd[4][8];
+    load_queries<4>(q16f, kvh * 4, hd, lane, qd);
     const f32pair magic2 = pair_of(CODE_MAGIC, CODE_MAGIC);
     float best = -INFINITY;                        // of head lane & 3
     for (; jb < nfill; jb += step) {
-        float v[32];                               // v[4u + g]: this lane's part of (key jb+u, head g)
-#pragma unroll
-        for (int up = 0; up < 4; ++up) {           // keys jb+2up, jb+2up+1
-            f32pair kf[8];
-            if (KMODE == 1) {
-                const __half2 *ha = reinterpret_cast<const __half2 *>(&raw16[2 * up]), *hb = reinterpret_cast<const __half2 *>(&raw16[2 * up + 1]);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float2 fa = __half22float2(ha[e]), fb = __half22float2(hb[e]);
-                    kf[2 * e] = pair_of(fa.x, fb.x); kf[2 * e + 1] = pair_of(fa.y, fb.y);
-                }
-            } else {
-                const uint32_t a0 = raw8[2 * up].x ^ 0x80808080u, a1 = raw8[2 * up].y ^ 0x80808080u;
-                const uint32_t b0 = raw8[2 * up + 1].x ^ 0x80808080u, b1 = raw8[2 * up + 1].y ^ 0x80808080u;
-                const f32pair sc2 = pair_of(half_bits_to_float(sc[2 * up]), half_bits_to_float(sc[2 * up + 1]));
-                kf[0] = pair_mul(sc2, pair_sub(pair_of(code_f<0>(a0), code_f<0>(b0)), magic2)); kf[1] = pair_mul(sc2, pair_sub(pair_of(code_f<1>(a0), code_f<1>(b0)), magic2));
-                kf[2] = pair_mul(sc2, pair_sub(pair_of(code_f<2>(a0), code_f<2>(b0)), magic2)); kf[3] = pair_mul(sc2, pair_sub(pair_of(code_f<3>(a0), code_f<3>(b0)), magic2));
-                kf[4] = pair_mul(sc2, pair_sub(pair_of(code_f<0>(a1), code_f<0>(b1)), magic2)); kf[5] = pair_mul(sc2, pair_sub(pair_of(code_f<1>(a1), code_f<1>(b1)), magic2));
-                kf[6] = pair_mul(sc2, pair_sub(pair_of(code_f<2>(a1), code_f<2>(b1)), magic2)); kf[7] = pair_mul(sc2, pair_sub(pair_of(code_f<3>(a1), code_f<3>(b1)), magic2));
-            }
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                f32pair acc = 0ull;
-#pragma unroll
-                for (int e = 0; e < 8; ++e) acc = pair_fma(qd[g][e], kf[e], acc);
-                split_pair(acc, v[8 * up + g], v[8 * up + 4 + g]);
-            }
-        }
-        if (jb + step < nfill) fetch(jb + step);
-        // transposed butterfly: at distance `off` a lane keeps the half of its values that its bit selects and adds the
-        // partner's copy of the same values; lane l ends with the total of value l
-#pragma unroll
-        for (int off = 16, n = 32; off >= 1; off >>= 1, n >>= 1) {
-            const bool upper = lane & off;
-#pragma unroll
-            for (int i = 0; i < n / 2; ++i) {
-                const float send = upper ? v[i] : v[i + n / 2];
-                const float keep = upper ? v[i + n / 2] : v[i];
-                v[i] = __fadd_rn(keep, __shfl_xor_sync(0xFFFFFFFFu, send, off));
-            }
-        }
+        float v[32];                               // v[4u + g]: (key jb + u, head g)
+        octet_parts<4>(keys, qd, magic2, v);
+        if (jb + step < nfill) keys.fetch(kv, a.n_kv, kvh, hd, lane, jb + step, nfill - 1);
+        octet_totals<32>(v, lane);                 // lane l: value l
         const int j = jb + (lane >> 2);
         if (j < nfill) {
             score[size_t(kvh * 4 + (lane & 3)) * a.cap + j] = v[0];
@@ -326,13 +256,6 @@ __global__ void __launch_bounds__(1024) k_attn_expsum(AttnDims a, AttnPos where,
         partial[size_t(h) * 128 + blockIdx.y * 16 + t] = __fadd_rn(__fadd_rn(__fadd_rn(v[0], v[4]), __fadd_rn(v[2], v[6])), __fadd_rn(__fadd_rn(v[1], v[5]), __fadd_rn(v[3], v[7])));
     }
 }
-// the rest of the tree: s = 64 .. 1 over a head's 128 sums
-__device__ __forceinline__ float tree128(float e0, float e1, float e2, float e3) {
-    float v = __fadd_rn(__fadd_rn(e0, e2), __fadd_rn(e1, e3));
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xFFFFFFFFu, v, s));
-    return v;
-}
 
 // PV: grid (n_kv, splits, columns); a thread owns DPT output dims of all GQA heads of the kv head and walks the split's keys
 // ascending: acc = acc + p*v with p = fp16(e / total), product and sum rounded (attn_pv_q8v.comp:85-112). V comes through a
@@ -374,7 +297,7 @@ __global__ void __launch_bounds__(256 / DPT) k_attn_pv(AttnDims a, AttnPos where
 #pragma unroll
         for (int k = 0; k < 4; ++k) pt[g][k] = partial[size_t(kvh * GQA + g) * 128 + (tid & 31) + 32 * k];
 #pragma unroll
-    for (int g = 0; g < GQA; ++g) tot[g] = tree128(pt[g][0], pt[g][1], pt[g][2], pt[g][3]);
+    for (int g = 0; g < GQA; ++g) tot[g] = warp_tree128(pt[g][0], pt[g][1], pt[g][2], pt[g][3]);
     for (int k = tid; k < n; k += T) {
         const float *e = pe + size_t(kvh * GQA) * a.cap + j0 + k;
         float x[GQA];

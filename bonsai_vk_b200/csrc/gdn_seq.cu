@@ -5,15 +5,9 @@
 // was launched once per position, about 12 us each: more than half of the 43 ms of a 100-token prompt, which now takes 14 ms.
 // Arithmetic and its order are those of k_gdn_core (ops.cu).
 #include "ops.cuh"
+#include "rotate_quant.cuh"
 
 namespace {
-
-__device__ __forceinline__ float tree128(float e0, float e1, float e2, float e3) {
-    float a = __fadd_rn(__fadd_rn(e0, e2), __fadd_rn(e1, e3));
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) a = __fadd_rn(a, __shfl_xor_sync(0xFFFFFFFFu, a, s));
-    return a;
-}
 
 // grid (2 x heads, positions / 4), 256 threads. Even CTAs: conv + silu + L2 norms of four positions of one value head (and of q / k
 // head h, where h is one). Odd CTAs: alpha and beta of one value head for the same positions, one warp per dot: as a second task of
@@ -75,7 +69,7 @@ __global__ void __launch_bounds__(256) k_gdn_seq_pre(bnk::GdnSeq a, int n) {
         const int p = warp >> 1, k = warp & 1;
         const float *s = sq[p] + k * 128;
         const float e0 = s[lane], e1 = s[lane + 32], e2 = s[lane + 64], e3 = s[lane + 96];
-        const float i = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(tree128(__fmul_rn(e0, e0), __fmul_rn(e1, e1), __fmul_rn(e2, e2), __fmul_rn(e3, e3)), 1e-12f)));
+        const float i = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(bnk::warp_tree128(__fmul_rn(e0, e0), __fmul_rn(e1, e1), __fmul_rn(e2, e2), __fmul_rn(e3, e3)), 1e-12f)));
         float *y = bnk::colp(a.qk, (c0 + p) * a.stride) + (k * a.qk_heads + h) * 128;
         y[lane] = __fmul_rn(e0, i); y[lane + 32] = __fmul_rn(e1, i); y[lane + 64] = __fmul_rn(e2, i); y[lane + 96] = __fmul_rn(e3, i);
     }
@@ -188,7 +182,7 @@ __global__ void __launch_bounds__(256) k_gdn_seq_post(bnk::GdnSeq a, const float
     float e[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) e[i] = o[l + 32 * i];
-    const float ss = tree128(__fmul_rn(e[0], e[0]), __fmul_rn(e[1], e[1]), __fmul_rn(e[2], e[2]), __fmul_rn(e[3], e[3]));
+    const float ss = bnk::warp_tree128(__fmul_rn(e[0], e[0]), __fmul_rn(e[1], e[1]), __fmul_rn(e[2], e[2]), __fmul_rn(e[3], e[3]));
     const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, 128.0f), eps)));
     const int sub = a.heads / a.qk_heads, hd = sub * (hs % a.qk_heads) + hs / a.qk_heads;
 #pragma unroll

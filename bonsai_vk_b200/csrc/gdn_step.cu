@@ -17,12 +17,6 @@ using namespace bnk;
 
 constexpr int T = 256;
 
-__device__ __forceinline__ float tree128(float e0, float e1, float e2, float e3) {
-    float a = __fadd_rn(__fadd_rn(e0, e2), __fadd_rn(e1, e3));
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) a = __fadd_rn(a, __shfl_xor_sync(0xFFFFFFFFu, a, s));
-    return a;
-}
 __device__ __forceinline__ void cp16(void *dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(uint32_t(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
 }
@@ -142,8 +136,8 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(T, 5) k_gdn_step(con
     {
 #pragma unroll
         for (int e = 0; e < 4; ++e) { qq[e] = sq[lane + 32 * e]; kk[e] = sk[lane + 32 * e]; }
-        const float iq = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(tree128(__fmul_rn(qq[0], qq[0]), __fmul_rn(qq[1], qq[1]), __fmul_rn(qq[2], qq[2]), __fmul_rn(qq[3], qq[3])), 1e-12f)));
-        const float ik = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(tree128(__fmul_rn(kk[0], kk[0]), __fmul_rn(kk[1], kk[1]), __fmul_rn(kk[2], kk[2]), __fmul_rn(kk[3], kk[3])), 1e-12f)));
+        const float iq = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(warp_tree128(__fmul_rn(qq[0], qq[0]), __fmul_rn(qq[1], qq[1]), __fmul_rn(qq[2], qq[2]), __fmul_rn(qq[3], qq[3])), 1e-12f)));
+        const float ik = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(warp_tree128(__fmul_rn(kk[0], kk[0]), __fmul_rn(kk[1], kk[1]), __fmul_rn(kk[2], kk[2]), __fmul_rn(kk[3], kk[3])), 1e-12f)));
 #pragma unroll
         for (int e = 0; e < 4; ++e) { qq[e] = __fmul_rn(qq[e], iq); kk[e] = __fmul_rn(kk[e], ik); }
     }
@@ -188,7 +182,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(T, 5) k_gdn_step(con
         float e[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) e[i] = so[i * 32 + lane];
-        const float ss = tree128(__fmul_rn(e[0], e[0]), __fmul_rn(e[1], e[1]), __fmul_rn(e[2], e[2]), __fmul_rn(e[3], e[3]));
+        const float ss = warp_tree128(__fmul_rn(e[0], e[0]), __fmul_rn(e[1], e[1]), __fmul_rn(e[2], e[2]), __fmul_rn(e[3], e[3]));
         const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, 128.0f), a.eps)));
         const int sub = a.heads / a.qk_heads, hd = sub * (h % a.qk_heads) + h / a.qk_heads, d = q4 * 32 + lane;
         a.y[hd * 128 + d] = __fmul_rn(gz, __fmul_rn(__fmul_rn(so[d], inv), nw));

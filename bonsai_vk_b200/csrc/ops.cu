@@ -195,15 +195,6 @@ __global__ void k_conv_silu(const float *__restrict__ x, const float *__restrict
     s[0] = s1; s[1] = s2; s[2] = xn;
 }
 
-// sum over 128 values held as 4 per lane (elements l, l+32, l+64, l+96) in the order of the
-// reference's shared-memory tree sh[l] += sh[l+s], s = 64..1 (gdn_delta.comp tree_reduce)
-__device__ __forceinline__ float warp_tree128(float e0, float e1, float e2, float e3) {
-    float a = __fadd_rn(__fadd_rn(e0, e2), __fadd_rn(e1, e3));
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) a = __fadd_rn(a, __shfl_xor_sync(0xFFFFFFFFu, a, s));
-    return a;
-}
-
 // L2 norm of 128-wide rows, mode 1 (runtime_vk/shaders/l2_norm.comp:59-78); one warp per row
 __global__ void k_l2_norm_rows(const float *__restrict__ x, int rows, float eps, float *__restrict__ y) {
     bnk::pdl_sync();
@@ -211,7 +202,7 @@ __global__ void k_l2_norm_rows(const float *__restrict__ x, int rows, float eps,
     if (row >= rows) return;
     const float *xr = x + size_t(row) * 128;
     const float a = xr[l], b = xr[l + 32], c = xr[l + 64], d = xr[l + 96];
-    const float ss = warp_tree128(__fmul_rn(a, a), __fmul_rn(b, b), __fmul_rn(c, c), __fmul_rn(d, d));
+    const float ss = bnk::warp_tree128(__fmul_rn(a, a), __fmul_rn(b, b), __fmul_rn(c, c), __fmul_rn(d, d));
     const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(ss, eps)));
     float *yr = y + size_t(row) * 128;
     yr[l] = __fmul_rn(a, inv); yr[l + 32] = __fmul_rn(b, inv); yr[l + 64] = __fmul_rn(c, inv); yr[l + 96] = __fmul_rn(d, inv);
@@ -232,11 +223,11 @@ __global__ void __launch_bounds__(256) k_gdn_delta(int heads, int qk_heads, cons
     float s[4], kk[4], qq[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) { s[e] = __fmul_rn(S[l + 32 * e], eg); kk[e] = kr[l + 32 * e]; qq[e] = qr[l + 32 * e]; }
-    const float pred = warp_tree128(__fmul_rn(s[0], kk[0]), __fmul_rn(s[1], kk[1]), __fmul_rn(s[2], kk[2]), __fmul_rn(s[3], kk[3]));
+    const float pred = bnk::warp_tree128(__fmul_rn(s[0], kk[0]), __fmul_rn(s[1], kk[1]), __fmul_rn(s[2], kk[2]), __fmul_rn(s[3], kk[3]));
     const float u = __fmul_rn(bt, __fsub_rn(v[h * 128 + j], pred));
 #pragma unroll
     for (int e = 0; e < 4; ++e) { s[e] = fmaf(kk[e], u, s[e]); S[l + 32 * e] = s[e]; }
-    const float ov = warp_tree128(__fmul_rn(s[0], qq[0]), __fmul_rn(s[1], qq[1]), __fmul_rn(s[2], qq[2]), __fmul_rn(s[3], qq[3]));
+    const float ov = bnk::warp_tree128(__fmul_rn(s[0], qq[0]), __fmul_rn(s[1], qq[1]), __fmul_rn(s[2], qq[2]), __fmul_rn(s[3], qq[3]));
     if (l == 0) o[h * 128 + j] = __fmul_rn(ov, scale);
 }
 
@@ -335,10 +326,10 @@ __global__ void __launch_bounds__(512, MINB) k_gdn_core(int heads, int qk_heads,
     float qq[4], kk[4];
     {
         const float a0 = sq[lane], a1 = sq[lane + 32], a2 = sq[lane + 64], a3 = sq[lane + 96];
-        const float iq = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(warp_tree128(__fmul_rn(a0, a0), __fmul_rn(a1, a1), __fmul_rn(a2, a2), __fmul_rn(a3, a3)), 1e-12f)));
+        const float iq = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(bnk::warp_tree128(__fmul_rn(a0, a0), __fmul_rn(a1, a1), __fmul_rn(a2, a2), __fmul_rn(a3, a3)), 1e-12f)));
         qq[0] = __fmul_rn(a0, iq); qq[1] = __fmul_rn(a1, iq); qq[2] = __fmul_rn(a2, iq); qq[3] = __fmul_rn(a3, iq);
         const float b0 = sk[lane], b1 = sk[lane + 32], b2 = sk[lane + 64], b3 = sk[lane + 96];
-        const float ik = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(warp_tree128(__fmul_rn(b0, b0), __fmul_rn(b1, b1), __fmul_rn(b2, b2), __fmul_rn(b3, b3)), 1e-12f)));
+        const float ik = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(bnk::warp_tree128(__fmul_rn(b0, b0), __fmul_rn(b1, b1), __fmul_rn(b2, b2), __fmul_rn(b3, b3)), 1e-12f)));
         kk[0] = __fmul_rn(b0, ik); kk[1] = __fmul_rn(b1, ik); kk[2] = __fmul_rn(b2, ik); kk[3] = __fmul_rn(b3, ik);
     }
     __syncthreads();
@@ -384,7 +375,7 @@ __global__ void __launch_bounds__(512, MINB) k_gdn_core(int heads, int qk_heads,
         float e[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) e[i] = so[lane + 32 * i];
-        const float ss = warp_tree128(__fmul_rn(e[0], e[0]), __fmul_rn(e[1], e[1]), __fmul_rn(e[2], e[2]), __fmul_rn(e[3], e[3]));
+        const float ss = bnk::warp_tree128(__fmul_rn(e[0], e[0]), __fmul_rn(e[1], e[1]), __fmul_rn(e[2], e[2]), __fmul_rn(e[3], e[3]));
         const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, 128.0f), eps)));
         const int sub = heads / qk_heads, hd = sub * (h % qk_heads) + h / qk_heads;
 #pragma unroll
@@ -407,7 +398,7 @@ __global__ void k_gdn_out(int heads, int qk_heads, const float *__restrict__ o, 
     float e[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) e[i] = orow[l + 32 * i];
-    const float ss = warp_tree128(__fmul_rn(e[0], e[0]), __fmul_rn(e[1], e[1]), __fmul_rn(e[2], e[2]), __fmul_rn(e[3], e[3]));
+    const float ss = bnk::warp_tree128(__fmul_rn(e[0], e[0]), __fmul_rn(e[1], e[1]), __fmul_rn(e[2], e[2]), __fmul_rn(e[3], e[3]));
     const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, 128.0f), eps)));
     // destination head hd reads source head hd/sub + nq*(hd%sub)  =>  source hs feeds hd = sub*(hs%nq) + hs/nq
     const int sub = heads / qk_heads;

@@ -143,13 +143,6 @@ template <bool CG> __device__ __forceinline__ float4 ldf4(const float *p) {
     return CG ? __ldcg(reinterpret_cast<const float4 *>(p)) : *reinterpret_cast<const float4 *>(p);
 }
 
-__device__ __forceinline__ float warp_tree128(float e0, float e1, float e2, float e3) {
-    float a = __fadd_rn(__fadd_rn(e0, e2), __fadd_rn(e1, e3));
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) a = __fadd_rn(a, __shfl_xor_sync(0xFFFFFFFFu, a, s));
-    return a;
-}
-
 // Sylvester-Walsh-Hadamard butterflies, h ascending (hat4096.comp:41-60), any thread mapping gives the
 // same floats because every stage is a set of independent (a+c, a-c) pairs.
 // N values = N / hb independent transforms of width hb side by side (a butterfly of distance h < hb never leaves its

@@ -10,12 +10,6 @@ using namespace bnk;
 constexpr int NT = 512;
 constexpr int IMG_COL = 160;                   // image bytes per column and block: 128 int8 codes + 4 x (fp32 d, fp32 -s)
 
-__device__ __forceinline__ void load8(const float *p, f32pair (&v)[4]) {
-    const ulonglong2 *q = reinterpret_cast<const ulonglong2 *>(p);
-    const ulonglong2 a = q[0], b = q[1];
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-
 __global__ void __launch_bounds__(NT) k_prep_cols(const PrepArgs a, int log_hb, float hat_inv, float inv_k, int ncp) {
     __shared__ __align__(16) float xs[XS8_SPAN];
     __shared__ float red[256];

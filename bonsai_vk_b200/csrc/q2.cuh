@@ -110,6 +110,19 @@ __device__ __forceinline__ void q2_prefetch_next(const Q2Next &n, int cta, int p
 }
 constexpr int Q2_MAGIC = 0x4B400000;           // bits of 12582912.0f: adding an int |i| < 2^22 gives the bits of 12582912 + i
 
+// bounded wait of the multi-column kernels: on giving up the error word is set and the caller goes on to its end without waiting
+// again (results are then invalid)
+__device__ __forceinline__ bool q2_wait(uint32_t bar, uint32_t parity, int *err, int limit = 1 << 22) {
+    for (int it = 0; it < limit; ++it) {
+        uint32_t ok;
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (__builtin_expect(ok != 0u, 1)) return true;
+    }
+    atomicExch(err, 2);
+    return false;
+}
+
 // D = A (u8) x B (s8) + C; the first instruction of a chain takes its C from constants
 __device__ __forceinline__ void q2_mma_first(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"

@@ -33,17 +33,6 @@ constexpr int SMEM_MAX = 227 << 10;
 constexpr int IMG_COL = 160;                   // image bytes per column and block (act_image.cuh)
 constexpr int MAX_TILES = 12;                  // row tiles per pass over K (a thread keeps their running sums in registers)
 
-__device__ __forceinline__ bool full_wait(uint32_t bar, uint32_t parity, int *err, int limit = 1 << 22) {
-    for (int it = 0; it < limit; ++it) {
-        uint32_t ok;
-        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (__builtin_expect(ok != 0u, 1)) return true;
-    }
-    atomicExch(err, 2);
-    return false;
-}
-
 // NATIVE: W holds the file's rows; a warp unpacks each of its pieces in a corner of shared memory of its own first
 template <int NCP, int MT, bool NATIVE>
 __global__ void __launch_bounds__(threads<NCP>(), 1) k_q2_gemm(const Q2GemmArgs a) {
@@ -95,7 +84,7 @@ __global__ void __launch_bounds__(threads<NCP>(), 1) k_q2_gemm(const Q2GemmArgs 
         for (int w = 0; w < nw; ++w) {
             const int g0 = w * kc, gn = min(kc, ng - g0);
             const int buf = nchunks > 1 ? q & 1 : 0;
-            if (alive && (nchunks > 1 || pass == 0)) alive = full_wait(bars + buf * 8, (q >> 1) & 1, a.err);
+            if (alive && (nchunks > 1 || pass == 0)) alive = q2_wait(bars + buf * 8, (q >> 1) & 1, a.err);
             const unsigned char *chunk = img + buf * kc * gbytes;
             for (int u = warp; u < gn * nur * H; u += NW) {
                 const int h = u % H, ur = (u / H) % nur, gl = u / (H * nur);
@@ -227,13 +216,13 @@ __global__ void __launch_bounds__(threads<NCP>(), 1) k_q2_gemm(const Q2GemmArgs 
     }
 }
 
-// A wait that nothing will ever satisfy, with a short limit: the give-up path of full_wait (error word = 2, kernel returns)
+// A wait that nothing will ever satisfy, with a short limit: the give-up path of q2_wait (error word = 2, kernel returns)
 __global__ void k_wait_selftest_gemm(int *err) {
     __shared__ uint64_t bar;
     const uint32_t b = uint32_t(__cvta_generic_to_shared(&bar));
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\nfence.mbarrier_init.release.cluster;" ::"r"(b) : "memory");
-        full_wait(b, 0, err, 1 << 10);
+        q2_wait(b, 0, err, 1 << 10);
     }
 }
 

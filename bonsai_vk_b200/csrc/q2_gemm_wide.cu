@@ -36,17 +36,6 @@ struct Split {                                         // see the launch
     int slots, wslots, imgs, wts;                      // image steps and groups of weights held; their shared memory offsets
 };
 
-__device__ __forceinline__ bool full_wait(uint32_t bar, uint32_t parity, int *err, int limit = 1 << 22) {
-    for (int it = 0; it < limit; ++it) {
-        uint32_t ok;
-        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (__builtin_expect(ok != 0u, 1)) return true;
-    }
-    atomicExch(err, 2);
-    return false;
-}
-
 __device__ __forceinline__ void bulk(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
@@ -96,7 +85,7 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm_wide(const Q2GemmArgs a, cons
         if (warp != NW || lane) return;
         int w_u = 0, w_i = 0, w_pass = 0, w_slot = 0, w_phase = 1;        // the next group of weights
         auto weights = [&]() {
-            if (alive && w_u >= sp.wslots) alive = full_wait(wempty + w_slot * 8, w_phase, a.err);
+            if (alive && w_u >= sp.wslots) alive = q2_wait(wempty + w_slot * 8, w_phase, a.err);
             if (!alive) return;
             const int tb = w_pass * sp.tiles, n = min(sp.tiles, nt - tb), ns = S > 1 ? (ng - w_i + gs - 1) / gs : 1;      // ns: segments that have a group i
             const uint8_t *src = a.W + (size_t(t0 + tb) * ng + w_i) * Q2_PIECE;
@@ -114,7 +103,7 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm_wide(const Q2GemmArgs a, cons
             if (w_u <= u) weights();
             const int ns = S > 1 ? (ng - i + gs - 1) / gs : 1;
             for (int jp = 0; jp < 2; ++jp) {
-                if (alive && 2 * u + jp >= slots) alive = full_wait(empty + slot * 8, phase, a.err);
+                if (alive && 2 * u + jp >= slots) alive = q2_wait(empty + slot * 8, phase, a.err);
                 if (!alive) return;
                 expect(full + slot * 8, ns * step);
                 for (int s = 0; s < ns; ++s) bulk(full + sp.imgs + (slot * S + s) * step, a.image + size_t((s * gs + i) * 2 + jp) * step, step, full + slot * 8);
@@ -138,8 +127,8 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm_wide(const Q2GemmArgs a, cons
             f32pair us[MT][CG][2];                 // v0 + v1 of rows g, g + 8
 #pragma unroll
             for (int jp = 0; jp < 2; ++jp) {
-                if (jp == 0 && alive) alive = full_wait(wfull + wslot * 8, wphase, a.err);
-                if (alive) alive = full_wait(full + slot * 8, phase, a.err);
+                if (jp == 0 && alive) alive = q2_wait(wfull + wslot * 8, wphase, a.err);
+                if (alive) alive = q2_wait(full + slot * 8, phase, a.err);
                 if (on && seg * gs + i < ng) {
                     const unsigned char *img = smem + sp.imgs + (slot * S + seg) * step + half * (CG * 1024) + (tig >> 1) * 128 + g * 16 + (tig & 1) * 8;
                     const unsigned char *scl = smem + sp.imgs + (slot * S + seg) * step + NCP * 128 + half * (CG * 256) + tig * 16;

@@ -46,11 +46,6 @@ constexpr int PBUF = XS8_SPAN;                 // floats of the transform's buff
 __device__ __forceinline__ unsigned long long gtime() { unsigned long long t; asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t)); return t; }
 #define Q2_STAMP(i) do { if (a.stamps && blockIdx.x == 0 && threadIdx.x == 0) a.stamps[i] = gtime(); } while (0)
 
-__device__ __forceinline__ void load8(const float *p, f32pair (&v)[4]) {
-    const ulonglong2 *q = reinterpret_cast<const ulonglong2 *>(p);
-    const ulonglong2 a = q[0], b = q[1];
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
 // barrier over the 16 compute warps (the copy warp never joins it)
 __device__ __forceinline__ void csync() { asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory"); }
 // bounded wait: on giving up the error word is set and the caller goes on to its end without waiting again (results are then

@@ -231,4 +231,19 @@ __device__ __forceinline__ float norm_tree256(const float *p, int lane) {
     return t;
 }
 
+// sum over 128 values held as 4 per lane (elements l, l + 32, l + 64, l + 96) in the order of the reference's shared-memory tree
+// sh[l] += sh[l + s], s = 64 .. 1 (gdn_delta.comp tree_reduce)
+__device__ __forceinline__ float warp_tree128(float e0, float e1, float e2, float e3) {
+    float a = __fadd_rn(__fadd_rn(e0, e2), __fadd_rn(e1, e3));
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) a = __fadd_rn(a, __shfl_xor_sync(0xFFFFFFFFu, a, s));
+    return a;
+}
+// eight consecutive values from a 16-byte aligned place
+__device__ __forceinline__ void load8(const float *p, f32pair (&v)[4]) {
+    const ulonglong2 *q = reinterpret_cast<const ulonglong2 *>(p);
+    const ulonglong2 a = q[0], b = q[1];
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+
 }  // namespace bnk
