@@ -471,7 +471,7 @@ def main():
                              "previous token is still in L2; one core behind the other's end, launch gap included)", "algorithmic_bytes": 4_194_304 + 98_304, "us": us_gdn,
                    "achieved": (4_194_304 + 98_304) / us_gdn / 1e3, "frac": (4_194_304 + 98_304) / us_gdn / 1e3 / peak}]
         line["cpu_baseline"] = cpu_gemv_tokens_per_s(seconds=12.0)
-        # the end-to-end CPU point: whole decode tokens of this workload through the CPU checker's forward (integer
+        # the end-to-end CPU point: whole decode tokens of this workload through the CPU oracle's forward (integer
         # block dots, fp32 scales - the same arithmetic as the GPU path), single-threaded: 2 tokens after a 1-token prompt
         try:
             from tests._oracle import OracleModel
@@ -484,7 +484,7 @@ def main():
             dt = (time.perf_counter() - t1) / 2
             om.close()
             line["cpu_baseline"]["full_token"] = {"value": 1.0 / dt, "unit": "tok/s", "cores": 1, "kind": "port",
-                                                  "sample": "2 whole decode tokens of the 9B-shape model through the CPU checker, single thread"}
+                                                  "sample": "2 whole decode tokens of the 9B-shape model through the CPU oracle, single thread"}
         except Exception as exc:
             line["cpu_baseline"]["full_token"] = {"error": str(exc)[:200]}
     m.close()
@@ -493,11 +493,12 @@ def main():
         try:
             for keys in (4096, 32768):
                 ms_a, nb = kernel_lab.attn_lab([str(keys), "10"], ctx=ctx, quiet=True)
-                others.append({"kernel": f"decode attention, one layer, {keys} keys (prep, scores, softmax sums, PV, combine; q8_0 K and V)",
+                how = "one cluster launch" if keys <= 8192 else "scores, softmax sums, PV, combine"
+                others.append({"kernel": f"decode attention, one layer, {keys} keys ({how}; q8_0 K and V)",
                                "algorithmic_bytes": nb, "us": ms_a * 1e3, "achieved": nb / ms_a / 1e6, "frac": nb / ms_a / 1e6 / peak})
             for ncol in (8, 32):
                 ms_g2, nb = kernel_lab.gemm_lab(["18944", "4096", str(ncol), "3"], ctx=ctx, quiet=True)
-                others.append({"kernel": f"k_q2_gemm: 18944 x 4096 projection, {ncol} sequences per pass (two-bit tiles, int8 tensor cores)",
+                others.append({"kernel": f"k_q2_gemm{'_wide' if ncol > 16 else ''}: 18944 x 4096 projection, {ncol} sequences per pass (two-bit tiles, int8 tensor cores)",
                                "algorithmic_bytes": nb, "us": ms_g2 * 1e3, "achieved": nb / ms_g2 / 1e6, "frac": nb / ms_g2 / 1e6 / peak})
         except Exception as exc:
             others.append({"error": str(exc)[:200]})

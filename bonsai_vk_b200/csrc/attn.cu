@@ -1,5 +1,5 @@
 // attn.cu - decode attention over the quantised KV cache: prep (head norm, rope, cache insert), scores, softmax numerators,
-// PV over splits of the keys, combine. The order of every floating-point sum is part of the contract with the CPU checker (the
+// PV over splits of the keys, combine. The order of every floating-point sum is part of the contract with the CPU oracle (the
 // file is compiled without fused-multiply-add contraction; fmaf is written where one is meant).
 //
 // One query token reads every key and value once: 71 MB at 32 768 keys, 11 us of memory. What bounds the kernels is CUDA-core

@@ -4,7 +4,7 @@
 // length; here the exchanges are four cluster barriers. With the insert in front, host side included: 1501 keys 16.9 -> 11.4 us,
 // 4096 keys 21.0 -> 17.6 us.
 //
-// Arithmetic and the order of every sum are those of attn.cu (and of the CPU checker): scores by an fmaf chain over 8 dims per
+// Arithmetic and the order of every sum are those of attn.cu (and of the CPU oracle): scores by an fmaf chain over 8 dims per
 // lane and the xor tree; 1024 "virtual threads" of ascending partial softmax sums combined by the tree 512 .. 1; probabilities
 // rounded to fp16; PV per split of the keys, ascending, product and sum rounded; splits added ascending; sigmoid gate.
 //

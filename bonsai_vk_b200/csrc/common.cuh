@@ -83,7 +83,7 @@ int bn_launch_check(bn_ctx *ctx, const char *what);
 
 // ---- device helpers ---------------------------------------------------------------------------
 #ifdef __CUDACC__
-// transcendental policy shared with the CPU checker: evaluate in double, round once to float
+// transcendental policy shared with the CPU oracle: evaluate in double, round once to float
 __device__ __forceinline__ float exp_f(float x) { return float(exp(double(x))); }
 __device__ __forceinline__ float log_f(float x) { return float(log(double(x))); }
 __device__ __forceinline__ float sigmoid_f(float x) { return __fdiv_rn(1.0f, __fadd_rn(1.0f, exp_f(-x))); }

@@ -1,7 +1,7 @@
 // ops.cu - the non-GEMV kernels of the decode path: Hadamard rotation, norms, elementwise fusions,
 // embedding gather, gated-delta-net update, decode attention over the quantised KV cache, argmax.
 //
-// Floating-point order is part of the contract with the CPU checker: sums use the fixed trees
+// Floating-point order is part of the contract with the CPU oracle: sums use the fixed trees
 // stated next to each kernel, transcendentals are evaluated in double and rounded once, and the
 // file is compiled without fused-multiply-add contraction (fmaf is written where one is meant).
 #include "ops.cuh"

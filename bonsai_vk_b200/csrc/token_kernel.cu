@@ -10,7 +10,7 @@
 // prologues and the non-projection phases: weights depend on nothing. (A 17th copy-only warp would cap the kernel at 96
 // registers per thread - 5 warps on one of the 4 schedulers - and the main loop then spills.)
 //
-// Arithmetic and its order are those of the stand-alone kernels in ops.cu (same CPU checker). Values that another CTA of
+// Arithmetic and its order are those of the stand-alone kernels in ops.cu (same CPU oracle). Values that another CTA of
 // the same launch wrote are always read through L2 (ld.global.cg): an SM's L1 is not coherent with other SMs' stores.
 //
 // No wait is unbounded: a grid barrier or ring wait that gives up sets the error word (code 4 / 1), raises the CTA's

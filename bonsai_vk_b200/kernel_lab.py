@@ -11,7 +11,7 @@
                                             ledger idea, BONSAI_PROFILE, bonsai_forward.h:650-662)
 
 Prints ms/op, Gop/s and GB/s of PTQ1_0 bytes from CUDA events. Timing rotates through enough copies of the matrix to
-exceed L2. (Results are checked against the CPU checker by the test-suite, not here.)
+exceed L2. (Results are checked against the CPU oracle by the test-suite, not here.)
 """
 from __future__ import annotations
 

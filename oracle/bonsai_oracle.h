@@ -204,7 +204,7 @@ static inline void block_dots_def(const uint8_t *pb, const uint32_t *xq, int32_t
 }
 
 // The same four numbers through a 256-entry table of each byte's five trits (built once from trit_of_byte):
-// the whole-token checker at the 9B shape evaluates 62 million row-blocks per token, which the per-element
+// the whole-token oracle at the 9B shape evaluates 62 million row-blocks per token, which the per-element
 // walk above is too slow for. Integer arithmetic, so equality with block_dots_def is exact; the tests compare
 // the two on random and on edge-case blocks.
 struct TritTable {
