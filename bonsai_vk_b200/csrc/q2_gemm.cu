@@ -28,15 +28,16 @@ using namespace bnk;
 // threads x 3 tiles 15.3 us (256 x 3: 16.2, 512 x 2: 16.3); 16 columns 512 x 2 21.0 us (256 x 3: 22.3). 32 columns, small matrices
 // only (see the launch): 512 x 2. Requesting a warp's next unit before the present one (weights in 60 more registers) changed
 // nothing: the other warps hide the loads.
-template <int NCP> __host__ __device__ constexpr int threads() { return NCP == 8 ? 384 : 512; }
+template <int NCP, bool NATIVE> __host__ __device__ constexpr int threads() { return NCP == 8 && !NATIVE ? 384 : 512; }
 constexpr int SMEM_MAX = 227 << 10;
 constexpr int IMG_COL = 160;                   // image bytes per column and block (act_image.cuh)
 constexpr int MAX_TILES = 12;                  // row tiles per pass over K (a thread keeps their running sums in registers)
 
-// NATIVE: W holds the file's rows; a warp unpacks each of its pieces in a corner of shared memory of its own first
+// NATIVE: W holds the file's rows; a warp unpacks each of its pieces in a corner of shared memory of its own first. Bound by that
+// unpacking, 250 instructions a piece: 16 warps also for 8 columns (128 x 12 288: 10.2 -> 9.1 us, 4096 rows and more the same).
 template <int NCP, int MT, bool NATIVE>
-__global__ void __launch_bounds__(threads<NCP>(), 1) k_q2_gemm(const Q2GemmArgs a) {
-    constexpr int NT = threads<NCP>(), NW = NT / 32;
+__global__ void __launch_bounds__(threads<NCP, NATIVE>(), 1) k_q2_gemm(const Q2GemmArgs a) {
+    constexpr int NT = threads<NCP, NATIVE>(), NW = NT / 32;
     constexpr int NG = NCP / 8, NGW = NG >= 2 ? 2 : 1, H = NG / NGW;      // column groups: all, per unit; units across the columns
     constexpr int ITEMS = (MAX_TILES * 16 * NCP + NT - 1) / NT;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -84,7 +85,10 @@ __global__ void __launch_bounds__(threads<NCP>(), 1) k_q2_gemm(const Q2GemmArgs 
         for (int w = 0; w < nw; ++w) {
             const int g0 = w * kc, gn = min(kc, ng - g0);
             const int buf = nchunks > 1 ? q & 1 : 0;
-            if (alive && (nchunks > 1 || pass == 0)) alive = q2_wait(bars + buf * 8, (q >> 1) & 1, a.err);
+            // the wave's image piece; NATIVE waits for it behind the first unit's unpacking, which needs the weights only
+            bool here = nchunks == 1 && pass > 0;
+            auto await_image = [&] { if (!here) { here = true; if (alive) alive = q2_wait(bars + buf * 8, (q >> 1) & 1, a.err); } };
+            if (!NATIVE) await_image();
             const unsigned char *chunk = img + buf * kc * gbytes;
             for (int u = warp; u < gn * nur * H; u += NW) {
                 const int h = u % H, ur = (u / H) % nur, gl = u / (H * nur);
@@ -112,6 +116,7 @@ __global__ void __launch_bounds__(threads<NCP>(), 1) k_q2_gemm(const Q2GemmArgs 
                     dw[m] = NATIVE ? *reinterpret_cast<const uint4 *>(p + Q2_SCALES + g * 16) : __ldg(reinterpret_cast<const uint4 *>(p + Q2_SCALES + g * 16));
                     if (NATIVE) __syncwarp();      // every lane has its part before the next piece is unpacked
                 }
+                if (NATIVE) await_image();
                 f32pair us[MT][NGW][2], ve[MT][NGW][2];                   // v0 + v1; v0 or v2 (rows g, g + 8)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -239,14 +244,14 @@ cudaError_t launch_t(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl) {
     a.tiles = std::min(a.share.q + (a.share.r > 0), MAX_TILES);
     // groups per wave: all of K where its image piece fits beside its group sums (one wave: no barrier in between, and the units
     // spread over more warps), else as many as fit with the image piece twice
-    const int gimg = 4 * NCP * IMG_COL, gsum = a.tiles * 16 * NCP * 4, stages = NATIVE ? threads<NCP>() / 32 * Q2_PIECE : 0;
+    const int gimg = 4 * NCP * IMG_COL, gsum = a.tiles * 16 * NCP * 4, stages = NATIVE ? threads<NCP, NATIVE>() / 32 * Q2_PIECE : 0;
     auto bytes = [&](int kc) { return 128 + kc * ((kc >= ng ? 1 : 2) * gimg + gsum) + stages; };
     a.kc = ng;
     if (bytes(ng) > SMEM_MAX) for (a.kc = std::min(ng - 1, 8); a.kc > 1 && bytes(a.kc) > SMEM_MAX;) a.kc = (a.kc + 1) / 2;
     if (a.next.W) a.next.share = {a.next.units / grid, a.next.units % grid};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(threads<NCP>());
+    cfg.blockDim = dim3(threads<NCP, NATIVE>());
     cfg.dynamicSmemBytes = std::max(bytes(a.kc), 116 << 10);             // one CTA per SM, as in q2_gemv.cu
     cfg.stream = st;
     cudaLaunchAttribute at[1];

@@ -1,0 +1,35 @@
+"""The several-column projection on both sides of each line of its dispatch: every column equals the single-column projection of its
+vector bit for bit (the same sums in the same order), whichever kernel took the call."""
+import numpy as np
+import pytest
+
+from bonsai_vk_b200 import Context, ptq
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,K,ncol,tiled", [
+    (1, 1024, 1, False), (100, 1024, 16, False), (100, 1024, 17, False),
+    (2368, 6144, 17, False), (2369, 6144, 17, False),            # 12 and 24 pieces per CTA of 148
+    (2368, 7168, 32, False),                                     # 14
+    (4737, 2048, 8, False), (700, 12288, 9, False),
+])
+def test_columns_equal_single_projections(M, K, ncol, tiled):
+    rng = np.random.default_rng(M + K + ncol)
+    rows = min(M, 1024)
+    W = np.ascontiguousarray(np.concatenate([ptq.synth_matrix(rng, rows, K)] * (-(-M // rows)), axis=0)[:M])
+    X = rng.standard_normal((ncol, K)).astype(np.float32)
+    ctx = Context(0)
+    wb, xb, image, out = ctx.from_numpy(W), ctx.from_numpy(X), ctx.alloc(ctx.gemm_image_bytes(K, ncol)), ctx.alloc(ncol * M * 4)
+    pack, one = ctx.alloc(ctx.act_pack_bytes(K)), ctx.alloc(M * 4)
+    wt = ctx.gemm_repack(wb, M, K) if tiled else wb
+    ctx.gemm_act_quant(xb, K, ncol, image)
+    ctx.gemm_q81(wt, M, K, image, ncol, out, tiled=tiled)
+    ctx.sync()
+    got = out.download(np.uint32, ncol * M).reshape(ncol, M)
+    for c in sorted({0, ncol // 2, ncol - 1}):
+        ctx.act_quant_q81(xb, K, pack, x_off=c * K * 4)
+        ctx.gemv_q81(wb, M, K, pack, one)
+        ctx.sync()
+        assert np.array_equal(got[c], one.download(np.uint32, M)), f"column {c}"
+    ctx.close()
