@@ -550,7 +550,7 @@ void enqueue_batch(bn_model *m, int ncol, bool one_sequence = false) {
     auto gemm = [&](const uint8_t *W, int M, int K, const uint8_t *img, float *out, const float *resid, const bnk::Q2Next &next, bool swiglu = false) {
         bnk::Q2GemmArgs a = {};
         a.W = W; a.M = M; a.K = K; a.swiglu = swiglu; a.image = img; a.ncol = ncol; a.out = out; a.out_stride = AS;
-        a.resid = resid; a.resid_stride = AS; a.next = next; a.err = m->ctx->err_dev;
+        a.resid = resid; a.resid_stride = AS; a.next = next; a.warm = 1; a.err = m->ctx->err_dev;
         cudaError_t e = bnk::launch_q2_gemm(st, m->ctx->sm_count, a, m->use_pdl);
         if (e != cudaSuccess && m->launch_err == cudaSuccess) m->launch_err = e;
     };

@@ -24,20 +24,24 @@
 namespace {
 using namespace bnk;
 
-// Threads and row tiles per unit, by measurement (24 576 x 4096, with the preparation of the columns as it was then): 8 columns 384
-// threads x 3 tiles 15.3 us (256 x 3: 16.2, 512 x 2: 16.3); 16 columns 512 x 2 21.0 us (256 x 3: 22.3). 32 columns, small matrices
-// only (see the launch): 512 x 2. Requesting a warp's next unit before the present one (weights in 60 more registers) changed
-// nothing: the other warps hide the loads.
-template <int NCP, bool NATIVE> __host__ __device__ constexpr int threads() { return NCP == 8 && !NATIVE ? 384 : 512; }
 constexpr int SMEM_MAX = 227 << 10;
 constexpr int IMG_COL = 160;                   // image bytes per column and block (act_image.cuh)
 constexpr int MAX_TILES = 12;                  // row tiles per pass over K (a thread keeps their running sums in registers)
 
+// FIRST: the load stays where it stands, in front of a wait
+template <bool FIRST> __device__ __forceinline__ uint4 weights16(const uint8_t *p) {
+    if (!FIRST) return __ldg(reinterpret_cast<const uint4 *>(p));
+    uint4 v;
+    asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
 // NATIVE: W holds the file's rows; a warp unpacks each of its pieces in a corner of shared memory of its own first. Bound by that
 // unpacking, 250 instructions a piece: 16 warps also for 8 columns (128 x 12 288: 10.2 -> 9.1 us, 4096 rows and more the same).
-template <int NCP, int MT, bool NATIVE>
-__global__ void __launch_bounds__(threads<NCP, NATIVE>(), 1) k_q2_gemm(const Q2GemmArgs a) {
-    constexpr int NT = threads<NCP, NATIVE>(), NW = NT / 32;
+// 12 warps (168 registers a thread) have room for a unit's weights to be on their way while the image is: LATE.
+template <int NCP, int MT, int NT, bool NATIVE>
+__global__ void __launch_bounds__(NT, 1) k_q2_gemm(const Q2GemmArgs a) {
+    constexpr int NW = NT / 32;
+    constexpr bool LATE = NATIVE || (NT == 384 && MT == 2);
     constexpr int NG = NCP / 8, NGW = NG >= 2 ? 2 : 1, H = NG / NGW;      // column groups: all, per unit; units across the columns
     constexpr int ITEMS = (MAX_TILES * 16 * NCP + NT - 1) / NT;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -85,10 +89,10 @@ __global__ void __launch_bounds__(threads<NCP, NATIVE>(), 1) k_q2_gemm(const Q2G
         for (int w = 0; w < nw; ++w) {
             const int g0 = w * kc, gn = min(kc, ng - g0);
             const int buf = nchunks > 1 ? q & 1 : 0;
-            // the wave's image piece; NATIVE waits for it behind the first unit's unpacking, which needs the weights only
+            // the wave's image piece, LATE: behind the loads (or the unpacking) of the first unit's weights
             bool here = nchunks == 1 && pass > 0;
             auto await_image = [&] { if (!here) { here = true; if (alive) alive = q2_wait(bars + buf * 8, (q >> 1) & 1, a.err); } };
-            if (!NATIVE) await_image();
+            if (!LATE) await_image();
             const unsigned char *chunk = img + buf * kc * gbytes;
             for (int u = warp; u < gn * nur * H; u += NW) {
                 const int h = u % H, ur = (u / H) % nur, gl = u / (H * nur);
@@ -112,11 +116,11 @@ __global__ void __launch_bounds__(threads<NCP, NATIVE>(), 1) k_q2_gemm(const Q2G
                         p = stage;
                     }
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) c[m][k] = NATIVE ? *reinterpret_cast<const uint4 *>(p + k * 512 + lane * 16) : __ldg(reinterpret_cast<const uint4 *>(p + k * 512 + lane * 16));
-                    dw[m] = NATIVE ? *reinterpret_cast<const uint4 *>(p + Q2_SCALES + g * 16) : __ldg(reinterpret_cast<const uint4 *>(p + Q2_SCALES + g * 16));
+                    for (int k = 0; k < 4; ++k) c[m][k] = NATIVE ? *reinterpret_cast<const uint4 *>(p + k * 512 + lane * 16) : weights16<LATE>(p + k * 512 + lane * 16);
+                    dw[m] = NATIVE ? *reinterpret_cast<const uint4 *>(p + Q2_SCALES + g * 16) : weights16<LATE>(p + Q2_SCALES + g * 16);
                     if (NATIVE) __syncwarp();      // every lane has its part before the next piece is unpacked
                 }
-                if (NATIVE) await_image();
+                if (LATE) await_image();
                 f32pair us[MT][NGW][2], ve[MT][NGW][2];                   // v0 + v1; v0 or v2 (rows g, g + 8)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -231,11 +235,11 @@ __global__ void k_wait_selftest_gemm(int *err) {
     }
 }
 
-template <int NCP, int MT, bool NATIVE = false>
+template <int NCP, int MT, int NT, bool NATIVE = false>
 cudaError_t launch_t(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl) {
     static bool attr_set = false;
     if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(k_q2_gemm<NCP, MT, NATIVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
+        cudaError_t e = cudaFuncSetAttribute(k_q2_gemm<NCP, MT, NT, NATIVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
@@ -244,14 +248,14 @@ cudaError_t launch_t(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl) {
     a.tiles = std::min(a.share.q + (a.share.r > 0), MAX_TILES);
     // groups per wave: all of K where its image piece fits beside its group sums (one wave: no barrier in between, and the units
     // spread over more warps), else as many as fit with the image piece twice
-    const int gimg = 4 * NCP * IMG_COL, gsum = a.tiles * 16 * NCP * 4, stages = NATIVE ? threads<NCP, NATIVE>() / 32 * Q2_PIECE : 0;
+    const int gimg = 4 * NCP * IMG_COL, gsum = a.tiles * 16 * NCP * 4, stages = NATIVE ? NT / 32 * Q2_PIECE : 0;
     auto bytes = [&](int kc) { return 128 + kc * ((kc >= ng ? 1 : 2) * gimg + gsum) + stages; };
     a.kc = ng;
     if (bytes(ng) > SMEM_MAX) for (a.kc = std::min(ng - 1, 8); a.kc > 1 && bytes(a.kc) > SMEM_MAX;) a.kc = (a.kc + 1) / 2;
     if (a.next.W) a.next.share = {a.next.units / grid, a.next.units % grid};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(threads<NCP, NATIVE>());
+    cfg.blockDim = dim3(NT);
     cfg.dynamicSmemBytes = std::max(bytes(a.kc), 116 << 10);             // one CTA per SM, as in q2_gemv.cu
     cfg.stream = st;
     cudaLaunchAttribute at[1];
@@ -260,7 +264,7 @@ cudaError_t launch_t(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl) {
     cfg.attrs = at;
     cfg.numAttrs = pdl ? 1 : 0;
     BN_COUNT(1);
-    return cudaLaunchKernelEx(&cfg, k_q2_gemm<NCP, MT, NATIVE>, a);
+    return cudaLaunchKernelEx(&cfg, k_q2_gemm<NCP, MT, NT, NATIVE>, a);
 }
 
 }  // namespace
@@ -269,21 +273,24 @@ namespace bnk {
 
 cudaError_t launch_q2_gemm(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl) {
     const int ncp = a.ncol <= 8 ? 8 : (a.ncol <= 16 ? 16 : 32), tiles = (a.M + 15) / 16;
-    // row tiles per unit: where a CTA has two tiles at most (the 4096-row projections) one, so that a wave has a unit for every
-    // warp (4096 x 12 288: 12.6 against 15.5 us at 8 columns); at 32 columns there are units enough and two are better (28.7
-    // against 31.8 us)
-    const bool few = tiles <= 2 * sm_count;
-    if (ncp == 8) return few ? launch_t<8, 1>(st, sm_count, a, pdl) : launch_t<8, 3>(st, sm_count, a, pdl);
-    if (ncp == 16) return few ? launch_t<16, 1>(st, sm_count, a, pdl) : launch_t<16, 2>(st, sm_count, a, pdl);
+    // Units of two row tiles (half the operand reads of one; three leave more warps without a unit) on 12 warps, whose first weights
+    // arrive beside the image. Layers of the 9B shape, with the preparation of the columns, weights in L2: 8 columns 43.0 us with
+    // units of three tiles (one where a CTA has two tiles at most) -> 39.3, 16 columns 58.9 with 16 warps -> 55.7. Otherwise: many
+    // tiles per CTA that come from DRAM (8 columns: the output head 82.6 us with units of three, 88 with two; 24 576 x 4096 13.5
+    // against 14.2 with the preparation), and 16 columns whose units fill 16 warps as well as 12 (rounds x warps, the tie:
+    // 24 576 x 4096 15.3 against 15.8 us).
+    const int nt = (tiles + sm_count - 1) / sm_count, units = (nt + 1) / 2 * (a.K / 512);
+    if (ncp == 8) return nt > (a.warm ? MAX_TILES : 6) ? launch_t<8, 3, 384>(st, sm_count, a, pdl) : launch_t<8, 2, 384>(st, sm_count, a, pdl);
+    if (ncp == 16) return (units + 15) / 16 * 16 <= (units + 11) / 12 * 12 ? launch_t<16, 2, 512>(st, sm_count, a, pdl) : launch_t<16, 2, 384>(st, sm_count, a, pdl);
     // 32 columns: a wave of all of K fits only the smallest matrices, where this kernel's units fill more warps (4096 x 4096, with the
     // preparation of the columns: 12.6 against 13.6 us); beyond, q2_gemm_wide.cu
-    return few && a.K <= 4096 ? launch_t<32, 2>(st, sm_count, a, pdl) : launch_q2_gemm_wide(st, sm_count, a, pdl);
+    return tiles <= 2 * sm_count && a.K <= 4096 ? launch_t<32, 2, 512>(st, sm_count, a, pdl) : launch_q2_gemm_wide(st, sm_count, a, pdl);
 }
 
 cudaError_t launch_q2_gemm_native(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl) {
-    if (a.ncol <= 8) return launch_t<8, 1, true>(st, sm_count, a, pdl);
-    if (a.ncol <= 16) return launch_t<16, 1, true>(st, sm_count, a, pdl);
-    return launch_t<32, 1, true>(st, sm_count, a, pdl);
+    if (a.ncol <= 8) return launch_t<8, 1, 512, true>(st, sm_count, a, pdl);
+    if (a.ncol <= 16) return launch_t<16, 1, 512, true>(st, sm_count, a, pdl);
+    return launch_t<32, 1, 512, true>(st, sm_count, a, pdl);
 }
 
 cudaError_t launch_wait_selftest_gemm(cudaStream_t st, int *err) {

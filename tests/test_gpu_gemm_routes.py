@@ -13,6 +13,10 @@ pytestmark = pytest.mark.gpu
     (2368, 6144, 17, False), (2369, 6144, 17, False),            # 12 and 24 pieces per CTA of 148
     (2368, 7168, 32, False),                                     # 14
     (4737, 2048, 8, False), (700, 12288, 9, False),
+    (14208, 1024, 8, True), (14209, 1024, 8, True),              # 6 and 7 row tiles per CTA
+    (28417, 1024, 5, True),                                      # 13: more than one pass
+    (4096, 2048, 16, True), (12288, 1024, 11, True),             # units for 12 warps, for 16
+    (17, 12288, 16, True), (2367, 12288, 8, True),               # K in waves
 ])
 def test_columns_equal_single_projections(M, K, ncol, tiled):
     rng = np.random.default_rng(M + K + ncol)
