@@ -62,7 +62,7 @@ struct Q2Args {
     float inv_k;                 // filled in by the launch: 1 / K when K is a power of two, else 0 (divide);
     int log_hat;                 // log2(hat_block);
     Q2Share share;               // the CTAs' shares of the row tiles;
-    int slots;                   // ring slots
+    int slots, fin;              // ring slots; bytes of group sums from a cluster's CTAs
     float *inv_out;              // Q2_NORM, optional: 1/sqrt(mean(x0^2) + eps)
     int late;                    // release the dependent launch behind this kernel's own dependency wait (see GdnStep)
     int lean;                    // leave room for the next kernel's CTA on the SM (a mixer follows)

@@ -21,6 +21,7 @@
 #include "phase_gemv.cuh"
 
 #include <algorithm>
+#include <array>
 
 namespace {
 using namespace bnk;
@@ -29,16 +30,18 @@ constexpr int NT = 512, NW = NT / 32;          // compute threads; a 17th warp i
 constexpr int CHUNK = NW * Q2_PIECE;           // one piece per warp, contiguous in memory: one bulk copy
 constexpr int EARLY = 1, MAX_SLOTS = 6, SMEM_MAX = 227 << 10;
 struct Lay {                                    // dynamic shared memory, bytes
-    int bars, codes, ds, red, xs, ring;
+    int bars, codes, ds, red, xs, fin, ring;
 };
-__host__ __device__ constexpr Lay layout(int K) {
+// fin: bytes of group sums that come from a cluster's CTAs
+__host__ __device__ constexpr Lay layout(int K, int fin = 0) {
     Lay l{};
     l.bars = 0;
     l.codes = 128;
     l.ds = l.codes + K;
     l.red = l.ds + (K / 32) * 4;
     l.xs = l.red + 256 * 4;
-    l.ring = (l.xs + (K + 4095) / 4096 * XS8_SPAN * 4 + 127) & ~127;
+    l.fin = l.xs + (K + 4095) / 4096 * XS8_SPAN * 4;
+    l.ring = (l.fin + fin + 127) & ~127;
     return l;
 }
 constexpr int PBUF = XS8_SPAN;                 // floats of the transform's buffer that hold group sums afterwards
@@ -65,15 +68,27 @@ __device__ __forceinline__ f32pair sign_pair(uint32_t sg, int k) {
     return (unsigned long long)((sg << (31 - 2 * k)) & 0x80000000u) | (unsigned long long)((sg << (30 - 2 * k)) & 0x80000000u) << 32;
 }
 
+// a CTA's rank in its cluster, its cluster's number
+template <int WHICH> __device__ __forceinline__ int special() {
+    int v;
+    if (WHICH == 0) asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(v));
+    else asm("mov.u32 %0, %%clusterid.x;" : "=r"(v));
+    return v;
+}
 // SPANS: spans of 4096 values whose inputs a thread holds at once (1: K <= 4096; 4: up to 16384)
 // LEAN: 80 registers instead of 94, so that beside the 17 warps (five of them on one of the SM's four schedulers, each with
 // 16 384 registers) the CTA of a latency-bound mixer kernel fits, and a shared-memory carve-out that leaves room for it: the
 // kernel behind the projections of a layer's input. It costs 0.6 us here (12 288 x 4096: 3.0 -> 3.6 us in the loop) and takes
 // 3.5 us off what follows.
-template <int SPANS, bool LEAN>
+// SPLIT: K is a whole number of spans and a cluster's CTAs share it, one span each: a CTA prepares its own 4096 values only (three
+// spans in every CTA took 4.5 us of the FFN's down projection, one takes 2) and takes its groups of the cluster's row tiles, as many
+// pieces as before. A tile's group sums go through distributed shared memory to the CTA that adds them, rank (tile mod CTAs);
+// one cluster barrier. Down projection of the 9B shape in its chain: 9.5 -> 7.0 us from the last CTA in front to its own last one.
+template <int SPANS, bool LEAN, bool SPLIT>
 __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Args a) {
     extern __shared__ __align__(128) unsigned char smem[];
-    const Lay L = layout(a.K);
+    const int parts = SPLIT ? a.K >> 12 : 1, K = SPLIT ? 4096 : a.K, rank = SPLIT ? special<0>() : 0;
+    const Lay L = layout(K, SPLIT ? a.fin : 0);
     unsigned char *codes = smem + L.codes;
     uint32_t *dsw = reinterpret_cast<uint32_t *>(smem + L.ds);
     float *red = reinterpret_cast<float *>(smem + L.red), *xs = reinterpret_cast<float *>(smem + L.xs);
@@ -81,18 +96,28 @@ __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Arg
     Q2_STAMP(0);
 
     // ---- this CTA's tiles ------------------------------------------------------------------------------------------
-    const int ng = a.K >> 9, cta = blockIdx.x, slots = a.slots;
+    const int ng = K >> 9, cta = SPLIT ? special<1>() : blockIdx.x, slots = a.slots;
     const int t0 = cta * a.share.q + min(cta, a.share.r), nt = a.share.q + (cta < a.share.r);
     const int npieces = nt * ng, nchunks = (npieces + NW - 1) / NW;
     const uint32_t full = uint32_t(__cvta_generic_to_shared(smem + L.bars)), empty = full + MAX_SLOTS * 8;
 
+    if (SPLIT) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // "I am running"
     if (warp == NW) {
         // ---- copy warp. Before the previous kernel is done: one chunk of weights into the ring (more would hold up the input
         // vector, which follows it through the same queue, by up to a microsecond) and the NEXT projection's weights (the
         // share that this CTA's successor reads) towards L2; the other slots once the input vector is in registers; refills.
-        const uint8_t *W = a.W + size_t(t0) * ng * Q2_PIECE;
+        const uint8_t *W = a.W + (SPLIT ? size_t(t0) * parts + rank : size_t(t0)) * ng * Q2_PIECE;
         auto request = [&](int i, int s) {
             const uint32_t bytes = uint32_t(min(NW, npieces - i * NW)) * Q2_PIECE;
+            if (SPLIT) {                           // (a chunk is two tiles' groups of this span)
+                constexpr uint32_t half = CHUNK / 2;
+                const uint32_t dst = uint32_t(__cvta_generic_to_shared(smem + L.ring)) + s * CHUNK;
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full + s * 8), "r"(bytes) : "memory");
+                for (uint32_t o = 0; o < bytes; o += half)
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                 ::"r"(dst + o), "l"(W + size_t(i * 2 + (o ? 1 : 0)) * parts * half), "r"(half), "r"(full + s * 8) : "memory");
+                return;
+            }
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full + s * 8), "r"(bytes) : "memory");
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                          ::"r"(uint32_t(__cvta_generic_to_shared(smem + L.ring)) + s * CHUNK), "l"(W + size_t(i) * CHUNK), "r"(bytes), "r"(full + s * 8) : "memory");
@@ -104,7 +129,7 @@ __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Arg
             }
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             for (int i = 0; i < min(EARLY, slots); ++i) request(i, i);
-            q2_prefetch_next(a.next, cta, 0, 1);
+            q2_prefetch_next(a.next, blockIdx.x, 0, 1);
         }
         __syncwarp();
         asm volatile("bar.arrive 2, %0;" ::"n"(NT + 32) : "memory");
@@ -116,17 +141,24 @@ __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Arg
             if (lane == 0) request(i, s);
             if (++s == slots) { s = 0; ph ^= 1; }
         }
+        if (SPLIT) {                               // (both cluster barriers with the other warps)
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        }
         return;
     }
 
     // constants of the preparation depend on no earlier kernel: norm weights with the signs applied to them (the sign of the
     // product is the product of the signs), or the signs as masks
-    const int base = tid * 8, nspan = SPANS == 1 ? 1 : (a.K + 4095) >> 12;
+    const int base = tid * 8, nspan = SPANS == 1 ? 1 : (K + 4095) >> 12;
+    const uint8_t *signs = a.sgn + rank * 512;
+    const float *x0 = a.x0 + rank * 4096;
     f32pair nw[4] = {0, 0, 0, 0};
     uint32_t sg[SPANS];
 #pragma unroll
-    for (int s = 0; s < SPANS; ++s) sg[s] = base + s * 4096 < a.K ? a.sgn[(base >> 3) + s * 512] : 0u;
-    if (SPANS == 1 && a.pro == Q2_NORM && base < a.K) load8(a.w + base, nw);
+    for (int s = 0; s < SPANS; ++s) sg[s] = base + s * 4096 < K ? signs[(base >> 3) + s * 512] : 0u;
+    if (SPANS == 1 && a.pro == Q2_NORM && base < K) load8(a.w + base, nw);
     Q2_STAMP(1);
     // The next kernel may start now: before its own wait it reads constants and words set before the pass (the rule at bnk::launch).
     if (!a.late) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -143,19 +175,19 @@ __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Arg
     f32pair v[SPANS][4];
 #pragma unroll
     for (int s = 0; s < SPANS; ++s)
-        if (base + s * 4096 < a.K) load8(a.x0 + base + s * 4096, v[s]);
+        if (base + s * 4096 < K) load8(x0 + base + s * 4096, v[s]);
         else {
 #pragma unroll
             for (int k = 0; k < 4; ++k) v[s][k] = 0ull;
         }
     // the residual of the row this thread finishes first
     float resid = 0.0f;
-    const int row0 = t0 * 16 + tid;
-    if (a.resid_out && tid < nt * 16 && row0 < a.M) resid = a.resid_in[row0];
+    const int row0 = SPLIT ? (t0 + (tid >> 4) * parts + rank) * 16 + (tid & 15) : t0 * 16 + tid;
+    if (a.resid_out && row0 < min((t0 + nt) * 16, a.M)) resid = a.resid_in[row0];
     f32pair inv2 = pair_of(1.0f, 1.0f);
     if (a.pro == Q2_NORM) {
         // rms_norm.comp order: 256 lanes sum the squares of their run of `per` consecutive values ascending, then the tree
-        const int per = (a.K + 255) >> 8;
+        const int per = (K + 255) >> 8;
         if (SPANS == 1 && per == 16) {             // K = 4096: a lane's run is two neighbouring threads' values
             float sq = 0.0f, e[8];
 #pragma unroll
@@ -170,14 +202,14 @@ __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Arg
             float sq = 0.0f;
             for (int i = 0; i < per; ++i) {
                 const int d = tid * per + i;
-                if (d < a.K) { const float x = a.x0[d]; sq = __fadd_rn(sq, __fmul_rn(x, x)); }
+                if (d < K) { const float x = x0[d]; sq = __fadd_rn(sq, __fmul_rn(x, x)); }
             }
             red[tid] = sq;
         }
         csync();
         const float ss = norm_tree256(red, lane);
-        const float inv = __frcp_rn(__fsqrt_rn(__fadd_rn(a.inv_k != 0.0f ? __fmul_rn(ss, a.inv_k) : __fdiv_rn(ss, float(a.K)), a.eps)));
-        if (a.inv_out && cta == 0 && tid == 0) a.inv_out[0] = inv;
+        const float inv = __frcp_rn(__fsqrt_rn(__fadd_rn(a.inv_k != 0.0f ? __fmul_rn(ss, a.inv_k) : __fdiv_rn(ss, float(K)), a.eps)));
+        if (a.inv_out && blockIdx.x == 0 && tid == 0) a.inv_out[0] = inv;
         inv2 = pair_of(inv, inv);
     }
     Q2_STAMP(3);
@@ -185,7 +217,7 @@ __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Arg
     for (int s = 0; s < SPANS; ++s) {
         if (s < nspan) {
             if (SPANS > 1) {
-                if (a.pro == Q2_NORM && base + s * 4096 < a.K) {
+                if (a.pro == Q2_NORM && base + s * 4096 < K) {
                     load8(a.w + base + s * 4096, nw);
 #pragma unroll
                     for (int k = 0; k < 4; ++k) v[s][k] = pair_mul(pair_mul(v[s][k], inv2), nw[k]);
@@ -214,7 +246,7 @@ __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Arg
         for (int k = 0; k < 4; ++k) y[k] = pair_mul(y[k], pair_of(a.hat_inv, a.hat_inv));
         const Q8x8 q = quant8_pairs(y);
         const int at = base + s * 4096;
-        if (at < a.K) {
+        if (at < K) {
             // codes of (block, sub-block b, elements 8t .. 8t + 7) at block * 128 + (b & 1) * 64 + t * 16 + (b >> 1) * 8
             const int b = (at >> 5) & 3, e8 = (at >> 3) & 3;
             *reinterpret_cast<uint2 *>(codes + (at & ~127) + (b & 1) * 64 + e8 * 16 + (b >> 1) * 8) = make_uint2(q.w0, q.w1);
@@ -248,7 +280,9 @@ __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Arg
     int u = warp, gr = warp % ng, slot = 0;
     uint32_t phase = 0;
     bool alive = true;
-    // one piece: its group sums p_g of 16 rows go to `dst`
+    // one piece: its group sums p_g of 16 rows go to `dst` (SPLIT: to the CTA that adds them)
+    const int per_part = parts == 2 ? 128 : (parts == 3 ? 86 : 64);      // tile / parts = tile * per_part >> 8 for the few tiles of a cluster
+    float *fin = reinterpret_cast<float *>(smem + L.fin);                 // [tile of this CTA][group of all K][16]
     auto piece = [&](float *dst) {
         if (gr != group) set_group(gr);
         gr += gstep; if (gr >= ng) gr -= ng;
@@ -288,9 +322,36 @@ __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Arg
         float va = block_sum(e[0], e[1], f[0], f[1], dw), vb = block_sum(e[2], e[3], f[2], f[3], dw >> 16);
         va = __fadd_rn(va, __shfl_xor_sync(0xFFFFFFFFu, va, 1)); vb = __fadd_rn(vb, __shfl_xor_sync(0xFFFFFFFFu, vb, 1));
         va = __fadd_rn(va, __shfl_xor_sync(0xFFFFFFFFu, va, 2)); vb = __fadd_rn(vb, __shfl_xor_sync(0xFFFFFFFFu, vb, 2));
-        if (tig < 2) dst[g + 8 * tig] = tig ? vb : va;
+        if (SPLIT) {
+            const int tile = u / 8, round = tile * per_part >> 8, to = tile - round * parts;
+            uint32_t at;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(uint32_t(__cvta_generic_to_shared(fin + ((round * parts + rank) * 8 + (u & 7)) * 16 + g + 8 * tig))), "r"(to));
+            if (tig < 2) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(tig ? vb : va) : "memory");
+        } else if (tig < 2) dst[g + 8 * tig] = tig ? vb : va;
     };
     Q2_STAMP(6);
+    if (SPLIT) {
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");              // every CTA is running
+        for (; u < npieces; u += NW) piece(nullptr);
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        const int n = parts * 8;
+        if (row0 < min((t0 + nt) * 16, a.M)) {
+            const float *own = fin + (tid >> 4) * n * 16 + (tid & 15);
+            float s = own[0];
+            for (int k = 1; k < n; k += 8) {       // (loads first, then the adds in ascending order)
+                float x[8];
+#pragma unroll
+                for (int b = 0; b < 8; ++b) x[b] = own[min(k + b, n - 1) * 16];
+#pragma unroll
+                for (int b = 0; b < 8; ++b) if (b < 7 || k + 7 < n) s = __fadd_rn(s, x[b]);
+            }
+            if (a.out) a.out[row0] = s;
+            if (a.resid_out) a.resid_out[row0] = __fadd_rn(s, resid);
+        }
+        Q2_STAMP(7);
+        return;
+    }
     for (int c0 = 0; c0 < nt; c0 += run) {
         const int c1 = min(nt, c0 + run), uend = c1 * ng, rows = (c1 - c0) * 16;
         // what the sums below need, worked out ahead of the barrier
@@ -376,20 +437,22 @@ __global__ void k_sign_bits(const int32_t *__restrict__ signs, int nwords, uint8
     bits[i] = uint8_t(b);
 }
 
-template <int SPANS, bool LEAN>
-cudaError_t launch_spans(cudaStream_t st, int sm_count, Q2Args a, bool pdl) {
+template <int SPANS, bool LEAN, bool SPLIT = false>
+cudaError_t launch_spans(cudaStream_t st, int sm_count, Q2Args a, bool pdl, int clusters = 0) {
     // as many chunks of weights as fit beside the rest, and at least half of an SM's shared memory in all, so that two CTAs of a
     // launch never share an SM (see above)
-    const int ng = a.K / 512, tiles = (a.M + 15) / 16, grid = tiles < sm_count ? tiles : sm_count;
-    a.share = {tiles / grid, tiles % grid};
-    const int chunks = ((a.share.q + (a.share.r > 0)) * ng + NW - 1) / NW;
-    a.slots = std::min({chunks, MAX_SLOTS, (SMEM_MAX - layout(a.K).ring) / CHUNK});
-    const int smem = std::max(layout(a.K).ring + a.slots * CHUNK, 116 << 10);
+    const int parts = SPLIT ? a.K / 4096 : 1, K = SPLIT ? 4096 : a.K, units = SPLIT ? clusters : sm_count;
+    const int ng = K / 512, tiles = (a.M + 15) / 16, split = tiles < units ? tiles : units, grid = split * parts;
+    a.share = {tiles / split, tiles % split};
+    const int most = a.share.q + (a.share.r > 0), chunks = (most * ng + NW - 1) / NW;
+    a.fin = SPLIT ? (most + parts - 1) / parts * (a.K / 512) * 64 : 0;
+    a.slots = std::min({chunks, MAX_SLOTS, (SMEM_MAX - layout(K, a.fin).ring) / CHUNK});
+    const int smem = std::max(layout(K, a.fin).ring + a.slots * CHUNK, 116 << 10);
     // once, to the largest value, whatever this launch needs: with a limit that grows from call to call a second thread could lower
     // it again under the first (an SM changes its carve-out only when it is empty, so every projection asks for the largest one)
     static const cudaError_t limits = [] {
-        cudaError_t e = cudaFuncSetAttribute(k_q2_gemv<SPANS, LEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
-        return e != cudaSuccess ? e : cudaFuncSetAttribute(k_q2_gemv<SPANS, LEAN>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        cudaError_t e = cudaFuncSetAttribute(k_q2_gemv<SPANS, LEAN, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(k_q2_gemv<SPANS, LEAN, SPLIT>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     }();
     if (limits != cudaSuccess) return limits;
     a.inv_k = (a.K & (a.K - 1)) == 0 ? 1.0f / float(a.K) : 0.0f;
@@ -400,13 +463,36 @@ cudaError_t launch_spans(cudaStream_t st, int sm_count, Q2Args a, bool pdl) {
     cfg.blockDim = dim3(NT + 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2];
+    int n = 0;
+    if (pdl) { at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[n++].val.programmaticStreamSerializationAllowed = 1; }
+    if (SPLIT) { at[n].id = cudaLaunchAttributeClusterDimension; at[n].val.clusterDim.x = parts; at[n].val.clusterDim.y = 1; at[n++].val.clusterDim.z = 1; }
     cfg.attrs = at;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = n;
     BN_COUNT(1);
-    return cudaLaunchKernelEx(&cfg, k_q2_gemv<SPANS, LEAN>, a);
+    return cudaLaunchKernelEx(&cfg, k_q2_gemv<SPANS, LEAN, SPLIT>, a);
+}
+
+// Clusters of `parts` CTAs, one CTA per SM, that start together behind a kernel whose CTAs end one by one: an eighth fewer than the
+// occupancy query finds room for. Counted over 330 down projections in a chain of the 9B shape's, with 3 CTAs and room for 45: 45
+// clusters had one held up until another ended in 262 of them (11.0 us on average), 43 in 28 (7.3 us), 40 in none (6.96 us), and
+// 34 take 7.24 us.
+int split_clusters(int parts) {
+    static const std::array<int, 9> most = [] {
+        std::array<int, 9> m{};
+        if (cudaFuncSetAttribute(k_q2_gemv<1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX) == cudaSuccess)
+            for (int p = 2; p <= 4; ++p) {
+                cudaLaunchConfig_t cfg = {};
+                cfg.gridDim = dim3(p * 64); cfg.blockDim = dim3(NT + 32); cfg.dynamicSmemBytes = SMEM_MAX;
+                cudaLaunchAttribute at[1];
+                at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = p; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+                cfg.attrs = at; cfg.numAttrs = 1;
+                if (cudaOccupancyMaxActiveClusters(&m[p], k_q2_gemv<1, false, true>, &cfg) != cudaSuccess) m[p] = 0;
+            }
+        cudaGetLastError();                        // (a refusal is an answer, not a failed call)
+        return m;
+    }();
+    return most[parts] - most[parts] / 8;
 }
 
 }  // namespace
@@ -418,6 +504,11 @@ bool q2_gemv_supported(int K, int hat_block) {
 }
 
 cudaError_t launch_q2_gemv(cudaStream_t st, int sm_count, const Q2Args &a, bool pdl) {
+    if (a.K > 4096 && a.K % 4096 == 0 && a.pro == Q2_PLAIN && !a.swiglu) {
+        // a span per CTA of a cluster where that costs no CTA more than one further piece per warp: 0.8 us against 2.4 us of preparation
+        const int parts = a.K / 4096, n = split_clusters(parts), tiles = (a.M + 15) / 16, most = n ? (tiles + n - 1) / n : 0;
+        if (n && most <= 12 && most * 8 <= (tiles + sm_count - 1) / sm_count * (a.K / 512) + NW) return launch_spans<1, false, true>(st, sm_count, a, pdl, n);
+    }
     if (a.K > 4096) return launch_spans<4, false>(st, sm_count, a, pdl);
     return a.lean ? launch_spans<1, true>(st, sm_count, a, pdl) : launch_spans<1, false>(st, sm_count, a, pdl);
 }
