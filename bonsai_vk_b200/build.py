@@ -6,6 +6,7 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -58,6 +59,22 @@ def build_host(force: bool = False) -> str:
     return HOST_BIN
 
 
+FASTCALL = os.path.join(HERE, "_fastcall.so")
+
+
+def build_fastcall(force: bool = False) -> str:
+    """The CPython call layer of the op-level entry points (host/fastcall.c); lib.py uses ctypes where it is missing."""
+    src = os.path.join(HERE, "host", "fastcall.c")
+    if not force and not _stale(FASTCALL, [src]):
+        return FASTCALL
+    cmd = ["gcc", "-O2", "-Wall", "-fPIC", "-shared", "-I" + sysconfig.get_paths()["include"], "-o", FASTCALL, src]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("gcc failed building _fastcall.so")
+    return FASTCALL
+
+
 def build_oracle() -> None:
     """Compile the CPU oracle under oracle/ (and the reference shim when the reference tree is
     present). Building the oracle is not using it: only tests and the benchmark baselines load it."""
@@ -73,5 +90,6 @@ def build_oracle() -> None:
 if __name__ == "__main__":
     build_lib(verbose="-v" in sys.argv, force=True)
     build_host(force=True)
+    build_fastcall(force=True)
     build_oracle()
     print("built", LIB)

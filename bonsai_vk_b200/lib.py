@@ -109,8 +109,24 @@ def load_library() -> C.CDLL:
         f.restype = res
         f.argtypes = args
     lib._bn_signatures = sig
+    lib._bn_fast = _call_layer(lib, sig)
     _lib = lib
     return lib
+
+
+def _call_layer(lib, sig):
+    """The entry points that are called once per kernel or two, taking handles as integers: host/fastcall.c, or without it the same
+    functions through ctypes (1.0 to 1.6 us more a call)."""
+    names = ("bn_act_quant_q81", "bn_gemv_q81", "bn_gemm_act_quant", "bn_gemm_q81", "bn_attn_insert", "bn_attn_attend")
+    at = {n: C.cast(getattr(lib, n), C.c_void_p).value for n in names}
+    try:
+        from . import _fastcall
+    except ImportError:
+        import types
+        plain = (C.c_int, C.c_size_t)
+        return types.SimpleNamespace(**{n: C.CFUNCTYPE(C.c_int, *[t if t in plain else C.c_void_p for t in sig[n][1]])(at[n]) for n in names})
+    _fastcall.bind(at)
+    return _fastcall
 
 
 def declared_symbols() -> list[str]:
@@ -136,7 +152,7 @@ class Buffer:
         self.nbytes = int(nbytes)
         h = C.c_void_p()
         _check(ctx.lib.bn_alloc(ctx.h, self.nbytes, C.byref(h)), "bn_alloc")
-        self.h = h
+        self.h, self.p = h, h.value
 
     def upload(self, arr: np.ndarray, off: int = 0):
         a = np.ascontiguousarray(arr)
@@ -155,7 +171,7 @@ class Buffer:
     def free(self):
         if self.h is not None:
             self.ctx.lib.bn_free(self.ctx.h, self.h)
-            self.h = None
+            self.h, self.p = None, 0
 
 
 class Context:
@@ -165,13 +181,13 @@ class Context:
         self.lib = load_library()
         h = C.c_void_p()
         _check(self.lib.bn_init(device, C.byref(h)), "bn_init")
-        self.h = h
+        self.h, self.p, self.fast = h, h.value, self.lib._bn_fast
         self.device = device
 
     def close(self):
         if self.h is not None:
             self.lib.bn_destroy(self.h)
-            self.h = None
+            self.h, self.p = None, 0
 
     def alloc(self, nbytes: int) -> Buffer:
         return Buffer(self, nbytes)
@@ -198,7 +214,7 @@ class Context:
         b.ctx, b.nbytes = self, int(nbytes)
         h = C.c_void_p()
         _check(self.lib.bn_wrap(self.h, C.c_void_p(device_ptr), int(nbytes), C.byref(h)), "bn_wrap")
-        b.h = h
+        b.h, b.p = h, h.value
         return b
 
     def info(self):
@@ -229,24 +245,24 @@ class Context:
         return int(self.lib.bn_act_pack_bytes(K))
 
     def act_quant_q81(self, x: Buffer, K: int, pack: Buffer, x_off: int = 0, pack_off: int = 0):
-        _check(self.lib.bn_act_quant_q81(self.h, x.h, x_off, K, pack.h, pack_off), "bn_act_quant_q81")
+        _check(self.fast.bn_act_quant_q81(self.p, x.p, x_off, K, pack.p, pack_off), "bn_act_quant_q81")
 
     def gemv_q81(self, w: Buffer, M: int, K: int, pack: Buffer, out: Buffer, w_off: int = 0, pack_off: int = 0,
                  out_off: int = 0, dots: Buffer | None = None, dots_off: int = 0):
-        _check(self.lib.bn_gemv_q81(self.h, w.h, w_off, M, K, pack.h, pack_off, out.h, out_off,
-                                    dots.h if dots is not None else None, dots_off), "bn_gemv_q81")
+        _check(self.fast.bn_gemv_q81(self.p, w.p, w_off, M, K, pack.p, pack_off, out.p, out_off,
+                                     dots.p if dots is not None else 0, dots_off), "bn_gemv_q81")
 
     def attn_sizes(self, dims: "AttnDimsC"):
         return int(self.lib.bn_attn_kv_bytes(C.byref(dims))), int(self.lib.bn_attn_scratch_bytes(C.byref(dims)))
 
     def attn_insert(self, dims, kv: Buffer, k_rows: Buffer, v_rows: Buffer, n: int, pos0: int, qg: Buffer, q_norm: Buffer,
                     k_norm: Buffer, scratch: Buffer, k_off: int = 0, v_off: int = 0):
-        _check(self.lib.bn_attn_insert(self.h, C.byref(dims), kv.h, 0, k_rows.h, k_off, v_rows.h, v_off, n, pos0, qg.h, 0,
-                                       q_norm.h, 0, k_norm.h, 0, scratch.h, 0), "bn_attn_insert")
+        _check(self.fast.bn_attn_insert(self.p, C.addressof(dims), kv.p, 0, k_rows.p, k_off, v_rows.p, v_off, n, pos0, qg.p, 0,
+                                        q_norm.p, 0, k_norm.p, 0, scratch.p, 0), "bn_attn_insert")
 
     def attn_attend(self, dims, kv: Buffer, pos: int, scratch: Buffer, pregate: "Buffer | None", gated: Buffer):
-        _check(self.lib.bn_attn_attend(self.h, C.byref(dims), kv.h, 0, pos, scratch.h, 0,
-                                       pregate.h if pregate is not None else None, 0, gated.h, 0), "bn_attn_attend")
+        _check(self.fast.bn_attn_attend(self.p, C.addressof(dims), kv.p, 0, pos, scratch.p, 0,
+                                        pregate.p if pregate is not None else 0, 0, gated.p, 0), "bn_attn_attend")
 
     def gemv_q81_static(self, w: Buffer, M: int, K: int, pack: Buffer, out: Buffer, w_off: int = 0, pack_off: int = 0,
                         out_off: int = 0):
@@ -261,12 +277,12 @@ def _gemm_methods():
     def gemm_act_quant(self, x: Buffer, K: int, ncol: int, image: Buffer, signs: "Buffer | None" = None, hat_block: int = 0,
                        x_stride: int = 0, x_off: int = 0, signs_off: int = 0):
         """ncol fp32 vectors -> the activation image of the multi-column projection (optional rotation first)."""
-        _check(self.lib.bn_gemm_act_quant(self.h, x.h, x_off, x_stride or K, K, ncol, signs.h if signs is not None else None,
-                                          signs_off, hat_block, image.h, 0), "bn_gemm_act_quant")
+        _check(self.fast.bn_gemm_act_quant(self.p, x.p, x_off, x_stride or K, K, ncol, signs.p if signs is not None else 0,
+                                           signs_off, hat_block, image.p, 0), "bn_gemm_act_quant")
 
     def gemm_q81(self, w: Buffer, M: int, K: int, image: Buffer, ncol: int, out: Buffer, out_stride: int = 0, w_off: int = 0,
                  tiled: bool = False):
-        _check(self.lib.bn_gemm_q81(self.h, w.h, w_off, 1 if tiled else 0, M, K, image.h, 0, ncol, out.h, 0, out_stride or M),
+        _check(self.fast.bn_gemm_q81(self.p, w.p, w_off, 1 if tiled else 0, M, K, image.p, 0, ncol, out.p, 0, out_stride or M),
                "bn_gemm_q81")
 
     def gemm_repack(self, w: Buffer, M: int, K: int, w_off: int = 0) -> Buffer:

@@ -1,0 +1,37 @@
+"""The call layer of the op-level entry points (host/fastcall.c) and its stand-in through ctypes: the same return codes, error texts and
+treatment of arguments, without a GPU (every call is refused before it reaches one)."""
+import ctypes as C
+import sys
+
+import pytest
+
+from bonsai_vk_b200 import build, lib
+
+CALLS = {"bn_act_quant_q81": 6, "bn_gemv_q81": 11, "bn_gemm_act_quant": 11, "bn_gemm_q81": 12, "bn_attn_insert": 18, "bn_attn_attend": 11}
+
+
+@pytest.fixture(params=["native", "ctypes"])
+def layer(request, monkeypatch):
+    build.build_lib()
+    build.build_fastcall()
+    L = lib.load_library()
+    if request.param == "ctypes":
+        monkeypatch.setitem(sys.modules, "bonsai_vk_b200._fastcall", None)
+        monkeypatch.delattr(sys.modules["bonsai_vk_b200"], "_fastcall", raising=False)
+    return L, lib._call_layer(L, L._bn_signatures)
+
+
+@pytest.mark.parametrize("name", CALLS)
+def test_null_context_is_refused(layer, name):
+    L, fast = layer
+    assert getattr(fast, name)(*([0] * CALLS[name])) == -2
+    assert L.bn_last_error().decode() == f"{name}: null context"
+
+
+@pytest.mark.parametrize("name", CALLS)
+def test_arguments_are_checked(layer, name):
+    _, fast = layer
+    with pytest.raises((TypeError, C.ArgumentError)):
+        getattr(fast, name)(*([0] * (CALLS[name] - 1)))
+    with pytest.raises((TypeError, C.ArgumentError)):
+        getattr(fast, name)(*([0] * (CALLS[name] - 1) + [0.5]))
