@@ -572,6 +572,7 @@ void enqueue_batch(bn_model *m, int ncol, bool one_sequence = false) {
             prep(bnk::PREP_NORM, m->RES, L.attn_norm, m->signs, h.hidden, m->IMG_H, m->G + 48);
             bnk::Q2Next next = q2_next(L.q2_out, h.hidden, IN, nullptr);
             next.state = gdn_state_of(m, L.idx); next.cols = one_sequence ? 1 : ncol; next.col_bytes = NH * D * D * 4; next.col_stride = cols.gdn;
+            next.rows[0] = L.alpha_w; next.rows[1] = L.beta_w; next.rows_bytes = NH * h.hidden * 4;
             gemm(L.q2_in, C + IN, h.hidden, m->IMG_H, m->QKV, nullptr, next);
             const bnk::GdnDims gd{NH, NQ, D};
             if (one_sequence) {

@@ -46,6 +46,9 @@ struct Q2Next {
     const float *state = nullptr;
     int cols = 0, col_bytes = 0;
     size_t col_stride = 0;                // bytes
+    // and the rows of that mixer's small projections: two matrices of `rows_bytes`
+    const float *rows[2] = {nullptr, nullptr};
+    int rows_bytes = 0;
 };
 struct Q2Args {
     const uint8_t *W;            // two-bit tiles
@@ -102,6 +105,10 @@ __device__ __forceinline__ void q2_prefetch_next(const Q2Next &n, int cta, int p
     for (int k = cta + part * int(gridDim.x), per = (n.col_bytes + 16383) >> 14; k < n.cols * per; k += parts * int(gridDim.x)) {
         const int o = k % per * 16384;
         q2_prefetch(reinterpret_cast<const uint8_t *>(n.state) + size_t(k / per) * n.col_stride + o, min(16384, n.col_bytes - o));
+    }
+    for (int o = (cta + part * int(gridDim.x)) * 4096; o < n.rows_bytes; o += parts * int(gridDim.x) * 4096) {
+        q2_prefetch(reinterpret_cast<const uint8_t *>(n.rows[0]) + o, min(4096, n.rows_bytes - o));
+        q2_prefetch(reinterpret_cast<const uint8_t *>(n.rows[1]) + o, min(4096, n.rows_bytes - o));
     }
     if (!n.W) return;
     const uint8_t *src = n.W + size_t(cta * n.share.q + min(cta, n.share.r)) * n.unit_bytes;
