@@ -86,7 +86,7 @@ struct Q2GemmArgs {
     const float *resid; size_t resid_stride;       // optional: out = sum + resid (may alias out)
     Q2Next next;
     int *err;
-    int warm;                                      // the projection in front has fetched W towards L2 (Q2Next)
+    int warm;                                      // the projection in front fetches W towards L2 (Q2Next), and no kernel that may still be running writes it
     int kc, tiles;                                 // filled in by the launch;
     Q2Share share;                                 // filled in by the launch: the CTAs' shares of the row tiles
 };
