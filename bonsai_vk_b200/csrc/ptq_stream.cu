@@ -3,10 +3,12 @@
 //
 // The arithmetic and the way the trits reach the tensor cores are those of ptq_gemv.cu: one multiply by 3^(t+1) turns two weight
 // bytes into an int8 operand register [r, T, r', T'] and the operand table of the activation pack (two columns per sub-block)
-// does the rest. What bounds it is instruction issue: per 16 x 128 weights 32 products, 8 byte permutes, 8 tensor-core steps, 7
-// loads and a quarter of the epilogue, 80 warp instructions in all, against 145 in the kernel this replaces (two blocks per
-// warp, sums across the warps of the CTA inside the loop, 16 bulk copies of 896 bytes per 16 rows): 248 320 x 4096 in 116 us
-// before. The tensor cores need 27 us of it (half of every operand is residue bytes), memory 34 us.
+// does the rest. What bounds it is instruction issue and latency: per 16 x 128 weights 32 products (two cycles of a scheduler each, as
+// shift-and-adds one), 8 byte permutes, 8 tensor-core steps, 7 loads and a quarter of the epilogue, 80 warp instructions in all,
+// against 145 in the kernel this replaces (two blocks per warp, sums across the warps of the CTA inside the loop, 16 bulk copies of
+// 896 bytes per 16 rows): 248 320 x 4096 in 116 us before. The tensor cores need 27 us of it (half of every operand is residue bytes),
+// memory 34 us. Measured beside it: pieces of a tile taken side by side, so that no line of DRAM comes in twice (232 MB are read for a
+// matrix of 117): with the warps' operands reloaded 96 us, from a table in shared memory and 16 warps 80 us.
 //
 // Work split. A CTA of 12 warps (16 of 128 registers each were slower: 16.1 against 13.9 us at 24 576 x 4096) owns a run of 16-row tiles over all of K. The pieces (16 rows x 4 blocks, the unit p_g of the
 // summation order) of a run are dealt to the warps group-major, so a warp stays with one group's operand table - 64 registers -
@@ -15,6 +17,7 @@
 // allows) into a ring of its warp's own. The pitch of 112 bytes is free of bank conflicts for every load of the loop: eight rows
 // start four banks apart and the four lanes of a row read words 0, 2, 3, 5 (one in each residue modulo 4).
 #include "ops.cuh"
+#include "q2.cuh"
 #include "rotate_quant.cuh"
 
 #include <algorithm>
@@ -47,31 +50,35 @@ template <int ALIGN> __device__ __forceinline__ void cp_async(uint32_t dst, cons
     else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(ALIGN) : "memory");
 }
 
-// two blocks of the same 16 rows: two chains of eight dependent tensor-core steps side by side (products v * 3^(t+1))
 struct Bytes { uint32_t h0, h1, h2, hq; };
 __device__ __forceinline__ Bytes split(uint32_t f, uint32_t s, uint32_t w6, uint32_t sel2) {
     return {__byte_perm(f, 0u, 0x4240u), __byte_perm(f, 0u, 0x4341u), __byte_perm(s, 0u, sel2), __byte_perm(w6, 0u, 0x4140u)};
 }
-__device__ __forceinline__ void block_dots2(int (&c)[4], int (&e)[4], const uint32_t *r0, const uint32_t *r1, int first, int second, uint32_t sel2, uint32_t cq,
-                                            const uint2 (&B)[8], const uint2 (&E)[8]) {
-    const Bytes a = split(r0[first], r0[second], r0[6], sel2), b = split(r1[first], r1[second], r1[6], sel2);
-    const Bytes f = split(r0[7 + first], r0[7 + second], r0[13], sel2), g = split(r1[7 + first], r1[7 + second], r1[13], sel2);
-    mma_first(c, a.h0 * 3u, b.h0 * 3u, a.h0 * 9u, b.h0 * 9u, B[0]);
-    mma_first(e, f.h0 * 3u, g.h0 * 3u, f.h0 * 9u, g.h0 * 9u, E[0]);
-    mma(c, a.h0 * 27u, b.h0 * 27u, a.h0 * 81u, b.h0 * 81u, B[1]);
-    mma(e, f.h0 * 27u, g.h0 * 27u, f.h0 * 81u, g.h0 * 81u, E[1]);
-    mma(c, a.h0 * 243u, b.h0 * 243u, a.h1 * 3u, b.h1 * 3u, B[2]);
-    mma(e, f.h0 * 243u, g.h0 * 243u, f.h1 * 3u, g.h1 * 3u, E[2]);
-    mma(c, a.h1 * 9u, b.h1 * 9u, a.h1 * 27u, b.h1 * 27u, B[3]);
-    mma(e, f.h1 * 9u, g.h1 * 9u, f.h1 * 27u, g.h1 * 27u, E[3]);
-    mma(c, a.h1 * 81u, b.h1 * 81u, a.h1 * 243u, b.h1 * 243u, B[4]);
-    mma(e, f.h1 * 81u, g.h1 * 81u, f.h1 * 243u, g.h1 * 243u, E[4]);
-    mma(c, a.h2 * 3u, b.h2 * 3u, a.h2 * 9u, b.h2 * 9u, B[5]);
-    mma(e, f.h2 * 3u, g.h2 * 3u, f.h2 * 9u, g.h2 * 9u, E[5]);
-    mma(c, a.h2 * 27u, b.h2 * 27u, a.h2 * 81u, b.h2 * 81u, B[6]);
-    mma(e, f.h2 * 27u, g.h2 * 27u, f.h2 * 81u, g.h2 * 81u, E[6]);
-    mma(c, a.h2 * 243u, b.h2 * 243u, a.hq * cq, b.hq * cq, B[7]);
-    mma(e, f.h2 * 243u, g.h2 * 243u, f.hq * cq, g.hq * cq, E[7]);
+// two blocks of the same 16 rows: two chains of eight dependent tensor-core steps side by side. Operand register r is the byte pairs
+// r / 5 times 3^(r % 5 + 1), the sixteenth the last two bytes at a level of the lane's own. MANY: each product from the one before, as a
+// shift-and-add.
+template <bool MANY> __device__ __forceinline__ void block_dots2(int (&c)[4], int (&e)[4], const uint32_t *r0, const uint32_t *r1, int first, int second,
+                                                                 uint32_t sel2, uint32_t cq, const uint2 (&B)[8], const uint2 (&E)[8]) {
+    const Bytes v[4] = {split(r0[first], r0[second], r0[6], sel2), split(r1[first], r1[second], r1[6], sel2),
+                        split(r0[7 + first], r0[7 + second], r0[13], sel2), split(r1[7 + first], r1[7 + second], r1[13], sel2)};
+    constexpr uint32_t pow3[5] = {3u, 9u, 27u, 81u, 243u};
+    uint32_t h[3][4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { h[0][k] = v[k].h0; h[1][k] = v[k].h1; h[2][k] = v[k].h2; }
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+        uint32_t x[2][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int r = 2 * m + i;
+                x[i][k] = r == 15 ? v[k].hq * cq : (MANY ? times3(h[r / 5 % 3][k]) : h[r / 5 % 3][k] * pow3[r % 5]);
+                if (MANY && r < 15) h[r / 5 % 3][k] = x[i][k];
+            }
+        if (m == 0) { mma_first(c, x[0][0], x[0][1], x[1][0], x[1][1], B[0]); mma_first(e, x[0][2], x[0][3], x[1][2], x[1][3], E[0]); }
+        else { mma(c, x[0][0], x[0][1], x[1][0], x[1][1], B[m]); mma(e, x[0][2], x[0][3], x[1][2], x[1][3], E[m]); }
+    }
 }
 // x[b]: this lane's sub-block (lane & 3) of block b -> the sum (t0 + t1) + (t2 + t3) of block lane & 3
 __device__ __forceinline__ float quad_transpose_sum(const float (&x)[4], bool odd, bool hi) {
@@ -80,7 +87,7 @@ __device__ __forceinline__ float quad_transpose_sum(const float (&x)[4], bool od
     return __fadd_rn(hi ? yb : ya, __shfl_xor_sync(0xFFFFFFFFu, hi ? ya : yb, 2));
 }
 
-template <int ALIGN>
+template <int ALIGN, bool MANY>
 __global__ void __launch_bounds__(NT, 1) k_ptq_stream(const StreamArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     uint4 *offs = reinterpret_cast<uint4 *>(smem + NW * ST * PIECE);       // where a lane's four 16-byte copies of a piece start
@@ -164,7 +171,7 @@ __global__ void __launch_bounds__(NT, 1) k_ptq_stream(const StreamArgs a) {
             const uint32_t *r0 = reinterpret_cast<const uint32_t *>(ring + slot * PIECE + g * 112), *r1 = r0 + 8 * 28;
             int c[4][4];
 #pragma unroll
-            for (int j = 0; j < 4; j += 2) block_dots2(c[j], c[j + 1], r0 + 7 * j, r1 + 7 * j, first, second, sel2, cq, B[j], B[j + 1]);
+            for (int j = 0; j < 4; j += 2) block_dots2<MANY>(c[j], c[j + 1], r0 + 7 * j, r1 + 7 * j, first, second, sel2, cq, B[j], B[j + 1]);
             const uint32_t da = r0[7 * tig + 6], db = r1[7 * tig + 6];
             float xa[4], xb[4];
 #pragma unroll
@@ -202,15 +209,15 @@ __global__ void __launch_bounds__(NT, 1) k_ptq_stream(const StreamArgs a) {
     }
 }
 
-template <int ALIGN>
+template <int ALIGN, bool MANY = false>
 cudaError_t launch_a(cudaStream_t st, int grid, size_t smem, const StreamArgs &a) {
     static bool set = false;
     if (!set) {
-        cudaError_t e = cudaFuncSetAttribute(k_ptq_stream<ALIGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, NW * ST * PIECE + 512 + MAX_PIECES * 64);
+        cudaError_t e = cudaFuncSetAttribute(k_ptq_stream<ALIGN, MANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, NW * ST * PIECE + 512 + MAX_PIECES * 64);
         if (e != cudaSuccess) return e;
         set = true;
     }
-    launch(k_ptq_stream<ALIGN>, dim3(grid), dim3(NT), smem, st, a);
+    launch(k_ptq_stream<ALIGN, MANY>, dim3(grid), dim3(NT), smem, st, a);
     return cudaGetLastError();
 }
 
@@ -231,7 +238,10 @@ cudaError_t ptq_stream(cudaStream_t st, int sm_count, const void *W, int M, int 
     const size_t smem = size_t(NW) * ST * PIECE + 512 + size_t(a.run) * ng * 64;
     // the widest copy that every row of every piece starts on
     const uintptr_t align = reinterpret_cast<uintptr_t>(W) | uintptr_t(a.nb * 28);
-    if (align % 16 == 0) return launch_a<16>(st, grid, smem, a);
+    // A chain of shift-and-adds per half-word pair where a CTA has many pieces (248 320 x 4096: 79.3 -> 75.3 us, 30 000 x 8192 23.9 ->
+    // 23.4), products side by side where the first piece's latency counts (1024 x 4096 3.2 against 3.4 us, 7000 x 3584 5.4 against
+    // 5.5) and where copies of 4 or 8 bytes take the issue slots (30 000 x 4736 20.3 against 20.7).
+    if (align % 16 == 0) return most * ng >= 10 * NW ? launch_a<16, true>(st, grid, smem, a) : launch_a<16>(st, grid, smem, a);
     if (align % 8 == 0) return launch_a<8>(st, grid, smem, a);
     return launch_a<4>(st, grid, smem, a);
 }

@@ -141,14 +141,20 @@ __device__ __forceinline__ void q2_mma(int (&d)[4], uint32_t a0, uint32_t a1, ui
         : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// x * 3 as a shift-and-add, which runs at twice the rate of a multiplication (left to itself the compiler makes it one again)
+__device__ __forceinline__ uint32_t times3(uint32_t x) {
+    uint32_t y;
+    asm("{\n.reg .u32 t;\nshl.b32 t, %1, 1;\nadd.u32 %0, t, %1;\n}\n" : "=r"(y) : "r"(x));
+    return y;
+}
 // four packed bytes: five base-3 digits per byte, each in a byte of its own word (T_t = (b * 3^(t+1)) >> 8 is the base-3 prefix of
 // byte b, digit t = T_t - 3 T_(t-1))
 __device__ __forceinline__ void q2_unpack4(uint32_t w, uint32_t *o, int stride) {
-    const uint32_t e = __byte_perm(w, 0u, 0x4240u), d = __byte_perm(w, 0u, 0x4341u);
-    uint32_t prev = 0u, p = 3u;
+    uint32_t e = __byte_perm(w, 0u, 0x4240u), d = __byte_perm(w, 0u, 0x4341u), prev = 0u;
 #pragma unroll
-    for (int t = 0; t < 5; ++t, p *= 3u) {
-        const uint32_t T = __byte_perm(e * p, d * p, 0x7351u);
+    for (int t = 0; t < 5; ++t) {
+        e = times3(e); d = times3(d);
+        const uint32_t T = __byte_perm(e, d, 0x7351u);
         o[t * stride] = T - 3u * prev;
         prev = T;
     }
