@@ -341,7 +341,7 @@ bool build_token_ops(bn_model *m) {
     const int QD = h.n_head * h.head_dim, KD = h.n_kv * h.head_dim;
     const int sm = m->ctx->sm_count;
     // Opt-in (BONSAI_TOKEN_KERNEL=1): measured on the 9B shape the one-launch token is slower than the launch-per-phase
-    // schedule with programmatic dependent launch (3.1 ms against 2.2 ms per token then, 1.19 now) - every phase pays a grid barrier and
+    // schedule with programmatic dependent launch (3.1 ms against 2.2 ms per token then, 1.10 now) - every phase pays a grid barrier and
     // nothing overlaps across phases - so the default stays the captured graph.
     if (!getenv("BONSAI_TOKEN_KERNEL")) return false;
     if (!m->fused || m->b0 != 0 || m->b1 != h.n_layer) return false;

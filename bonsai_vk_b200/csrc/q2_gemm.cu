@@ -8,13 +8,13 @@
 // ANDs per 16 rows. The accumulators of mma.sync are registers, in the layout the combination wants; tcgen05 would bring them
 // through tensor memory and hand-offs between warps: the kernel that did so, with the operand decoded into tensor memory, took
 // 28 / 33 us for 24 576 x 4096 at 8 / 16 columns (a tcgen05.mma of 128 rows costs 190 cycles whatever its column count, and the
-// tensor pipe is idle either way). Here, weights from DRAM, back to back, without the preparation of the columns: 11.1 / 15.5 us;
-// 4096 x 12 288: 7.2 / 12.9 us.
+// tensor pipe is idle either way). Here, weights from DRAM, back to back, without the preparation of the columns: 11.1 / 15.4 us;
+// 4096 x 12 288: 7.2 / 11.5 us.
 //
 // Work split. A CTA of 12 or 16 warps owns a run of row tiles over all of K. K is walked in waves of `kc` groups (512 weights each);
 // a wave's piece of the activation image is double-buffered in shared memory. A wave's units (MT row tiles, one group, up to 16
 // columns) are dealt to the warps; a unit keeps everything in registers and leaves its group sums p_g in shared memory, where
-// after a barrier every thread adds its own (row, column)s' in ascending order. MT = 2 or 3 row tiles share a group's operands and
+// after a barrier every thread adds its own (row, column)s' in ascending order. MT = 2 (or 3, or for native rows 1) row tiles share a group's operands and
 // scales: with one, shared-memory reads (24 wavefronts per 16 rows x 8 columns x 128 weights) would bound the loop.
 #include "q2.cuh"
 #include "rotate_quant.cuh"
