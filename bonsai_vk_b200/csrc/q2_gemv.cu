@@ -75,6 +75,9 @@ template <int WHICH> __device__ __forceinline__ int special() {
     else asm("mov.u32 %0, %%clusterid.x;" : "=r"(v));
     return v;
 }
+// to the other CTAs of the cluster: this one is running. Nothing is published with it: as a release it waits for the accesses before
+// it, 0.3 us of every launch (48 tokens 52.8 ms, relaxed 52.4).
+__device__ __forceinline__ void running() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 // SPANS: spans of 4096 values whose inputs a thread holds at once (1: K <= 4096; 4: up to 16384)
 // LEAN: 80 registers instead of 94, so that beside the 17 warps (five of them on one of the SM's four schedulers, each with
 // 16 384 registers) the CTA of a latency-bound mixer kernel fits, and a shared-memory carve-out that leaves room for it: the
@@ -101,7 +104,7 @@ __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Arg
     const int npieces = nt * ng, nchunks = (npieces + NW - 1) / NW;
     const uint32_t full = uint32_t(__cvta_generic_to_shared(smem + L.bars)), empty = full + MAX_SLOTS * 8;
 
-    if (SPLIT) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // "I am running"
+    if (SPLIT) running();
     if (warp == NW) {
         // ---- copy warp. Before the previous kernel is done: one chunk of weights into the ring (more would hold up the input
         // vector, which follows it through the same queue, by up to a microsecond) and the NEXT projection's weights (the
@@ -142,6 +145,7 @@ __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Arg
             if (++s == slots) { s = 0; ph ^= 1; }
         }
         if (SPLIT) {                               // (both cluster barriers with the other warps)
+            __syncwarp();
             asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
             asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
             asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -333,6 +337,7 @@ __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Arg
     if (SPLIT) {
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");              // every CTA is running
         for (; u < npieces; u += NW) piece(nullptr);
+        __syncwarp();
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         const int n = parts * 8;
