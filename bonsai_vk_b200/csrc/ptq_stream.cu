@@ -54,14 +54,35 @@ struct Bytes { uint32_t h0, h1, h2, hq; };
 __device__ __forceinline__ Bytes split(uint32_t f, uint32_t s, uint32_t w6, uint32_t sel2) {
     return {__byte_perm(f, 0u, 0x4240u), __byte_perm(f, 0u, 0x4341u), __byte_perm(s, 0u, sel2), __byte_perm(w6, 0u, 0x4140u)};
 }
-// two blocks of the same 16 rows: two chains of eight dependent tensor-core steps side by side. Operand register r is the byte pairs
-// r / 5 times 3^(r % 5 + 1), the sixteenth the last two bytes at a level of the lane's own. MANY: each product from the one before, as a
-// shift-and-add.
-template <bool MANY> __device__ __forceinline__ void block_dots2(int (&c)[4], int (&e)[4], const uint32_t *r0, const uint32_t *r1, int first, int second,
-                                                                 uint32_t sel2, uint32_t cq, const uint2 (&B)[8], const uint2 (&E)[8]) {
+// two blocks of the same 16 rows: two chains of eight dependent tensor-core steps side by side (products v * 3^(t+1), written out: as the
+// loop below 1 % slower)
+__device__ __forceinline__ void block_dots2(int (&c)[4], int (&e)[4], const uint32_t *r0, const uint32_t *r1, int first, int second, uint32_t sel2, uint32_t cq,
+                                            const uint2 (&B)[8], const uint2 (&E)[8]) {
+    const Bytes a = split(r0[first], r0[second], r0[6], sel2), b = split(r1[first], r1[second], r1[6], sel2);
+    const Bytes f = split(r0[7 + first], r0[7 + second], r0[13], sel2), g = split(r1[7 + first], r1[7 + second], r1[13], sel2);
+    mma_first(c, a.h0 * 3u, b.h0 * 3u, a.h0 * 9u, b.h0 * 9u, B[0]);
+    mma_first(e, f.h0 * 3u, g.h0 * 3u, f.h0 * 9u, g.h0 * 9u, E[0]);
+    mma(c, a.h0 * 27u, b.h0 * 27u, a.h0 * 81u, b.h0 * 81u, B[1]);
+    mma(e, f.h0 * 27u, g.h0 * 27u, f.h0 * 81u, g.h0 * 81u, E[1]);
+    mma(c, a.h0 * 243u, b.h0 * 243u, a.h1 * 3u, b.h1 * 3u, B[2]);
+    mma(e, f.h0 * 243u, g.h0 * 243u, f.h1 * 3u, g.h1 * 3u, E[2]);
+    mma(c, a.h1 * 9u, b.h1 * 9u, a.h1 * 27u, b.h1 * 27u, B[3]);
+    mma(e, f.h1 * 9u, g.h1 * 9u, f.h1 * 27u, g.h1 * 27u, E[3]);
+    mma(c, a.h1 * 81u, b.h1 * 81u, a.h1 * 243u, b.h1 * 243u, B[4]);
+    mma(e, f.h1 * 81u, g.h1 * 81u, f.h1 * 243u, g.h1 * 243u, E[4]);
+    mma(c, a.h2 * 3u, b.h2 * 3u, a.h2 * 9u, b.h2 * 9u, B[5]);
+    mma(e, f.h2 * 3u, g.h2 * 3u, f.h2 * 9u, g.h2 * 9u, E[5]);
+    mma(c, a.h2 * 27u, b.h2 * 27u, a.h2 * 81u, b.h2 * 81u, B[6]);
+    mma(e, f.h2 * 27u, g.h2 * 27u, f.h2 * 81u, g.h2 * 81u, E[6]);
+    mma(c, a.h2 * 243u, b.h2 * 243u, a.hq * cq, b.hq * cq, B[7]);
+    mma(e, f.h2 * 243u, g.h2 * 243u, f.hq * cq, g.hq * cq, E[7]);
+}
+// the same with each product from the one before, as a shift-and-add; operand register r is the byte pairs r / 5 times 3^(r % 5 + 1), the
+// sixteenth the last two bytes at a level of the lane's own
+__device__ __forceinline__ void block_dots2_chained(int (&c)[4], int (&e)[4], const uint32_t *r0, const uint32_t *r1, int first, int second, uint32_t sel2, uint32_t cq,
+                                            const uint2 (&B)[8], const uint2 (&E)[8]) {
     const Bytes v[4] = {split(r0[first], r0[second], r0[6], sel2), split(r1[first], r1[second], r1[6], sel2),
                         split(r0[7 + first], r0[7 + second], r0[13], sel2), split(r1[7 + first], r1[7 + second], r1[13], sel2)};
-    constexpr uint32_t pow3[5] = {3u, 9u, 27u, 81u, 243u};
     uint32_t h[3][4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) { h[0][k] = v[k].h0; h[1][k] = v[k].h1; h[2][k] = v[k].h2; }
@@ -73,8 +94,8 @@ template <bool MANY> __device__ __forceinline__ void block_dots2(int (&c)[4], in
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const int r = 2 * m + i;
-                x[i][k] = r == 15 ? v[k].hq * cq : (MANY ? times3(h[r / 5 % 3][k]) : h[r / 5 % 3][k] * pow3[r % 5]);
-                if (MANY && r < 15) h[r / 5 % 3][k] = x[i][k];
+                x[i][k] = r == 15 ? v[k].hq * cq : times3(h[r / 5 % 3][k]);
+                if (r < 15) h[r / 5 % 3][k] = x[i][k];
             }
         if (m == 0) { mma_first(c, x[0][0], x[0][1], x[1][0], x[1][1], B[0]); mma_first(e, x[0][2], x[0][3], x[1][2], x[1][3], E[0]); }
         else { mma(c, x[0][0], x[0][1], x[1][0], x[1][1], B[m]); mma(e, x[0][2], x[0][3], x[1][2], x[1][3], E[m]); }
@@ -171,7 +192,10 @@ __global__ void __launch_bounds__(NT, 1) k_ptq_stream(const StreamArgs a) {
             const uint32_t *r0 = reinterpret_cast<const uint32_t *>(ring + slot * PIECE + g * 112), *r1 = r0 + 8 * 28;
             int c[4][4];
 #pragma unroll
-            for (int j = 0; j < 4; j += 2) block_dots2<MANY>(c[j], c[j + 1], r0 + 7 * j, r1 + 7 * j, first, second, sel2, cq, B[j], B[j + 1]);
+            for (int j = 0; j < 4; j += 2) {
+                if (MANY) block_dots2_chained(c[j], c[j + 1], r0 + 7 * j, r1 + 7 * j, first, second, sel2, cq, B[j], B[j + 1]);
+                else block_dots2(c[j], c[j + 1], r0 + 7 * j, r1 + 7 * j, first, second, sel2, cq, B[j], B[j + 1]);
+            }
             const uint32_t da = r0[7 * tig + 6], db = r1[7 * tig + 6];
             float xa[4], xb[4];
 #pragma unroll
