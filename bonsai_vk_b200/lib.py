@@ -138,6 +138,14 @@ def declared_symbols() -> list[str]:
     return sorted(set(re.findall(r"\b(bn_[a-z0-9_]+)\s*\(", text)))
 
 
+def _dims_address(dims) -> int:
+    """The address of an AttnDimsC. The call layer takes it as a number, so what else would be read as sizes is refused here."""
+    at = C.addressof(dims)
+    if not isinstance(dims, AttnDimsC):
+        raise C.ArgumentError(f"expected AttnDimsC instance instead of {type(dims).__name__}")
+    return at
+
+
 def _check(rc: int, what: str):
     if rc != 0:
         msg = load_library().bn_last_error().decode()
@@ -257,11 +265,11 @@ class Context:
 
     def attn_insert(self, dims, kv: Buffer, k_rows: Buffer, v_rows: Buffer, n: int, pos0: int, qg: Buffer, q_norm: Buffer,
                     k_norm: Buffer, scratch: Buffer, k_off: int = 0, v_off: int = 0):
-        _check(self.fast.bn_attn_insert(self.p, C.addressof(dims), kv.p, 0, k_rows.p, k_off, v_rows.p, v_off, n, pos0, qg.p, 0,
+        _check(self.fast.bn_attn_insert(self.p, _dims_address(dims), kv.p, 0, k_rows.p, k_off, v_rows.p, v_off, n, pos0, qg.p, 0,
                                         q_norm.p, 0, k_norm.p, 0, scratch.p, 0), "bn_attn_insert")
 
     def attn_attend(self, dims, kv: Buffer, pos: int, scratch: Buffer, pregate: "Buffer | None", gated: Buffer):
-        _check(self.fast.bn_attn_attend(self.p, C.addressof(dims), kv.p, 0, pos, scratch.p, 0,
+        _check(self.fast.bn_attn_attend(self.p, _dims_address(dims), kv.p, 0, pos, scratch.p, 0,
                                         pregate.p if pregate is not None else 0, 0, gated.p, 0), "bn_attn_attend")
 
     def gemv_q81_static(self, w: Buffer, M: int, K: int, pack: Buffer, out: Buffer, w_off: int = 0, pack_off: int = 0,

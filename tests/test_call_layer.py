@@ -2,10 +2,11 @@
 treatment of arguments, without a GPU (every call is refused before it reaches one)."""
 import ctypes as C
 import sys
+import types
 
 import pytest
 
-from bonsai_vk_b200 import build, lib
+from bonsai_vk_b200 import BonsaiError, Context, build, lib
 
 CALLS = {"bn_act_quant_q81": 6, "bn_gemv_q81": 11, "bn_gemm_act_quant": 11, "bn_gemm_q81": 12, "bn_attn_insert": 18, "bn_attn_attend": 11}
 
@@ -35,3 +36,25 @@ def test_arguments_are_checked(layer, name):
         getattr(fast, name)(*([0] * (CALLS[name] - 1)))
     with pytest.raises((TypeError, C.ArgumentError)):
         getattr(fast, name)(*([0] * (CALLS[name] - 1) + [0.5]))
+
+
+class _Short(C.Structure):
+    _fields_ = [("n_head", C.c_int32)]
+
+
+class _Longer(lib.AttnDimsC):
+    _fields_ = [("more", C.c_int32)]
+
+
+@pytest.mark.parametrize("dims,refusal", [
+    (lib.AttnDimsC(), None), (_Longer(), None),
+    (lib.HParamsC(), C.ArgumentError), (_Short(), C.ArgumentError), (C.c_int(16), C.ArgumentError), (C.pointer(lib.AttnDimsC()), C.ArgumentError),
+    ((lib.AttnDimsC * 2)(), C.ArgumentError), (None, TypeError), (16, TypeError)])
+def test_attention_takes_its_own_dims_only(layer, dims, refusal):
+    """Only an AttnDimsC may be read as sizes; a call that gets that far is refused for its null context."""
+    L, fast = layer
+    c, b = types.SimpleNamespace(fast=fast, lib=L, p=0), types.SimpleNamespace(p=0)
+    with pytest.raises(refusal or BonsaiError):
+        Context.attn_insert(c, dims, b, b, b, 1, 0, b, b, b, b)
+    with pytest.raises(refusal or BonsaiError):
+        Context.attn_attend(c, dims, b, 0, b, None, b)
