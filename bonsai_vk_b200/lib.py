@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
 
 import numpy as np
@@ -152,7 +153,29 @@ def _check(rc: int, what: str):
         raise BonsaiError(f"{what} failed ({rc}): {msg}")
 
 
-class Buffer:
+class _Handle:
+    """`h`, the library's handle, and `p`, the same as the number that the call layer takes (0: none): kept beside a handle that is
+    assigned, looked up each time while there is none, since a ctypes pointer may be filled in behind the assignment."""
+    _h = None
+
+    @property
+    def h(self):
+        return self._h
+
+    @h.setter
+    def h(self, handle):
+        self._h = handle
+        self.__dict__.pop("p", None)
+        if self.p:
+            self.__dict__["p"] = self.p
+
+    def __getattr__(self, name):
+        if name != "p":
+            raise AttributeError(f"{type(self).__name__!r} object has no attribute {name!r}")
+        return (self._h.value if isinstance(self._h, C.c_void_p) else self._h) or 0
+
+
+class Buffer(_Handle):
     """Device buffer owned by the library; named by handle + byte offset in every op."""
 
     def __init__(self, ctx: "Context", nbytes: int):
@@ -160,7 +183,7 @@ class Buffer:
         self.nbytes = int(nbytes)
         h = C.c_void_p()
         _check(ctx.lib.bn_alloc(ctx.h, self.nbytes, C.byref(h)), "bn_alloc")
-        self.h, self.p = h, h.value
+        self.h = h
 
     def upload(self, arr: np.ndarray, off: int = 0):
         a = np.ascontiguousarray(arr)
@@ -179,23 +202,27 @@ class Buffer:
     def free(self):
         if self.h is not None:
             self.ctx.lib.bn_free(self.ctx.h, self.h)
-            self.h, self.p = None, 0
+            self.h = None
 
 
-class Context:
+class Context(_Handle):
     """One context per GPU (reference: the single Vulkan device + queue of vk_ctx_init)."""
 
     def __init__(self, device: int = 0):
         self.lib = load_library()
         h = C.c_void_p()
         _check(self.lib.bn_init(device, C.byref(h)), "bn_init")
-        self.h, self.p, self.fast = h, h.value, self.lib._bn_fast
+        self.h = h
         self.device = device
+
+    @functools.cached_property
+    def fast(self):
+        return self.lib._bn_fast
 
     def close(self):
         if self.h is not None:
             self.lib.bn_destroy(self.h)
-            self.h, self.p = None, 0
+            self.h = None
 
     def alloc(self, nbytes: int) -> Buffer:
         return Buffer(self, nbytes)
@@ -222,7 +249,7 @@ class Context:
         b.ctx, b.nbytes = self, int(nbytes)
         h = C.c_void_p()
         _check(self.lib.bn_wrap(self.h, C.c_void_p(device_ptr), int(nbytes), C.byref(h)), "bn_wrap")
-        b.h, b.p = h, h.value
+        b.h = h
         return b
 
     def info(self):

@@ -6,7 +6,7 @@ import types
 
 import pytest
 
-from bonsai_vk_b200 import BonsaiError, Context, build, lib
+from bonsai_vk_b200 import BonsaiError, Buffer, Context, build, lib
 
 CALLS = {"bn_act_quant_q81": 6, "bn_gemv_q81": 11, "bn_gemm_act_quant": 11, "bn_gemm_q81": 12, "bn_attn_insert": 18, "bn_attn_attend": 11}
 
@@ -58,3 +58,19 @@ def test_attention_takes_its_own_dims_only(layer, dims, refusal):
         Context.attn_insert(c, dims, b, b, b, 1, 0, b, b, b, b)
     with pytest.raises(refusal or BonsaiError):
         Context.attn_attend(c, dims, b, 0, b, None, b)
+
+
+def test_number_follows_the_handle():
+    """Objects whose handle was made elsewhere work, and a handle that is taken away is gone for every call."""
+    build.build_lib()
+    c, b = Context.__new__(Context), Buffer.__new__(Buffer)
+    c.lib = lib.load_library()
+    c.h, b.h = None, C.c_void_p(0x7000)
+    assert (c.p, b.p) == (0, 0x7000) and b.h.value == 0x7000
+    with pytest.raises(BonsaiError, match="null context"):
+        c.gemv_q81(b, 16, 512, b, b)
+    b.h = None
+    assert b.p == 0
+    b.h = C.c_void_p()
+    b.h.value = 0x8000                                      # (as a call that takes C.byref(b.h) does)
+    assert b.p == 0x8000
