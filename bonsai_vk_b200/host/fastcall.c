@@ -9,24 +9,32 @@
 #include <stddef.h>
 #include <stdint.h>
 
-typedef void *P;
-typedef size_t Z;
+/* the whole numbers of a call as 64-bit patterns; 0 where an argument is none */
+static int whole(PyObject *const *a, Py_ssize_t n, uint64_t *v) {
+    for (Py_ssize_t i = 0; i < n; ++i) {
+        v[i] = PyLong_AsUnsignedLongLongMask(a[i]);
+        if (v[i] == (uint64_t)-1 && PyErr_Occurred()) return 0;
+    }
+    return 1;
+}
+#define P(i) ((void *)(uintptr_t)v[i])
+#define Z(i) ((size_t)v[i])
+#define I(i) ((int)(uint32_t)v[i])
 
-/* argument i as a 64-bit pattern; errors are collected and looked at once */
-static uint64_t arg(PyObject *const *a, Py_ssize_t i) { return PyLong_AsUnsignedLongLongMask(a[i]); }
-#define AP(i) ((P)(uintptr_t)arg(a, i))
-#define AZ(i) ((Z)arg(a, i))
-#define AI(i) ((int)(uint32_t)arg(a, i))
-
-/* one entry point: NAME, number of arguments, the C prototype and the converted arguments */
-#define ENTRY(NAME, N, PROTO, DECL, ARGS)                                                        \
+/* one entry point: NAME, number of arguments, the C prototype and the converted arguments. What is no whole number (a ctypes instance,
+ * or a mistake) goes to the ctypes function, which takes or refuses it. */
+#define ENTRY(NAME, N, PROTO, ARGS)                                                              \
     static int(*p_##NAME) PROTO;                                                                 \
+    static PyObject *c_##NAME;                                                                   \
     static PyObject *f_##NAME(PyObject *self, PyObject *const *a, Py_ssize_t n) {                \
         (void)self;                                                                              \
         if (n != N) return PyErr_Format(PyExc_TypeError, #NAME " takes %d arguments, got %zd", N, n); \
         if (!p_##NAME) return PyErr_Format(PyExc_RuntimeError, #NAME " is not bound");          \
-        DECL;                                                                                    \
-        if (PyErr_Occurred()) return NULL;                                                       \
+        uint64_t v[N];                                                                           \
+        if (!whole(a, N, v)) {                                                                   \
+            PyErr_Clear();                                                                       \
+            return PyObject_Vectorcall(c_##NAME, a, N, NULL);                                    \
+        }                                                                                        \
         int rc;                                                                                  \
         Py_BEGIN_ALLOW_THREADS                                                                   \
         rc = p_##NAME ARGS;                                                                      \
@@ -34,37 +42,33 @@ static uint64_t arg(PyObject *const *a, Py_ssize_t i) { return PyLong_AsUnsigned
         return PyLong_FromLong(rc);                                                              \
     }
 
-ENTRY(bn_act_quant_q81, 6, (P, P, Z, int, P, Z),
-      P c = AP(0); P x = AP(1); Z xo = AZ(2); int K = AI(3); P p = AP(4); Z po = AZ(5),
-      (c, x, xo, K, p, po))
-ENTRY(bn_gemv_q81, 11, (P, P, Z, int, int, P, Z, P, Z, P, Z),
-      P c = AP(0); P w = AP(1); Z wo = AZ(2); int M = AI(3); int K = AI(4); P p = AP(5); Z po = AZ(6); P o = AP(7); Z oo = AZ(8); P d = AP(9); Z dof = AZ(10),
-      (c, w, wo, M, K, p, po, o, oo, d, dof))
-ENTRY(bn_gemm_act_quant, 11, (P, P, Z, Z, int, int, P, Z, int, P, Z),
-      P c = AP(0); P x = AP(1); Z xo = AZ(2); Z xs = AZ(3); int K = AI(4); int nc = AI(5); P s = AP(6); Z so = AZ(7); int hb = AI(8); P im = AP(9); Z io = AZ(10),
-      (c, x, xo, xs, K, nc, s, so, hb, im, io))
-ENTRY(bn_gemm_q81, 12, (P, P, Z, int, int, int, P, Z, int, P, Z, Z),
-      P c = AP(0); P w = AP(1); Z wo = AZ(2); int t = AI(3); int M = AI(4); int K = AI(5); P im = AP(6); Z io = AZ(7); int nc = AI(8); P o = AP(9); Z oo = AZ(10); Z os = AZ(11),
-      (c, w, wo, t, M, K, im, io, nc, o, oo, os))
-ENTRY(bn_attn_insert, 18, (P, P, P, Z, P, Z, P, Z, int, int, P, Z, P, Z, P, Z, P, Z),
-      P c = AP(0); P d = AP(1); P kv = AP(2); Z kvo = AZ(3); P k = AP(4); Z ko = AZ(5); P v = AP(6); Z vo = AZ(7); int m = AI(8); int pos = AI(9); P q = AP(10); Z qo = AZ(11);
-      P qn = AP(12); Z qno = AZ(13); P kn = AP(14); Z kno = AZ(15); P s = AP(16); Z so = AZ(17),
-      (c, d, kv, kvo, k, ko, v, vo, m, pos, q, qo, qn, qno, kn, kno, s, so))
-ENTRY(bn_attn_attend, 11, (P, P, P, Z, int, P, Z, P, Z, P, Z),
-      P c = AP(0); P d = AP(1); P kv = AP(2); Z kvo = AZ(3); int pos = AI(4); P s = AP(5); Z so = AZ(6); P pg = AP(7); Z pgo = AZ(8); P g = AP(9); Z go = AZ(10),
-      (c, d, kv, kvo, pos, s, so, pg, pgo, g, go))
+ENTRY(bn_act_quant_q81, 6, (void *, void *, size_t, int, void *, size_t),
+      (P(0), P(1), Z(2), I(3), P(4), Z(5)))
+ENTRY(bn_gemv_q81, 11, (void *, void *, size_t, int, int, void *, size_t, void *, size_t, void *, size_t),
+      (P(0), P(1), Z(2), I(3), I(4), P(5), Z(6), P(7), Z(8), P(9), Z(10)))
+ENTRY(bn_gemm_act_quant, 11, (void *, void *, size_t, size_t, int, int, void *, size_t, int, void *, size_t),
+      (P(0), P(1), Z(2), Z(3), I(4), I(5), P(6), Z(7), I(8), P(9), Z(10)))
+ENTRY(bn_gemm_q81, 12, (void *, void *, size_t, int, int, int, void *, size_t, int, void *, size_t, size_t),
+      (P(0), P(1), Z(2), I(3), I(4), I(5), P(6), Z(7), I(8), P(9), Z(10), Z(11)))
+ENTRY(bn_attn_insert, 18, (void *, void *, void *, size_t, void *, size_t, void *, size_t, int, int, void *, size_t, void *, size_t, void *, size_t, void *, size_t),
+      (P(0), P(1), P(2), Z(3), P(4), Z(5), P(6), Z(7), I(8), I(9), P(10), Z(11), P(12), Z(13), P(14), Z(15), P(16), Z(17)))
+ENTRY(bn_attn_attend, 11, (void *, void *, void *, size_t, int, void *, size_t, void *, size_t, void *, size_t),
+      (P(0), P(1), P(2), Z(3), I(4), P(5), Z(6), P(7), Z(8), P(9), Z(10)))
 
-/* bind({name: address}) */
+/* bind({name: (address, ctypes function)}) */
 static PyObject *bind(PyObject *self, PyObject *table) {
     (void)self;
     if (!PyDict_Check(table)) return PyErr_Format(PyExc_TypeError, "bind takes a dict");
 #define BIND(NAME)                                                                               \
     do {                                                                                         \
-        PyObject *v = PyDict_GetItemString(table, #NAME);                                        \
-        if (!v) return PyErr_Format(PyExc_KeyError, #NAME);                                      \
-        void *f = PyLong_AsVoidPtr(v);                                                           \
+        PyObject *at, *slow, *e = PyDict_GetItemString(table, #NAME);                            \
+        if (!e) return PyErr_Format(PyExc_KeyError, #NAME);                                      \
+        if (!PyArg_ParseTuple(e, "OO", &at, &slow)) return NULL;                                 \
+        void *f = PyLong_AsVoidPtr(at);                                                          \
         if (PyErr_Occurred()) return NULL;                                                       \
         *(void **)&p_##NAME = f;                                                                 \
+        Py_INCREF(slow);                                                                         \
+        Py_XSETREF(c_##NAME, slow);                                                              \
     } while (0)
     BIND(bn_act_quant_q81); BIND(bn_gemv_q81); BIND(bn_gemm_act_quant); BIND(bn_gemm_q81); BIND(bn_attn_insert); BIND(bn_attn_attend);
     Py_RETURN_NONE;

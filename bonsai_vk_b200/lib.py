@@ -120,13 +120,14 @@ def _call_layer(lib, sig):
     functions through ctypes (1.0 to 1.6 us more a call)."""
     names = ("bn_act_quant_q81", "bn_gemv_q81", "bn_gemm_act_quant", "bn_gemm_q81", "bn_attn_insert", "bn_attn_attend")
     at = {n: C.cast(getattr(lib, n), C.c_void_p).value for n in names}
+    plain = (C.c_int, C.c_size_t)
+    slow = {n: C.CFUNCTYPE(C.c_int, *[t if t in plain else C.c_void_p for t in sig[n][1]])(at[n]) for n in names}
     try:
         from . import _fastcall
     except ImportError:
         import types
-        plain = (C.c_int, C.c_size_t)
-        return types.SimpleNamespace(**{n: C.CFUNCTYPE(C.c_int, *[t if t in plain else C.c_void_p for t in sig[n][1]])(at[n]) for n in names})
-    _fastcall.bind(at)
+        return types.SimpleNamespace(**slow)
+    _fastcall.bind({n: (at[n], slow[n]) for n in names})
     return _fastcall
 
 
