@@ -65,9 +65,10 @@ FASTCALL = os.path.join(HERE, "_fastcall.so")
 def build_fastcall(force: bool = False) -> str:
     """The CPython call layer of the op-level entry points (host/fastcall.c); lib.py uses ctypes where it is missing."""
     src = os.path.join(HERE, "host", "fastcall.c")
-    if not force and not _stale(FASTCALL, [src]):
+    if not force and not _stale(FASTCALL, [src] + glob.glob(os.path.join(ROOT, "include", "*.h"))):
         return FASTCALL
-    cmd = ["gcc", "-O2", "-Wall", "-fPIC", "-shared", "-I" + sysconfig.get_paths()["include"], "-o", FASTCALL, src]
+    cmd = ["gcc", "-O2", "-Wall", "-Wconversion", "-Werror", "-fPIC", "-shared", "-I" + os.path.join(ROOT, "include"),
+           "-isystem", sysconfig.get_paths()["include"], "-o", FASTCALL, src]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)

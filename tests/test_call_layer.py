@@ -89,3 +89,29 @@ def test_number_follows_the_handle():
     b.h = C.c_void_p()
     b.h.value = 0x8000                                      # (as a call that takes C.byref(b.h) does)
     assert b.p == 0x8000
+
+
+@pytest.mark.parametrize("name", CALLS)
+def test_arguments_arrive_in_order_and_whole(name):
+    """Each argument, at its parameter's full width, against a function of the binding's signature in the entry point's place."""
+    build.build_lib()
+    build.build_fastcall()
+    L = lib.load_library()
+    from bonsai_vk_b200 import _fastcall
+    types_ = [t if t in (C.c_int, C.c_size_t) else C.c_void_p for t in L._bn_signatures[name][1]]
+    sent = [-7 - i if t is C.c_int else (0x0123456789ABCD00 << 4) + i for i, t in enumerate(types_)]
+    got = []
+    stub = C.CFUNCTYPE(C.c_int, *types_)(lambda *a: got.extend(a) or -77)
+    try:
+        _fastcall.bind({n: (C.cast(stub, C.c_void_p).value, stub) for n in CALLS})
+        assert getattr(_fastcall, name)(*sent) == -77 and got == sent
+    finally:
+        lib._call_layer(L, L._bn_signatures)
+
+
+def test_call_layer_is_rebuilt_for_another_header(monkeypatch):
+    """The layer's types are the header's: a changed header makes the built file stale."""
+    seen = []
+    monkeypatch.setattr(build, "_stale", lambda target, sources: seen.extend(sources))
+    build.build_fastcall()
+    assert any(s.endswith("bonsai_cuda.h") for s in seen)
