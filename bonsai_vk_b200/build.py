@@ -59,7 +59,7 @@ def build_host(force: bool = False) -> str:
     return HOST_BIN
 
 
-FASTCALL = os.path.join(HERE, "_fastcall.so")
+FASTCALL = os.path.join(HERE, "_fastcall" + sysconfig.get_config_var("EXT_SUFFIX"))     # named for this interpreter: others do not load it
 
 
 def build_fastcall(force: bool = False) -> str:
@@ -69,6 +69,9 @@ def build_fastcall(force: bool = False) -> str:
         return FASTCALL
     cmd = ["gcc", "-O2", "-Wall", "-Wconversion", "-Werror", "-fPIC", "-shared", "-I" + os.path.join(ROOT, "include"),
            "-isystem", sysconfig.get_paths()["include"], "-o", FASTCALL, src]
+    for old in (FASTCALL, os.path.join(HERE, "_fastcall.so")):             # (the second: a name that any interpreter would load)
+        if os.path.exists(old):
+            os.remove(old)
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)

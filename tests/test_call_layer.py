@@ -1,6 +1,7 @@
 """The call layer of the op-level entry points (host/fastcall.c) and its stand-in through ctypes: the same return codes, error texts and
 treatment of arguments, without a GPU (every call is refused before it reaches one)."""
 import ctypes as C
+import importlib.machinery
 import sys
 import types
 
@@ -115,3 +116,7 @@ def test_call_layer_is_rebuilt_for_another_header(monkeypatch):
     monkeypatch.setattr(build, "_stale", lambda target, sources: seen.extend(sources))
     build.build_fastcall()
     assert any(s.endswith("bonsai_cuda.h") for s in seen)
+
+
+def test_call_layer_is_named_for_its_interpreter():
+    assert build.FASTCALL.endswith("_fastcall" + importlib.machinery.EXTENSION_SUFFIXES[0]) and "cpython" in build.FASTCALL
