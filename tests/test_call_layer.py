@@ -120,3 +120,18 @@ def test_call_layer_is_rebuilt_for_another_header(monkeypatch):
 
 def test_call_layer_is_named_for_its_interpreter():
     assert build.FASTCALL.endswith("_fastcall" + importlib.machinery.EXTENSION_SUFFIXES[0]) and "cpython" in build.FASTCALL
+
+
+@pytest.mark.parametrize("failure", [OSError("no gcc"), types.SimpleNamespace(returncode=1, stdout="", stderr="Python.h: No such file")])
+def test_build_goes_on_without_the_call_layer(monkeypatch, tmp_path, failure):
+    def run(*a, **k):
+        if isinstance(failure, OSError):
+            raise failure
+        return failure
+    monkeypatch.setattr(build, "HERE", str(tmp_path))
+    monkeypatch.setattr(build, "FASTCALL", str(tmp_path / "_fastcall.so"))
+    (tmp_path / "_fastcall.so").write_bytes(b"an older one")
+    monkeypatch.setattr(build.subprocess, "run", run)
+    with pytest.warns(UserWarning, match="ctypes"):
+        assert build.build_fastcall(force=True) is None
+    assert not (tmp_path / "_fastcall.so").exists()
