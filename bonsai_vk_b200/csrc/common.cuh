@@ -30,6 +30,8 @@ struct bn_ctx {
     size_t scratch_bytes;
     // the device error word that bounded waits set
     int *err_dev;
+    // bn_selftest_refusal
+    bool refuse_launch;
 };
 
 void bn_set_error(const char *fmt, ...);

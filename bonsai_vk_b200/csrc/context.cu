@@ -81,6 +81,7 @@ int bn_init(int device, bn_ctx **out) {
     c->launches = 0;
     c->scratch = nullptr;
     c->scratch_bytes = 0;
+    c->refuse_launch = false;
     e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) { delete c; return bn_cuda_fail(e, "cudaStreamCreate"); }
     c->own_stream = true;
@@ -138,6 +139,12 @@ int bn_free(bn_ctx *ctx, bn_buf *buf) {
 }
 
 size_t bn_buf_size(const bn_buf *buf) { return buf ? buf->bytes : 0; }
+
+int bn_selftest_refusal(bn_ctx *ctx) {
+    BN_REQUIRE(ctx, BN_ERR_ARG, "bn_selftest_refusal: null context");
+    ctx->refuse_launch = true;
+    return BN_OK;
+}
 
 int bn_wrap(bn_ctx *ctx, void *device_ptr, size_t bytes, bn_buf **out) {
     BN_REQUIRE(ctx && device_ptr && bytes && out, BN_ERR_ARG, "bn_wrap: bad argument");

@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <string>
 #include <vector>
@@ -221,7 +222,8 @@ bnk::Q2Args phase_base(bn_model *m, const uint8_t *W, int M, int K) {
 }
 void launch(bn_model *m, const bnk::Q2Args &a) {
     if (m->mixers_only) return;
-    cudaError_t e = bnk::launch_q2_gemv(m->ctx->stream, m->ctx->sm_count, a, m->use_pdl);
+    cudaError_t e = m->ctx->refuse_launch ? cudaErrorInvalidConfiguration : bnk::launch_q2_gemv(m->ctx->stream, m->ctx->sm_count, a, m->use_pdl);
+    m->ctx->refuse_launch = false;
     if (e != cudaSuccess && m->launch_err == cudaSuccess) m->launch_err = e;
 }
 bool adjacent(const uint32_t *a, size_t a_bytes, const uint32_t *b) {
@@ -622,30 +624,45 @@ __global__ void k_fill_u16(uint16_t *p, size_t n, uint16_t v) {
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) p[i] = v;
 }
 
+// what the launches of a schedule left behind: errors of the runtime, and those that launch() recorded
+cudaError_t schedule_error(bn_model *m) {
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = m->launch_err;
+    m->launch_err = cudaSuccess;
+    return e;
+}
+
+// a schedule as an executable graph; none is made of one that lost a launch
+int capture(bn_model *m, const char *what, cudaGraphExec_t *out, int *launches, const std::function<void()> &schedule) {
+    cudaGraph_t g = nullptr;
+    const unsigned long long before = g_bn_launches;
+    schedule_error(m);                    // (earlier calls' errors, which those reported)
+    BN_CUDA(cudaStreamBeginCapture(m->ctx->stream, cudaStreamCaptureModeThreadLocal));
+    schedule();
+    const cudaError_t s = schedule_error(m);
+    cudaError_t e = cudaStreamEndCapture(m->ctx->stream, &g);
+    if (e == cudaSuccess) e = s;
+    *launches = int(g_bn_launches - before);
+    g_bn_launches = before;               // captured, not launched
+    if (e == cudaSuccess) e = cudaGraphInstantiate(out, g, 0);
+    if (g) cudaGraphDestroy(g);
+    return e == cudaSuccess ? BN_OK : bn_cuda_fail(e, what);
+}
+
 // the whole token (schedule + hand-over of the pick to TOK / POS / HIST) as one CUDA graph, captured on first use
 int ensure_token_graph(bn_model *m) {
     if (m->token_graph) return BN_OK;
-    cudaStream_t st = m->ctx->stream;
-    cudaGraph_t g = nullptr;
-    const unsigned long long before = g_bn_launches;
     if (getenv("BONSAI_STAMP_GRAPH")) {      // profiling aid: the captured kernels keep writing their time stamps
         BN_CUDA(cudaMalloc(&m->stamps, 256 * 8 * sizeof(unsigned long long)));
         BN_CUDA(cudaMemset(m->stamps, 0, 256 * 8 * sizeof(unsigned long long)));
         m->stamp_idx = 0;
     }
-    BN_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    enqueue_token(m, -1, true);
-    m->graph_stamps = m->stamps;
-    m->stamps = nullptr;
-    bnk::launch(k_advance, dim3(1), dim3(32), 0, st, m->TOK, m->POS, m->NEXT, m->HIST, m->STEP);
-    cudaError_t e = cudaStreamEndCapture(st, &g);
-    if (e != cudaSuccess) return bn_cuda_fail(e, "cudaStreamEndCapture(token)");
-    m->graph_launches = int(g_bn_launches - before);
-    g_bn_launches = before;               // captured, not launched
-    e = cudaGraphInstantiate(&m->token_graph, g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess) return bn_cuda_fail(e, "cudaGraphInstantiate(token)");
-    return BN_OK;
+    return capture(m, "capture of the token schedule", &m->token_graph, &m->graph_launches, [m] {
+        enqueue_token(m, -1, true);
+        m->graph_stamps = m->stamps;
+        m->stamps = nullptr;
+        bnk::launch(k_advance, dim3(1), dim3(32), 0, m->ctx->stream, m->TOK, m->POS, m->NEXT, m->HIST, m->STEP);
+    });
 }
 
 }  // namespace
@@ -937,9 +954,7 @@ int bn_model_token(bn_model *m, int tok, int pos, int stop_after_block, int *nex
     BN_CUDA(cudaMemcpyAsync(m->POS, &tp[1], 4, cudaMemcpyHostToDevice, st));
     BN_CUDA(cudaStreamSynchronize(st));     // tp lives on this stack frame
     enqueue_token(m, stop_after_block, true);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = m->launch_err;
-    m->launch_err = cudaSuccess;
+    const cudaError_t e = schedule_error(m);
     if (e != cudaSuccess) return bn_cuda_fail(e, "token schedule");
     if (next_tok) {
         BN_CUDA(cudaMemcpyAsync(next_tok, m->NEXT, 4, cudaMemcpyDeviceToHost, st));
@@ -992,8 +1007,6 @@ int bn_model_stage_prepare(bn_model *m, int stream0, int ncol) {
     const int S = h.n_streams > 0 ? h.n_streams : 1;
     BN_REQUIRE(ncol >= 0 && stream0 >= 0 && stream0 + (ncol > 0 ? ncol : 1) <= S, BN_ERR_ARG,
                "bn_model_stage_prepare: sequences %d..%d outside [0, %d)", stream0, stream0 + (ncol > 0 ? ncol : 1) - 1, S);
-    cudaStream_t st = m->ctx->stream;
-    cudaGraph_t g = nullptr;
     cudaGraphExec_t ge = nullptr;
     m->cur = stream0;
     if (ncol == 0) {
@@ -1005,18 +1018,9 @@ int bn_model_stage_prepare(bn_model *m, int stream0, int ncol) {
         BN_REQUIRE(m->fused, BN_ERR_STATE, "bn_model_stage_prepare: the multi-sequence pass needs the fused layer kernels");
         if (m->batch_graphs.count(long(stream0) * 64 + ncol)) return BN_OK;
     }
-    const unsigned long long before = g_bn_launches;
-    BN_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    if (ncol == 0) enqueue_token(m, -1, true); else enqueue_batch(m, ncol);
-    cudaError_t e = cudaStreamEndCapture(st, &g);
-    if (e == cudaSuccess) e = m->launch_err;
-    m->launch_err = cudaSuccess;
-    if (e != cudaSuccess) return bn_cuda_fail(e, "cudaStreamEndCapture(stage)");
-    (ncol == 0 ? m->graph_launches : m->batch_graph_launches) = int(g_bn_launches - before);
-    g_bn_launches = before;               // captured, not launched
-    e = cudaGraphInstantiate(&ge, g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess) return bn_cuda_fail(e, "cudaGraphInstantiate(stage)");
+    const int rc = capture(m, "capture of the stage schedule", &ge, ncol == 0 ? &m->graph_launches : &m->batch_graph_launches,
+                           [=] { if (ncol == 0) enqueue_token(m, -1, true); else enqueue_batch(m, ncol); });
+    if (rc != BN_OK) return rc;
     if (ncol == 0) m->stage_graphs[stream0] = ge; else m->batch_graphs.emplace(long(stream0) * 64 + ncol, ge);
     return BN_OK;
 }
@@ -1043,7 +1047,7 @@ int bn_model_stage(bn_model *m, int stream, int tok, int pos, const bn_buf *in, 
     cudaError_t e = cudaSuccess;
     if (getenv("BONSAI_NO_STAGE_GRAPH")) {
         enqueue_token(m, -1, true);
-        e = cudaGetLastError();
+        e = schedule_error(m);
     } else {
         // the ~100 launches of a stage are replayed as one graph: the host only feeds copies and NCCL calls. The graph
         // must exist already (bn_model_stage_prepare): building one here could synchronise a device whose stream holds a
@@ -1053,8 +1057,6 @@ int bn_model_stage(bn_model *m, int stream, int tok, int pos, const bn_buf *in, 
         e = cudaGraphLaunch(m->stage_graphs[stream], st);
         BN_COUNT(m->graph_launches);
     }
-    if (e == cudaSuccess) e = m->launch_err;
-    m->launch_err = cudaSuccess;
     if (e != cudaSuccess) return bn_cuda_fail(e, "stage schedule");
     if (last) BN_CUDA(cudaMemcpyAsync(bn_ptr<char>(out, out_off), m->NEXT, 4, cudaMemcpyDeviceToDevice, st));
     else BN_CUDA(cudaMemcpyAsync(bn_ptr<char>(out, out_off), m->RES, size_t(h.hidden) * 4, cudaMemcpyDeviceToDevice, st));
@@ -1094,7 +1096,7 @@ int bn_model_stage_batch(bn_model *m, int stream0, int ncol, const int *tok, con
     cudaError_t e = cudaSuccess;
     if (getenv("BONSAI_NO_STAGE_GRAPH")) {
         enqueue_batch(m, ncol);
-        e = cudaGetLastError();
+        e = schedule_error(m);
     } else {
         auto it = m->batch_graphs.find(long(stream0) * 64 + ncol);
         BN_REQUIRE(it != m->batch_graphs.end(), BN_ERR_STATE,
@@ -1103,8 +1105,6 @@ int bn_model_stage_batch(bn_model *m, int stream0, int ncol, const int *tok, con
         e = cudaGraphLaunch(it->second, st);
         BN_COUNT(m->batch_graph_launches);
     }
-    if (e == cudaSuccess) e = m->launch_err;
-    m->launch_err = cudaSuccess;
     if (e != cudaSuccess) return bn_cuda_fail(e, "stage batch schedule");
     if (last) BN_CUDA(cudaMemcpy2DAsync(bn_ptr<char>(out, out_off), 4, m->NEXT, m->arena_bytes, 4, ncol, cudaMemcpyDeviceToDevice, st));
     else BN_CUDA(cudaMemcpy2DAsync(bn_ptr<char>(out, out_off), size_t(h.hidden) * 4, m->RES, m->arena_bytes, size_t(h.hidden) * 4, ncol,
@@ -1131,9 +1131,7 @@ int bn_model_prefill(bn_model *m, const int *toks, int n, int pos0, int *next_to
     k_set_cols<<<1, 32, 0, st>>>(m->TOK, m->POS, m->arena_bytes, n, ci, nullptr, h.vocab, m->ctx->err_dev);
     BN_COUNT(1);
     enqueue_batch(m, n, true);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = m->launch_err;
-    m->launch_err = cudaSuccess;
+    cudaError_t e = schedule_error(m);
     if (e != cudaSuccess) return bn_cuda_fail(e, "prefill schedule");
     // the pick after the block: output norm + head + first maximum on the last column's residual, through the
     // single-sequence kernels (whose buffers are column 0's)
@@ -1145,11 +1143,13 @@ int bn_model_prefill(bn_model *m, const int *toks, int n, int pos0, int *next_to
     }
     norm_project(m, m->q2_head, h.vocab, m->out_norm, m->LOGITS, next_after(m, m->b0 - 1));
     bnk::argmax_first(st, m->LOGITS, h.vocab, m->NEXT, m->AMV, m->AMI);
+    e = schedule_error(m);
+    if (e != cudaSuccess) return bn_cuda_fail(e, "prefill pick");
     if (next_tok) {
         BN_CUDA(cudaMemcpyAsync(next_tok, m->NEXT, 4, cudaMemcpyDeviceToHost, st));
         BN_CUDA(cudaStreamSynchronize(st));
     }
-    return bn_launch_check(m->ctx, "bn_model_prefill");
+    return BN_OK;
 }
 
 int bn_model_set_head_rows(bn_model *m, int row_begin, int row_end) {
@@ -1253,6 +1253,7 @@ int bn_model_gemv_sweep(bn_model *m, int reps, float *ms_per_sweep) {
     cudaEvent_t e0, e1;
     BN_CUDA(cudaEventCreate(&e0));
     BN_CUDA(cudaEventCreate(&e1));
+    schedule_error(m);                   // (earlier calls' errors, which those reported)
     sweep();
     BN_CUDA(cudaEventRecord(e0, st));
     for (int r = 0; r < reps; ++r) sweep();
@@ -1262,6 +1263,8 @@ int bn_model_gemv_sweep(bn_model *m, int reps, float *ms_per_sweep) {
     BN_CUDA(cudaEventElapsedTime(&ms, e0, e1));
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    const cudaError_t e = schedule_error(m);
+    if (e != cudaSuccess) return bn_cuda_fail(e, "bn_model_gemv_sweep");
     *ms_per_sweep = ms / float(reps);
     return BN_OK;
 }
@@ -1315,9 +1318,12 @@ int bn_model_profile_token(bn_model *m, int tok, int pos, unsigned long long *st
     BN_CUDA(cudaStreamSynchronize(st));
     m->stamp_idx = 0;
     unsigned long long *keep = m->stamps;
+    schedule_error(m);                   // (earlier calls' errors, which those reported)
     enqueue_token(m, -1, true);
     const int n = m->stamp_idx;
     m->stamps = nullptr;                 // later tokens run unstamped
+    const cudaError_t e = schedule_error(m);
+    if (e != cudaSuccess) { cudaStreamSynchronize(st); cudaFree(keep); return bn_cuda_fail(e, "bn_model_profile_token"); }
     BN_CUDA(cudaStreamSynchronize(st));
     *n_phases = n < max_phases ? n : max_phases;
     BN_CUDA(cudaMemcpy(stamps_out, keep, size_t(*n_phases) * 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost));

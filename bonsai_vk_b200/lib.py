@@ -93,6 +93,7 @@ def load_library() -> C.CDLL:
         "bn_model_stage_prepare": (i32, [vp, i32, i32]),
         "bn_model_stage": (i32, [vp, i32, i32, i32, vp, sz, vp, sz]),
         "bn_model_stage_batch": (i32, [vp, i32, i32, vp, vp, vp, sz, vp, sz]),
+        "bn_selftest_refusal": (i32, [vp]),
         "bn_model_reset_stream": (i32, [vp, i32]),
         "bn_model_prefill": (i32, [vp, vp, i32, i32, C.POINTER(i32)]),
         "bn_model_set_head_rows": (i32, [vp, i32, i32]),
@@ -239,6 +240,11 @@ class Context(_Handle):
         """Queue a kernel whose bounded wait must give up (0: copy-ring wait, 1: tensor-core pipeline wait); the next
         sync() then raises BonsaiError with code BN_ERR_TIMEOUT and the context stays usable."""
         _check(self.lib.bn_selftest_wait(self.h, which), "bn_selftest_wait")
+
+    def selftest_refusal(self):
+        """The next single-sequence projection of a model of this context is refused; the call that launches or captures it
+        must raise BonsaiError, and the model stays usable."""
+        _check(self.lib.bn_selftest_refusal(self.h), "bn_selftest_refusal")
 
     def use_stream(self, cuda_stream: int):
         """Run this context's kernels on a stream owned by the caller (e.g. torch's current stream)."""

@@ -69,6 +69,9 @@ int bn_sync(bn_ctx *ctx);
  * BN_ERR_TIMEOUT and clears the word, and the context stays usable. (The reference has no counterpart: its waits are
  * Vulkan fences with an unbounded timeout, bonsai_weights.h:287.) */
 int bn_selftest_wait(bn_ctx *ctx, int which);
+/* The next single-sequence projection that a model of this context launches is refused as the runtime refuses a bad launch (nothing
+ * is launched in its place): the call that was launching or capturing it must fail, and keep nothing that it captured. */
+int bn_selftest_refusal(bn_ctx *ctx);
 
 /* page-locked host staging memory (reference: the mapped host_buf, bonsai_weights.h:199) */
 int bn_host_alloc(size_t bytes, void **out);
