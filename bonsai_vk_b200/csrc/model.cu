@@ -820,6 +820,7 @@ int bn_model_finalize(bn_model *m) {
     m->FU = m->FG + h.ffn;           // [gate | up]
     m->fused = h.act_mode == 0 && getenv("BONSAI_NO_FUSE") == nullptr && bnk::q2_gemv_supported(h.hidden, h.hat_block) &&
                bnk::q2_gemv_supported(h.ffn, h.hat_block);
+    if (m->fused) bnk::q2_gemv_prepare();
     m->use_pdl = getenv("BONSAI_NO_PDL") == nullptr;
     bnk::g_pdl = m->use_pdl;
     // persistent state

@@ -74,6 +74,8 @@ struct Q2Args {
     unsigned long long *stamps;  // optional, 8 device time stamps of CTA 0 (see PhaseArgs)
 };
 bool q2_gemv_supported(int K, int hat_block);
+// asks what launches depend on (how many clusters fit): once, ahead of any capture
+void q2_gemv_prepare();
 cudaError_t launch_q2_gemv(cudaStream_t st, int sm_count, const Q2Args &a, bool pdl);
 
 struct Q2GemmArgs {

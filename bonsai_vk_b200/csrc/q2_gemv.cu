@@ -485,16 +485,16 @@ cudaError_t launch_spans(cudaStream_t st, int sm_count, Q2Args a, bool pdl, int 
 int split_clusters(int parts) {
     static const std::array<int, 9> most = [] {
         std::array<int, 9> m{};
-        if (cudaFuncSetAttribute(k_q2_gemv<1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX) == cudaSuccess)
-            for (int p = 2; p <= 4; ++p) {
-                cudaLaunchConfig_t cfg = {};
-                cfg.gridDim = dim3(p * 64); cfg.blockDim = dim3(NT + 32); cfg.dynamicSmemBytes = SMEM_MAX;
-                cudaLaunchAttribute at[1];
-                at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = p; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-                cfg.attrs = at; cfg.numAttrs = 1;
-                if (cudaOccupancyMaxActiveClusters(&m[p], k_q2_gemv<1, false, true>, &cfg) != cudaSuccess) m[p] = 0;
-            }
-        cudaGetLastError();                        // (a refusal is an answer, not a failed call)
+        cudaError_t e = cudaFuncSetAttribute(k_q2_gemv<1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
+        for (int p = 2; p <= 4 && e == cudaSuccess; ++p) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(p * 64); cfg.blockDim = dim3(NT + 32); cfg.dynamicSmemBytes = SMEM_MAX;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = p; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+            cfg.attrs = at; cfg.numAttrs = 1;
+            if ((e = cudaOccupancyMaxActiveClusters(&m[p], k_q2_gemv<1, false, true>, &cfg)) != cudaSuccess) m[p] = 0;
+        }
+        if (e != cudaSuccess) cudaGetLastError();  // (a refusal is an answer, not a failed call)
         return m;
     }();
     return most[parts] - most[parts] / 8;
@@ -507,6 +507,8 @@ namespace bnk {
 bool q2_gemv_supported(int K, int hat_block) {
     return K >= 512 && K % 512 == 0 && K <= 16384 && hat_block >= 16 && hat_block <= 4096 && (hat_block & (hat_block - 1)) == 0 && K % hat_block == 0;
 }
+
+void q2_gemv_prepare() { split_clusters(2); }
 
 cudaError_t launch_q2_gemv(cudaStream_t st, int sm_count, const Q2Args &a, bool pdl) {
     if (a.K > 4096 && a.K % 4096 == 0 && a.pro == Q2_PLAIN && !a.swiglu) {
