@@ -63,20 +63,13 @@ int bn_gemm_q81(bn_ctx *ctx, const bn_buf *w, size_t w_off, int w_tiled, int M, 
         q.out = bn_ptr<float>(out, out_off) + r0; q.out_stride = out_stride; q.err = ctx->err_dev;
         return q;
     };
-    // Native rows of up to 16 columns: the projection's warps unpack the pieces that they use. One launch less, and no tiles through
-    // memory: 3000 x 5120 x 11 13.4 -> 10.1 us with the preparation of the columns, 1500 x 4096 x 8 9.7 -> 6.4, 24 576 x 4096 x 8
-    // 25.5 -> 22.9, 24 576 x 12 288 x 16 95 -> 88; between 0.98 and 1.05 of the other way's time where 16 columns meet 24 576 x 5120 or
-    // 8192 x 12 288. From 17 columns on every piece is unpacked twice (a unit has 16 columns), which pays while a CTA has few
-    // pieces (row tiles x groups of 512 weights): 1500 x 4096 x 24 17.5 -> 10.7 us with 8 of them, 8192 x 1024 11.3 -> 9.9 with 8,
-    // 700 x 5120 14.6 -> 13.8 with 10, but 3000 x 4096 14.2 -> 15.1 with 16 and 24 576 x 4096 42 -> 61. There the rows are unpacked
-    // into two-bit tiles first, in chunks of at most 48 MB of scratch, which stay in L2 - unless the call is inside a capture (a
-    // graph may outlive the scratch), or there is no memory left for it.
-    const int tiles_cta = ((M + 15) / 16 + ctx->sm_count - 1) / ctx->sm_count;
-    const bool in_place = ncol <= 16 || tiles_cta * (K / 512) <= 12;
+    // Native rows are unpacked by the warps that use them (one launch less, no tiles through memory) where q2_gemm_in_place says so. The
+    // others are unpacked into two-bit tiles first, in chunks of at most 48 MB of scratch, which stay in L2 - unless the call is inside
+    // a capture (a graph may outlive the scratch), or there is no memory left for it.
     const int step = int(std::max<size_t>(1, (size_t(48) << 20) / (size_t(K / 512) * bnk::Q2_PIECE))) * 16;
     cudaError_t e = cudaSuccess;
     if (w_tiled) e = bnk::launch_q2_gemm(ctx->stream, ctx->sm_count, args(bn_ptr<uint8_t>(w, w_off), 0, M), bnk::g_pdl);
-    else if (in_place || !bn_scratch_available(ctx, bnk::q2_bytes(std::min(M, step), K)))
+    else if (bnk::q2_gemm_in_place(ctx->sm_count, M, K, ncol, M <= step) || !bn_scratch_available(ctx, bnk::q2_bytes(std::min(M, step), K)))
         e = bnk::launch_q2_gemm_native(ctx->stream, ctx->sm_count, args(bn_ptr<uint8_t>(w, w_off), 0, M), bnk::g_pdl);
     else {
         uint8_t *tiles = reinterpret_cast<uint8_t *>(ctx->scratch);

@@ -94,6 +94,8 @@ struct Q2GemmArgs {
 };
 cudaError_t launch_q2_gemm(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl);
 // the same with W in the file's native rows (16-byte aligned, K % 1024 == 0): each warp unpacks its pieces itself, no scratch
+// whether that is the faster way: `one_chunk`, the matrix unpacked into tiles beforehand would fit the scratch at once
+bool q2_gemm_in_place(int sm_count, int M, int K, int ncol, bool one_chunk);
 cudaError_t launch_q2_gemm_native(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl);
 cudaError_t launch_q2_gemm_wide(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl);      // 17 to 32 columns (q2_gemm_wide.cu)
 

@@ -235,6 +235,17 @@ __global__ void k_wait_selftest_gemm(int *err) {
     }
 }
 
+// Groups per wave: all of K where its image piece fits beside its group sums (one wave: no barrier in between, and the units spread over
+// more warps), else as many as fit with the image piece twice. tiles: row tiles per pass, stages: bytes in which warps unpack.
+int wave_bytes(int ng, int kc, int tiles, int ncp, int stages) {
+    return 128 + kc * ((kc >= ng ? 1 : 2) * 4 * ncp * IMG_COL + tiles * 16 * ncp * 4) + stages;
+}
+int wave_groups(int ng, int tiles, int ncp, int stages) {
+    int kc = ng;
+    if (wave_bytes(ng, kc, tiles, ncp, stages) > SMEM_MAX) for (kc = std::min(ng - 1, 8); kc > 1 && wave_bytes(ng, kc, tiles, ncp, stages) > SMEM_MAX;) kc = (kc + 1) / 2;
+    return kc;
+}
+constexpr int NATIVE_NT = 512;
 template <int NCP, int MT, int NT, bool NATIVE = false>
 cudaError_t launch_t(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl) {
     static bool attr_set = false;
@@ -246,17 +257,13 @@ cudaError_t launch_t(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl) {
     const int ng = a.K / 512, tiles = (a.M + 15) / 16, grid = std::min(tiles, sm_count);
     a.share = {tiles / grid, tiles % grid};
     a.tiles = std::min(a.share.q + (a.share.r > 0), MAX_TILES);
-    // groups per wave: all of K where its image piece fits beside its group sums (one wave: no barrier in between, and the units
-    // spread over more warps), else as many as fit with the image piece twice
-    const int gimg = 4 * NCP * IMG_COL, gsum = a.tiles * 16 * NCP * 4, stages = NATIVE ? NT / 32 * Q2_PIECE : 0;
-    auto bytes = [&](int kc) { return 128 + kc * ((kc >= ng ? 1 : 2) * gimg + gsum) + stages; };
-    a.kc = ng;
-    if (bytes(ng) > SMEM_MAX) for (a.kc = std::min(ng - 1, 8); a.kc > 1 && bytes(a.kc) > SMEM_MAX;) a.kc = (a.kc + 1) / 2;
+    const int stages = NATIVE ? NT / 32 * Q2_PIECE : 0;
+    a.kc = wave_groups(ng, a.tiles, NCP, stages);
     if (a.next.W) a.next.share = {a.next.units / grid, a.next.units % grid};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(NT);
-    cfg.dynamicSmemBytes = std::max(bytes(a.kc), 116 << 10);             // one CTA per SM, as in q2_gemv.cu
+    cfg.dynamicSmemBytes = std::max(wave_bytes(ng, a.kc, a.tiles, NCP, stages), 116 << 10);             // one CTA per SM, as in q2_gemv.cu
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -287,10 +294,25 @@ cudaError_t launch_q2_gemm(cudaStream_t st, int sm_count, const Q2GemmArgs &a, b
     return tiles <= 2 * sm_count && a.K <= 4096 ? launch_t<32, 2, 512>(st, sm_count, a, pdl) : launch_q2_gemm_wide(st, sm_count, a, pdl);
 }
 
+// Against unpacking into tiles first, with the preparation of the columns, rows from DRAM (us, tiles -> in place):
+//   up to 8 columns   always: 1500 x 4096 10.3 -> 5.9, 3000 x 5120 9.6 -> 8.0, 24 576 x 4096 25.5 -> 22.8, 8192 x 12 288 26.5 -> 24.2
+//                     (four row tiles a CTA and K from 14 336 on, where K goes in waves: between 0.94 and 1.09 of the other way)
+//   9 to 16 columns   while K goes in one wave (20 000 x 5120 30.3 -> 27.9, 24 576 x 4096 31.0 -> 30.0), a CTA has up to three row tiles
+//                     (7000 x 12 288 31.2 -> 28.9) or the tiles would take several chunks (24 576 x 12 288 95.5 -> 89.4). Otherwise every
+//                     wave ends in a barrier behind one or two units a warp, and unpacking is the part that waits: 16 384 x 6144
+//                     30.1 -> 32.5, 14 000 x 7168 28.3 -> 32.3, 8192 x 12 288 32.9 -> 34.9; of 226 such shapes the worst loses 4 %
+//   17 and more       every piece is unpacked twice (a unit has 16 columns), which pays while a CTA has few pieces (row tiles x groups of
+//                     512 weights): 1500 x 4096 x 24 17.9 -> 9.8 with 8 of them, 512 x 5120 14.9 -> 13.7 with 10, but 3000 x 5120
+//                     17.6 -> 18.4 with 20 and 24 576 x 4096 41.8 -> 61.9
+bool q2_gemm_in_place(int sm_count, int M, int K, int ncol, bool one_chunk) {
+    const int ng = K / 512, tiles = ((M + 15) / 16 + sm_count - 1) / sm_count;
+    if (ncol > 16) return tiles * ng <= 12;
+    return ncol <= 8 || tiles <= 3 || !one_chunk || wave_groups(ng, std::min(tiles, MAX_TILES), 16, NATIVE_NT / 32 * Q2_PIECE) == ng;
+}
 cudaError_t launch_q2_gemm_native(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl) {
-    if (a.ncol <= 8) return launch_t<8, 1, 512, true>(st, sm_count, a, pdl);
-    if (a.ncol <= 16) return launch_t<16, 1, 512, true>(st, sm_count, a, pdl);
-    return launch_t<32, 1, 512, true>(st, sm_count, a, pdl);
+    if (a.ncol <= 8) return launch_t<8, 1, NATIVE_NT, true>(st, sm_count, a, pdl);
+    if (a.ncol <= 16) return launch_t<16, 1, NATIVE_NT, true>(st, sm_count, a, pdl);
+    return launch_t<32, 1, NATIVE_NT, true>(st, sm_count, a, pdl);
 }
 
 cudaError_t launch_wait_selftest_gemm(cudaStream_t st, int *err) {
