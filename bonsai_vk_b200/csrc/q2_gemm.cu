@@ -14,7 +14,7 @@
 // Work split. A CTA of 12 or 16 warps owns a run of row tiles over all of K. K is walked in waves of `kc` groups (512 weights each);
 // a wave's piece of the activation image is double-buffered in shared memory. A wave's units (MT row tiles, one group, up to 16
 // columns) are dealt to the warps; a unit keeps everything in registers and leaves its group sums p_g in shared memory, where
-// after a barrier every thread adds its own (row, column)s' in ascending order. MT = 2 (or 3, or for native rows 1) row tiles share a group's operands and
+// after a barrier every thread adds its own (row, column)s' in ascending order. MT = 2 or 3 (1 for native rows, and where a CTA has few) row tiles share a group's operands and
 // scales: with one, shared-memory reads (24 wavefronts per 16 rows x 8 columns x 128 weights) would bound the loop.
 #include "q2.cuh"
 #include "rotate_quant.cuh"
@@ -37,11 +37,11 @@ template <bool FIRST> __device__ __forceinline__ uint4 weights16(const uint8_t *
 }
 // NATIVE: W holds the file's rows; a warp unpacks each of its pieces in a corner of shared memory of its own first. Bound by that
 // unpacking, 250 instructions a piece: 16 warps also for 8 columns (128 x 12 288: 10.2 -> 9.1 us, 4096 rows and more the same).
-// 12 warps (168 registers a thread) have room for a unit's weights to be on their way while the image is: LATE.
+// 12 warps (168 registers a thread), or units of one tile, have room for a unit's weights to be on their way while the image is: LATE.
 template <int NCP, int MT, int NT, bool NATIVE>
 __global__ void __launch_bounds__(NT, 1) k_q2_gemm(const Q2GemmArgs a) {
     constexpr int NW = NT / 32;
-    constexpr bool LATE = NATIVE || (NT == 384 && MT == 2);
+    constexpr bool LATE = NATIVE || MT == 1 || (NT == 384 && MT == 2);
     constexpr int NG = NCP / 8, NGW = NG >= 2 ? 2 : 1, H = NG / NGW;      // column groups: all, per unit; units across the columns
     constexpr int ITEMS = (MAX_TILES * 16 * NCP + NT - 1) / NT;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -245,6 +245,12 @@ int wave_groups(int ng, int tiles, int ncp, int stages) {
     if (wave_bytes(ng, kc, tiles, ncp, stages) > SMEM_MAX) for (kc = std::min(ng - 1, 8); kc > 1 && wave_bytes(ng, kc, tiles, ncp, stages) > SMEM_MAX;) kc = (kc + 1) / 2;
     return kc;
 }
+// units one behind the other in a warp, over all waves of one pass
+int unit_rounds(int ng, int tiles, int ncp, int mt, int warps) {
+    const int kc = wave_groups(ng, tiles, ncp, 0);
+    auto rounds = [&](int groups) { return ((tiles + mt - 1) / mt * groups + warps - 1) / warps; };
+    return ng / kc * rounds(kc) + (ng % kc ? rounds(ng % kc) : 0);
+}
 constexpr int NATIVE_NT = 512;
 template <int NCP, int MT, int NT, bool NATIVE = false>
 cudaError_t launch_t(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl) {
@@ -280,15 +286,28 @@ namespace bnk {
 
 cudaError_t launch_q2_gemm(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl) {
     const int ncp = a.ncol <= 8 ? 8 : (a.ncol <= 16 ? 16 : 32), tiles = (a.M + 15) / 16;
-    // Units of two row tiles (half the operand reads of one; three leave more warps without a unit) on 12 warps, whose first weights
-    // arrive beside the image. Layers of the 9B shape, with the preparation of the columns, weights in L2: 8 columns 43.0 us with
-    // units of three tiles (one where a CTA has two tiles at most) -> 39.3, 16 columns 58.9 with 16 warps -> 55.7. Otherwise: many
-    // tiles per CTA that come from DRAM (8 columns: the output head 82.6 us with units of three, 88 with two; 24 576 x 4096 13.5
-    // against 14.2 with the preparation), and 16 columns whose units fill 16 warps as well as 12 (rounds x warps, the tie:
-    // 24 576 x 4096 15.3 against 15.8 us).
-    const int nt = (tiles + sm_count - 1) / sm_count, units = (nt + 1) / 2 * (a.K / 512);
-    if (ncp == 8) return nt > (a.warm ? MAX_TILES : 6) ? launch_t<8, 3, 384>(st, sm_count, a, pdl) : launch_t<8, 2, 384>(st, sm_count, a, pdl);
-    if (ncp == 16) return (units + 15) / 16 * 16 <= (units + 11) / 12 * 12 ? launch_t<16, 2, 512>(st, sm_count, a, pdl) : launch_t<16, 2, 384>(st, sm_count, a, pdl);
+    // Units of several row tiles share operand reads, units of one spread over more warps. Times with the preparation of the columns.
+    // One tile, 16 warps: a CTA with one tile (a second one in a unit is the first again: 1024 x 4096 x 8 5.3 us with units of two, 4.9
+    // with one, 1024 x 8192 x 16 9.0 and 7.5), or so few units that most warps have none (3000 x 1024 x 8 4.4 and 4.0).
+    // 8 columns, 12 warps: two or three tiles by the rounds of a warp times what a unit costs, its tiles and about one more for its
+    // operands: 5500 x 4096 6.8 us with two, 6.3 with three; 8192 x 4096 7.1 and 8.4; 20 000 x 4096 from L2 11.0 and 9.6. Where that
+    // is even (24 576 x 4096 from L2, say, where they are equal in a serving step): three if they divide the tiles. Three also for many
+    // tiles that come from DRAM (the output head 82.6 us with three, 88 with two) and for several passes.
+    // 16 columns, two tiles: the number of warps that leaves fewer of them without a unit in the last round, 16 on a tie (24 576 x 4096
+    // 18.8 against 19.0 us; 4096 x 4096 6.8 with 12, 7.6 with 16).
+    const int nt = (tiles + sm_count - 1) / sm_count, ng = a.K / 512, n = std::min(nt, MAX_TILES);
+    const bool single = nt == 1 || nt * ng <= 4;
+    if (ncp == 8) {
+        if (single) return launch_t<8, 1, 512>(st, sm_count, a, pdl);
+        const int two = unit_rounds(ng, n, 8, 2, 12) * 3, three = unit_rounds(ng, n, 8, 3, 12) * 4;
+        const bool by_three = nt > (a.warm ? MAX_TILES : 6) || three < two || (three == two && nt % 3 == 0);
+        return by_three ? launch_t<8, 3, 384>(st, sm_count, a, pdl) : launch_t<8, 2, 384>(st, sm_count, a, pdl);
+    }
+    if (ncp == 16) {
+        if (single) return launch_t<16, 1, 512>(st, sm_count, a, pdl);
+        return unit_rounds(ng, n, 16, 2, 16) * 16 <= unit_rounds(ng, n, 16, 2, 12) * 12 ? launch_t<16, 2, 512>(st, sm_count, a, pdl)
+                                                                                         : launch_t<16, 2, 384>(st, sm_count, a, pdl);
+    }
     // 32 columns: a wave of all of K fits only the smallest matrices, where this kernel's units fill more warps (4096 x 4096, with the
     // preparation of the columns: 12.6 against 13.6 us); beyond, q2_gemm_wide.cu
     return tiles <= 2 * sm_count && a.K <= 4096 ? launch_t<32, 2, 512>(st, sm_count, a, pdl) : launch_q2_gemm_wide(st, sm_count, a, pdl);

@@ -28,6 +28,10 @@ def test_native_rows_take_the_faster_way(M, K, ncol, launches):
     (28417, 1024, 5, True),                                      # 13: more than one pass
     (4096, 2048, 16, True), (12288, 1024, 11, True),             # units for 12 warps, for 16
     (17, 12288, 16, True), (2367, 12288, 8, True),               # K in waves
+    (2368, 8192, 16, True), (2369, 8192, 16, True),              # one and two tiles: units of one, of two
+    (2368, 4096, 3, True), (2369, 4096, 3, True), (4736, 1024, 8, True), (4737, 1024, 8, True), (4736, 1024, 9, True),
+    (7104, 3072, 8, True), (7104, 4096, 8, True), (11841, 8192, 8, True), (14208, 8192, 2, True),      # units of two and three by rounds
+    (11841, 8192, 12, True), (4737, 16384, 8, True), (4736, 14336, 16, True),        # K in waves
 ])
 def test_columns_equal_single_projections(M, K, ncol, tiled, launches=None):
     rng = np.random.default_rng(M + K + ncol)
