@@ -1218,6 +1218,13 @@ int bn_model_fill_kv(bn_model *m, int stream, int n_positions) {
     return bn_launch_check(m->ctx, "bn_model_fill_kv");
 }
 
+int bn_projection_split(bn_ctx *ctx, int M, int K, int *clusters, int *tiles) {
+    BN_REQUIRE(ctx && clusters && tiles && M > 0, BN_ERR_ARG, "bn_projection_split: bad argument");
+    const bnk::Q2Split s = bnk::q2_gemv_split(ctx->sm_count, M, K);
+    *clusters = s.clusters; *tiles = s.tiles;
+    return BN_OK;
+}
+
 int bn_model_gemv_sweep(bn_model *m, int reps, float *ms_per_sweep) {
     BN_REQUIRE(m && m->finalized && ms_per_sweep && reps > 0, BN_ERR_ARG, "bn_model_gemv_sweep: bad argument");
     BN_REQUIRE(m->b0 == 0 && m->b1 == m->hp.n_layer, BN_ERR_STATE, "bn_model_gemv_sweep: whole model only");

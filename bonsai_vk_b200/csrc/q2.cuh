@@ -76,6 +76,9 @@ struct Q2Args {
 bool q2_gemv_supported(int K, int hat_block);
 // asks what launches depend on (how many clusters fit): once, ahead of any capture
 void q2_gemv_prepare();
+// how a projection of a plain input shares K among the CTAs of clusters: how many clusters (0: it does not), most row tiles of one
+struct Q2Split { int clusters = 0, tiles = 0; };
+Q2Split q2_gemv_split(int sm_count, int M, int K);
 cudaError_t launch_q2_gemv(cudaStream_t st, int sm_count, const Q2Args &a, bool pdl);
 
 struct Q2GemmArgs {

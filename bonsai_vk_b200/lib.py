@@ -102,6 +102,7 @@ def load_library() -> C.CDLL:
         "bn_model_fill_kv": (i32, [vp, i32, i32]),
         "bn_wrap": (i32, [vp, vp, sz, C.POINTER(vp)]),
         "bn_use_stream": (i32, [vp, vp]),
+        "bn_projection_split": (i32, [vp, i32, i32, C.POINTER(i32), C.POINTER(i32)]),
         "bn_model_gemv_sweep": (i32, [vp, i32, C.POINTER(C.c_float)]),
         "bn_model_mixer_sweep": (i32, [vp, i32, C.POINTER(C.c_float), C.POINTER(C.c_float)]),
         "bn_model_profile_token": (i32, [vp, i32, i32, vp, i32, C.POINTER(i32)]),
@@ -263,6 +264,12 @@ class Context(_Handle):
         sm, fr, tot = C.c_int(), C.c_size_t(), C.c_size_t()
         _check(self.lib.bn_device_info(self.h, C.byref(sm), C.byref(fr), C.byref(tot)), "bn_device_info")
         return {"sm_count": sm.value, "free_bytes": fr.value, "total_bytes": tot.value}
+
+    def projection_split(self, M: int, K: int) -> tuple[int, int]:
+        """(clusters, most row tiles of one) of a model's plain M x K projection; (0, 0): K is not shared among CTAs."""
+        n, t = C.c_int(), C.c_int()
+        _check(self.lib.bn_projection_split(self.h, M, K, C.byref(n), C.byref(t)), "bn_projection_split")
+        return n.value, t.value
 
     @property
     def launches(self) -> int:

@@ -288,6 +288,9 @@ int bn_model_decode(bn_model *m, int first_tok, int pos0, int n_steps, int *out_
  * runtime_vk/bonsai_vk.cpp:1452): launch every PTQ1_0 projection of one token back to back on the
  * model's own weights, `reps` times after one untimed pass, and return the CUDA-event time of one sweep */
 int bn_model_gemv_sweep(bn_model *m, int reps, float *ms_per_sweep);
+/* How a model's projection of a plain input (M rows, K values; the FFN's down projection, say) shares K among the CTAs of clusters:
+ * how many clusters are launched (0: every CTA takes all of K) and the most row tiles that one of them has. */
+int bn_projection_split(bn_ctx *ctx, int M, int K, int *clusters, int *tiles);
 /* lab: device time of what runs between a block's projections, per layer, averaged over `reps` sweeps of all layers of
  * the kind: the gated-delta-net core (reads and writes the layer's recurrent state once) and the attention chain (K/V
  * insert + decode over the prefix that ends at the current position). The recurrent cores run one behind the other's end, so
