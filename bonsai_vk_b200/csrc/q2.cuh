@@ -34,14 +34,16 @@ void pack_sign_bits(cudaStream_t st, const int32_t *signs, int n, uint8_t *bits)
 enum Q2Prologue { Q2_PLAIN = 0, Q2_NORM = 1 };
 // what follows this projection in the schedule: its weights (and norm weights) are prefetched into L2 from here
 struct Q2Share { int q, r; };             // CTA c takes q units, the first r CTAs one more
-constexpr int Q2_NEXT_BYTES = 256 << 10;  // per CTA: 38 MB in all, more than any projection of a block; the output head would push everything else out of L2
+// per CTA: 38 MB in all (31 from a split projection's 120), more than any projection of a block; the whole output head would push
+// everything else out of L2
+constexpr int Q2_NEXT_BYTES = 256 << 10;
 struct Q2Next {
     const uint8_t *W = nullptr;
     int units = 0, unit_bytes = 0;        // row tiles and their bytes
     int max_bytes = Q2_NEXT_BYTES;        // per CTA
     const float *w = nullptr;
     int w_bytes = 0;
-    Q2Share share = {0, 0};               // filled in by the launch
+    Q2Share share = {0, 0};               // filled in by the launch: the units dealt to THIS launch's CTAs
     // recurrent state that the mixer behind this projection reads: `cols` pieces, any CTA any part of them
     const float *state = nullptr;
     int cols = 0, col_bytes = 0;
@@ -106,8 +108,12 @@ cudaError_t launch_q2_gemm_wide(cudaStream_t st, int sm_count, Q2GemmArgs a, boo
 __device__ __forceinline__ void q2_prefetch(const uint8_t *p, int bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
-// thread `part` of `parts`: the share of the next projection's weights that CTA `cta`'s successor reads, and its norm weights, and
-// this CTA's part of the state, towards L2 (several threads, because a prefetch costs the one that asks for it some 70 cycles)
+// thread `part` of `parts`: CTA `cta`'s share of the next projection's weights, and its norm weights, and this CTA's part of the state,
+// towards L2 (several threads, because a prefetch costs the one that asks for it some 70 cycles). Shares are this grid's: below
+// Q2_NEXT_BYTES all weights are asked for, whatever the shares. The output head's are 1.8 MB, so behind the split down projection (120
+// CTAs, the head has 148) their first 256 KB are not what the head's CTAs read first. Shares of the head's grid, the 28 beyond this one's
+// dealt out in pieces, made every token slower, since each projection runs that code ahead of its dependency wait: 48 tokens 52.5 ->
+// 52.8 ms, 100-token prefill 13.66 -> 13.75 ms.
 __device__ __forceinline__ void q2_prefetch_next(const Q2Next &n, int cta, int part, int parts) {
     for (int k = cta + part * int(gridDim.x), per = (n.col_bytes + 16383) >> 14; k < n.cols * per; k += parts * int(gridDim.x)) {
         const int o = k % per * 16384;

@@ -107,8 +107,8 @@ __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Arg
     if (SPLIT) running();
     if (warp == NW) {
         // ---- copy warp. Before the previous kernel is done: one chunk of weights into the ring (more would hold up the input
-        // vector, which follows it through the same queue, by up to a microsecond) and the NEXT projection's weights (the
-        // share that this CTA's successor reads) towards L2; the other slots once the input vector is in registers; refills.
+        // vector, which follows it through the same queue, by up to a microsecond) and the NEXT projection's weights (a
+        // share of this grid) towards L2; the other slots once the input vector is in registers; refills.
         const uint8_t *W = a.W + (SPLIT ? size_t(t0) * parts + rank : size_t(t0)) * ng * Q2_PIECE;
         auto request = [&](int i, int s) {
             const uint32_t bytes = uint32_t(min(NW, npieces - i * NW)) * Q2_PIECE;
