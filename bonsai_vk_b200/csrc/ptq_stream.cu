@@ -3,16 +3,18 @@
 //
 // The arithmetic and the way the trits reach the tensor cores are those of ptq_gemv.cu: one multiply by 3^(t+1) turns two weight
 // bytes into an int8 operand register [r, T, r', T'] and the operand table of the activation pack (two columns per sub-block)
-// does the rest. What bounds it is instruction issue and latency: per 16 x 128 weights 32 products (two cycles of a scheduler each, as
-// shift-and-adds one), 8 byte permutes, 8 tensor-core steps, 7 loads and a quarter of the epilogue, 80 warp instructions in all,
-// against 145 in the kernel this replaces (two blocks per warp, sums across the warps of the CTA inside the loop, 16 bulk copies of
-// 896 bytes per 16 rows): 248 320 x 4096 in 116 us before. The tensor cores need 27 us of it (half of every operand is residue bytes),
-// memory 34 us. Measured beside it: pieces of a tile taken side by side, so that no line of DRAM comes in twice (232 MB are read for a
-// matrix of 117): with the warps' operands reloaded 96 us, from a table in shared memory and 16 warps 80 us.
+// does the rest. What bounds it is instruction issue and, nearly as much, memory: per 16 x 128 weights 32 products (two cycles of a
+// scheduler each, as shift-and-adds one), 8 byte permutes, 8 tensor-core steps, 7 loads and a quarter of the epilogue, 80 warp
+// instructions in all, against 145 in the kernel this replaces (two blocks per warp, sums across the warps of the CTA inside the loop,
+// 16 bulk copies of 896 bytes per 16 rows): 248 320 x 4096 in 116 us before. The tensor cores need 27 us of it (half of every operand
+// is residue bytes). A line of DRAM holds parts of two pieces of a row, which are taken at different times: 445 MB are read for this
+// matrix of 222 (131 072 x 4096: 232 MB for 117), 68 us at the copy rate. Measured beside it: pieces of a tile taken side by side, so
+// that no line comes in twice: with the warps' operands reloaded 96 us, from a table in shared memory and 16 warps 80 us.
 //
-// Work split. A CTA of 12 warps (16 of 128 registers each were slower: 16.1 against 13.9 us at 24 576 x 4096) owns a run of 16-row tiles over all of K. The pieces (16 rows x 4 blocks, the unit p_g of the
-// summation order) of a run are dealt to the warps group-major, so a warp stays with one group's operand table - 64 registers -
-// for most of its pieces; group sums meet in shared memory, where one thread per row adds them in ascending order.
+// Work split. A CTA of 12 warps (16 of 128 registers each were slower: 16.1 against 13.9 us at 24 576 x 4096) owns a run of 16-row tiles
+// over all of K. The pieces (16 rows x 4 blocks, the unit p_g of the summation order) of a run are dealt to the warps group-major, so a
+// warp stays with one group's operand table - 64 registers - for most of its pieces; group sums meet in shared memory, where one thread
+// per row adds them in ascending order.
 // Data movement. A piece is 16 rows of 112 bytes, brought by cp.async (16, 8 or 4 bytes at a time, whichever the rows' alignment
 // allows) into a ring of its warp's own. The pitch of 112 bytes is free of bank conflicts for every load of the loop: eight rows
 // start four banks apart and the four lanes of a row read words 0, 2, 3, 5 (one in each residue modulo 4).
@@ -262,8 +264,9 @@ cudaError_t ptq_stream(cudaStream_t st, int sm_count, const void *W, int M, int 
     const size_t smem = size_t(NW) * ST * PIECE + 512 + size_t(a.run) * ng * 64;
     // the widest copy that every row of every piece starts on
     const uintptr_t align = reinterpret_cast<uintptr_t>(W) | uintptr_t(a.nb * 28);
-    // A chain of shift-and-adds per half-word pair where a CTA has many pieces (248 320 x 4096: 79.3 -> 75.3 us, 30 000 x 8192 23.9 ->
-    // 23.4), products side by side where the first piece's latency counts (1024 x 4096 3.2 against 3.4 us, 7000 x 3584 5.4 against
+    // A chain of shift-and-adds per half-word pair where a CTA has many pieces (248 320 x 4096: 81.6 -> 77.5 us in a loop over the matrix,
+    // 87.1 -> 84.3 with two matrices in turn, 88.9 -> 87.2 with the quantiser in front; 30 000 x 8192 23.9 -> 23.4 in the loop),
+    // products side by side where the first piece's latency counts (1024 x 4096 3.2 against 3.4 us, 7000 x 3584 5.4 against
     // 5.5) and where copies of 4 or 8 bytes take the issue slots (30 000 x 4736 20.3 against 20.7).
     if (align % 16 == 0) return most * ng >= 10 * NW ? launch_a<16, true>(st, grid, smem, a) : launch_a<16>(st, grid, smem, a);
     if (align % 8 == 0) return launch_a<8>(st, grid, smem, a);
