@@ -1,4 +1,4 @@
-"""ctypes binding of libbonsai_cuda.so (C ABI: include/bonsai_cuda.h)."""
+"""Python binding of libbonsai_cuda.so (C ABI: include/bonsai_cuda.h): ctypes, and host/fastcall.c for the op-level entry points."""
 from __future__ import annotations
 
 import ctypes as C

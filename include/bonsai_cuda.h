@@ -134,9 +134,9 @@ int bn_gemm_act_quant(bn_ctx *ctx, const bn_buf *x, size_t x_off, size_t x_strid
  * 512 weights of K one contiguous piece; rows beyond M are zero. About a fifth larger than the matrix itself. */
 size_t bn_gemm_tiled_bytes(int M, int K);
 int bn_gemm_repack(bn_ctx *ctx, const bn_buf *w, size_t w_off, int M, int K, bn_buf *tiled, size_t tiled_off);
-/* w_tiled = 0: w is the native row-major matrix; 1: w is the copy made by bn_gemm_repack. Native rows of up to 16
- * columns, or of more where the matrix is small, are unpacked by the kernel itself; others into up to 48 MB of memory that the
- * context keeps, unless the call is inside a stream capture or that memory is not to be had: a captured graph refers to nothing of
+/* w_tiled = 0: w is the native row-major matrix; 1: w is the copy made by bn_gemm_repack. Native rows are
+ * unpacked by the kernel itself where that is the faster way (few columns, or small matrices); others into up to 48 MB of memory
+ * that the context keeps, unless the call is inside a stream capture or that memory is not to be had: a captured graph refers to nothing of
  * the context's. Same results.
  * out: column c at out + c * out_stride floats, M values each */
 int bn_gemm_q81(bn_ctx *ctx, const bn_buf *w, size_t w_off, int w_tiled, int M, int K, const bn_buf *image, size_t image_off,
