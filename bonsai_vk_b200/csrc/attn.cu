@@ -15,26 +15,30 @@ __device__ __forceinline__ void pdl_early() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// q8_0 of one 32-element block held one value per lane (recipe: attn_norm_rope2.comp:39-49,184-217)
+// q8_0 of one 32-element block held one value per lane (recipe: attn_norm_rope2.comp:39-49,184-217). Division and rounding are
+// those of the projections' quantiser (rotate_quant.cuh); the largest magnitude of the warp is one instruction, which leaves NaNs out
+// as fmaxf does.
 __device__ __forceinline__ void q80_store(float v, int lane, int8_t *codes, uint16_t *scale) {
-    float amax = fabsf(v);
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, s));
-    const float d = amax > 1e-35f ? __fdiv_rn(amax, 127.0f) : 0.0f;
-    const float id = d != 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
-    float r = roundf(__fmul_rn(v, id));
-    r = fminf(fmaxf(r, -127.0f), 127.0f);
-    codes[lane] = int8_t(int(r));
+    float amax;
+    asm("redux.sync.max.abs.f32 %0, %1, 0xffffffff;" : "=f"(amax) : "f"(v));
+    const bool some = amax > 1e-35f;
+    const float d = some ? div127(amax) : 0.0f, id = some ? __frcp_rn(d) : 0.0f;
+    codes[lane] = int8_t(code_byte(__fmul_rn(v, id)));
     if (lane == 0) *scale = (uint16_t)float_to_half_bits(d);
 }
 
-// one CTA per head row (n_head query rows, then n_kv key rows) and column or token; blockDim = head_dim = 256.
+// one CTA per head row (n_head query rows, then n_kv key rows) and column or token; a thread per dim (head_dim = 256), and a ninth warp
+// for the serial sum, beside which the others deal with the row that needs no norm (gate, or quantised V).
 // Query rows: RMS norm * weight, NeoX rope on the first n_rot dims, fp16 rounding, gate split; the row's softmax maximum is
 // cleared. Key rows: the same norm / rope, then cache insert (fp16 or q8_0) of K and of the raw V row.
 // Columns (cols.n > 0) are sequences; tokens (the op-level insert) are consecutive positions whose rows follow each other, and
 // only the last one's query is kept. The rope factors need the position only (set before the pass: the rule at bnk::launch)
 // and are worked out before the wait: a double-precision power, sine and cosine are most of this kernel's chain.
-__global__ void __launch_bounds__(256) k_attn_prep(AttnDims a, AttnPos where, const float *__restrict__ qg, const float *__restrict__ kin,
+// What bounds it is that chain (256 dependent additions, 0.7 us) and the quantiser behind it. With V quantised last, by divisions and five
+// shuffles, a key row's CTA took 1.5 us from the dependency wait on; an insert and an attention over 64 keys 9.72 -> 9.53 us, 500 keys
+// 10.18 -> 9.93.
+constexpr int PREP_T = 288;
+__global__ void __launch_bounds__(PREP_T) k_attn_prep(AttnDims a, AttnPos where, const float *__restrict__ qg, const float *__restrict__ kin,
                                                    const float *__restrict__ vin, const float *__restrict__ qn_w, const float *__restrict__ kn_w,
                                                    KvLayer kv, float *__restrict__ q16f, float *__restrict__ gate, unsigned *__restrict__ mx, Cols cols) {
     const int tok = cols.n > 0 ? 0 : blockIdx.z;
@@ -43,16 +47,16 @@ __global__ void __launch_bounds__(256) k_attn_prep(AttnDims a, AttnPos where, co
     __shared__ float sx[256];
     __shared__ float ssum;
     const int d = threadIdx.x, hd = a.head_dim, w = blockIdx.x;
-    const bool is_q = w < a.n_head;
+    const bool is_q = w < a.n_head, elem = d < 256;
     const int h = is_q ? w : w - a.n_head;
     if (is_q && tok + 1 < int(gridDim.z) && cols.n == 0) return;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int pos = where.get() + tok;
     const float *nwp = is_q ? qn_w : kn_w;
     const int half = a.n_rot >> 1, p = d < half ? d : d - half, pd = d < half ? d + half : d - half;
-    const float nw = nwp[d];
+    const float nw = elem ? nwp[d] : 0.0f, inv_hd = 1.0f / float(hd);      // (a power of two: the product with it is the quotient)
     float c = 1.0f, s = 0.0f, nwr = 0.0f;
-    if (d < a.n_rot) {
+    if (d < a.n_rot) {                             // (the ninth warp has no dims: n_rot <= 256)
         const float ex = __fdiv_rn(__fmul_rn(-2.0f, float(p)), float(a.n_rot));
         const float th = float(pow(double(a.rope_base), double(ex)));
         const float ang = __fmul_rn(float(pos), th);
@@ -61,24 +65,44 @@ __global__ void __launch_bounds__(256) k_attn_prep(AttnDims a, AttnPos where, co
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const float *src = is_q ? qg + size_t(h) * 2 * hd : kin + (size_t(tok) * a.n_kv + h) * hd;
-    const float x = src[d], vr = is_q ? src[hd + d] : vin[(size_t(tok) * a.n_kv + h) * hd + d];
-    sx[d] = x;
-    part[d] = __fmul_rn(x, x);
+    const size_t row = (size_t(pos) * a.n_kv + h) * hd;
+    const int lane = d & 31, blk = d >> 5;
+    float x = 0.0f, vr = 0.0f;
+    if (elem) {
+        x = src[d];
+        vr = is_q ? src[hd + d] : vin[(size_t(tok) * a.n_kv + h) * hd + d];
+        sx[d] = x;
+        part[d] = __fmul_rn(x, x);
+    }
     __syncthreads();
-    // the 256 squares are added serially in ascending order, as the reference's CPU mirror adds them
-    // (attn_vk.h:102-108), so that the fp16 operands below are the mirror's bit for bit
-    if (d == 0) {
+    if (elem) {
+        if (is_q) {
+            gate[size_t(h) * hd + d] = vr;
+            if (d == 0) mx[h] = 0u;
+        } else if (a.v_mode == 1) reinterpret_cast<__half *>(kv.v_data)[row + d] = __float2half_rn(vr);
+        else q80_store(vr, lane, reinterpret_cast<int8_t *>(kv.v_data) + row + blk * 32, kv.v_scale + row / 32 + blk);
+    } else if (lane == 0) {
+        // the 256 squares are added serially in ascending order, as the reference's CPU mirror adds them
+        // (attn_vk.h:102-108), so that the fp16 operands below are the mirror's bit for bit
         float acc = 0.0f;
         const float4 *p4 = reinterpret_cast<const float4 *>(part);
-#pragma unroll 8
-        for (int i = 0; i < 64; ++i) {
-            const float4 v = p4[i];
-            acc = __fadd_rn(acc, v.x); acc = __fadd_rn(acc, v.y); acc = __fadd_rn(acc, v.z); acc = __fadd_rn(acc, v.w);
+        float4 v[8], n[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = p4[i];
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {              // (the next eight loads in front of these additions)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) n[i] = p4[min(b + 1, 7) * 8 + i];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { acc = __fadd_rn(acc, v[i].x); acc = __fadd_rn(acc, v[i].y); acc = __fadd_rn(acc, v[i].z); acc = __fadd_rn(acc, v[i].w); }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = n[i];
         }
         ssum = acc;
     }
     __syncthreads();
-    const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ssum, float(hd)), a.eps)));
+    if (!elem) return;
+    const float inv = __frcp_rn(__fsqrt_rn(__fadd_rn(__fmul_rn(ssum, inv_hd), a.eps)));
     float y = __fmul_rn(__fmul_rn(x, inv), nw);
     if (d < a.n_rot) {
         const float xp = __fmul_rn(__fmul_rn(sx[pd], inv), nwr);
@@ -86,16 +110,10 @@ __global__ void __launch_bounds__(256) k_attn_prep(AttnDims a, AttnPos where, co
     }
     if (is_q) {
         q16f[size_t(h) * hd + d] = __half2float(__float2half_rn(y));
-        gate[size_t(h) * hd + d] = vr;
-        if (d == 0) mx[h] = 0u;
         return;
     }
-    const size_t row = (size_t(pos) * a.n_kv + h) * hd;
-    const int lane = d & 31, blk = d >> 5;
     if (a.k_mode == 1) reinterpret_cast<__half *>(kv.k_data)[row + d] = __float2half_rn(y);
     else q80_store(y, lane, reinterpret_cast<int8_t *>(kv.k_data) + row + blk * 32, kv.k_scale + row / 32 + blk);
-    if (a.v_mode == 1) reinterpret_cast<__half *>(kv.v_data)[row + d] = __float2half_rn(vr);
-    else q80_store(vr, lane, reinterpret_cast<int8_t *>(kv.v_data) + row + blk * 32, kv.v_scale + row / 32 + blk);
 }
 
 // Scores: a warp takes octets of consecutive keys of one kv head (attn_octet.cuh), the next octet's rows in flight while it works
@@ -448,8 +466,8 @@ void attn_prep(cudaStream_t st, AttnDims a, const float *qg, const float *kin, c
     unsigned *mx = reinterpret_cast<unsigned *>(esum + size_t(a.n_head) * 128);
     const dim3 grid(a.n_head + a.n_kv, 1, cols.n > 0 ? cols.z() : tokens);
     // (one token's few CTAs run beside the projection in front of them)
-    if (grid.z == 1) launch(k_attn_prep, grid, dim3(256), 0, st, a, where, qg, kin, vin, qn_w, kn_w, kv, q16f, gate, mx, cols);
-    else launch_spread<k_attn_prep>(grid, dim3(256), 0, st, a, where, qg, kin, vin, qn_w, kn_w, kv, q16f, gate, mx, cols);
+    if (grid.z == 1) launch(k_attn_prep, grid, dim3(PREP_T), 0, st, a, where, qg, kin, vin, qn_w, kn_w, kv, q16f, gate, mx, cols);
+    else launch_spread<k_attn_prep>(grid, dim3(PREP_T), 0, st, a, where, qg, kin, vin, qn_w, kn_w, kv, q16f, gate, mx, cols);
 }
 void attn_decode(cudaStream_t st, AttnDims a, const float *q16f, const float *gate, AttnPos where, KvLayer kv,
                  float *score, float *p16f, float *esum, float *pv_part, int splits, float *pregate, float *gated, Cols cols) {
