@@ -470,10 +470,10 @@ void attn_prep(cudaStream_t st, AttnDims a, const float *qg, const float *kin, c
     else launch_spread<k_attn_prep>(grid, dim3(PREP_T), 0, st, a, where, qg, kin, vin, qn_w, kn_w, kv, q16f, gate, mx, cols);
 }
 void attn_decode(cudaStream_t st, AttnDims a, const float *q16f, const float *gate, AttnPos where, KvLayer kv,
-                 float *score, float *p16f, float *esum, float *pv_part, int splits, float *pregate, float *gated, Cols cols) {
+                 float *score, float *p16f, float *esum, float *pv_part, int splits, float *pregate, float *gated, int *err, Cols cols) {
     // one query token: one launch up to 8192 positions. With several columns (serving, prefill) the chain of kernels below
     // fills the GPU better than 64 large CTAs per column (8 columns at 2048 positions: 2.46 against 2.62 ms a pass).
-    if (cols.z() == 1 && attn_cluster(st, a, q16f, gate, where, kv, splits, pregate, gated, cols)) return;
+    if (cols.z() == 1 && attn_cluster(st, a, q16f, gate, where, kv, splits, pregate, gated, cols, err)) return;
     // grids are sized for the cache capacity; CTAs beyond the filled prefix return at once.
     // esum: [n_head][128] partial softmax sums, then n_head row maxima (cleared by attn_prep and again by the combine kernel)
     unsigned *mx = reinterpret_cast<unsigned *>(esum + size_t(a.n_head) * 128);

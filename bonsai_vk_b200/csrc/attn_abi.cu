@@ -105,7 +105,7 @@ int bn_attn_attend(bn_ctx *ctx, const bn_attn_dims *d, const bn_buf *kv, size_t 
     bnk::attn_decode(ctx->stream, to_dims(*d), reinterpret_cast<float *>(sb + S.q16f), reinterpret_cast<float *>(sb + S.gate),
                      {nullptr, pos}, kv_of(*d, kv, kv_off), reinterpret_cast<float *>(sb + S.score),
                      reinterpret_cast<float *>(sb + S.pe), reinterpret_cast<float *>(sb + S.esum), reinterpret_cast<float *>(sb + S.pv),
-                     splits_for(d->cap), pregate ? bn_ptr<float>(pregate, pg_off) : nullptr, bn_ptr<float>(gated, g_off));
+                     splits_for(d->cap), pregate ? bn_ptr<float>(pregate, pg_off) : nullptr, bn_ptr<float>(gated, g_off), ctx->err_dev);
     return bn_launch_check(ctx, "bn_attn_attend");
 }
 

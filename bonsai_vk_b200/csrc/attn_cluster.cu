@@ -1,8 +1,11 @@
 // attn_cluster.cu - decode attention of one query token in ONE launch, for caches of up to 8192 positions: a thread-block cluster
 // of 16 CTAs per kv head keeps scores, numerators, probabilities and partial outputs in distributed shared memory. The chain of
 // four kernels in attn.cu costs about 3.5 us of latency per kernel on the device and 2.2 us each on the host, whatever the
-// length; here the exchanges are four cluster barriers. With the insert in front, host side included: 1501 keys 16.9 -> 11.4 us,
-// 4096 keys 21.0 -> 17.6 us.
+// length; here the CTAs exchange four times (maxima, numerators, sums, partial outputs) by stores into each other's shared memory that
+// an mbarrier over there counts, so an exchange costs one way across the cluster. As plain stores and a cluster barrier it cost the
+// stores' acknowledgement and the barrier's round trip as well, some 0.4 us each: with the insert in front 1501 keys (8192 positions)
+// 11.5 -> 9.9 us, 4096 keys 17.4 -> 15.3, 64 keys 9.5 -> 7.9 (the scales of V by asynchronous copies, 0.4 us of it, included).
+// What bounds it: latency below 1000 keys, then instruction issue of scores and values on its 64 SMs.
 //
 // Arithmetic and the order of every sum are those of attn.cu (and of the CPU oracle): scores by an fmaf chain over 8 dims per
 // lane and the xor tree; 1024 "virtual threads" of ascending partial softmax sums combined by the tree 512 .. 1; probabilities
@@ -30,7 +33,7 @@ __host__ __device__ __forceinline__ Shape shape_of(int splits, int cap) {
     s.rcap = s.spc * ((cap + splits - 1) / splits);
     return s;
 }
-struct Lay { int v, vsc, eg, eb, sums, mx, part, red, total; };
+struct Lay { int v, vsc, eg, eb, sums, mx, part, red, bars, total; };
 template <int GQA, int VMODE> __host__ __device__ __forceinline__ Lay layout(const Shape &s, int splits, int cap) {
     Lay l;
     int o = 0;
@@ -46,6 +49,7 @@ template <int GQA, int VMODE> __host__ __device__ __forceinline__ Lay layout(con
     o = (o + 15) & ~15;
     l.part = o; o += splits * (GQA * HD / CL) * 4;
     l.red = o; o += 2 * GQA * 4;
+    l.bars = o = (o + 7) & ~7; o += 4 * 8;
     l.total = o;
     return l;
 }
@@ -55,10 +59,25 @@ __device__ __forceinline__ uint32_t remote(const void *p, int rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(uint32_t(__cvta_generic_to_shared(p))), "r"(rank));
     return r;
 }
-__device__ __forceinline__ void put(uint32_t addr, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
-__device__ __forceinline__ void put2(uint32_t addr, float a, float b) { asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(a), "f"(b) : "memory"); }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// stores into another CTA of the cluster, counted by a barrier there
+__device__ __forceinline__ void put(uint32_t addr, float v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(__float_as_uint(v)), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void put2(uint32_t addr, float a, float b, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(addr), "r"(__float_as_uint(a)), "r"(__float_as_uint(b)), "r"(bar) : "memory");
+}
+// bounded wait for an exchange's bytes; on giving up the error word is set and the caller goes on without waiting again (results
+// are then invalid)
+__device__ __forceinline__ bool arrived(uint32_t bar, int *err, int limit = 1 << 22) {
+    for (int it = 0; it < limit; ++it) {
+        uint32_t ok;
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(ok) : "r"(bar) : "memory");
+        if (__builtin_expect(ok != 0u, 1)) return true;
+    }
+    atomicExch(err, 5);
+    return false;
+}
 
 struct Args {
     AttnDims a;
@@ -69,6 +88,7 @@ struct Args {
     float scale, nz;                           // nz = -0: see k_attn_pv in attn.cu
     float *pregate, *gated;
     Cols cols;
+    int *err;
 };
 
 template <int GQA, int KMODE, int VMODE>
@@ -90,14 +110,29 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
     unsigned *red = reinterpret_cast<unsigned *>(smem + L.red);
     float *tot = reinterpret_cast<float *>(red + GQA);
     const int rank = blockIdx.x, kvh = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    cluster_arrive();                          // "I am running": waited for before the first store into a neighbour
-    if (tid < GQA) red[tid] = 0u;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int nfill = where.get() + 1, splits = g.splits, per = (nfill + splits - 1) / splits;
+    // (the position was set before the pass: the rule at bnk::launch)
+    const int nfill = where.get() + 1, splits = g.splits, per = (nfill + splits - 1) / splits, used = (nfill + per - 1) / per;
     const int grp = rank / sh.nsl, sl = rank - grp * sh.nsl;             // which splits, which dims of them
     const int r0 = min(nfill, grp * sh.spc * per), n = min(nfill, (grp + 1) * sh.spc * per) - r0;
     const int o0 = r0 + n * sl / sh.nsl, o1 = r0 + n * (sl + 1) / sh.nsl; // keys this CTA scores
+    // the four exchanges and the bytes that come with each: maxima; numerators (of this CTA's residues, and of a split that it shares);
+    // sums; partial outputs
+    const uint32_t bars = uint32_t(__cvta_generic_to_shared(smem + L.bars));
+    if (tid == 0) {
+        const int own = (nfill >> 7) * RL + max(0, min(RL, (nfill & 127) - rank * RL));
+        const int bytes[4] = {CL * GQA * 4, (own + (sh.nsl > 1 ? n : 0)) * GQA * 4, GQA * 128 * 4, used * OPC * 4};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + i * 8));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < 4; ++i) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bars + i * 8), "r"(bytes[i]) : "memory");
+    }
+    if (tid < GQA) red[tid] = 0u;
+    // "I am running, my barriers count": waited for before the first store into a neighbour
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    bool alive = true;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 
     // ---- K octets of the first round and the V slice on their way ------------------------------------------------------
     // (KeyOctet::fetch and, below, load_queries in place: called, they make the fp16 kernel up to 2 % slower, 11.7 against 11.4 us at
@@ -126,13 +161,22 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
             const int k = i >> csh, b = (i & (ch - 1)) * 16;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + k * rb + b), "l"(src + k * stride + b) : "memory");
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
     }
+    // its scales: eight, four (with the copies) or one per key (through a register, stored behind the scores)
     const int nsc = sh.D >= 32 ? sh.D / 32 : 1, ssh = 31 - __clz(nsc);
+    const uint16_t *vsrc = kv.v_scale + (size_t(r0) * a.n_kv + kvh) * (HD / 32) + sl * sh.D / 32;
+    uint16_t vs0 = 0;
     if (VMODE == 0) {
-        const uint16_t *src = kv.v_scale + (size_t(r0) * a.n_kv + kvh) * (HD / 32) + sl * sh.D / 32;
-        for (int i = tid; i < n << ssh; i += T) vsc[i] = src[size_t(i >> ssh) * a.n_kv * (HD / 32) + (i & (nsc - 1))];
+        const uint32_t dst = uint32_t(__cvta_generic_to_shared(vsc));
+        if (nsc == 1) { if (tid < n) vs0 = vsrc[size_t(tid) * a.n_kv * (HD / 32)]; }
+        else
+            for (int i = tid; i < n; i += T) {
+                const uint16_t *s = vsrc + size_t(i) * a.n_kv * (HD / 32);
+                if (nsc == 8) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * 16), "l"(s) : "memory");
+                else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + i * 8), "l"(s) : "memory");
+            }
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
 
     // ---- scores ------------------------------------------------------------------------------------------------------------
     const f32pair magic2 = pair_of(CODE_MAGIC, CODE_MAGIC);
@@ -164,15 +208,16 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
         if (hp == 0) __syncthreads();          // red is cleared
         if (lane < 4) atomicMax(red + hp * G + (lane >> GSH), ord(best));
     }
+    if (VMODE == 0 && nsc == 1)
+        for (int i = tid; i < n; i += T) vsc[i] = i == tid ? vs0 : vsrc[size_t(i) * a.n_kv * (HD / 32)];
     __syncthreads();
-    cluster_wait();                            // every CTA is running
-    for (int i = tid; i < CL * GQA; i += T) put(remote(mxs + rank * GQA + i % GQA, i / GQA), unord(red[i % GQA]));
-    cluster_arrive();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // every CTA is running
+    for (int i = tid; i < CL * GQA; i += T) put(remote(mxs + rank * GQA + i % GQA, i / GQA), unord(red[i % GQA]), remote(smem + L.bars, i / GQA));
     // (the gate of the outputs that this CTA finishes, off the tail)
     const int orow = (kvh * GQA * HD) + rank * OPC + tid;
     float gt = 0.0f;
     if (tid < OPC) gt = __fdiv_rn(1.0f, __fadd_rn(1.0f, exp_f(-gate[orow])));
-    cluster_wait();
+    alive = arrived(bars, g.err);
 
     // ---- numerators: to the CTAs that share the split and to the one that sums the residue ------------------------------------
     {
@@ -184,13 +229,12 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
             // (o0 - r0) * GQA is a multiple of GQA, so i % GQA == h
             const int j = r0 + i / GQA, res = j & 127;
             const float e = exp_f(__fsub_rn(__fmul_rn(eg[i], g.scale), mx));
-            put(remote(eb + (h * ((a.cap + 127) >> 7) + (j >> 7)) * RL + res % RL, res / RL), e);
+            put(remote(eb + (h * ((a.cap + 127) >> 7) + (j >> 7)) * RL + res % RL, res / RL), e, remote(smem + L.bars + 8, res / RL));
             if (sh.nsl == 1) eg[i] = e;
-            else for (int p = 0; p < sh.nsl; ++p) put(remote(eg + i, grp * sh.nsl + p), e);
+            else for (int p = 0; p < sh.nsl; ++p) put(remote(eg + i, grp * sh.nsl + p), e, remote(smem + L.bars + 8, grp * sh.nsl + p));
         }
     }
-    cluster_arrive();
-    cluster_wait();
+    if (alive) alive = arrived(bars + 8, g.err);
     // ---- softmax sums: thread (head, residue, a) adds the keys of virtual thread 128 a + residue ascending ---------------------
     if (tid < GQA * RL * 8) {
         const int av = tid & 7, rl = (tid >> 3) % RL, h = (tid >> 3) / RL, res = rank * RL + rl;
@@ -199,12 +243,11 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
         for (int m = av; m * 128 + res < nfill; m += 8) s = __fadd_rn(s, p[m * RL]);
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1) s = __fadd_rn(s, __shfl_xor_sync(0xFFFFFFFFu, s, o));      // tree steps 512, 256, 128
-        put(remote(sums + h * 128 + res, av), s);
-        put(remote(sums + h * 128 + res, av + 8), s);
+        put(remote(sums + h * 128 + res, av), s, remote(smem + L.bars + 16, av));
+        put(remote(sums + h * 128 + res, av + 8), s, remote(smem + L.bars + 16, av + 8));
     }
-    cluster_arrive();
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    cluster_wait();
+    if (alive) alive = arrived(bars + 16, g.err);
     if (warp < GQA) {
         const float *p = sums + warp * 128 + lane;
         float s = __fadd_rn(__fadd_rn(p[0], p[64]), __fadd_rn(p[32], p[96]));
@@ -262,7 +305,7 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
                 float x, y;
                 split_pair(acc[h], x, y);
                 const int o = h * HD + d;
-                put2(remote(part + (grp * 4 + s) * OPC + o % OPC, o / OPC), x, y);
+                put2(remote(part + (grp * 4 + s) * OPC + o % OPC, o / OPC), x, y, remote(smem + L.bars + 24, o / OPC));
             }
         }
     } else if (sh.nsl == 2) {                  // 128 threads (one warp per scheduler): one dim, all heads
@@ -281,7 +324,7 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
 #pragma unroll
             for (int h = 0; h < GQA; ++h) {
                 const int o = h * HD + sl * 128 + tid;
-                put(remote(part + grp * OPC + o % OPC, o / OPC), acc[h]);
+                put(remote(part + grp * OPC + o % OPC, o / OPC), acc[h], remote(smem + L.bars + 24, o / OPC));
             }
         }
     } else if (tid < 16 * GQA) {               // one split: a thread owns one dim of one head
@@ -290,13 +333,13 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
 #pragma unroll 8
         for (int k = 0; k < n; ++k) acc = __fadd_rn(acc, __fmul_rn(eg[k * GQA + h], value(k, d)));
         const int o = h * HD + sl * 16 + d;
-        put(remote(part + o % OPC, o / OPC), acc);
+        put(remote(part + o % OPC, o / OPC), acc, remote(smem + L.bars + 24, o / OPC));
     }
-    cluster_arrive();
-    cluster_wait();
-    // ---- splits ascending, gate (nobody reads a neighbour's memory from here on) ---------------------------------------------------
+    // a CTA that has its part of every exchange has all that is stored into it; one that gave up waits for the others to end
+    if (alive) alive = arrived(bars + 24, g.err);
+    if (!alive) asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+    // ---- splits ascending, gate ----------------------------------------------------------------------------------------------------
     if (tid < OPC) {
-        const int used = (nfill + per - 1) / per;
         float s = part[tid];
         int i = 1;
         for (; i + 8 <= used; i += 8) {
@@ -309,6 +352,16 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
         for (; i < used; ++i) s = __fadd_rn(s, part[i * OPC + tid]);
         if (g.pregate) colp(g.pregate, col * g.cols.arena)[orow] = s;
         colp(g.gated, col * g.cols.arena)[orow] = __fmul_rn(s, gt);
+    }
+}
+
+// A wait that nothing will ever satisfy, with a short limit: the give-up path of arrived()
+__global__ void k_wait_selftest_exchange(int *err) {
+    __shared__ uint64_t bar;
+    const uint32_t b = uint32_t(__cvta_generic_to_shared(&bar));
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\nfence.mbarrier_init.release.cluster;" ::"r"(b) : "memory");
+        arrived(b, err, 1 << 10);
     }
 }
 
@@ -355,10 +408,16 @@ bool launch_g(cudaStream_t st, const Args &g) {
 
 namespace bnk {
 
-bool attn_cluster(cudaStream_t st, AttnDims a, const float *q16f, const float *gate, AttnPos where, KvLayer kv, int splits, float *pregate, float *gated, Cols cols) {
+cudaError_t launch_wait_selftest_exchange(cudaStream_t st, int *err) {
+    BN_COUNT(1);
+    k_wait_selftest_exchange<<<1, 32, 0, st>>>(err);
+    return cudaGetLastError();
+}
+
+bool attn_cluster(cudaStream_t st, AttnDims a, const float *q16f, const float *gate, AttnPos where, KvLayer kv, int splits, float *pregate, float *gated, Cols cols, int *err) {
     if (a.cap > 8192 || (splits != 1 && splits != 8 && splits != 64)) return false;
     if (getenv("BONSAI_ATTN_CHAIN")) return false;                         // the answer "does not fit", for comparisons
-    const Args g = {a, where, q16f, gate, kv, splits, 1.0f / sqrtf(float(a.head_dim)), -0.0f, pregate, gated, cols};
+    const Args g = {a, where, q16f, gate, kv, splits, 1.0f / sqrtf(float(a.head_dim)), -0.0f, pregate, gated, cols, err};
     switch (a.n_head / a.n_kv) {
         case 1: return launch_g<1>(st, g);
         case 2: return launch_g<2>(st, g);

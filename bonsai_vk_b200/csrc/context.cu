@@ -211,7 +211,7 @@ int bn_sync(bn_ctx *ctx) {
             return BN_ERR_ARG;
         }
         bn_set_error("a bounded device-side wait gave up (%s); results of the last kernels are invalid",
-                     flag == 2 ? "tensor-core projection pipeline" : flag == 4 ? "grid barrier of the whole-token kernel" : "copy ring");
+                     flag == 2 ? "tensor-core projection pipeline" : flag == 4 ? "grid barrier of the whole-token kernel" : flag == 5 ? "exchange of the attention clusters" : "copy ring");
         return BN_ERR_TIMEOUT;
     }
     return BN_OK;

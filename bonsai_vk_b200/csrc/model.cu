@@ -204,7 +204,7 @@ void attn_plain(bn_model *m, const bn_model::Layer &L) {
     project(m, L.k_w, KD, h.hidden, m->PACK_H, m->KBUF);
     project(m, L.v_w, KD, h.hidden, m->PACK_H, m->VBUF);
     bnk::attn_prep(st, a, m->QKV, m->KBUF, m->VBUF, L.q_norm, L.k_norm, {m->POS, 0}, kv, m->Q16F, m->GATEB, m->ESUM);
-    bnk::attn_decode(st, a, m->Q16F, m->GATEB, {m->POS, 0}, kv, m->SCORE, m->P16F, m->ESUM, m->PVPART, m->pv_splits, nullptr, m->GOUT);
+    bnk::attn_decode(st, a, m->Q16F, m->GATEB, {m->POS, 0}, kv, m->SCORE, m->P16F, m->ESUM, m->PVPART, m->pv_splits, nullptr, m->GOUT, m->ctx->err_dev);
     rot_project(m, m->GOUT, m->signs, QD, m->PACK_H, L.o_w, h.hidden, m->D);
     bnk::add_inplace(st, m->RES, m->D, h.hidden);
 }
@@ -306,7 +306,7 @@ void attn_fused(bn_model *m, const bn_model::Layer &L) {
     norm_project(m, L.q2_in, 2 * QD + 2 * KD, L.attn_norm, m->QKV, q2_next(L.q2_out, h.hidden, QD, nullptr), BEFORE_ATTENTION);
     if (!m->phases_only) {
         bnk::attn_prep(st, ad, m->QKV, m->KBUF, m->VBUF, L.q_norm, L.k_norm, {m->POS, 0}, kv, m->Q16F, m->GATEB, m->ESUM);
-        bnk::attn_decode(st, ad, m->Q16F, m->GATEB, {m->POS, 0}, kv, m->SCORE, m->P16F, m->ESUM, m->PVPART, m->pv_splits, nullptr, m->GOUT);
+        bnk::attn_decode(st, ad, m->Q16F, m->GATEB, {m->POS, 0}, kv, m->SCORE, m->P16F, m->ESUM, m->PVPART, m->pv_splits, nullptr, m->GOUT, m->ctx->err_dev);
     }
     project_add(m, L.q2_out, QD, m->GOUT, q2_next(L.q2_ffn, 2 * h.ffn, h.hidden, L.post_norm));
 }
@@ -567,7 +567,7 @@ void enqueue_batch(bn_model *m, int ncol, bool one_sequence = false) {
             prep(bnk::PREP_NORM, m->RES, L.attn_norm, m->signs, h.hidden, m->IMG_H, nullptr);
             gemm(L.q2_in, 2 * QD + 2 * KD, h.hidden, m->IMG_H, m->QKV, nullptr, q2_next(L.q2_out, h.hidden, QD, nullptr));
             bnk::attn_prep(st, ad, m->QKV, m->KBUF, m->VBUF, L.q_norm, L.k_norm, {m->POS, 0}, kv, m->Q16F, m->GATEB, m->ESUM, cols);
-            bnk::attn_decode(st, ad, m->Q16F, m->GATEB, {m->POS, 0}, kv, m->SCORE, m->P16F, m->ESUM, m->PVPART, m->pv_splits, nullptr, m->GOUT, cols);
+            bnk::attn_decode(st, ad, m->Q16F, m->GATEB, {m->POS, 0}, kv, m->SCORE, m->P16F, m->ESUM, m->PVPART, m->pv_splits, nullptr, m->GOUT, m->ctx->err_dev, cols);
             prep(bnk::PREP_PLAIN, m->GOUT, nullptr, m->signs, QD, m->IMG_H, nullptr);
             gemm(L.q2_out, h.hidden, QD, m->IMG_H, m->RES, m->RES, q2_next(L.q2_ffn, 2 * h.ffn, h.hidden, L.post_norm));
         } else {

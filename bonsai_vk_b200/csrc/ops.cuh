@@ -162,10 +162,11 @@ void attn_prep(cudaStream_t st, AttnDims a, const float *qg, const float *kin, c
 void attn_decode(cudaStream_t st, AttnDims a, const float *q16f, const float *gate, AttnPos where, KvLayer kv,
                  float *score /*[nh][cap]*/, float *p16f /*[nh][cap]*/, float *esum /*[nh][128] partial softmax sums + [nh] row maxima*/,
                  float *pv_part /*[splits][nh][hd]*/, int splits,
-                 float *pregate /*[nh][hd] or null*/, float *gated, Cols cols = {});
+                 float *pregate /*[nh][hd] or null*/, float *gated, int *err, Cols cols = {});
 // the same in one launch (attn_cluster.cu), without scratch; false: this capacity, or this device, is not for it
 bool attn_cluster(cudaStream_t st, AttnDims a, const float *q16f, const float *gate, AttnPos where, KvLayer kv, int splits, float *pregate,
-                  float *gated, Cols cols);
+                  float *gated, Cols cols, int *err);
+cudaError_t launch_wait_selftest_exchange(cudaStream_t st, int *err);
 // cand (optional): per column (value, row0 + index) of the maximum, for an output head whose rows are sharded
 void argmax_first(cudaStream_t st, const float *x, int n, int *out_idx, float *scratch_val, int *scratch_idx, Cols cols = {},
                   float *cand = nullptr, int row0 = 0);
