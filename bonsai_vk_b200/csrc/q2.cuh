@@ -68,6 +68,7 @@ struct Q2Args {
     int log_hat;                 // log2(hat_block);
     Q2Share share;               // the CTAs' shares of the row tiles;
     int slots, fin;              // ring slots; bytes of group sums from a cluster's CTAs
+    int run, gstep;              // row tiles per run of group sums; warps modulo groups (divisions that would sit in front of the first piece)
     float *inv_out;              // Q2_NORM, optional: 1/sqrt(mean(x0^2) + eps)
     int late;                    // release the dependent launch behind this kernel's own dependency wait (see GdnStep)
     int lean;                    // leave room for the next kernel's CTA on the SM (a mixer follows)

@@ -280,8 +280,9 @@ __global__ void __launch_bounds__(LEAN ? 768 : NT + 32, 1) k_q2_gemv(const Q2Arg
     };
     const f32pair magic2 = pair_of(__int_as_float(Q2_MAGIC), __int_as_float(Q2_MAGIC));
     // tiles per run of group sums: what the transform's buffer holds
-    const int run = max(1, PBUF / (16 * ng)), gstep = NW % ng;
-    int u = warp, gr = warp % ng, slot = 0;
+    const int run = a.run, gstep = a.gstep;
+    int u = warp, gr = warp, slot = 0;
+    while (gr >= ng) gr -= ng;                     // (eight groups at K = 4096: one step at most)
     uint32_t phase = 0;
     bool alive = true;
     // one piece: its group sums p_g of 16 rows go to `dst` (SPLIT: to the CTA that adds them)
@@ -462,6 +463,7 @@ cudaError_t launch_spans(cudaStream_t st, int sm_count, Q2Args a, bool pdl, int 
     if (limits != cudaSuccess) return limits;
     a.inv_k = (a.K & (a.K - 1)) == 0 ? 1.0f / float(a.K) : 0.0f;
     a.log_hat = 31 - __builtin_clz(unsigned(a.hat_block));
+    a.run = std::max(1, PBUF / (16 * ng)); a.gstep = NW % ng;
     if (a.next.W) a.next.share = {a.next.units / grid, a.next.units % grid};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
