@@ -7,8 +7,10 @@
 //     before the wait  state rows into registers, conv taps, the norm of the residual, the two small projections (alpha, beta)
 //                      and their gate functions
 //     after it         conv + silu, L2 norms, delta rule, head norm over the cluster, ssm_norm, swiglu(z, .), permutation
-// From the end of the projection in front to the end of the one behind (9B shape): 12.7 us before, 8.7 us now, of which 0.9 us
-// go back in the first projection, which now shares its SMs. Arithmetic and its order are those of k_gdn_core (ops.cu).
+// From the end of the projection in front to the end of the one behind (9B shape): 12.7 us before, 8.7 us then, of which 0.9 us
+// go back in the first projection, which shares its SMs; another 0.7 us went with the cluster barrier behind the outputs (counted
+// stores now: a barrier waits for the stores' acknowledgement, then makes a round trip), the divisions of the head's place and two
+// divisions by square roots: 48 greedy tokens 51.0 -> 50.2 ms. Arithmetic and its order are those of k_gdn_core (ops.cu).
 #include "ops.cuh"
 #include "rotate_quant.cuh"
 
@@ -27,11 +29,25 @@ __device__ __forceinline__ void push(float *p, int cta, float v) {
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(v) : "memory");
 }
 
+// the same, counted by a barrier there
+__device__ __forceinline__ void push_counted(float *p, int cta, float v, const uint64_t *bar) {
+    uint32_t dst, b;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(uint32_t(__cvta_generic_to_shared(p))), "r"(cta));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(uint32_t(__cvta_generic_to_shared(bar))), "r"(cta));
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst), "r"(__float_as_uint(v)), "r"(b) : "memory");
+}
+
 __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(T, 5) k_gdn_step(const GdnStep a) {
     extern __shared__ float4 dyn[];                // [2][hidden / 4]: normed residual, row h of alpha or beta
     __shared__ float red[256], sq[128], sk[128], sv[32], so[128], sgb[2];     // so: the head's 128 outputs, every quarter pushed here by its CTA
     const int h = blockIdx.x >> 2, q4 = blockIdx.x & 3, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int hq = h % a.qk_heads, n4 = a.hidden >> 2;
+    __shared__ uint64_t outs;                      // counts the bytes of so[]
+    if (tid == 0) {
+        const uint32_t b = uint32_t(__cvta_generic_to_shared(&outs));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\nfence.mbarrier_init.release.cluster;" ::"r"(b) : "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], 512;" ::"r"(b) : "memory");
+    }
     // "I am running": the matching wait sits in front of the first store into a neighbour's shared memory
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -136,8 +152,8 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(T, 5) k_gdn_step(con
     {
 #pragma unroll
         for (int e = 0; e < 4; ++e) { qq[e] = sq[lane + 32 * e]; kk[e] = sk[lane + 32 * e]; }
-        const float iq = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(warp_tree128(__fmul_rn(qq[0], qq[0]), __fmul_rn(qq[1], qq[1]), __fmul_rn(qq[2], qq[2]), __fmul_rn(qq[3], qq[3])), 1e-12f)));
-        const float ik = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(warp_tree128(__fmul_rn(kk[0], kk[0]), __fmul_rn(kk[1], kk[1]), __fmul_rn(kk[2], kk[2]), __fmul_rn(kk[3], kk[3])), 1e-12f)));
+        const float iq = __frcp_rn(__fsqrt_rn(__fadd_rn(warp_tree128(__fmul_rn(qq[0], qq[0]), __fmul_rn(qq[1], qq[1]), __fmul_rn(qq[2], qq[2]), __fmul_rn(qq[3], qq[3])), 1e-12f)));
+        const float ik = __frcp_rn(__fsqrt_rn(__fadd_rn(warp_tree128(__fmul_rn(kk[0], kk[0]), __fmul_rn(kk[1], kk[1]), __fmul_rn(kk[2], kk[2]), __fmul_rn(kk[3], kk[3])), 1e-12f)));
 #pragma unroll
         for (int e = 0; e < 4; ++e) { qq[e] = __fmul_rn(qq[e], iq); kk[e] = __fmul_rn(kk[e], ik); }
     }
@@ -168,23 +184,34 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(T, 5) k_gdn_step(con
     if (lane < 16) {                               // lane = (CTA, row): push this warp's four outputs into all four so[]
         const int row = lane & 3;
         const float o = __fmul_rn(row == 0 ? pr[0] : (row == 1 ? pr[1] : (row == 2 ? pr[2] : pr[3])), a.scale);
-        push(so + q4 * 32 + warp * 4 + row, lane >> 2, o);
+        push_counted(so + q4 * 32 + warp * 4 + row, lane >> 2, o, &outs);
     }
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
         for (int e = 0; e < 4; ++e) Sr[r * 128 + 32 * e] = S[r][e];
-    float gz = 0.0f, nw = 0.0f;                    // this CTA's share of the gate, off the tail (a double-precision exp)
-    if (warp == 1) { gz = silu_f(zz); nw = a.ssm_norm[q4 * 32 + lane]; }
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");      // the head's 128 outputs are in every CTA's so[]
+    float gz = 0.0f, nw = 0.0f;                    // this CTA's share of the gate, and its place, off the tail (a double-precision exp; divisions)
+    int hd = 0;
+    if (warp == 1) { gz = silu_f(zz); nw = a.ssm_norm[q4 * 32 + lane]; hd = a.heads / a.qk_heads * hq + h / a.qk_heads; }
+    // the head's 128 outputs are in every CTA's so[] (counted stores: a cluster barrier waits for their acknowledgement first)
+    bool alive = false;
+    for (int it = 0; it < (1 << 22) && !alive; ++it) {
+        uint32_t ok;
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(ok) : "r"(uint32_t(__cvta_generic_to_shared(&outs))) : "memory");
+        alive = ok != 0u;
+    }
+    if (!alive) {                                  // given up: the others end first
+        atomicExch(a.err, 1);
+        asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+    }
     if (warp == 1) {
         float e[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) e[i] = so[i * 32 + lane];
         const float ss = warp_tree128(__fmul_rn(e[0], e[0]), __fmul_rn(e[1], e[1]), __fmul_rn(e[2], e[2]), __fmul_rn(e[3], e[3]));
-        const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, 128.0f), a.eps)));
-        const int sub = a.heads / a.qk_heads, hd = sub * (h % a.qk_heads) + h / a.qk_heads, d = q4 * 32 + lane;
+        const float inv = __frcp_rn(__fsqrt_rn(__fadd_rn(__fmul_rn(ss, 1.0f / 128.0f), a.eps)));
+        const int d = q4 * 32 + lane;
         a.y[hd * 128 + d] = __fmul_rn(gz, __fmul_rn(__fmul_rn(so[d], inv), nw));
     }
 }

@@ -287,7 +287,7 @@ void gdn_fused(bn_model *m, const bn_model::Layer &L) {
             bnk::GdnStep s = {};
             s.heads = NH; s.qk_heads = NQ; s.hidden = h.hidden; s.qkv = m->QKV; s.z = m->Z; s.conv_w = L.conv_w; s.hist0 = h0; s.hist1 = h1; s.pos = m->POS;
             s.x = m->RES; s.norm_w = L.attn_norm; s.alpha_w = L.alpha_w; s.beta_w = L.beta_w; s.dt_bias = L.dt_bias; s.ssm_a = L.ssm_a;
-            s.state = gdn_state_of(m, L.idx); s.ssm_norm = L.ssm_norm; s.eps = h.rms_eps; s.scale = 1.0f / sqrtf(float(D)); s.y = m->X1;
+            s.state = gdn_state_of(m, L.idx); s.ssm_norm = L.ssm_norm; s.eps = h.rms_eps; s.scale = 1.0f / sqrtf(float(D)); s.y = m->X1; s.err = m->ctx->err_dev;
             bnk::gdn_step(m->ctx->stream, s, m->mixers_only);
         }
         else

@@ -126,6 +126,7 @@ struct GdnStep {
     const float *ssm_norm;
     float eps, scale;
     float *y;
+    int *err;                              // device error word (a bounded wait)
 };
 void gdn_step(cudaStream_t st, const GdnStep &a, bool alone = false);
 // the mixer for n <= 32 consecutive positions of one sequence (gdn_seq.cu): column c's activations at + c * stride bytes
