@@ -43,6 +43,11 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm(const Q2GemmArgs a) {
     constexpr int NW = NT / 32;
     constexpr bool LATE = NATIVE || MT == 1 || (NT == 384 && MT == 2);
     constexpr int NG = NCP / 8, NGW = NG >= 2 ? 2 : 1, H = NG / NGW;      // column groups: all, per unit; units across the columns
+    // A unit's group by a division, or by a multiplier that waits in shared memory (in a register it spills 16 columns' units). The
+    // division is up to a tenth of a unit: 12 288 x 4096 x 8 8.84 -> 8.67 us, native 3000 x 5120 x 4 8.76 -> 8.35, 16 columns native
+    // 4096 x 12 288 20.8 -> 20.4. Two builds are faster with it: three tiles (20 000 x 12 288 x 8 26.6 us, 28.6 without) and 16 columns
+    // on 12 warps (9000 x 2048 7.01, 7.18).
+    constexpr bool DIVIDE = MT == 3 || (NCP == 16 && MT == 2 && NT == 384);
     constexpr int ITEMS = (MAX_TILES * 16 * NCP + NT - 1) / NT;
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tig = lane & 3, cta = blockIdx.x;
@@ -55,8 +60,8 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm(const Q2GemmArgs a) {
     float *sums = reinterpret_cast<float *>(img + (nchunks > 1 ? 2 : 1) * kc * gbytes);
     unsigned char *stage = reinterpret_cast<unsigned char *>(sums + size_t(kc) * a.tiles * 16 * NCP) + warp * Q2_PIECE;       // NATIVE only
     const size_t rowbytes = size_t(a.K >> 7) * 28;
-    auto request = [&](int q) {                                            // image piece of chunk q (wave q % nw) into buffer q & 1
-        const int g0 = (q % nw) * kc, n = min(kc, ng - g0);
+    auto request = [&](int q, int w) {                                     // image piece of chunk q (its wave w) into buffer q & 1
+        const int g0 = w * kc, n = min(kc, ng - g0);
         const uint32_t bytes = uint32_t(n) * gbytes, bar = bars + (q & 1) * 8;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -65,6 +70,9 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm(const Q2GemmArgs a) {
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars));
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8));
+        // i / nur = i * per >> 16 for the few hundred units of a wave (nur <= 12); the last pass may have fewer tiles
+        auto per = [&](int n) { return 65536 / ((n + MT - 1) / MT) + 1; };
+        asm volatile("st.shared.v2.s32 [%0], {%1, %2};" ::"r"(bars + 16), "r"(per(min(a.tiles, nt))), "r"(per(nt - (npass - 1) * a.tiles)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (lane == 0) {
@@ -77,7 +85,7 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm(const Q2GemmArgs a) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __syncthreads();
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (tid == 0) for (int q = 0; q < min(2, nchunks); ++q) request(q);
+    if (tid == 0) for (int q = 0; q < min(2, nchunks); ++q) request(q, q < nw ? q : 0);
 
     const f32pair magic2 = pair_of(__int_as_float(Q2_MAGIC), __int_as_float(Q2_MAGIC));
     bool alive = true;
@@ -85,6 +93,7 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm(const Q2GemmArgs a) {
     for (int pass = 0; pass < npass; ++pass) {
         const int tb = pass * a.tiles, n = min(a.tiles, nt - tb), nur = (n + MT - 1) / MT;      // this pass's tiles, units of rows
         const uint8_t *W = a.W + size_t(t0 + tb) * ng * Q2_PIECE;
+        const uint32_t per_at = bars + (pass + 1 == npass ? 20 : 16);
         float acc[ITEMS];
         for (int w = 0; w < nw; ++w) {
             const int g0 = w * kc, gn = min(kc, ng - g0);
@@ -95,7 +104,13 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm(const Q2GemmArgs a) {
             if (!LATE) await_image();
             const unsigned char *chunk = img + buf * kc * gbytes;
             for (int u = warp; u < gn * nur * H; u += NW) {
-                const int h = u % H, ur = (u / H) % nur, gl = u / (H * nur);
+                int gl;
+                if (DIVIDE) gl = u / H / nur;
+                else {
+                    asm volatile("ld.shared.s32 %0, [%1];" : "=r"(gl) : "r"(per_at));
+                    gl = u / H * gl >> 16;
+                }
+                const int h = u % H, ur = u / H - gl * nur;
                 const uint8_t *src = W + (size_t(ur * MT) * ng + g0 + gl) * Q2_PIECE;
                 uint4 c[MT][4], dw[MT];
 #pragma unroll
@@ -183,7 +198,7 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm(const Q2GemmArgs a) {
             }
             __syncthreads();                       // the wave's group sums are there, its image piece is no longer read
             if (nchunks > 1) {
-                if (tid == 0 && q + 2 < nchunks) request(q + 2);
+                if (tid == 0 && q + 2 < nchunks) request(q + 2, (q + 2) % nw);
                 ++q;
             }
             const int items = n * NG * 128;
