@@ -240,7 +240,11 @@ __global__ void __launch_bounds__(256) k_gdn_delta(int heads, int qk_heads, cons
 // Arithmetic and its order are those of the stand-alone kernels above.
 // MINB = CTAs per SM the register budget is set for: 1 for a single sequence (32 CTAs in all; the loads hoisted above
 // the dependency wait keep ~90 registers live, measured 4 % of a token faster than the 64-register build), 2 when many
-// sequences fill the GPU with CTAs (measured 3 % of a 32-sequence pass faster than one CTA per SM).
+// sequences fill the GPU with CTAs (measured 3 % of a 32-sequence pass faster than one CTA per SM). With several sequences the
+// projection in front is the several-column one, which releases its dependents behind its own dependency wait, so the residual and its norm
+// factor, which the kernel in front of that one wrote, may be read before the wait here: the two dot products, their gate functions and
+// the row's loads pass while the projection's last CTAs run. With the outputs' gate off the tail (it was one warp's, behind everything)
+// a step of 8 sequences takes 1.995 instead of 2.012 ms, a recurrent block of 2 / 8 / 32 sequences 65.3 / 67.9 / 161.5 -> 63.6 / 65.8 / 158.2 us.
 template <int MINB>
 __global__ void __launch_bounds__(512, MINB) k_gdn_core(int heads, int qk_heads, int hidden, const float *__restrict__ qkv,
                                                   const float *__restrict__ conv_w, float *__restrict__ hist0,
@@ -252,7 +256,9 @@ __global__ void __launch_bounds__(512, MINB) k_gdn_core(int heads, int qk_heads,
                                                   const float *__restrict__ z, const float *__restrict__ ssm_norm, float eps,
                                                   float *__restrict__ y, float scale, bnk::Cols cols) {
     { const size_t col = blockIdx.z; qkv = bnk::colp(qkv, col * cols.arena); hist0 = bnk::colp(hist0, col * cols.conv); hist1 = bnk::colp(hist1, col * cols.conv); pos_ptr = bnk::colp(pos_ptr, col * cols.arena); x = bnk::colp(x, col * cols.arena); inv_ptr = bnk::colp(inv_ptr, col * cols.arena); state = bnk::colp(state, col * cols.gdn); z = bnk::colp(z, col * cols.arena); y = bnk::colp(y, col * cols.arena); }
-    __shared__ float sq[128], sk[128], sv[128], so[128], sgb[2];
+    constexpr bool PRE = MINB == 2;
+    __shared__ float sq[128], sk[128], sv[128], so[128], sz[128], sgb[2];
+    __shared__ int place;
     extern __shared__ float4 dyn[];                // [3][hidden/4]: normed residual, row h of ssm_alpha, row h of ssm_beta
     const int h = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int hq = h % qk_heads, n4 = hidden / 4;
@@ -282,33 +288,24 @@ __global__ void __launch_bounds__(512, MINB) k_gdn_core(int heads, int qk_heads,
         const float4 *ra = reinterpret_cast<const float4 *>(alpha_w + size_t(h) * hidden), *rb = reinterpret_cast<const float4 *>(beta_w + size_t(h) * hidden);
         for (int i = tid; i < n4; i += 512) { dyn[n4 + i] = ra[i]; dyn[2 * n4 + i] = rb[i]; }
     }
-    bnk::pdl_sync();
-    {   // the normed residual goes to shared memory for the two dependent dot-product chains
-        const float inv = inv_ptr[0];
+    if (tid == 0) place = heads / qk_heads * hq + h / qk_heads;              // the head's place in the v-grouped permutation
+    const float nwz = tid >= 384 ? ssm_norm[tid - 384] : 0.0f;
+    auto residual = [&] {   // the normed residual goes to shared memory for the two dependent dot-product chains
+        const float inv = __ldcg(inv_ptr);
         const float4 *xv = reinterpret_cast<const float4 *>(x), *nw = reinterpret_cast<const float4 *>(norm_w);
         for (int i = tid; i < n4; i += 512) {
-            const float4 a4 = xv[i], w4 = nw[i];
+            const float4 a4 = __ldcg(xv + i), w4 = nw[i];
             dyn[i] = make_float4(__fmul_rn(__fmul_rn(a4.x, inv), w4.x), __fmul_rn(__fmul_rn(a4.y, inv), w4.y),
                                  __fmul_rn(__fmul_rn(a4.z, inv), w4.z), __fmul_rn(__fmul_rn(a4.w, inv), w4.w));
         }
-    }
-    const bool own_qk = h < qk_heads;              // the first of the v-heads sharing q/k head hq writes its taps
-    if (tid < 384) {
-        const float xn = qkv[cch];
-        float acc = __fmul_rn(cw0, tap0);
-        acc = __fadd_rn(acc, __fmul_rn(cw1, tap1));
-        acc = __fadd_rn(acc, __fmul_rn(cw2, tap2));
-        acc = __fadd_rn(acc, __fmul_rn(cw3, xn));
-        if (tid >= 256 || own_qk) { float *sw = hist_wr + 3 * size_t(cch); sw[0] = tap1; sw[1] = tap2; sw[2] = xn; }
-        const float cv = silu_f(acc);
-        if (tid < 128) sq[tid] = cv; else if (tid < 256) sk[tid - 128] = cv; else sv[tid - 256] = cv;
-    }
-    __syncthreads();
-    if (warp >= 14) {
+    };
+    auto gates = [&] {
+        if (warp < 14) return;
         // row h of ssm_alpha (warp 14) or ssm_beta (warp 15) times the normed residual: lane l takes float4 groups
         // l, l+32, ... with one fmaf per element, then a 32-lane xor tree (k_gemv_f32_small)
         const float4 *wr = dyn + (warp == 14 ? n4 : 2 * n4);
         float acc = 0.0f;
+#pragma unroll 4
         for (int i = lane; i < n4; i += 32) {
             const float4 w4 = wr[i], a4 = dyn[i];
             acc = fmaf(w4.x, a4.x, acc); acc = fmaf(w4.y, a4.y, acc); acc = fmaf(w4.z, a4.z, acc); acc = fmaf(w4.w, a4.w, acc);
@@ -319,21 +316,41 @@ __global__ void __launch_bounds__(512, MINB) k_gdn_core(int heads, int qk_heads,
             if (warp == 14) {
                 const float al = __fadd_rn(acc, dt_bias[h]);
                 const float sp = al > 20.0f ? al : log_f(__fadd_rn(1.0f, exp_f(al)));
-                sgb[0] = __fmul_rn(sp, ssm_a[h]);
+                sgb[0] = exp_f(__fmul_rn(sp, ssm_a[h]));
             } else sgb[1] = sigmoid_f(acc);
         }
+    };
+    if (PRE) {
+        residual();
+        __syncthreads();
+        gates();
     }
+    bnk::pdl_sync();
+    if (!PRE) residual();
+    const bool own_qk = h < qk_heads;              // the first of the v-heads sharing q/k head hq writes its taps
+    if (tid < 384) {
+        const float xn = qkv[cch];
+        float acc = __fmul_rn(cw0, tap0);
+        acc = __fadd_rn(acc, __fmul_rn(cw1, tap1));
+        acc = __fadd_rn(acc, __fmul_rn(cw2, tap2));
+        acc = __fadd_rn(acc, __fmul_rn(cw3, xn));
+        if (tid >= 256 || own_qk) { float *sw = hist_wr + 3 * size_t(cch); sw[0] = tap1; sw[1] = tap2; sw[2] = xn; }
+        const float cv = silu_f(acc);
+        if (tid < 128) sq[tid] = cv; else if (tid < 256) sk[tid - 128] = cv; else sv[tid - 256] = cv;
+    } else sz[tid - 384] = silu_f(z[h * 128 + tid - 384]);                   // (the gate of the outputs, off the tail)
+    __syncthreads();
+    if (!PRE) gates();
     float qq[4], kk[4];
     {
         const float a0 = sq[lane], a1 = sq[lane + 32], a2 = sq[lane + 64], a3 = sq[lane + 96];
-        const float iq = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(bnk::warp_tree128(__fmul_rn(a0, a0), __fmul_rn(a1, a1), __fmul_rn(a2, a2), __fmul_rn(a3, a3)), 1e-12f)));
+        const float iq = __frcp_rn(__fsqrt_rn(__fadd_rn(bnk::warp_tree128(__fmul_rn(a0, a0), __fmul_rn(a1, a1), __fmul_rn(a2, a2), __fmul_rn(a3, a3)), 1e-12f)));
         qq[0] = __fmul_rn(a0, iq); qq[1] = __fmul_rn(a1, iq); qq[2] = __fmul_rn(a2, iq); qq[3] = __fmul_rn(a3, iq);
         const float b0 = sk[lane], b1 = sk[lane + 32], b2 = sk[lane + 64], b3 = sk[lane + 96];
-        const float ik = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(bnk::warp_tree128(__fmul_rn(b0, b0), __fmul_rn(b1, b1), __fmul_rn(b2, b2), __fmul_rn(b3, b3)), 1e-12f)));
+        const float ik = __frcp_rn(__fsqrt_rn(__fadd_rn(bnk::warp_tree128(__fmul_rn(b0, b0), __fmul_rn(b1, b1), __fmul_rn(b2, b2), __fmul_rn(b3, b3)), 1e-12f)));
         kk[0] = __fmul_rn(b0, ik); kk[1] = __fmul_rn(b1, ik); kk[2] = __fmul_rn(b2, ik); kk[3] = __fmul_rn(b3, ik);
     }
     __syncthreads();
-    const float eg = exp_f(sgb[0]), bt = sgb[1];
+    const float eg = sgb[0], bt = sgb[1];
     // four rows at a time; their trees share six shuffles (a level's two values change hands between the lanes that go on with
     // one and those that go on with the other), as the shuffles' throughput bounds this part
     const bool b4 = lane & 16, b3 = lane & 8;
@@ -370,20 +387,15 @@ __global__ void __launch_bounds__(512, MINB) k_gdn_core(int heads, int qk_heads,
         if (!(lane & 7)) so[warp * 8 + r0 + (lane >> 4) + ((lane >> 3) & 1) * 2] = __fmul_rn(ov, scale);
     }
     __syncthreads();
-    if (warp == 0) {
+    if (tid >= 384) {
         // per-head RMS (no weight), * ssm_norm, swiglu(z, .), destination head of the v-grouped permutation
         float e[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) e[i] = so[lane + 32 * i];
         const float ss = bnk::warp_tree128(__fmul_rn(e[0], e[0]), __fmul_rn(e[1], e[1]), __fmul_rn(e[2], e[2]), __fmul_rn(e[3], e[3]));
-        const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, 128.0f), eps)));
-        const int sub = heads / qk_heads, hd = sub * (h % qk_heads) + h / qk_heads;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int d = lane + 32 * i;
-            const float nrm = __fmul_rn(__fmul_rn(e[i], inv), ssm_norm[d]);
-            y[hd * 128 + d] = __fmul_rn(silu_f(z[h * 128 + d]), nrm);
-        }
+        const float inv = __frcp_rn(__fsqrt_rn(__fadd_rn(__fmul_rn(ss, 1.0f / 128.0f), eps)));
+        const int d = tid - 384;
+        y[place * 128 + d] = __fmul_rn(sz[d], __fmul_rn(__fmul_rn(so[d], inv), nwz));
     }
 }
 

@@ -18,7 +18,9 @@ namespace bnk {
 //     token and position (k_set_cols, k_set_tok_pos), and every pass begins behind a plain launch, a copy or a graph launch,
 //     which waits for all that was enqueued before it. Those must stay plain: with this attribute they would be part of the chain.
 //     (In a pass whose first launch follows k_set_cols directly that launch is embed_rotate, which waits before it releases.)
-//   * the residual, in gdn_step alone: the projection in front of it releases it late (Q2Args::late).
+//   * the residual, in gdn_step alone: the projection in front of it releases it late (Q2Args::late);
+//   * the residual and its norm factor, in k_gdn_core of several sequences: the projections of several columns release their dependents
+//     behind their own wait, and the kernel that wrote the factor stands in front of them.
 extern bool g_pdl;
 template <class... KArgs, class... Args>
 inline void launch_as(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {

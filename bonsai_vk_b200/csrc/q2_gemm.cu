@@ -82,9 +82,11 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm(const Q2GemmArgs a) {
         for (int o = warp * 16384; o < bytes; o += NW * 16384) q2_prefetch(own + o, min(16384, bytes - o));
         q2_prefetch_next(a.next, cta, warp, NW);
     }
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __syncthreads();
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    // Released here, the kernel behind this one may read ahead of its own wait what was complete before this one's (k_gdn_core does);
+    // it has no room on an SM before this CTA ends anyway.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (tid == 0) for (int q = 0; q < min(2, nchunks); ++q) request(q, q < nw ? q : 0);
 
     const f32pair magic2 = pair_of(__int_as_float(Q2_MAGIC), __int_as_float(Q2_MAGIC));

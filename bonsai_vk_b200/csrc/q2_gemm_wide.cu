@@ -69,7 +69,6 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm_wide(const Q2GemmArgs a, cons
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     bool alive = true;
 
     if (warp >= NW) {
@@ -121,6 +120,7 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm_wide(const Q2GemmArgs a, cons
     // ---- sums ----------------------------------------------------------------------------------------------------------------------
     asm volatile("setmaxnreg.inc.sync.aligned.u32 160;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");        // (behind the wait: see k_q2_gemm; the copies' warps end without it)
     f32pair acc[MT][CG][2];
     int slot = 0, phase = 0, wslot = 0, wphase = 0;                      // slots of the step and the group, and the parity of their use
     for (int pass = 0; pass < npass; ++pass) {
