@@ -280,8 +280,8 @@ __global__ void __launch_bounds__(1024) k_attn_expsum(AttnDims a, AttnPos where,
 // ring of two 32-key tiles in shared memory (cp.async; small enough that the 1024 CTAs of a long context are all resident),
 // probabilities are staged as one [key][head] row, so a key costs a thread three shared-memory loads whatever the number of
 // dims. The rounded products of two dims are one fma.f32x2 with -0 (x * y - 0 is the rounded product; the -0 is an
-// argument `nz`, because the assembler contracts a packed multiply, or one with a constant -0, with the packed add behind it). DPT = 4 where splits and columns fill the GPU with 64-thread CTAs,
-// else 1 (short caches: the keys' serial chain is what takes the time).
+// argument `nz`, because the assembler contracts a packed multiply, or one with a constant -0, with the packed add behind it). DPT: two or four
+// where splits and columns fill the GPU (pv_any), else 1 (short caches: the keys' serial chain is what takes the time).
 constexpr int PV_TILE = 32;
 template <int GQA, int DPT, int VMODE>
 __global__ void __launch_bounds__(256 / DPT) k_attn_pv(AttnDims a, AttnPos where, const float *__restrict__ pe, const float *__restrict__ partial,
@@ -369,6 +369,18 @@ __global__ void __launch_bounds__(256 / DPT) k_attn_pv(AttnDims a, AttnPos where
                     acc2[g][0] = pair_add(acc2[g][0], pair_fma(pp, v01, nzero));
                     acc2[g][1] = pair_add(acc2[g][1], pair_fma(pp, v23, nzero));
                 }
+            } else if (DPT == 2) {
+                f32pair v;
+                if (VMODE == 0) {
+                    const float s = half_bits_to_float(*reinterpret_cast<const uint16_t *>(tile + VB + k * 16 + (tid >> 4) * 2));
+                    const uint32_t c = uint32_t(*reinterpret_cast<const uint16_t *>(tile + k * 256 + tid * 2)) ^ 0x8080u;
+                    v = pair_mul(pair_of(s, s), pair_sub(pair_of(code_f<0>(c), code_f<1>(c)), magic2));
+                } else {
+                    const uint32_t c = *reinterpret_cast<const uint32_t *>(tile + k * 512 + tid * 4);
+                    v = pair_of(half_bits_to_float(c), half_bits_to_float(c >> 16));
+                }
+#pragma unroll
+                for (int g = 0; g < GQA; ++g) acc2[g][0] = pair_add(acc2[g][0], pair_fma(pair_of(p[g], p[g]), v, nzero));
             } else {
                 float v;
                 if (VMODE == 0) {
@@ -385,6 +397,7 @@ __global__ void __launch_bounds__(256 / DPT) k_attn_pv(AttnDims a, AttnPos where
     for (int g = 0; g < GQA; ++g) {
         float *o = part + (size_t(sp) * a.n_head + kvh * GQA + g) * hd + tid * DPT;
         if (DPT == 4) *reinterpret_cast<ulonglong2 *>(o) = make_ulonglong2(acc2[g][0], acc2[g][1]);
+        else if (DPT == 2) *reinterpret_cast<f32pair *>(o) = acc2[g][0];
         else o[0] = acc[g];
     }
 }
@@ -451,10 +464,20 @@ void pv(cudaStream_t st, AttnDims a, AttnPos where, const float *pe, const float
 }
 template <int GQA>
 void pv_any(cudaStream_t st, AttnDims a, AttnPos where, const float *pe, const float *partial, KvLayer kv, int splits, float *part, Cols cols) {
-    // four dims per thread from three 64-thread CTAs per two SMs on (8 columns x 8 splits x 4 heads: 28 -> 22 us)
-    const bool wide = size_t(a.n_kv) * splits * cols.z() >= 200;
-    if (a.v_mode == 0) { if (wide) pv<GQA, 4, 0>(st, a, where, pe, partial, kv, splits, part, cols); else pv<GQA, 1, 0>(st, a, where, pe, partial, kv, splits, part, cols); }
-    else { if (wide) pv<GQA, 4, 1>(st, a, where, pe, partial, kv, splits, part, cols); else pv<GQA, 1, 1>(st, a, where, pe, partial, kv, splits, part, cols); }
+    // Several dims per thread from three CTAs per two SMs on (8 columns x 8 splits x 4 heads: 28 -> 22 us). Two dims where four or eight
+    // heads share a value, up to 4096 CTAs: twice the warps for an eighth more instructions (30 000 keys 45.1 us with four dims, 43.4 with
+    // two, eight heads 47.0 and 46.0; 8 columns at 2048 positions 85.6 and 83.1 us a block; 16 columns at 8192, 4096 CTAs, the same, 32
+    // columns 356 and 362). Fewer heads have too little work per value for that (two heads: 50.6 and 51.4).
+    const size_t ctas = size_t(a.n_kv) * splits * cols.z();
+    const int dims = ctas < 200 ? 1 : (GQA >= 4 && ctas <= 4096 ? 2 : 4);
+    constexpr int TWO = GQA >= 4 ? 2 : 4;
+    if (a.v_mode == 0) {
+        if (dims == 1) pv<GQA, 1, 0>(st, a, where, pe, partial, kv, splits, part, cols);
+        else if (dims == 2) pv<GQA, TWO, 0>(st, a, where, pe, partial, kv, splits, part, cols);
+        else pv<GQA, 4, 0>(st, a, where, pe, partial, kv, splits, part, cols);
+    } else if (dims == 1) pv<GQA, 1, 1>(st, a, where, pe, partial, kv, splits, part, cols);
+    else if (dims == 2) pv<GQA, TWO, 1>(st, a, where, pe, partial, kv, splits, part, cols);
+    else pv<GQA, 4, 1>(st, a, where, pe, partial, kv, splits, part, cols);
 }
 
 }  // namespace
