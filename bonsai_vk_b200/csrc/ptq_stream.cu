@@ -15,9 +15,13 @@
 // over all of K. The pieces (16 rows x 4 blocks, the unit p_g of the summation order) of a run are dealt to the warps group-major, so a
 // warp stays with one group's operand table - 64 registers - for most of its pieces; group sums meet in shared memory, where one thread
 // per row adds them in ascending order.
-// Data movement. A piece is 16 rows of 112 bytes, brought by cp.async (16, 8 or 4 bytes at a time, whichever the rows' alignment
-// allows) into a ring of its warp's own. The pitch of 112 bytes is free of bank conflicts for every load of the loop: eight rows
-// start four banks apart and the four lanes of a row read words 0, 2, 3, 5 (one in each residue modulo 4).
+// Data movement. A piece is 16 rows of 112 bytes, brought by cp.async into a ring of its warp's own: 16 or 8 bytes at a time where the
+// rows' alignment allows, else the eight 16-byte granules that hold a row's 112 bytes (ALIGN 0), from which a lane reads at its row's
+// place. Four bytes at a time, 14 copies a piece instead of four, took the issue slots: 30 000 x 4736 22.6 -> 18.1 us, 50 000 x 6528
+// 43.1 -> 32.0, 100 000 x 2176 34.8 -> 26.7. Rows of more alignment lose by it (1000 x 8192 6.9 against 7.5, 20 000 x 12 288 26.5 against
+// 27.7; 60 000 x 1280 13.8 against 13.5). The pitches of 112
+// and 144 bytes are free of bank conflicts for every load of the loop: eight rows start four banks apart and the four lanes of a row
+// read words 0, 2, 3, 5 (one in each residue modulo 4).
 #include "ops.cuh"
 #include "q2.cuh"
 #include "rotate_quant.cuh"
@@ -27,7 +31,9 @@
 namespace {
 using namespace bnk;
 
-constexpr int NT = 384, NW = NT / 32, ST = 5, PIECE = 16 * 112, MAX_PIECES = 1536, MAGIC = 0x4B400000;   // bits of 12582912.0f
+constexpr int NT = 384, NW = NT / 32, MAX_PIECES = 1536, MAGIC = 0x4B400000;   // bits of 12582912.0f
+
+template <int ALIGN> struct Ring { static constexpr int STAGES = ALIGN ? 5 : 4, PITCH = ALIGN ? 112 : 144, PIECE = 16 * PITCH, BYTES = NW * STAGES * PIECE; };
 
 struct StreamArgs {
     const unsigned char *W;
@@ -112,9 +118,10 @@ __device__ __forceinline__ float quad_transpose_sum(const float (&x)[4], bool od
 
 template <int ALIGN, bool MANY>
 __global__ void __launch_bounds__(NT, 1) k_ptq_stream(const StreamArgs a) {
+    constexpr int ST = Ring<ALIGN>::STAGES, PITCH = Ring<ALIGN>::PITCH, PIECE = Ring<ALIGN>::PIECE;
     extern __shared__ __align__(16) unsigned char smem[];
-    uint4 *offs = reinterpret_cast<uint4 *>(smem + NW * ST * PIECE);       // where a lane's four 16-byte copies of a piece start
-    float *sums = reinterpret_cast<float *>(smem + NW * ST * PIECE + 512); // [group][tile of the run][16]
+    uint4 *offs = reinterpret_cast<uint4 *>(smem + Ring<ALIGN>::BYTES);    // where a lane's four 16-byte copies of a piece start
+    float *sums = reinterpret_cast<float *>(smem + Ring<ALIGN>::BYTES + 512); // [group][tile of the run][16]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tig = lane & 3, cta = blockIdx.x;
     const int nb = a.nb, ng = (nb + 3) >> 2;
     const int t0 = cta * a.q + min(cta, a.r), nt = a.q + (cta < a.r);
@@ -140,6 +147,12 @@ __global__ void __launch_bounds__(NT, 1) k_ptq_stream(const StreamArgs a) {
     const bool odd = tig & 1, hi = tig & 2;
     const unsigned char *ring = smem + warp * ST * PIECE;
     const uint32_t ring_s = uint32_t(__cvta_generic_to_shared(ring));
+    // ALIGN 0: lane (row, granule) of every fourth row; rows four apart (4 x 28 bytes per block) start at the same place in a granule, and
+    // so do a row's pieces. `at`: where this lane finds its words of row g (and, eight pitches on, of row g + 8)
+    const uintptr_t w0 = reinterpret_cast<uintptr_t>(a.W), w1 = w0 + size_t(a.M) * rowbytes;
+    const uintptr_t grow = w0 + size_t(lane >> 3) * rowbytes;
+    const bool needed = (lane & 7) < 7 || (grow & 15);                     // (a row that starts on a granule has seven)
+    const int at = g * PITCH + (ALIGN ? 0 : int((w0 + size_t(g) * rowbytes) & 15));
     uint2 B[4][8];
     float d[4], ns[4];
     int group = -1;
@@ -163,11 +176,25 @@ __global__ void __launch_bounds__(NT, 1) k_ptq_stream(const StreamArgs a) {
         int fg = p0 / n, ft = p0 - fg * n, fs = 0, fp = p0;       // next piece to request: group, tile, slot
         auto request = [&] {
             if (fp < p1) {
-                constexpr int CH = 112 / ALIGN;                   // copies per row
+                constexpr int W = ALIGN ? ALIGN : 4, CH = 112 / W; // copies per row
                 const unsigned char *src = a.W + size_t(t0 + c0 + ft) * 16 * rowbytes + size_t(fg) * 112;
-                const int rmax = a.M - 1 - (t0 + c0 + ft) * 16, have = ALIGN == 16 ? CH : min(4, nb - fg * 4) * 28 / ALIGN;
+                const int rmax = a.M - 1 - (t0 + c0 + ft) * 16, have = ALIGN == 16 ? CH : min(4, nb - fg * 4) * 28 / W;
                 const uint32_t dst = ring_s + fs * PIECE;
-                if (ALIGN == 16 && rmax >= 15) {
+                if (ALIGN == 0) {
+                    const int row0 = (t0 + c0 + ft) * 16;
+                    uintptr_t s = ((grow + size_t(row0) * rowbytes + size_t(fg) * 112) & ~uintptr_t(15)) + (lane & 7) * 16;
+                    const uint32_t to = dst + (lane >> 3) * PITCH + (lane & 7) * 16;
+                    if (row0 > 0 && rmax > 15) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i, s += 4 * rowbytes) if (needed) cp_async<16>(to + i * 4 * PITCH, reinterpret_cast<const void *>(s));
+                    } else                     // the matrix's first and last rows: the words of a granule that reaches out of it one by one
+#pragma unroll 1
+                        for (int i = 0; i < 4; ++i, s += 4 * rowbytes) {
+                            if (!needed || (lane >> 3) + 4 * i > rmax) continue;
+                            if (s >= w0 && s + 16 <= w1) cp_async<16>(to + i * 4 * PITCH, reinterpret_cast<const void *>(s));
+                            else for (int k = 0; k < 16; k += 4) if (s + k >= w0 && s + k < w1) cp_async<4>(to + i * 4 * PITCH + k, reinterpret_cast<const void *>(s + k));
+                        }
+                } else if (ALIGN == 16 && rmax >= 15) {
                     const uint4 o = offs[lane];
                     cp_async<16>(dst + lane * 16, src + o.x); cp_async<16>(dst + lane * 16 + 512, src + o.y); cp_async<16>(dst + lane * 16 + 1024, src + o.z);
                     if (lane < 16) cp_async<16>(dst + lane * 16 + 1536, src + o.w);
@@ -175,7 +202,7 @@ __global__ void __launch_bounds__(NT, 1) k_ptq_stream(const StreamArgs a) {
 #pragma unroll
                 for (int i = 0; i < (16 * CH + 31) / 32; ++i) {
                     const int c = i * 32 + lane, row = c / CH, k = c - row * CH;
-                    if (c < 16 * CH && (ALIGN == 16 || k < have)) cp_async<ALIGN>(dst + c * ALIGN, src + size_t(min(row, rmax)) * rowbytes + k * ALIGN);
+                    if (c < 16 * CH && (ALIGN == 16 || k < have)) cp_async<W>(dst + c * W, src + size_t(min(row, rmax)) * rowbytes + k * W);
                 }
                 ++fp; if (++ft == n) { ft = 0; ++fg; }
                 if (++fs == ST) fs = 0;
@@ -191,7 +218,7 @@ __global__ void __launch_bounds__(NT, 1) k_ptq_stream(const StreamArgs a) {
             asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
             __syncwarp();                      // every lane's copies are there, and every lane is done with the slot requested next
             request();
-            const uint32_t *r0 = reinterpret_cast<const uint32_t *>(ring + slot * PIECE + g * 112), *r1 = r0 + 8 * 28;
+            const uint32_t *r0 = reinterpret_cast<const uint32_t *>(ring + slot * PIECE + at), *r1 = r0 + 8 * PITCH / 4;
             int c[4][4];
 #pragma unroll
             for (int j = 0; j < 4; j += 2) {
@@ -236,10 +263,11 @@ __global__ void __launch_bounds__(NT, 1) k_ptq_stream(const StreamArgs a) {
 }
 
 template <int ALIGN, bool MANY = false>
-cudaError_t launch_a(cudaStream_t st, int grid, size_t smem, const StreamArgs &a) {
+cudaError_t launch_a(cudaStream_t st, int grid, const StreamArgs &a) {
+    const size_t smem = size_t(Ring<ALIGN>::BYTES) + 512 + size_t(a.run) * ((a.nb + 3) / 4) * 64;
     static bool set = false;
     if (!set) {
-        cudaError_t e = cudaFuncSetAttribute(k_ptq_stream<ALIGN, MANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, NW * ST * PIECE + 512 + MAX_PIECES * 64);
+        cudaError_t e = cudaFuncSetAttribute(k_ptq_stream<ALIGN, MANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<ALIGN>::BYTES + 512 + MAX_PIECES * 64);
         if (e != cudaSuccess) return e;
         set = true;
     }
@@ -261,16 +289,16 @@ cudaError_t ptq_stream(cudaStream_t st, int sm_count, const void *W, int M, int 
     a.q = tiles / grid; a.r = tiles % grid;
     const int most = a.q + (a.r > 0);
     a.run = std::min(most, MAX_PIECES / ng);
-    const size_t smem = size_t(NW) * ST * PIECE + 512 + size_t(a.run) * ng * 64;
-    // the widest copy that every row of every piece starts on
+    // the widest copy that every row of every piece starts on (4 bytes: granules)
     const uintptr_t align = reinterpret_cast<uintptr_t>(W) | uintptr_t(a.nb * 28);
     // A chain of shift-and-adds per half-word pair where a CTA has many pieces (248 320 x 4096: 81.6 -> 77.5 us in a loop over the matrix,
     // 87.1 -> 84.3 with two matrices in turn, 88.9 -> 87.2 with the quantiser in front; 30 000 x 8192 23.9 -> 23.4 in the loop),
     // products side by side where the first piece's latency counts (1024 x 4096 3.2 against 3.4 us, 7000 x 3584 5.4 against
-    // 5.5) and where copies of 4 or 8 bytes take the issue slots (30 000 x 4736 20.3 against 20.7).
-    if (align % 16 == 0) return most * ng >= 10 * NW ? launch_a<16, true>(st, grid, smem, a) : launch_a<16>(st, grid, smem, a);
-    if (align % 8 == 0) return launch_a<8>(st, grid, smem, a);
-    return launch_a<4>(st, grid, smem, a);
+    // 5.5) and where copies of 8 bytes take the issue slots.
+    const bool many = most * ng >= 10 * NW;
+    if (align % 16 == 0) return many ? launch_a<16, true>(st, grid, a) : launch_a<16>(st, grid, a);
+    if (align % 8 == 0) return launch_a<8>(st, grid, a);
+    return many ? launch_a<0, true>(st, grid, a) : launch_a<0>(st, grid, a);
 }
 
 }  // namespace bnk
