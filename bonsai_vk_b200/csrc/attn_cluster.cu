@@ -1,5 +1,5 @@
 // attn_cluster.cu - decode attention of one query token in ONE launch, for caches of up to 8192 positions: a thread-block cluster
-// of 16 CTAs per kv head keeps scores, numerators, probabilities and partial outputs in distributed shared memory. The chain of
+// of 16 CTAs per kv head (or several, for parts of its query heads) keeps scores, numerators, probabilities and partial outputs in distributed shared memory. The chain of
 // four kernels in attn.cu costs about 3.5 us of latency per kernel on the device and 2.2 us each on the host, whatever the
 // length; here the CTAs exchange four times (maxima, numerators, sums, partial outputs) by stores into each other's shared memory that
 // an mbarrier over there counts, so an exchange costs one way across the cluster. As plain stores and a cluster barrier it cost the
@@ -85,6 +85,7 @@ struct Args {
     const float *q16f, *gate;
     KvLayer kv;
     int splits;
+    int log_parts;                             // clusters per kv head, GQA of its query heads each
     float scale, nz;                           // nz = -0: see k_attn_pv in attn.cu
     float *pregate, *gated;
     Cols cols;
@@ -109,7 +110,7 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
     float *mxs = reinterpret_cast<float *>(smem + L.mx), *part = reinterpret_cast<float *>(smem + L.part);
     unsigned *red = reinterpret_cast<unsigned *>(smem + L.red);
     float *tot = reinterpret_cast<float *>(red + GQA);
-    const int rank = blockIdx.x, kvh = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = blockIdx.x, kvh = blockIdx.y >> g.log_parts, head0 = blockIdx.y * GQA, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // (the position was set before the pass: the rule at bnk::launch)
     const int nfill = where.get() + 1, splits = g.splits, per = (nfill + splits - 1) / splits, used = (nfill + per - 1) / per;
     const int grp = rank / sh.nsl, sl = rank - grp * sh.nsl;             // which splits, which dims of them
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
         f32pair qd[G][8];
 #pragma unroll
         for (int h = 0; h < G; ++h) {
-            const float4 *qv = reinterpret_cast<const float4 *>(q16f + size_t(kvh * GQA + hp * G + h) * HD + lane * 8);
+            const float4 *qv = reinterpret_cast<const float4 *>(q16f + size_t(head0 + hp * G + h) * HD + lane * 8);
             const float4 q0 = qv[0], q1 = qv[1];
             qd[h][0] = pair_of(q0.x, q0.x); qd[h][1] = pair_of(q0.y, q0.y); qd[h][2] = pair_of(q0.z, q0.z); qd[h][3] = pair_of(q0.w, q0.w);
             qd[h][4] = pair_of(q1.x, q1.x); qd[h][5] = pair_of(q1.y, q1.y); qd[h][6] = pair_of(q1.z, q1.z); qd[h][7] = pair_of(q1.w, q1.w);
@@ -214,7 +215,7 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // every CTA is running
     for (int i = tid; i < CL * GQA; i += T) put(remote(mxs + rank * GQA + i % GQA, i / GQA), unord(red[i % GQA]), remote(smem + L.bars, i / GQA));
     // (the gate of the outputs that this CTA finishes, off the tail)
-    const int orow = (kvh * GQA * HD) + rank * OPC + tid;
+    const int orow = head0 * HD + rank * OPC + tid;
     float gt = 0.0f;
     if (tid < OPC) gt = __fdiv_rn(1.0f, __fadd_rn(1.0f, exp_f(-gate[orow])));
     alive = arrived(bars, g.err);
@@ -365,38 +366,61 @@ __global__ void k_wait_selftest_exchange(int *err) {
     }
 }
 
+// clusters of the largest CTAs that run at once (0: none); asked once, before the first launch: 16 CTAs are beyond the portable
+// cluster size, and a launch that does not fit would leave an error behind, or an invalid capture
+template <int GQA, int KMODE, int VMODE>
+int clusters_at_once() {
+    static const int n = [] {
+        auto kernel = k_attn_cluster<GQA, KMODE, VMODE>;
+        cudaLaunchConfig_t most = {};
+        most.gridDim = dim3(CL, 64); most.blockDim = dim3(T); most.dynamicSmemBytes = SMEM_MAX;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = CL; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        most.attrs = at; most.numAttrs = 1;
+        int clusters = 0;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX) == cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&clusters, kernel, &most) == cudaSuccess && clusters > 0) return clusters;
+        cudaGetLastError();                    // (a refusal is an answer, not a failed call)
+        return 0;
+    }();
+    return n;
+}
 template <int GQA, int KMODE, int VMODE>
 bool launch_c(cudaStream_t st, const Args &g, size_t smem) {
     auto kernel = k_attn_cluster<GQA, KMODE, VMODE>;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(CL, g.a.n_kv, g.cols.z()); cfg.blockDim = dim3(T); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cfg.gridDim = dim3(CL, g.a.n_kv << g.log_parts, g.cols.z()); cfg.blockDim = dim3(T); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = CL; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
-    // asked once, before the first launch, for the largest CTA: 16 CTAs are beyond the portable cluster size, and a launch that
-    // does not fit would leave an error behind, or an invalid capture
-    static const bool fits = [&] {
-        cudaLaunchConfig_t most = cfg;
-        most.dynamicSmemBytes = SMEM_MAX;
-        int clusters = 0;
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX) == cudaSuccess &&
-            cudaOccupancyMaxActiveClusters(&clusters, kernel, &most) == cudaSuccess && clusters > 0) return true;
-        cudaGetLastError();                    // (a refusal is an answer, not a failed call)
-        return false;
-    }();
-    if (!fits) return false;
     cfg.numAttrs = g_pdl ? 2 : 1;
     BN_COUNT(1);
     cudaLaunchKernelEx(&cfg, kernel, g);       // (a failure now is one of the caller's, who asks for the last error)
     return true;
 }
 template <int GQA>
-bool launch_g(cudaStream_t st, const Args &g) {
+int clusters_of(const Args &g) {
+    if (g.a.k_mode) return g.a.v_mode ? clusters_at_once<GQA, 1, 1>() : clusters_at_once<GQA, 1, 0>();
+    return g.a.v_mode ? clusters_at_once<GQA, 0, 1>() : clusters_at_once<GQA, 0, 0>();
+}
+template <int GQA>
+bool launch_g(cudaStream_t st, Args g) {
+    if constexpr (GQA > 1) {
+        // Two clusters with half the heads each where they run at once (K and V are read twice, from L2): few kv heads leave the GPU idle.
+        // One of eight heads, with the insert: 64 keys 9.5 -> 7.7 us, 1501 13.9 -> 8.8, 4096 23.1 -> 12.8. (Four kv heads would need
+        // eight clusters; fewer fit.)
+        if ((g.a.n_kv << (g.log_parts + 1)) * int(g.cols.z()) <= clusters_of<GQA / 2>(g)) {
+            Args half = g;
+            ++half.log_parts;
+            if (launch_g<GQA / 2>(st, half)) return true;
+        }
+    }
+    if (!clusters_of<GQA>(g)) return false;
     const Shape sh = shape_of(g.splits, g.a.cap);
     const size_t smem = size_t((g.a.v_mode ? layout<GQA, 1>(sh, g.splits, g.a.cap) : layout<GQA, 0>(sh, g.splits, g.a.cap)).total);
     if (smem > SMEM_MAX) return false;
@@ -417,7 +441,7 @@ cudaError_t launch_wait_selftest_exchange(cudaStream_t st, int *err) {
 bool attn_cluster(cudaStream_t st, AttnDims a, const float *q16f, const float *gate, AttnPos where, KvLayer kv, int splits, float *pregate, float *gated, Cols cols, int *err) {
     if (a.cap > 8192 || (splits != 1 && splits != 8 && splits != 64)) return false;
     if (getenv("BONSAI_ATTN_CHAIN")) return false;                         // the answer "does not fit", for comparisons
-    const Args g = {a, where, q16f, gate, kv, splits, 1.0f / sqrtf(float(a.head_dim)), -0.0f, pregate, gated, cols, err};
+    const Args g = {a, where, q16f, gate, kv, splits, 0, 1.0f / sqrtf(float(a.head_dim)), -0.0f, pregate, gated, cols, err};
     switch (a.n_head / a.n_kv) {
         case 1: return launch_g<1>(st, g);
         case 2: return launch_g<2>(st, g);
