@@ -54,9 +54,10 @@ __global__ void __launch_bounds__(512) k_rotate_quant(const float *__restrict__ 
     if (y) for (int i = threadIdx.x; i < block; i += blockDim.x) y[base + i] = s[i];
     if (q81) {
         const int grp = threadIdx.x >> 7, i = threadIdx.x & 127;       // 4 groups of 128 threads
+        const bnk::TableSlots slots = bnk::table_slots(i);
         for (int b = grp; b < block / 128; b += 4) {
             const size_t gb = base / 128 + b;
-            bnk::quant_block_128(s[b * 128 + i], i, qs + grp * 128, q81 + gb * bnk::Q81_DWORDS,
+            bnk::quant_block_128(s[b * 128 + i], i, slots, qs + grp * 128, q81 + gb * bnk::Q81_DWORDS,
                                  table + gb * bnk::BF_WORDS, 1 + grp);
         }
     }
