@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(NT, 1) k_ptq_stream(const StreamArgs a) {
     const uintptr_t w0 = reinterpret_cast<uintptr_t>(a.W), w1 = w0 + size_t(a.M) * rowbytes;
     const uintptr_t grow = w0 + size_t(lane >> 3) * rowbytes;
     const bool needed = (lane & 7) < 7 || (grow & 15);                     // (a row that starts on a granule has seven)
+    const int after = nb == 1 ? 4 : (nb == 2 ? 2 : 1);                     // rows behind a tile that its last row's granules may reach into: 100 bytes
     const int at = g * PITCH + (ALIGN ? 0 : int((w0 + size_t(g) * rowbytes) & 15));
     uint2 B[4][8];
     float d[4], ns[4];
@@ -184,7 +185,7 @@ __global__ void __launch_bounds__(NT, 1) k_ptq_stream(const StreamArgs a) {
                     const int row0 = (t0 + c0 + ft) * 16;
                     uintptr_t s = ((grow + size_t(row0) * rowbytes + size_t(fg) * 112) & ~uintptr_t(15)) + (lane & 7) * 16;
                     const uint32_t to = dst + (lane >> 3) * PITCH + (lane & 7) * 16;
-                    if (row0 > 0 && rmax > 15) {
+                    if (row0 > 0 && rmax >= 15 + after) {
 #pragma unroll
                         for (int i = 0; i < 4; ++i, s += 4 * rowbytes) if (needed) cp_async<16>(to + i * 4 * PITCH, reinterpret_cast<const void *>(s));
                     } else                     // the matrix's first and last rows: the words of a granule that reaches out of it one by one
