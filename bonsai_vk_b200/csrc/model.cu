@@ -553,7 +553,7 @@ void enqueue_batch(bn_model *m, int ncol, bool one_sequence = false) {
         bnk::Q2GemmArgs a = {};
         a.W = W; a.M = M; a.K = K; a.swiglu = swiglu; a.image = img; a.ncol = ncol; a.out = out; a.out_stride = AS;
         a.resid = resid; a.resid_stride = AS; a.next = next; a.warm = 1; a.err = m->ctx->err_dev;
-        cudaError_t e = bnk::launch_q2_gemm(st, m->ctx->sm_count, a, m->use_pdl);
+        cudaError_t e = bnk::launch_q2_gemm(st, m->ctx->sm_count, a, m->use_pdl, true);
         if (e != cudaSuccess && m->launch_err == cudaSuccess) m->launch_err = e;
     };
     if (m->b0 == 0) {
@@ -1183,7 +1183,7 @@ int bn_model_head_batch(bn_model *m, int ncol, const bn_buf *in, size_t in_off, 
     const int rows = m->head_r1 - m->head_r0;
     bnk::Q2GemmArgs a = {};
     a.W = m->q2_shard; a.M = rows; a.K = h.hidden; a.image = m->IMG_HD; a.ncol = ncol; a.out = m->LOGITS; a.out_stride = AS; a.err = m->ctx->err_dev;
-    cudaError_t e = bnk::launch_q2_gemm(st, m->ctx->sm_count, a, m->use_pdl);
+    cudaError_t e = bnk::launch_q2_gemm(st, m->ctx->sm_count, a, m->use_pdl, true);
     if (e != cudaSuccess) return bn_cuda_fail(e, "bn_model_head_batch");
     bnk::argmax_first(st, m->LOGITS, rows, m->NEXT, m->AMV, m->AMI, cols, m->CAND, m->head_r0);
     BN_CUDA(cudaMemcpyAsync(bn_ptr<char>(out, out_off), m->CAND, size_t(ncol) * 8, cudaMemcpyDeviceToDevice, st));

@@ -98,7 +98,9 @@ struct Q2GemmArgs {
     int kc, tiles;                                 // filled in by the launch;
     Q2Share share;                                 // filled in by the launch: the CTAs' shares of the row tiles
 };
-cudaError_t launch_q2_gemm(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl);
+// late: the dependent launch is released behind this kernel's own dependency wait in every build, so that the kernel behind may read ahead
+// of its wait what was complete before this one's (k_gdn_core). All of a model's projections are: see k_q2_gemm.
+cudaError_t launch_q2_gemm(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl, bool late = false);
 // the same with W in the file's native rows (16-byte aligned, K % 1024 == 0): each warp unpacks its pieces itself, no scratch
 // whether that is the faster way: `one_chunk`, the matrix unpacked into tiles beforehand would fit the scratch at once
 bool q2_gemm_in_place(int sm_count, int M, int K, int ncol, bool one_chunk);

@@ -38,7 +38,11 @@ template <bool FIRST> __device__ __forceinline__ uint4 weights16(const uint8_t *
 // NATIVE: W holds the file's rows; a warp unpacks each of its pieces in a corner of shared memory of its own first. Bound by that
 // unpacking, 250 instructions a piece: 16 warps also for 8 columns (128 x 12 288: 10.2 -> 9.1 us, 4096 rows and more the same).
 // 12 warps (168 registers a thread), or units of one tile, have room for a unit's weights to be on their way while the image is: LATE.
-template <int NCP, int MT, int NT, bool NATIVE>
+// EARLY: the dependent launch is released ahead of this kernel's own dependency wait. Late is what k_gdn_core needs, and costs nothing
+// but in the build of 16 columns and two tiles on 12 warps, alone with its preparation (12 288 x 4096 11.60 us early, 11.75 late;
+// 10 000 x 6144 14.53 and 14.70). A model's passes run the late build throughout: with both in turn four blocks of 12 sequences take
+// 330.5 us, with the late one 328.7.
+template <int NCP, int MT, int NT, bool NATIVE, bool EARLY>
 __global__ void __launch_bounds__(NT, 1) k_q2_gemm(const Q2GemmArgs a) {
     constexpr int NW = NT / 32;
     constexpr bool LATE = NATIVE || MT == 1 || (NT == 384 && MT == 2);
@@ -70,9 +74,11 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm(const Q2GemmArgs a) {
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars));
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8));
-        // i / nur = i * per >> 16 for the few hundred units of a wave (nur <= 12); the last pass may have fewer tiles
-        auto per = [&](int n) { return 65536 / ((n + MT - 1) / MT) + 1; };
-        asm volatile("st.shared.v2.s32 [%0], {%1, %2};" ::"r"(bars + 16), "r"(per(min(a.tiles, nt))), "r"(per(nt - (npass - 1) * a.tiles)) : "memory");
+        if (!DIVIDE) {
+            // i / nur = i * per >> 16 for the few hundred units of a wave (nur <= 12); the last pass may have fewer tiles
+            auto per = [&](int n) { return 65536 / ((n + MT - 1) / MT) + 1; };
+            asm volatile("st.shared.v2.s32 [%0], {%1, %2};" ::"r"(bars + 16), "r"(per(min(a.tiles, nt))), "r"(per(nt - (npass - 1) * a.tiles)) : "memory");
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (lane == 0) {
@@ -82,11 +88,12 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm(const Q2GemmArgs a) {
         for (int o = warp * 16384; o < bytes; o += NW * 16384) q2_prefetch(own + o, min(16384, bytes - o));
         q2_prefetch_next(a.next, cta, warp, NW);
     }
+    if (EARLY) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __syncthreads();
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    // Released here, the kernel behind this one may read ahead of its own wait what was complete before this one's (k_gdn_core does);
-    // it has no room on an SM before this CTA ends anyway.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // Released here, the kernel behind this one may read ahead of its own wait what was complete before this one's (k_gdn_core does).
+    // Where this grid has a CTA on every SM the dependents have no room before one ends anyway.
+    if (!EARLY) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (tid == 0) for (int q = 0; q < min(2, nchunks); ++q) request(q, q < nw ? q : 0);
 
     const f32pair magic2 = pair_of(__int_as_float(Q2_MAGIC), __int_as_float(Q2_MAGIC));
@@ -107,12 +114,12 @@ __global__ void __launch_bounds__(NT, 1) k_q2_gemm(const Q2GemmArgs a) {
             const unsigned char *chunk = img + buf * kc * gbytes;
             for (int u = warp; u < gn * nur * H; u += NW) {
                 int gl;
-                if (DIVIDE) gl = u / H / nur;
+                if (DIVIDE) gl = u / (H * nur);
                 else {
                     asm volatile("ld.shared.s32 %0, [%1];" : "=r"(gl) : "r"(per_at));
                     gl = u / H * gl >> 16;
                 }
-                const int h = u % H, ur = u / H - gl * nur;
+                const int h = u % H, ur = DIVIDE ? (u / H) % nur : u / H - gl * nur;
                 const uint8_t *src = W + (size_t(ur * MT) * ng + g0 + gl) * Q2_PIECE;
                 uint4 c[MT][4], dw[MT];
 #pragma unroll
@@ -269,11 +276,11 @@ int unit_rounds(int ng, int tiles, int ncp, int mt, int warps) {
     return ng / kc * rounds(kc) + (ng % kc ? rounds(ng % kc) : 0);
 }
 constexpr int NATIVE_NT = 512;
-template <int NCP, int MT, int NT, bool NATIVE = false>
+template <int NCP, int MT, int NT, bool NATIVE = false, bool EARLY = false>
 cudaError_t launch_t(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl) {
     static bool attr_set = false;
     if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(k_q2_gemm<NCP, MT, NT, NATIVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
+        cudaError_t e = cudaFuncSetAttribute(k_q2_gemm<NCP, MT, NT, NATIVE, EARLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
@@ -294,14 +301,14 @@ cudaError_t launch_t(cudaStream_t st, int sm_count, Q2GemmArgs a, bool pdl) {
     cfg.attrs = at;
     cfg.numAttrs = pdl ? 1 : 0;
     BN_COUNT(1);
-    return cudaLaunchKernelEx(&cfg, k_q2_gemm<NCP, MT, NT, NATIVE>, a);
+    return cudaLaunchKernelEx(&cfg, k_q2_gemm<NCP, MT, NT, NATIVE, EARLY>, a);
 }
 
 }  // namespace
 
 namespace bnk {
 
-cudaError_t launch_q2_gemm(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl) {
+cudaError_t launch_q2_gemm(cudaStream_t st, int sm_count, const Q2GemmArgs &a, bool pdl, bool late) {
     const int ncp = a.ncol <= 8 ? 8 : (a.ncol <= 16 ? 16 : 32), tiles = (a.M + 15) / 16;
     // Units of several row tiles share operand reads, units of one spread over more warps. Times with the preparation of the columns.
     // One tile, 16 warps: a CTA with one tile (a second one in a unit is the first again: 1024 x 4096 x 8 5.3 us with units of two, 4.9
@@ -322,8 +329,8 @@ cudaError_t launch_q2_gemm(cudaStream_t st, int sm_count, const Q2GemmArgs &a, b
     }
     if (ncp == 16) {
         if (single) return launch_t<16, 1, 512>(st, sm_count, a, pdl);
-        return unit_rounds(ng, n, 16, 2, 16) * 16 <= unit_rounds(ng, n, 16, 2, 12) * 12 ? launch_t<16, 2, 512>(st, sm_count, a, pdl)
-                                                                                         : launch_t<16, 2, 384>(st, sm_count, a, pdl);
+        if (unit_rounds(ng, n, 16, 2, 16) * 16 <= unit_rounds(ng, n, 16, 2, 12) * 12) return launch_t<16, 2, 512>(st, sm_count, a, pdl);
+        return late ? launch_t<16, 2, 384>(st, sm_count, a, pdl) : launch_t<16, 2, 384, false, true>(st, sm_count, a, pdl);
     }
     // 32 columns: a wave of all of K fits only the smallest matrices, where this kernel's units fill more warps (4096 x 4096, with the
     // preparation of the columns: 12.6 against 13.6 us); beyond, q2_gemm_wide.cu
