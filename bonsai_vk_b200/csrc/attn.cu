@@ -459,17 +459,22 @@ template <int GQA, int DPT, int VMODE>
 void pv(cudaStream_t st, AttnDims a, AttnPos where, const float *pe, const float *partial, KvLayer kv, int splits, float *part, Cols cols) {
     constexpr int TILE_BYTES = PV_TILE * (VMODE == 0 ? 256 + 16 : 512);
     const size_t smem = 2 * TILE_BYTES + size_t(GQA) * ((a.cap + splits - 1) / splits) * 4;
-    // (1024 CTAs of two warps at 32 768 positions: seven per SM everywhere instead of up to eleven, 57 -> 49 us a layer)
+    // (1024 CTAs at 32 768 positions: seven per SM everywhere instead of up to eleven; of two warps, four dims a thread, 57 -> 49 us a layer)
     launch_spread<k_attn_pv<GQA, DPT, VMODE>, 8>(dim3(a.n_kv, splits, cols.z()), dim3(256 / DPT), smem, st, a, where, pe, partial, kv, splits, part, -0.0f, cols);
 }
 template <int GQA>
 void pv_any(cudaStream_t st, AttnDims a, AttnPos where, const float *pe, const float *partial, KvLayer kv, int splits, float *part, Cols cols) {
-    // Several dims per thread from three CTAs per two SMs on (8 columns x 8 splits x 4 heads: 28 -> 22 us). Two dims where four or eight
-    // heads share a value, up to 4096 CTAs: twice the warps for an eighth more instructions (30 000 keys 45.1 us with four dims, 43.4 with
-    // two, eight heads 47.0 and 46.0; 8 columns at 2048 positions 85.6 and 83.1 us a block; 16 columns at 8192, 4096 CTAs, the same, 32
-    // columns 356 and 362). Fewer heads have too little work per value for that (two heads: 50.6 and 51.4).
-    const size_t ctas = size_t(a.n_kv) * splits * cols.z();
-    const int dims = ctas < 200 ? 1 : (GQA >= 4 && ctas <= 4096 ? 2 : 4);
+    // Several dims per thread from three CTAs per two SMs on (8 columns x 8 splits x 4 heads: 28 -> 22 us). Two dims is twice the warps
+    // for an eighth more instructions. Four heads a value gain by it up to 4096 CTAs (32 000 keys, four dims and two: 44.0 and 42.1 us with
+    // four kv heads, 23.7 and 22.1 with one; 8 columns at 2048 positions 85.6 and 83.1 us a block; 16 columns at 8192, 4096 CTAs, the same,
+    // 32 columns 356 and 362) - unless one column's CTAs are more than four an SM and leave a tenth of the last round empty, which
+    // the fewer warps hide (three kv heads, 768 CTAs: 12 000 of 16 384 keys 21.8 and 22.3). Eight heads a value issue enough with four
+    // dims: two up to three CTAs an SM (256 CTAs, 32 000 keys 48.8 and 48.0; 384, three sequences at 8192 253.5 and 251.6 us a stage; 512,
+    // 768, 2048, 32 000 keys 73.6 and 75.1, 103.0 and 105.4, 245 and 252). Fewer heads have too little work per value (two heads: 50.6
+    // and 51.4).
+    const size_t ctas = size_t(a.n_kv) * splits * cols.z(), per = (ctas + 147) / 148;
+    const bool uneven = cols.z() == 1 && per > 4 && ctas * 10 < per * 148 * 9;
+    const int dims = ctas < 200 ? 1 : ((GQA == 4 && ctas <= 4096 && !uneven) || (GQA == 8 && per <= 3) ? 2 : 4);
     constexpr int TWO = GQA >= 4 ? 2 : 4;
     if (a.v_mode == 0) {
         if (dims == 1) pv<GQA, 1, 0>(st, a, where, pe, partial, kv, splits, part, cols);
