@@ -16,6 +16,7 @@
 // A CTA scores the keys of its splits (its share of them where CTAs share a split) and brings their V slice into shared memory
 // with cp.async meanwhile. Numerators go to the CTAs that share the split and to the CTA that sums their residue modulo 128.
 #include "attn_octet.cuh"
+#include "exchange.cuh"
 
 #include <cstdlib>
 
@@ -54,30 +55,7 @@ template <int GQA, int VMODE> __host__ __device__ __forceinline__ Lay layout(con
     return l;
 }
 
-__device__ __forceinline__ uint32_t remote(const void *p, int rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(uint32_t(__cvta_generic_to_shared(p))), "r"(rank));
-    return r;
-}
-// stores into another CTA of the cluster, counted by a barrier there
-__device__ __forceinline__ void put(uint32_t addr, float v, uint32_t bar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(__float_as_uint(v)), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void put2(uint32_t addr, float a, float b, uint32_t bar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(addr), "r"(__float_as_uint(a)), "r"(__float_as_uint(b)), "r"(bar) : "memory");
-}
-// bounded wait for an exchange's bytes; on giving up the error word is set and the caller goes on without waiting again (results
-// are then invalid)
-__device__ __forceinline__ bool arrived(uint32_t bar, int *err, int limit = 1 << 22) {
-    for (int it = 0; it < limit; ++it) {
-        uint32_t ok;
-        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}\n"
-                     : "=r"(ok) : "r"(bar) : "memory");
-        if (__builtin_expect(ok != 0u, 1)) return true;
-    }
-    atomicExch(err, 5);
-    return false;
-}
+constexpr int ERR = ERR_ATTN_EXCHANGE;
 
 struct Args {
     AttnDims a;
@@ -218,7 +196,7 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
     const int orow = head0 * HD + rank * OPC + tid;
     float gt = 0.0f;
     if (tid < OPC) gt = __fdiv_rn(1.0f, __fadd_rn(1.0f, exp_f(-gate[orow])));
-    alive = arrived(bars, g.err);
+    alive = arrived<ERR>(bars, g.err);
 
     // ---- numerators: to the CTAs that share the split and to the one that sums the residue ------------------------------------
     {
@@ -235,7 +213,7 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
             else for (int p = 0; p < sh.nsl; ++p) put(remote(eg + i, grp * sh.nsl + p), e, remote(smem + L.bars + 8, grp * sh.nsl + p));
         }
     }
-    if (alive) alive = arrived(bars + 8, g.err);
+    if (alive) alive = arrived<ERR>(bars + 8, g.err);
     // ---- softmax sums: thread (head, residue, a) adds the keys of virtual thread 128 a + residue ascending ---------------------
     if (tid < GQA * RL * 8) {
         const int av = tid & 7, rl = (tid >> 3) % RL, h = (tid >> 3) / RL, res = rank * RL + rl;
@@ -248,7 +226,7 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
         put(remote(sums + h * 128 + res, av + 8), s, remote(smem + L.bars + 16, av + 8));
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (alive) alive = arrived(bars + 16, g.err);
+    if (alive) alive = arrived<ERR>(bars + 16, g.err);
     if (warp < GQA) {
         const float *p = sums + warp * 128 + lane;
         float s = __fadd_rn(__fadd_rn(p[0], p[64]), __fadd_rn(p[32], p[96]));
@@ -337,7 +315,7 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
         put(remote(part + o % OPC, o / OPC), acc, remote(smem + L.bars + 24, o / OPC));
     }
     // a CTA that has its part of every exchange has all that is stored into it; one that gave up waits for the others to end
-    if (alive) alive = arrived(bars + 24, g.err);
+    if (alive) alive = arrived<ERR>(bars + 24, g.err);
     if (!alive) asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
     // ---- splits ascending, gate ----------------------------------------------------------------------------------------------------
     if (tid < OPC) {
@@ -353,16 +331,6 @@ __global__ void __launch_bounds__(T, 1) k_attn_cluster(const Args g) {
         for (; i < used; ++i) s = __fadd_rn(s, part[i * OPC + tid]);
         if (g.pregate) colp(g.pregate, col * g.cols.arena)[orow] = s;
         colp(g.gated, col * g.cols.arena)[orow] = __fmul_rn(s, gt);
-    }
-}
-
-// A wait that nothing will ever satisfy, with a short limit: the give-up path of arrived()
-__global__ void k_wait_selftest_exchange(int *err) {
-    __shared__ uint64_t bar;
-    const uint32_t b = uint32_t(__cvta_generic_to_shared(&bar));
-    if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\nfence.mbarrier_init.release.cluster;" ::"r"(b) : "memory");
-        arrived(b, err, 1 << 10);
     }
 }
 
@@ -434,7 +402,7 @@ namespace bnk {
 
 cudaError_t launch_wait_selftest_exchange(cudaStream_t st, int *err) {
     BN_COUNT(1);
-    k_wait_selftest_exchange<<<1, 32, 0, st>>>(err);
+    k_wait_selftest_exchange<ERR><<<1, 32, 0, st>>>(err);
     return cudaGetLastError();
 }
 

@@ -1,5 +1,6 @@
 // context.cu - context, memory, transfer and event entry points of libbonsai_cuda.
 #include "common.cuh"
+#include "exchange.cuh"
 
 #include <stdarg.h>
 #include <string.h>
@@ -211,7 +212,8 @@ int bn_sync(bn_ctx *ctx) {
             return BN_ERR_ARG;
         }
         bn_set_error("a bounded device-side wait gave up (%s); results of the last kernels are invalid",
-                     flag == 2 ? "tensor-core projection pipeline" : flag == 4 ? "grid barrier of the whole-token kernel" : flag == 5 ? "exchange of the attention clusters" : "copy ring");
+                     flag == 2 ? "tensor-core projection pipeline" : flag == 4 ? "grid barrier of the whole-token kernel"
+                     : flag == bnk::ERR_ATTN_EXCHANGE ? "exchange of the attention clusters" : flag == bnk::ERR_STEP_EXCHANGE ? "exchange of the recurrent step" : "copy ring");
         return BN_ERR_TIMEOUT;
     }
     return BN_OK;

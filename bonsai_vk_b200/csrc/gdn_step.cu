@@ -11,30 +11,21 @@
 // go back in the first projection, which shares its SMs; another 0.7 us went with the cluster barrier behind the outputs (counted
 // stores now: a barrier waits for the stores' acknowledgement, then makes a round trip), the divisions of the head's place and two
 // divisions by square roots: 48 greedy tokens 51.0 -> 50.2 ms. Arithmetic and its order are those of k_gdn_core (ops.cu).
+#include "exchange.cuh"
 #include "ops.cuh"
 #include "rotate_quant.cuh"
 
 namespace {
 using namespace bnk;
 
-constexpr int T = 256;
+constexpr int T = 256, ERR = ERR_STEP_EXCHANGE;
 
 __device__ __forceinline__ void cp16(void *dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(uint32_t(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
 }
 // v to the place of `p` in the shared memory of CTA `cta` of the cluster
 __device__ __forceinline__ void push(float *p, int cta, float v) {
-    uint32_t dst;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(uint32_t(__cvta_generic_to_shared(p))), "r"(cta));
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(v) : "memory");
-}
-
-// the same, counted by a barrier there
-__device__ __forceinline__ void push_counted(float *p, int cta, float v, const uint64_t *bar) {
-    uint32_t dst, b;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(uint32_t(__cvta_generic_to_shared(p))), "r"(cta));
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(uint32_t(__cvta_generic_to_shared(bar))), "r"(cta));
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst), "r"(__float_as_uint(v)), "r"(b) : "memory");
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote(p, cta)), "f"(v) : "memory");
 }
 
 __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(T, 5) k_gdn_step(const GdnStep a) {
@@ -184,7 +175,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(T, 5) k_gdn_step(con
     if (lane < 16) {                               // lane = (CTA, row): push this warp's four outputs into all four so[]
         const int row = lane & 3;
         const float o = __fmul_rn(row == 0 ? pr[0] : (row == 1 ? pr[1] : (row == 2 ? pr[2] : pr[3])), a.scale);
-        push_counted(so + q4 * 32 + warp * 4 + row, lane >> 2, o, &outs);
+        put(remote(so + q4 * 32 + warp * 4 + row, lane >> 2), o, remote(&outs, lane >> 2));
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r)
@@ -194,17 +185,8 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(T, 5) k_gdn_step(con
     int hd = 0;
     if (warp == 1) { gz = silu_f(zz); nw = a.ssm_norm[q4 * 32 + lane]; hd = a.heads / a.qk_heads * hq + h / a.qk_heads; }
     // the head's 128 outputs are in every CTA's so[] (counted stores: a cluster barrier waits for their acknowledgement first)
-    bool alive = false;
-    for (int it = 0; it < (1 << 22) && !alive; ++it) {
-        uint32_t ok;
-        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}\n"
-                     : "=r"(ok) : "r"(uint32_t(__cvta_generic_to_shared(&outs))) : "memory");
-        alive = ok != 0u;
-    }
-    if (!alive) {                                  // given up: the others end first
-        atomicExch(a.err, 1);
-        asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
-    }
+    if (!arrived<ERR>(uint32_t(__cvta_generic_to_shared(&outs)), a.err))
+        asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");      // (given up: the others end first)
     if (warp == 1) {
         float e[4];
 #pragma unroll
@@ -219,6 +201,12 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(T, 5) k_gdn_step(con
 }  // namespace
 
 namespace bnk {
+
+cudaError_t launch_wait_selftest_step(cudaStream_t st, int *err) {
+    BN_COUNT(1);
+    k_wait_selftest_exchange<ERR><<<1, 32, 0, st>>>(err);
+    return cudaGetLastError();
+}
 
 void gdn_step(cudaStream_t st, const GdnStep &a, bool alone) {
     static bool attr = false;

@@ -85,9 +85,10 @@ int bn_gemm_q81(bn_ctx *ctx, const bn_buf *w, size_t w_off, int w_tiled, int M, 
 
 int bn_selftest_wait(bn_ctx *ctx, int which) {
     BN_REQUIRE(ctx, BN_ERR_ARG, "bn_selftest_wait: null context");
-    BN_REQUIRE(which >= 0 && which <= 2, BN_ERR_ARG, "bn_selftest_wait: which=%d (0 = copy-ring wait, 1 = tensor-core pipeline wait, 2 = attention's exchange)", which);
-    cudaError_t e = which == 0 ? bnk::launch_wait_selftest_ring(ctx->stream, ctx->err_dev)
-                               : which == 1 ? bnk::launch_wait_selftest_gemm(ctx->stream, ctx->err_dev) : bnk::launch_wait_selftest_exchange(ctx->stream, ctx->err_dev);
+    BN_REQUIRE(which >= 0 && which <= 3, BN_ERR_ARG, "bn_selftest_wait: which=%d (0 = copy-ring wait, 1 = tensor-core pipeline wait, 2 = attention's exchange, 3 = the recurrent step's)", which);
+    auto launch = which == 0 ? bnk::launch_wait_selftest_ring : which == 1 ? bnk::launch_wait_selftest_gemm
+                : which == 2 ? bnk::launch_wait_selftest_exchange : bnk::launch_wait_selftest_step;
+    cudaError_t e = launch(ctx->stream, ctx->err_dev);
     if (e != cudaSuccess) return bn_cuda_fail(e, "bn_selftest_wait");
     return BN_OK;
 }

@@ -131,6 +131,7 @@ struct GdnStep {
     int *err;                              // device error word (a bounded wait)
 };
 void gdn_step(cudaStream_t st, const GdnStep &a, bool alone = false);
+cudaError_t launch_wait_selftest_step(cudaStream_t st, int *err);
 // the mixer for n <= 32 consecutive positions of one sequence (gdn_seq.cu): column c's activations at + c * stride bytes
 struct GdnSeq {
     int heads, qk_heads, hidden;

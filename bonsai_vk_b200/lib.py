@@ -242,7 +242,7 @@ class Context(_Handle):
         _check(self.lib.bn_sync(self.h), "bn_sync")
 
     def selftest_wait(self, which: int):
-        """Queue a kernel whose bounded wait must give up (0: copy-ring wait, 1: tensor-core pipeline wait, 2: attention's exchange); the next
+        """Queue a kernel whose bounded wait must give up (0: copy-ring wait, 1: tensor-core pipeline wait, 2: attention's exchange, 3: the recurrent step's); the next
         sync() then raises BonsaiError with code BN_ERR_TIMEOUT and the context stays usable."""
         _check(self.lib.bn_selftest_wait(self.h, which), "bn_selftest_wait")
 

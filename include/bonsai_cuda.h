@@ -65,8 +65,9 @@ int bn_memset(bn_ctx *ctx, bn_buf *dst, size_t off, int byte, size_t n);
 int bn_sync(bn_ctx *ctx);
 /* Failure detection without a fault: queues one tiny kernel whose only wait can never complete, with the wait's limit
  * cut to a few milliseconds (which = 0: the copy-ring wait of the single-column projection; 1: the pipeline wait of the
- * tensor-core projection; 2: the wait for an exchange of the attention clusters). The kernel gives up, sets the context's error word and returns; the next bn_sync reports
- * BN_ERR_TIMEOUT and clears the word, and the context stays usable. (The reference has no counterpart: its waits are
+ * tensor-core projection; 2: the wait for an exchange of the attention clusters; 3: for that of the recurrent
+ * step). The kernel gives up, sets the context's error word and returns; the next bn_sync reports BN_ERR_TIMEOUT and
+ * clears the word, and the context stays usable. (The reference has no counterpart: its waits are
  * Vulkan fences with an unbounded timeout, bonsai_weights.h:287.) */
 int bn_selftest_wait(bn_ctx *ctx, int which);
 /* The next single-sequence projection that a model of this context launches is refused as the runtime refuses a bad launch (nothing

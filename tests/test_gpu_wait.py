@@ -32,3 +32,11 @@ def test_bounded_wait_gives_up_and_context_survives(ctx, oracle, which, where):
     assert np.array_equal(out.download(np.float32, M).view(np.uint32), ref.view(np.uint32))
     for b in (wb, xb, pack, out):
         b.free()
+
+
+def test_the_recurrent_exchange_has_a_name_of_its_own(ctx):
+    ctx.sync()
+    ctx.selftest_wait(3)
+    with pytest.raises(BonsaiError, match="exchange of the recurrent step"):
+        ctx.sync()
+    ctx.sync()
