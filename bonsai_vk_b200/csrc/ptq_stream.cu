@@ -16,12 +16,13 @@
 // warp stays with one group's operand table - 64 registers - for most of its pieces; group sums meet in shared memory, where one thread
 // per row adds them in ascending order.
 // Data movement. A piece is 16 rows of 112 bytes, brought by cp.async into a ring of its warp's own: 16 or 8 bytes at a time where the
-// rows' alignment allows, else the eight 16-byte granules that hold a row's 112 bytes (ALIGN 0), from which a lane reads at its row's
-// place. Four bytes at a time, 14 copies a piece instead of four, took the issue slots: 30 000 x 4736 22.6 -> 18.1 us, 50 000 x 6528
-// 43.1 -> 32.0, 100 000 x 2176 34.8 -> 26.7. Rows of more alignment lose by it (1000 x 8192 6.9 against 7.5, 20 000 x 12 288 26.5 against
-// 27.7; 60 000 x 1280 13.8 against 13.5). The pitches of 112
-// and 144 bytes are free of bank conflicts for every load of the loop: eight rows start four banks apart and the four lanes of a row
-// read words 0, 2, 3, 5 (one in each residue modulo 4).
+// rows' alignment allows, else the up to eight 16-byte granules that hold a row's bytes (ALIGN 0, granules.cuh), from which a lane reads
+// at its row's place. Four bytes at a time, 14 copies a piece instead of four, took the issue slots: 30 000 x 4736 22.6 -> 18.1 us, 50 000
+// x 6528 43.1 -> 32.0, 100 000 x 2176 34.8 -> 26.7. Rows of more alignment lose by it (1000 x 8192 6.9 against 7.5, 20 000 x 12 288 26.5
+// against 27.7; 60 000 x 1280 13.8 against 13.5). The pitch of 112 bytes is free of bank conflicts for every load of the loop: eight rows
+// start four banks apart and the four lanes of a row read words 0, 2, 3, 5 (one in each residue modulo 4). So is that of 144, but the rows
+// of an odd number of blocks lie at different places in their granules, which makes most loads conflicts of two.
+#include "granules.cuh"
 #include "ops.cuh"
 #include "q2.cuh"
 #include "rotate_quant.cuh"
@@ -147,13 +148,14 @@ __global__ void __launch_bounds__(NT, 1) k_ptq_stream(const StreamArgs a) {
     const bool odd = tig & 1, hi = tig & 2;
     const unsigned char *ring = smem + warp * ST * PIECE;
     const uint32_t ring_s = uint32_t(__cvta_generic_to_shared(ring));
-    // ALIGN 0: lane (row, granule) of every fourth row; rows four apart (4 x 28 bytes per block) start at the same place in a granule, and
-    // so do a row's pieces. `at`: where this lane finds its words of row g (and, eight pitches on, of row g + 8)
-    const uintptr_t w0 = reinterpret_cast<uintptr_t>(a.W), w1 = w0 + size_t(a.M) * rowbytes;
-    const uintptr_t grow = w0 + size_t(lane >> 3) * rowbytes;
-    const bool needed = (lane & 7) < 7 || (grow & 15);                     // (a row that starts on a granule has seven)
-    const int after = nb == 1 ? 4 : (nb == 2 ? 2 : 1);                     // rows behind a tile that its last row's granules may reach into: 100 bytes
-    const int at = g * PITCH + (ALIGN ? 0 : int((w0 + size_t(g) * rowbytes) & 15));
+    // `at`: where this lane finds its words of row g (and, eight pitches on, of row g + 8). ALIGN 0, nfull and nlast: whether the granule
+    // that this lane copies holds any of a full group's blocks, of the last group's (worked out per piece, a CTA's first piece came 0.1 us
+    // later; with all eight granules of a short last group 200 000 x 640 took 20.4 instead of 19.0 us)
+    const uintptr_t w0 = reinterpret_cast<uintptr_t>(a.W);
+    const Granules gran = {w0, w0 + size_t(a.M) * rowbytes, rowbytes, a.M, nb};
+    const int place = gran.place(lane >> 3);
+    const bool nfull = gran.holds(place, 0, lane & 7), nlast = gran.holds(place, ng - 1, lane & 7);
+    const int at = g * PITCH + (ALIGN ? 0 : gran.place(g));
     uint2 B[4][8];
     float d[4], ns[4];
     int group = -1;
@@ -182,19 +184,10 @@ __global__ void __launch_bounds__(NT, 1) k_ptq_stream(const StreamArgs a) {
                 const int rmax = a.M - 1 - (t0 + c0 + ft) * 16, have = ALIGN == 16 ? CH : min(4, nb - fg * 4) * 28 / W;
                 const uint32_t dst = ring_s + fs * PIECE;
                 if (ALIGN == 0) {
-                    const int row0 = (t0 + c0 + ft) * 16;
-                    uintptr_t s = ((grow + size_t(row0) * rowbytes + size_t(fg) * 112) & ~uintptr_t(15)) + (lane & 7) * 16;
                     const uint32_t to = dst + (lane >> 3) * PITCH + (lane & 7) * 16;
-                    if (row0 > 0 && rmax >= 15 + after) {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i, s += 4 * rowbytes) if (needed) cp_async<16>(to + i * 4 * PITCH, reinterpret_cast<const void *>(s));
-                    } else                     // the matrix's first and last rows: the words of a granule that reaches out of it one by one
-#pragma unroll 1
-                        for (int i = 0; i < 4; ++i, s += 4 * rowbytes) {
-                            if (!needed || (lane >> 3) + 4 * i > rmax) continue;
-                            if (s >= w0 && s + 16 <= w1) cp_async<16>(to + i * 4 * PITCH, reinterpret_cast<const void *>(s));
-                            else for (int k = 0; k < 16; k += 4) if (s + k >= w0 && s + k < w1) cp_async<4>(to + i * 4 * PITCH + k, reinterpret_cast<const void *>(s + k));
-                        }
+                    gran.copies((t0 + c0 + ft) * 16, fg, lane, fg + 1 < ng ? nfull : nlast,
+                                [&](int i, uintptr_t s) { cp_async<16>(to + i * 4 * PITCH, reinterpret_cast<const void *>(s)); },
+                                [&](int i, int k, uintptr_t s) { cp_async<4>(to + i * 4 * PITCH + k, reinterpret_cast<const void *>(s)); });
                 } else if (ALIGN == 16 && rmax >= 15) {
                     const uint4 o = offs[lane];
                     cp_async<16>(dst + lane * 16, src + o.x); cp_async<16>(dst + lane * 16 + 512, src + o.y); cp_async<16>(dst + lane * 16 + 1024, src + o.z);
