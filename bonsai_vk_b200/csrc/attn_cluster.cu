@@ -380,8 +380,10 @@ template <int GQA>
 bool launch_g(cudaStream_t st, Args g) {
     if constexpr (GQA > 1) {
         // Two clusters with half the heads each where they run at once (K and V are read twice, from L2): few kv heads leave the GPU idle.
-        // One of eight heads, with the insert: 64 keys 9.5 -> 7.7 us, 1501 13.9 -> 8.8, 4096 23.1 -> 12.8. (Four kv heads would need
-        // eight clusters; fewer fit.)
+        // One kv head of eight heads, with the insert: 64 keys 9.5 -> 7.7 us, 1501 13.9 -> 8.8, 4096 23.1 -> 12.8. 4000 keys (one cluster
+        // a kv head -> several): two kv heads of eight 22.2 -> 14.7, of four 14.5 -> 12.2, of two 12.0 -> 11.0; three of eight 22.3 -> 14.7,
+        // of four 14.7 -> 12.2, of two 12.1 -> 11.0. Of 80 shapes of one to three kv heads two lose by it, 300 keys at 8 splits (10.1 ->
+        // 10.3). (Four kv heads would need eight clusters; fewer fit.)
         if ((g.a.n_kv << (g.log_parts + 1)) * int(g.cols.z()) <= clusters_of<GQA / 2>(g)) {
             Args half = g;
             ++half.log_parts;
